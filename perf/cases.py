@@ -297,23 +297,29 @@ def _run_turn(state):
     return out
 
 
+class _KeepingLogits:
+    """A batch under way whose every step's logits are kept."""
+
+    def __init__(self, run, logits):
+        self.run, self.logits, self.depth = run, logits, run.depth
+
+    def start(self, slots, prompts, limits):
+        self.run.start(slots, prompts, limits)
+        self.logits.append(self.run.last_logits.clone())
+
+    def launch(self, slots):
+        self.run.launch(slots)
+        self.logits.append(self.run.last_logits.clone())
+
+    def collect(self):
+        return self.run.collect()
+
+
 def _run_generate(state):
     case, eng, logits = state["case"], state["eng"], []
-
-    def keeping_logits(engine, opts, stops, n):
-        r = engine.begin_run(opts.sampler, stops)
-
-        def kept(call):
-            def go(*args):
-                call(*args)
-                logits.append(r.last_logits.clone())
-            return go
-        r.start, r.launch = kept(r.start), kept(r.launch)
-        return r
-
     sampler = wick.SamplerConfig.greedy() if case["sampling"] == "greedy" else wick.SamplerConfig()
     got = wick.generate(eng, state["prompts"], wick.GenOptions(max_tokens=case["steps"], sampler=sampler, max_batch=case["batch"]),
-                        run_factory=keeping_logits)
+                        run_factory=lambda engine, opts, stops, n: _KeepingLogits(engine.begin_run(opts.sampler, stops), logits))
     return {"tokens": [torch.tensor(r.tokens) for r in got], "logits": logits}
 
 
