@@ -307,9 +307,10 @@ def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 # ---------------------------------------------------------------------------
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, *, gated: bool = False,
-              out: Optional[torch.Tensor] = None) -> torch.Tensor:
+              out: Optional[torch.Tensor] = None, w_static: bool = False) -> torch.Tensor:
     """x [m, k] times w [n, k] transposed on the CUDA cores, float32 accumulation.
-    gated: w is [2n, k] (gate rows, then up rows); returns silu(x gate^T) * (x up^T)."""
+    gated: w is [2n, k] (gate rows, then up rows); returns silu(x gate^T) * (x up^T).
+    w_static: no kernel ever writes w (weights)."""
     _cuda("x", x)
     _cuda("w", w, x.dtype)
     m, k = x.shape
@@ -324,7 +325,7 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, *, gated
     if name not in ("wick_gemm_simt_bf16_bf16", "wick_gemm_simt_bf16_f32", "wick_gemm_simt_f32_f32",
                     "wick_gemm_simt_bf16_bf16_gated", "wick_gemm_simt_f32_f32_gated"):
         raise KernelError(f"no matrix product from {x.dtype} to {out_dtype}" + (" (gated)" if gated else ""))
-    _simt().call(name, "pppiiip", _p(x), _p(w), _p(out), m, n, k, _stream())
+    _simt().call(name, "pppiiiip", _p(x), _p(w), _p(out), m, n, k, 1 if w_static else 0, _stream())
     return out
 
 

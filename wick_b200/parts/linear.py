@@ -62,7 +62,7 @@ class Linear:
             tc = self._tensor_core()
             if tc is not None:
                 return tc.forward(x, out_dtype)
-        return ops.gemm_simt(x, self.weight, out_dtype, gated=self.gated)
+        return ops.gemm_simt(x, self.weight, out_dtype, gated=self.gated, w_static=True)
 
     def forward_delta(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
         """[n, in] -> float32 [splits, n, out]: partial sums over slices of the
@@ -75,4 +75,4 @@ class Linear:
                 if residual is not None and tc.forward_add(x, residual):
                     return None
                 return tc.forward_delta(x)
-        return ops.gemm_simt(x, self.weight, torch.float32).unsqueeze(0)
+        return ops.gemm_simt(x, self.weight, torch.float32, w_static=True).unsqueeze(0)
