@@ -58,3 +58,41 @@ def test_float32_products_of_misaligned_rows_take_the_general_form():
     x, w = torch.randn(5 * 64 + 1).to(DEV)[1:].view(5, 64), torch.randn(24, 64).to(DEV)
     assert x.data_ptr() % 16 != 0
     assert (ops.gemm_simt(x, w, torch.float32).double() - x.double() @ w.double().T).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("H, R, r, q_lens, starts, window, sink", [
+    (32, 576, 512, [1, 1, 1], [0, 700, 2100], 2048, False),          # runs of keys, a window's edge
+    (40, 576, 512, [1], [33], 0, False),                             # a second, partial group of heads
+    (16, 320, 256, [1, 1], [31, 32], 20, True),                      # one group of 16 heads, a window that starts inside a tile
+    (7, 80, 64, [3, 70], [62, 0], 0, True),                          # few heads, the smallest value, new tokens of one sequence
+    (5, 64, 64, [200], [5], 50, False),                              # many tokens: one run each, the value is the whole row
+    (33, 144, 128, [2], [127], 64, True),
+])
+def test_attention_over_rows_on_the_tensor_cores(H, R, r, q_lens, starts, window, sink):
+    """float32 queries as three bfloat16 numbers each: no further from 64 bits than float32 arithmetic is."""
+    g = torch.Generator().manual_seed(H)
+    assert ops.attention_latent_supported(R, r)
+    batch, pages, n_pages = batch_of(q_lens, starts)
+    store = torch.full((n_pages, PAGE, R), float("nan")).bfloat16()
+    rows = []
+    for b, (q, s) in enumerate(zip(q_lens, starts)):
+        rows.append(torch.randn(s + q, R, generator=g).bfloat16())
+        for p in range(s + q):
+            store[pages[b][p // PAGE], p % PAGE] = rows[b][p]
+    n = sum(q_lens)
+    q = torch.randn(n, H, R, generator=g)
+    sinks = torch.randn(H, generator=g) if sink else None
+    scale = R ** -0.5
+    out = ops.attention_multi(q.to(DEV), store.to(DEV), batch, scale, maps=1, kv_heads=1, v_dim=r, window=window,
+                              sink=sinks.to(DEV) if sink else None, rows_of=R, out_dtype=torch.float32).double().cpu()
+    t = 0
+    for b, (ql, s) in enumerate(zip(q_lens, starts)):
+        k = rows[b].double()
+        for p in range(s, s + ql):
+            lo = max(0, p - window + 1) if window else 0
+            z = q[t].double() @ k[lo:p + 1].T * scale
+            e = torch.exp(z - 20.0)                     # (scores of order one to ten: no maximum is needed in 64 bits)
+            den = e.sum(1, keepdim=True) + (torch.exp(sinks.double()[:, None] - 20.0) if sink else 0.0)
+            ref = (e / den) @ k[lo:p + 1, :r]
+            assert (out[t] - ref).abs().max() < 1e-5 * float(ref.abs().max()), (b, p)
+            t += 1

@@ -21,6 +21,7 @@
 //
 // Scores, softmax, weights, sums and norms are float32.  A token's arithmetic does not depend
 // on what else the step holds, up to the number of warps that share its keys.
+#include "attn_latent.cuh"
 #include "common.cuh"
 
 namespace wick {
@@ -1121,6 +1122,22 @@ int attn_multi(const void* q, const void* store, void* out, float* partial, cons
 #undef WICK_AM
 }
 
+template <int MT>
+int attn_latent_launch(const latent::Params& P, int n, int runs, cudaStream_t s) {
+    const size_t smem = latent::smem_bytes<MT>(P.R);
+    static bool raised = false;
+    if (!raised) {
+        WICK_CUDA(cudaFuncSetAttribute(latent::attn_latent_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)latent::smem_bytes<MT>(latent::MAX_ROW)));
+        raised = true;
+    }
+    WICK_CUDA(launch(latent::attn_latent_kernel<MT>, dim3((unsigned)(n * ceil_div(P.H, 16 * MT)), runs), dim3(32 * latent::WARPS), smem, s, P));
+    if (int rc = check_launch("attn_latent")) return rc;
+    if (!P.partial) return 0;
+    WICK_CUDA(launch(attn_multi_merge_kernel<float, 1, 4>, dim3(ceil_div((int64_t)n * P.H * ((P.r + 127) / 128), 4)), dim3(128), 0, s, (const float*)P.partial,
+                     P.out, n * P.H, P.H, P.r, runs, P.sink, 0.f, 0.f, 1.f, (const float*)nullptr));
+    return check_launch("attn_latent_merge");
+}
+
 template <typename T>
 int latent_finish(const float* parts, int splits, int n, int cols, int qr, int r, int dr, int Hg, const float* q_w, const float* kv_w,
                   float eps, const float* cos_t, const float* sin_t, int pairing, void* cq_out, float* gate_out, void* rows,
@@ -1214,6 +1231,23 @@ WICK_ATTN_MULTI(wick_attn_multi2_f32, float, float, float, 2)
 WICK_ATTN_MULTI(wick_attn_multi1_bf16, bf16, float, float, 1)
 WICK_ATTN_MULTI(wick_attn_multi1_f32, float, float, float, 1)
 WICK_ATTN_MULTI(wick_attn_multi1_act_bf16, bf16, bf16, bf16, 1)
+
+// float32 queries [n, H, R] over pages of 64 rows of R bfloat16 numbers, the first r of which are the value; results float32 [n, H, r].
+// start: the positions of a sequence from which on this step writes rows.  partial: n * H * runs * (4 + r rounded up to 128) floats, for runs > 1.
+WICK_API int wick_attn_latent_bf16(const float* q, const void* store, float* out, const int* seq_of_token, const int* positions,
+                                   const int* page_table, const int* start, int table_width, int n, int H, int R, int r, float scale,
+                                   int window, int keep_first, const float* sink, int runs, float* partial, void* s) {
+    WICK_REQUIRE(H > 0 && R % 16 == 0 && R <= latent::MAX_ROW && r % 64 == 0 && r > 0 && r <= latent::MAX_R && r <= R,
+                 "attn_latent: rows of %d numbers with values of %d are not built", R, r);
+    WICK_REQUIRE((((uintptr_t)q | (uintptr_t)store | (uintptr_t)out | (uintptr_t)partial) & 15) == 0, "attn_latent: a misaligned array");
+    WICK_REQUIRE(window >= 0 && keep_first >= 0, "attn_latent: bad window");
+    WICK_REQUIRE(runs >= 1 && runs <= 64 && (runs == 1 || partial), "attn_latent: %d runs of keys need a place for their records", runs);
+    WICK_REQUIRE((int64_t)n * H <= 0x7fffffff, "attn_latent: too many (token, head) pairs");
+    if (n == 0) return 0;
+    const latent::Params P = {q, (const bf16*)store, out, runs > 1 ? partial : nullptr, seq_of_token, positions, page_table, start, sink,
+                              table_width, H, R, r, window, keep_first, scale};
+    return H > 16 ? attn_latent_launch<2>(P, n, runs, (cudaStream_t)s) : attn_latent_launch<1>(P, n, runs, (cudaStream_t)s);
+}
 
 #define WICK_LATENT(T, SUFFIX)                                                                                                   \
     WICK_API int wick_latent_finish_##SUFFIX(const float* parts, int splits, int n, int cols, int qr, int r, int dr, int Hg,  \

@@ -744,6 +744,9 @@ def attention_multi(q: torch.Tensor, store: torch.Tensor, batch, scale: float, *
     if gate is not None:
         _cuda("gate", gate, torch.float32, (n, H))
         _need(maps == 1, "the factor per head belongs to one map")
+    if (rows_of is not None and maps == 1 and T == torch.bfloat16 and q.dtype == torch.float32 and not soft_cap and gate is None
+            and attention_latent_supported(d, v_dim) and (q.data_ptr() | store.data_ptr()) % 16 == 0 and not plain_kernels()):
+        return _attention_latent(q, store, batch, scale, v_dim, window, keep_first, sink)
     out = torch.empty((n, H, v_dim), dtype=out_dtype, device=q.device)
     # A step of few tokens: eight warps a block, heads that read the same rows together, and the visible keys cut into
     # runs (a block each, records merged by a second kernel) until the step fills the device about twice.  How many keys
@@ -912,6 +915,33 @@ def combine_maps(a: torch.Tensor, lam: float, eps: float, factor: float, *, lib:
     out = torch.empty((n, H, e), dtype=torch.bfloat16, device=a.device)
     _flex(*lib).call("wick_combine_maps_bf16", "pplifffp", _p(a), _p(out), n * H, e, float(lam), float(eps),
                      float(factor), _stream())
+    return out
+
+
+def attention_latent_supported(row: int, v_dim: int) -> bool:
+    """Whether rows of ``row`` bfloat16 numbers whose first ``v_dim`` are the value go through the tensor-core kernel."""
+    return row % 16 == 0 and row <= 576 and v_dim % 64 == 0 and 0 < v_dim <= min(512, row)
+
+
+LATENT_BLOCKS = 148         # blocks of a step of few tokens
+
+
+def _attention_latent(q, store, batch, scale, v_dim, window, keep_first, sink) -> torch.Tensor:
+    n, H, R = q.shape
+    out = torch.empty((n, H, v_dim), dtype=torch.float32, device=q.device)
+    # A block takes a token's up to 32 heads and fills an SM; the visible keys are cut into runs until every SM has one.  (8 tokens of
+    # 1,500 positions: 74 blocks 32.8 us, 148 25.7, 296 38.3; 4 of 700 to 1,500: 22.8, 24.8, 31.0.)
+    bound = getattr(batch, "kv_bound", None) or batch.max_kv_len
+    keys = min(bound, window + keep_first) if window > 0 else bound
+    runs = max(1, min(LATENT_BLOCKS // (n * ((H + 31) // 32)), (max(1, keys) + 31) // 32, 64))
+    partial = None
+    if runs > 1:
+        need = n * H * runs * (4 + (v_dim + 127) // 128 * 128)
+        ws = getattr(batch, "workspace", None)
+        partial = ws.get("attention_multi", need, torch.float32) if ws is not None else torch.empty(need, dtype=torch.float32, device=q.device)
+    _layer().call("wick_attn_latent_bf16", "pppppppiiiiifiipipp", _p(q), _p(store), _p(out), _p(batch.seq_of_token), _p(batch.positions),
+                  _p(batch.page_table), _p(batch.start), batch.table_width, n, H, R, v_dim, float(scale), int(window), int(keep_first),
+                  _p(sink), runs, _p(partial), _stream(), kernels=2 if partial is not None else 1)
     return out
 
 
