@@ -96,3 +96,42 @@ def test_attention_over_rows_on_the_tensor_cores(H, R, r, q_lens, starts, window
             ref = (e / den) @ k[lo:p + 1, :r]
             assert (out[t] - ref).abs().max() < 1e-5 * float(ref.abs().max()), (b, p)
             t += 1
+
+
+@pytest.mark.parametrize("E, top, ff, width, shared", [(5, 3, 136, 264, False), (8, 2, 192, 1024, True), (1, 1, 64, 128, False), (16, 2, 72, 512, False)])
+@pytest.mark.parametrize("n", [1, 2, 17, 64, 65, 128, 129])
+def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
+    """Experts that no token uses are left alone; results beyond a token's own experts are never read (they hold NaN before)."""
+    from wick_b200.models.spec import PartSpec
+    from wick_b200.parts.base import BuildContext, build_part
+    from wick_b200.parts import feedforward  # noqa: F401
+    g = torch.Generator().manual_seed(E + n)
+    part = build_part("ffn", PartSpec("table_moe", dict(width=width, vocab=50, experts=E, top=top, intermediate=ff,
+                                                        shared=PartSpec("gated_mlp", dict(width=width, intermediate=64, activation="silu",
+                                                                                          names=dict(gate="gate_proj.weight", up="up_proj.weight", down="down_proj.weight"))) if shared else None)),
+                      BuildContext(dtype=torch.bfloat16, device=torch.device(DEV)))
+    tensors = {}
+
+    def get(name):
+        if name == "table":
+            return torch.rand(50, E, generator=g).argsort(1)[:, :top].int()
+        rows, cols = (width, 64 if "shared" in name else ff) if "down" in name else (64 if "shared" in name else ff, width)
+        return tensors.setdefault(name, (torch.randn(rows, cols, generator=g) / math.sqrt(cols)).bfloat16().to(DEV))
+    part.load(get)
+    x = torch.randn(n, width, generator=g).bfloat16().to(DEV)
+    tok = torch.randint(0, 50, (n,), generator=g).int().to(DEV)
+    torch.full((1 << 22,), float("nan"), device=DEV)                   # (scratch that the step may be given again)
+    got = part.forward(x, types.SimpleNamespace(tokens=tok, host=None)).sum(0)
+    ops.check_status()
+
+    def expert(pre, h):
+        a = gated(torch.cat([h @ tensors[pre + "gate_proj.weight"].double().T, h @ tensors[pre + "up_proj.weight"].double().T], 1))
+        return a @ tensors[pre + "down_proj.weight"].double().T
+    ref = expert("shared.", x.double()) if shared else torch.zeros(n, width, dtype=torch.float64, device=DEV)
+    for t in range(n):
+        for e in part.table[int(tok[t])].tolist():
+            ref[t] += expert(f"experts.{e}.", x[t:t + 1].double())[0] / top
+    assert (got.double() - ref).norm() < 5e-3 * ref.norm()             # (the inner activations are rounded to bfloat16)
+    if n <= 64:
+        one = part.forward(x[:1].contiguous(), types.SimpleNamespace(tokens=tok[:1].contiguous(), host=None)).sum(0)
+        assert torch.equal(one, got[:1]), "a token's bits do not depend on the others"

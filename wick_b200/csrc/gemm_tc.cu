@@ -24,6 +24,8 @@
 // flight land, frees its tensor memory and returns.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "sm100.cuh"
 #include "tcgen05.cuh"
@@ -58,6 +60,17 @@ struct GemmParams {
     int* status;
 };
 
+// (A struct of its own: with these fields in GemmParams the kernels that do not use them came out with up to half as many registers
+// again, and the decode products were 1 to 3 % slower.)
+struct GroupedParams : GemmParams {
+    // Grouped (several matrices of A one after the other, see wick_gemm_tc_grouped): the m tiles of one matrix, its padded
+    // rows, the rows of B it is multiplied with (0: all matrices with the same rows), elements of out between two matrices'
+    // results; the step's token ids and the table that names each id's `top` matrices.
+    int group_tiles, group_rows, group_b_rows, top, n_tokens;
+    long long group_out;
+    const int *tokens, *table;
+};
+
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -66,9 +79,14 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // tile, split) with the m tile varying fastest, so that blocks running at the
 // same time share B tiles through the L2 cache.  With two accumulators in tensor
 // memory the epilogue of one tile overlaps the main loop of the next.
-template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32>
+//
+// Grouped: the m tiles run over several matrices (experts), all multiplied with the same few rows of B or each with rows of
+// its own.  A block whose matrix no token of the step uses leaves at once, and of the others' results only those of tokens
+// that use the matrix are written.
+template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool GROUPED = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+               const std::conditional_t<GROUPED, GroupedParams, GemmParams> p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full_bar[MAX_STAGES];
     __shared__ uint64_t empty_bar[MAX_STAGES];
@@ -79,7 +97,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __shared__ int ok_w[4];
     __shared__ float xch[2][64][17];           // gated == 3: up values on their way to the warps that hold the gate values
 
+    __shared__ unsigned uses[GROUPED ? 8 : 1];   // grouped: a bit per token that uses this block's matrix
+
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int group = 0, bx = blockIdx.x;                          // this block's matrix, its m tile there
+    if constexpr (GROUPED) {
+        group = bx / p.group_tiles;
+        bx -= group * p.group_tiles;
+        // (the step's description is the host's or step_prepare's: it may be read before griddepcontrol.wait)
+        if (threadIdx.x < 8) uses[threadIdx.x] = 0;
+        __syncthreads();
+        bool mine = false;
+        for (int i = threadIdx.x; i < p.n_tokens * p.top; i += NUM_THREADS) {
+            const int t = i / p.top;
+            if (p.table[(long long)p.tokens[t] * p.top + (i - t * p.top)] == group) {
+                mine = true;
+                atomicOr(&uses[t >> 5], 1u << (t & 31));
+            }
+        }
+        if (!__syncthreads_or(mine)) return;
+    }
     const int tile_m = GATED == 3 ? BM / 2 : BM;
     const int a_tiles = GATED == 1 ? 2 : 1, b_tiles = GATED == 2 ? 2 : 1;
     const uint32_t a_bytes = BM * BK * 2, b_bytes = (uint32_t)p.bn * BK * 2;
@@ -102,7 +139,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             y = (w / p.grid_m) % p.grid_n;
             z = w / (p.grid_m * p.grid_n);
         } else {                                             // one tile per block: a three-dimensional grid
-            x = blockIdx.x;
+            x = GROUPED ? bx : (int)blockIdx.x;
             y = blockIdx.y;
             z = blockIdx.z;
         }
@@ -142,6 +179,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int w = w_first; w < w_end && ok; w += w_step) {
                 int m0, n0, kb_begin, n_kb, z;
                 tile_coords(w, m0, n0, kb_begin, n_kb, z);
+                if constexpr (GROUPED) {                     // (from here on rows of the operands, not of the result)
+                    m0 += group * p.group_rows;
+                    n0 += group * p.group_b_rows;
+                }
                 // Coordinates of the box that holds rows row.. of k-block kb: in a row-major
                 // operand (kb * 64, row); in a packed one the tile (row / 128, kb) lies as
                 // 128 contiguous lines of 128 bytes.
@@ -245,6 +286,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int m = m0 + q * 32 + lane;
             const uint32_t lane_addr = tmem_base + buf * acc_cols + ((uint32_t)(q * 32) << 16);
             char* out_base = (char*)p.out + (size_t)z * p.split_stride * (OUT_F32 ? 4 : 2);
+            if constexpr (GROUPED) out_base += (size_t)group * p.group_out * (OUT_F32 ? 4 : 2);
             // One answer for the four epilogue warps, so that they leave the loop together.
             const bool ok_warp = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1, &abort_flag, p.status, 3));
             bool ok = ok_warp;
@@ -276,7 +318,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         for (int jj = 0; jj < 8; ++jj) {
                             const int j = upper ? 8 + jj : jj;
                             const int n = n0 + c0 + j;
-                            if (n < p.b_rows) {
+                            bool wanted = n < p.b_rows;
+                            if constexpr (GROUPED) wanted = wanted && (uses[n >> 5] >> (n & 31) & 1u);
+                            if (wanted) {
                                 const float mine = upper ? v[8 + jj] : v[jj], other = xb[xrow][j];
                                 const float g = upper ? other : mine, u = upper ? mine : other;
                                 const float r = g / (1.0f + expf(-g)) * u;
@@ -327,7 +371,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                             for (int j = 0; j < 16; ++j) {
                                 const int n = n0 + c0 + j;
-                                if (n < p.b_rows) {
+                                bool wanted = n < p.b_rows;
+                                if constexpr (GROUPED) wanted = wanted && (uses[n >> 5] >> (n & 31) & 1u);
+                                if (wanted) {
                                     const long long off = (long long)n * p.ldo + m;
                                     if (OUT_F32) ((float*)out_base)[off] = v[j];
                                     else ((__nv_bfloat16*)out_base)[off] = __float2bfloat16_rn(v[j]);
@@ -383,10 +429,16 @@ using namespace wick;
 // a_total_rows / b_total_rows then count padded rows.  A weight tile then comes from DRAM as
 // one contiguous piece instead of 128 pieces of 128 bytes.
 // status: device int that receives a non-zero code if a wait inside the kernel gave up.
-WICK_API int wick_gemm_tc(const void* a, long long a_total_rows, int a_rows, const void* b, long long b_total_rows,
-                          int b_rows, int k, int bn, int gated, int pair_offset, int transposed, int out_f32,
-                          int a_static, int b_static, int a_packed, int b_packed, void* out, long long ldo, int splits, long long split_stride, int max_smem_bytes, int* status,
-                          void* stream) {
+struct Groups {
+    int n, rows, b_rows, top, n_tokens;            // n: 0 where A is one matrix
+    long long out;
+    const int *tokens, *table;
+};
+
+static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const void* b, long long b_total_rows,
+                        int b_rows, int k, int bn, int gated, int pair_offset, int transposed, int out_f32,
+                        int a_static, int b_static, int a_packed, int b_packed, void* out, long long ldo, int splits, long long split_stride, int max_smem_bytes, int* status,
+                        const Groups& G, void* stream) {
     WICK_REQUIRE(bn % 16 == 0 && bn >= 16 && bn <= 256, "gemm_tc: tile width %d must be a multiple of 16 in [16, 256]", bn);
     WICK_REQUIRE(!(gated == 2 && bn > 128) , "gemm_tc: a gated pair needs two accumulators: tile width <= 128");
     WICK_REQUIRE(gated >= 0 && gated <= 3 && splits >= 1, "gemm_tc: bad options");
@@ -425,6 +477,25 @@ WICK_API int wick_gemm_tc(const void* a, long long a_total_rows, int a_rows, con
     const long long total = (long long)p.grid_m * p.grid_n * splits;
     WICK_REQUIRE(total < (1ll << 30), "gemm_tc: too many tiles");
     p.total_tiles = (int)total;
+    if (G.n) {
+        GroupedParams g;
+        static_cast<GemmParams&>(g) = p;
+        g.group_tiles = p.grid_m; g.group_rows = G.rows; g.group_b_rows = G.b_rows; g.group_out = G.out;
+        g.top = G.top; g.n_tokens = G.n_tokens; g.tokens = G.tokens; g.table = G.table;
+        WICK_REQUIRE(a_packed && transposed && (gated == 0 || gated == 3) && (out_f32 != 0) == (gated == 0), "gemm_tc: grouped products are built for packed matrices, transposed results");
+        WICK_REQUIRE((long long)G.n * G.rows <= a_total_rows && G.rows % 128 == 0 && G.n_tokens == b_rows && b_rows <= 256 && G.top > 0, "gemm_tc: bad groups");
+        WICK_REQUIRE(total * G.n < (1ll << 30) && splits <= 65535 && p.grid_n <= 65535, "gemm_tc: too many tiles");
+        const dim3 grid(p.grid_m * G.n, p.grid_n, splits);
+        static bool raised = false;
+        if (!raised) {
+            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false, 3, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false, 0, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+            raised = true;
+        }
+        if (gated) WICK_CUDA(launch(gemm_tc_kernel<false, 3, true, false, true>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, g));
+        else WICK_CUDA(launch(gemm_tc_kernel<false, 0, true, true, true>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, g));
+        return check_launch("gemm_tc_grouped");
+    }
     // persistent blocks: as many as can be resident at once (one or two per SM by shared memory)
     const int resident = sm_count() * ((smem + 12 * 1024) * 2 <= 227 * 1024 ? 2 : 1);
     // Decode orientation (and anything that fits at once): one tile per block, so
@@ -457,4 +528,28 @@ WICK_API int wick_gemm_tc(const void* a, long long a_total_rows, int a_rows, con
     WICK_GEMM_CASE(true, 2, false, true) WICK_GEMM_CASE(true, 2, false, false)
 #undef WICK_GEMM_CASE
     return fail("gemm_tc: no kernel for pair mode %d with %s output", gated, transposed ? "transposed" : "row-major");
+}
+
+WICK_API int wick_gemm_tc(const void* a, long long a_total_rows, int a_rows, const void* b, long long b_total_rows,
+                          int b_rows, int k, int bn, int gated, int pair_offset, int transposed, int out_f32,
+                          int a_static, int b_static, int a_packed, int b_packed, void* out, long long ldo, int splits, long long split_stride, int max_smem_bytes, int* status,
+                          void* stream) {
+    const Groups none = {};
+    return gemm_tc_host(a, a_total_rows, a_rows, b, b_total_rows, b_rows, k, bn, gated, pair_offset, transposed, out_f32, a_static, b_static,
+                        a_packed, b_packed, out, ldo, splits, split_stride, max_smem_bytes, status, none, stream);
+}
+
+// Few tokens (at most 256) times the matrices of the experts that a table names for their ids: a holds n_groups packed matrices
+// of group_rows padded rows one after the other; a gated pair (silu(g) * u, bfloat16 out) or plain (float32 out).  Matrix e's
+// results lie at out + e * n_tokens * a_rows, token by token; only those of tokens whose id names e are written.  splits: runs of the
+// inner dimension, left as partial sums n_groups * n_tokens * a_rows apart (not for gated pairs).
+// per_group_b: matrix e is multiplied with rows e * n_tokens .. of b, otherwise all of them with the first n_tokens rows.
+WICK_API int wick_gemm_tc_grouped(const void* a, int n_groups, int group_rows, int a_rows, const void* b, long long b_total_rows,
+                                  int per_group_b, int n_tokens, int k, int bn, int gated, int pair_offset, void* out,
+                                  const int* tokens, const int* table, int top, int splits, int max_smem_bytes, int* status, void* stream) {
+    WICK_REQUIRE(n_groups > 0 && tokens && table, "gemm_tc: bad groups");
+    WICK_REQUIRE(bn >= n_tokens, "gemm_tc: a grouped product takes its tokens in one tile");
+    const Groups G = {n_groups, group_rows, per_group_b ? n_tokens : 0, top, n_tokens, (long long)n_tokens * a_rows, tokens, table};
+    return gemm_tc_host(a, (long long)n_groups * group_rows, a_rows, b, b_total_rows, n_tokens, k, bn, gated ? 3 : 0, pair_offset, 1, gated ? 0 : 1,
+                        1, 0, 1, 0, out, a_rows, splits, gated ? 0 : (long long)n_groups * n_tokens * a_rows, max_smem_bytes, status, G, stream);
 }

@@ -325,6 +325,55 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
 }
 
 
+// The same where y holds every expert's rows by token, as y_splits partial sums [n_experts][n][width]: a token's c-th row is that of
+// its id's c-th expert.  grid (n, ceil(width / 1024)): a thread takes four neighbours (VEC) or one element at a time.
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+moe_combine_table_kernel(const float* __restrict__ y, int y_splits, const int* __restrict__ tokens, const int* __restrict__ table, int top,
+                         int n_experts, float weight, const float* __restrict__ base, int base_splits, int64_t base_stride,
+                         float* __restrict__ out, int width) {
+    constexpr int V = VEC ? 4 : 1;
+    pdl_trigger();
+    const int t = blockIdx.x, n = gridDim.x;
+    const int* mine = table + (int64_t)tokens[t] * top;                  // (the step's description: no kernel in flight writes it)
+    pdl_wait();
+    y = fresh(y);
+    base = fresh(base);
+    const int64_t y_stride = (int64_t)n_experts * n * width;
+    auto add = [&](float (&v)[V], const float* p) {
+        if (VEC) {
+            const float4 d = ld4(p);
+            v[0] += d.x; v[V > 1 ? 1 : 0] += d.y; v[V > 2 ? 2 : 0] += d.z; v[V > 3 ? 3 : 0] += d.w;
+        } else {
+            v[0] += *p;
+        }
+    };
+    for (int j = (blockIdx.y * blockDim.x + threadIdx.x) * V; j < width; j += gridDim.y * blockDim.x * V) {
+        float sum[V], v[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) sum[i] = v[i] = 0.f;
+#pragma unroll 2
+        for (int c = 0; c < top; ++c) {
+            const int ex = mine[c];
+            if (ex < 0 || ex >= n_experts) continue;
+            float r[V];
+#pragma unroll
+            for (int i = 0; i < V; ++i) r[i] = 0.f;
+#pragma unroll 2
+            for (int s = 0; s < y_splits; ++s) add(r, y + s * y_stride + ((int64_t)ex * n + t) * width + j);
+#pragma unroll
+            for (int i = 0; i < V; ++i) sum[i] += r[i];
+        }
+#pragma unroll 8
+        for (int s = 0; s < base_splits; ++s) add(v, base + s * base_stride + (int64_t)t * width + j);
+        float* o = out + (int64_t)t * width + j;
+#pragma unroll
+        for (int i = 0; i < V; ++i) v[i] += weight * sum[i];
+        if (VEC) st4(o, v[0], v[V > 1 ? 1 : 0], v[V > 2 ? 2 : 0], v[V > 3 ? 3 : 0]);
+        else *o = v[0];
+    }
+}
+
 // ---- experts chosen by a router ---------------------------------------------------------------
 // One warp per token.  z = the router's logits (float32 partial sums, added in index order) over all its outputs;
 // s = softmax(z) over the outputs (`scoring` 0) or sigmoid(z) of each (`scoring` 1); the choice score of an output is
@@ -722,6 +771,18 @@ WICK_API int wick_moe_combine(const float* y, const int* row_of, int top, float 
     WICK_CUDA(launch(moe_combine_kernel, dim3(n), dim3(256), 0, (cudaStream_t)s, y, row_of, top, weight, base, base_splits,
                      (int64_t)n * width, out, width));
     return check_launch("moe_combine");
+}
+
+// y: y_splits partial sums [n_experts][n][width], a token's rows those of the experts that table [vocab, top] names for its id.
+WICK_API int wick_moe_combine_table(const float* y, int y_splits, const int* tokens, const int* table, int top, int n_experts, float weight,
+                                    const float* base, int base_splits, float* out, int n, int width, void* s) {
+    if (n == 0) return 0;
+    const bool vec = width % 4 == 0 && (((uintptr_t)y | (uintptr_t)base | (uintptr_t)out) & 15) == 0;
+    if (vec) WICK_CUDA(launch(moe_combine_table_kernel<true>, dim3(n, ceil_div(width, 1024)), dim3(256), 0, (cudaStream_t)s, y, y_splits, tokens, table, top,
+                              n_experts, weight, base, base_splits, (int64_t)n * width, out, width));
+    else WICK_CUDA(launch(moe_combine_table_kernel<false>, dim3(n, ceil_div(width, 1024)), dim3(256), 0, (cudaStream_t)s, y, y_splits, tokens, table, top,
+                          n_experts, weight, base, base_splits, (int64_t)n * width, out, width));
+    return check_launch("moe_combine_table");
 }
 
 // parts: float32 [splits, n, ld] (the router's logits as partial sums in a row's first n_out columns; a row may hold further

@@ -1305,7 +1305,7 @@ def moe_gather(x: torch.Tensor, row_of: torch.Tensor, n_rows: int) -> torch.Tens
     n, width = x.shape
     _cuda("row_of", row_of, torch.int32)
     top = row_of.shape[1]
-    xs = torch.zeros((n_rows, width), dtype=x.dtype, device=x.device)      # (rows between the experts' stay zero)
+    xs = torch.empty((n_rows, width), dtype=x.dtype, device=x.device)      # (nobody reads what becomes of the rows between the experts')
     _layer().call(f"wick_moe_gather_{_dt(x)}", "ppipiip", _p(x), _p(row_of), top, _p(xs), n, width, _stream())
     return xs
 
@@ -1324,6 +1324,25 @@ def moe_combine(y: torch.Tensor, row_of: torch.Tensor, weight: float, base: Opti
     out = torch.empty((n, width), dtype=torch.float32, device=y.device)
     _layer().call("wick_moe_combine", "ppifpipiip", _p(y), _p(row_of), top, float(weight), _p(base), splits, _p(out), n, width,
                   _stream())
+    return out
+
+
+def moe_combine_table(y: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, weight: float,
+                      base: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """float32 out[t] = sum(base[:, t]) + weight * sum over c of y[:, table[tokens[t], c], t] (the partial sums in index order);
+    y: float32 [splits, experts, n, width]."""
+    _cuda("y", y, torch.float32)
+    y_splits, experts, n, width = y.shape
+    _cuda("tokens", tokens, torch.int32, (n,))
+    _cuda("table", table, torch.int32)
+    splits = 0
+    if base is not None:
+        _cuda("base", base, torch.float32)
+        _need(base.dim() == 3 and tuple(base.shape[1:]) == (n, width), f"base must be [splits, {n}, {width}]")
+        splits = base.shape[0]
+    out = torch.empty((n, width), dtype=torch.float32, device=y.device)
+    _layer().call("wick_moe_combine_table", "pippiifpipiip", _p(y), y_splits, _p(tokens), _p(table), table.shape[1], experts, float(weight),
+                  _p(base), splits, _p(out), n, width, _stream())
     return out
 
 

@@ -150,6 +150,39 @@ def gemm_tc_pair(a: torch.Tensor, b: torch.Tensor, b_rows: int, *, out: torch.Te
                 _p(st), _stream())
 
 
+def gemm_tc_experts(a: torch.Tensor, n_experts: int, rows: int, b: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, *,
+                    gated: bool, per_expert_b: bool, k: int, splits: int = 1) -> torch.Tensor:
+    """Few tokens times the matrices of the experts that ``table`` (int32 [vocab, top]) names for their ids ``tokens`` (int32 [n]):
+    ``a`` holds the experts' packed matrices (:func:`pack`) of ``rows`` outputs one after the other.  b: [n, k], or with
+    ``per_expert_b`` [n_experts * n, k] (an expert's rows by token).  ``splits`` (plain matrices):
+    runs of the inner dimension.  Returns bfloat16
+    [n_experts, n, rows], silu(g) * u, for gated pairs, otherwise float32 partial sums [splits, n_experts, n, rows]; only the
+    places of tokens whose id names the expert hold numbers."""
+    for nm, t in (("a", a), ("b", b)):
+        if not (t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()):
+            raise KernelError(f"gemm_tc_experts: {nm} must be a contiguous bfloat16 CUDA tensor")
+    for nm, t in (("tokens", tokens), ("table", table)):
+        if not (t.is_cuda and t.dtype == torch.int32 and t.is_contiguous()):
+            raise KernelError(f"gemm_tc_experts: {nm} must be a contiguous int32 CUDA tensor")
+    n = tokens.numel()
+    if a.dim() != 4 or a.shape[0] % n_experts or a.shape[1] != (k + 63) // 64 or b.dim() != 2 or b.shape[1] != k \
+            or b.shape[0] != (n * n_experts if per_expert_b else n) or n > FEW_MAX or table.dim() != 2:
+        raise KernelError("gemm_tc_experts: sizes that do not go together")
+    group_rows = a.shape[0] // n_experts * 128
+    out = torch.empty((n_experts, n, rows) if gated else (splits, n_experts, n, rows),
+                      dtype=torch.bfloat16 if gated else torch.float32, device=b.device)
+    if n == 0:
+        return out
+    st = status_tensor(a.device)
+    _lib().call("wick_gemm_tc_grouped", "piiipliiiiiipppiiipp", _p(a), n_experts, group_rows, rows, _p(b), b.shape[0], 1 if per_expert_b else 0,
+                n, k, _ceil16(n), 1 if gated else 0, (rows + 127) // 128 * 128, _p(out), _p(tokens), _p(table), table.shape[1],
+                splits, (100 if n <= 128 else 200) * 1024, _p(st), _stream())
+    return out
+
+
+FEW_MAX = 128               # tokens of gemm_tc_experts at most
+
+
 def _ceil16(n: int) -> int:
     return (n + 15) // 16 * 16
 
@@ -267,3 +300,11 @@ def plan_for(weight: torch.Tensor, gated: bool = False) -> Optional[Plan]:
     if gated and weight.shape[0] % 2 != 0:
         return None
     return Plan(weight, gated)
+def even_splits(wanted: int, k_blocks: int) -> int:
+    """At most ``wanted`` runs of ``k_blocks`` steps, none of them empty."""
+    s = max(1, wanted)
+    while s > 1 and (s - 1) * -(-k_blocks // s) >= k_blocks:
+        s -= 1
+    return s
+
+

@@ -186,19 +186,42 @@ class TableMoE(FeedForward):
             if base.dim() == 2:
                 base = base.unsqueeze(0)
         n = x.shape[0]
-        if self.up_tiles is not None and n >= self.SORTED_FROM:
+        if self.up_tiles is not None and n > self.FEW_MAX:
             return self._forward_sorted(x, batch, base)
+        if self.up_tiles is not None:
+            return self._forward_few(x, batch, base)
         hidden = ops.moe_table_up(x, batch.tokens, self.table, self.gate_up)
         return ops.moe_table_down(hidden, batch.tokens, self.table, self.down, 1.0 / self.top, base).unsqueeze(0)
 
-    # From this many tokens on a step sorts its rows by expert, every expert's rows starting at a
+    # Up to this many tokens every expert that the step uses is multiplied with all of them, in the orientation of the dense
+    # products of few tokens (the matrices stream through the 128-row side once; what other tokens make of an expert is not
+    # written).  The runs of the inner dimension depend on the matrices alone, so that a token's bits do not depend on the step.
+    FEW_MAX = 128
+
+    def _few_splits(self, n):
+        """Runs of the down product's inner dimension: two, where its tiles alone leave SMs without a block, fixed for the sizes of
+        decode steps so that a token's bits do not depend on the step.  (Experts of 1,536 x 2,048, 8 tokens: 36.5 us in one run,
+        33.7 in two, 38.2 in four; the gated product in two runs is faster up to four tokens only.)"""
+        from ..ops import gemm_tc
+        k_blocks = (self.intermediate + 63) // 64
+        return gemm_tc.even_splits(min(2, k_blocks // 4), k_blocks) if n <= gemm_tc.SMALL else 1
+
+    def _forward_few(self, x, batch, base):
+        from ..ops import gemm_tc
+        f, w = self.intermediate, self.width
+        hidden = gemm_tc.gemm_tc_experts(self.up_tiles, self.experts, f, x, batch.tokens, self.table, gated=True, per_expert_b=False, k=w)
+        y = gemm_tc.gemm_tc_experts(self.down_tiles, self.experts, w, hidden.view(-1, f), batch.tokens, self.table, gated=False,
+                                    per_expert_b=True, k=f, splits=self._few_splits(x.shape[0]))
+        return ops.moe_combine_table(y, batch.tokens, self.table, 1.0 / self.top, base).unsqueeze(0)
+
+    # With more tokens a step sorts its rows by expert, every expert's rows starting at a
     # multiple of 256, and runs ONE tensor-core product over all of them: a tile of 256 rows is
     # multiplied with the matrices of the expert the tile belongs to.  How many rows that makes
     # depends on the step's tokens: the host counts them from the step's token ids where the step's
     # description has them (the table is a constant); otherwise (a captured step, whose tokens the
     # host never sees) the product runs over the most rows there can be, and the tiles beyond the
-    # last expert's hold zeros.  Fewer tokens go through the kernels that walk the matrices by expert.
-    SORTED_FROM = 16
+    # last expert's hold zeros.  The 32-bit path and sizes the tensor-core
+    # kernels do not take go through the kernels that walk the matrices by expert.
     ROW_TILE = 256
 
     def _forward_sorted(self, x, batch, base):
