@@ -98,6 +98,23 @@ def test_attention_over_rows_on_the_tensor_cores(H, R, r, q_lens, starts, window
             t += 1
 
 
+@pytest.mark.parametrize("ff, width, t", [(64, 512, 1), (200, 1024, 16), (320, 2048, 17), (65, 576, 128), (1000, 264, 5)])
+def test_gated_products_of_few_tokens_joined_over_a_cluster(ff, width, t):
+    """Few tiles of a gated pair: runs of the inner dimension meet inside the kernel; a token's bits do not depend on the others."""
+    from wick_b200.ops import gemm_tc as G
+    g = torch.Generator().manual_seed(ff)
+    w = (torch.randn(2 * ff, width, generator=g) / math.sqrt(width)).bfloat16().to(DEV)
+    x = torch.randn(t, width, generator=g).bfloat16().to(DEV)
+    plan = G.plan_for(w, gated=True)
+    assert plan.joined_splits == {512: 2, 1024: 4, 2048: 8, 576: 2, 264: 1}[width]
+    got = plan.forward(x, torch.bfloat16)
+    ref = gated(x.double() @ w.double().T)
+    G.check_status()
+    assert (got.double() - ref).abs().max() < 2 ** -8 * max(1.0, float(ref.abs().max()))
+    if t <= G.SMALL:
+        assert torch.equal(plan.forward(x[:1].contiguous(), torch.bfloat16), got[:1])
+
+
 @pytest.mark.parametrize("E, top, ff, width, shared", [(5, 3, 136, 264, False), (8, 2, 192, 1024, True), (1, 1, 64, 128, False), (16, 2, 72, 512, False)])
 @pytest.mark.parametrize("n", [1, 2, 17, 64, 65, 128, 129])
 def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):

@@ -83,7 +83,13 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // Grouped: the m tiles run over several matrices (experts), all multiplied with the same few rows of B or each with rows of
 // its own.  A block whose matrix no token of the step uses leaves at once, and of the others' results only those of tokens
 // that use the matrix are written.
-template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool GROUPED = false>
+//
+// Joined (a gated pair that shares a tile, transposed bfloat16 result): the runs of the inner dimension along blockIdx.z are a
+// cluster; every block leaves its accumulator in its shared memory (the ring is idle by then), and the blocks finish a share of the
+// tokens each, adding the runs' sums in index order over distributed shared memory.  A pair cannot be left as partial sums, and
+// without runs a narrow matrix fills a part of the device only: 5,120 + 5,120 rows of 2,048 at one token are 80 blocks,
+// 16.5 us; as 240 blocks 11.7 us.
+template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool GROUPED = false, bool JOINED = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const std::conditional_t<GROUPED, GroupedParams, GemmParams> p) {
@@ -290,14 +296,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // One answer for the four epilogue warps, so that they leave the loop together.
             const bool ok_warp = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1, &abort_flag, p.status, 3));
             bool ok = ok_warp;
-            if (my_tiles > 1 || GATED == 3) {            // (a block with one plain tile has nothing left to agree on)
+            if (my_tiles > 1 || (GATED == 3 && !JOINED)) {            // (a block with one plain tile has nothing left to agree on)
                 if (lane == 0) ok_w[q] = ok_warp ? 1 : 0;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 ok = ok_w[0] && ok_w[1] && ok_w[2] && ok_w[3];
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
             tc_fence_after();
-            if (GATED == 3) {
+            if (JOINED) {
+                // column n of the accumulator at tiles[n][128 rows]
+                float* acc = reinterpret_cast<float*>(tiles);
+                for (int c0 = 0; c0 < p.bn; c0 += 16) {
+                    float v[16];
+                    tc_ld16(lane_addr + c0, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[(c0 + j) * BM + q * 32 + lane] = v[j];
+                }
+            } else if (GATED == 3) {
                 // Lanes 0-63 of the accumulator hold gate rows, lanes 64-127 the up rows of the
                 // same outputs (transposed output only).  Of every 16 columns the warps of the gate
                 // rows finish and store the first 8, the warps of the up rows the last 8 (the
@@ -391,6 +406,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     }
 
+    if constexpr (JOINED) {
+        static_assert(!GROUPED, "built for one matrix");
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const int runs = (int)gridDim.z, rank = (int)blockIdx.z, m0 = (int)blockIdx.x * (BM / 2);
+        const int n0 = blockIdx.y * p.bn;
+        const uint32_t here = smem_u32(tiles);
+        auto sum = [&](int at) {
+            float v = 0.f;
+#pragma unroll 8
+            for (int z = 0; z < runs; ++z) {
+                uint32_t there;
+                float d;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here + 4u * (uint32_t)at), "r"(z));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(d) : "r"(there) : "memory");
+                v = z == 0 ? d : v + d;
+            }
+            return v;
+        };
+        __nv_bfloat16* o = (__nv_bfloat16*)p.out;
+        const int tokens = min(p.bn, p.b_rows - n0);
+        for (int x = rank * NUM_THREADS + (int)threadIdx.x; x < tokens * (BM / 2); x += runs * NUM_THREADS) {
+            const int n = x / (BM / 2), m = x % (BM / 2);
+            if (m0 + m >= p.a_rows) continue;
+            const float g = sum(n * BM + m), u = sum(n * BM + BM / 2 + m);
+            o[(long long)(n0 + n) * p.ldo + m0 + m] = __float2bfloat16_rn(g / (1.0f + expf(-g)) * u);
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // (nobody leaves while it is read)
+    }
+
     tc_fence_before();
     __syncthreads();
     if (abort_flag) {
@@ -435,6 +480,30 @@ struct Groups {
     const int *tokens, *table;
 };
 
+// The blocks along z are a cluster.
+static int launch_joined(dim3 grid, int smem, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, cudaStream_t s) {
+    static bool raised = false;
+    if (!raised) {
+        WICK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false, 3, true, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+        raised = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = grid.z;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    WICK_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false, 3, true, false, false, true>, map_a, map_b, p));
+    return check_launch("gemm_tc_joined");
+}
+
 static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const void* b, long long b_total_rows,
                         int b_rows, int k, int bn, int gated, int pair_offset, int transposed, int out_f32,
                         int a_static, int b_static, int a_packed, int b_packed, void* out, long long ldo, int splits, long long split_stride, int max_smem_bytes, int* status,
@@ -445,7 +514,8 @@ static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const
     WICK_REQUIRE(gated != 3 || transposed, "gemm_tc: the shared-tile pair is built for the transposed output only");
     WICK_REQUIRE(gated != 1 || transposed, "gemm_tc: a pair in the 128-row operand goes with the transposed output");
     WICK_REQUIRE(gated != 2 || !transposed, "gemm_tc: a pair in the narrow operand goes with the row-major output");
-    WICK_REQUIRE(splits == 1 || (out_f32 && !gated), "gemm_tc: a split inner dimension needs plain float32 partial sums");
+    // (a gated pair that shares a tile: the runs of the inner dimension are joined inside the kernel, by a cluster)
+    WICK_REQUIRE(splits == 1 || (out_f32 && !gated) || (gated == 3 && !out_f32 && splits <= 8), "gemm_tc: a split inner dimension needs plain float32 partial sums");
     WICK_REQUIRE(a_rows > 0 && b_rows >= 0 && k > 0, "gemm_tc: bad sizes");
     if (b_rows == 0) return 0;
     const int k_blocks = ceil_div(k, BK);
@@ -466,6 +536,9 @@ static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     if (stages > per_split) stages = per_split < 2 ? 2 : per_split;
     WICK_REQUIRE(stages >= 2, "gemm_tc: %d bytes of shared memory hold fewer than two stages of %d bytes", budget, stage_bytes);
+    const bool joined = gated == 3 && splits > 1;
+    if (joined && stages * stage_bytes < bn * BM * 4) stages = ceil_div(bn * BM * 4, stage_bytes);      // (the ring holds the accumulator at the end)
+    WICK_REQUIRE(!joined || stages <= MAX_STAGES, "gemm_tc: the joined tile does not fit the ring");
     const int smem = stages * stage_bytes + 1024;
     GemmParams p;
     p.a_rows = a_rows; p.b_rows = b_rows; p.bn = bn; p.k_blocks = k_blocks; p.k_blocks_per_split = per_split;
@@ -482,7 +555,7 @@ static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const
         static_cast<GemmParams&>(g) = p;
         g.group_tiles = p.grid_m; g.group_rows = G.rows; g.group_b_rows = G.b_rows; g.group_out = G.out;
         g.top = G.top; g.n_tokens = G.n_tokens; g.tokens = G.tokens; g.table = G.table;
-        WICK_REQUIRE(a_packed && transposed && (gated == 0 || gated == 3) && (out_f32 != 0) == (gated == 0), "gemm_tc: grouped products are built for packed matrices, transposed results");
+        WICK_REQUIRE(a_packed && transposed && (gated == 0 || gated == 3) && (out_f32 != 0) == (gated == 0) && !joined, "gemm_tc: grouped products are built for packed matrices, transposed results");
         WICK_REQUIRE((long long)G.n * G.rows <= a_total_rows && G.rows % 128 == 0 && G.n_tokens == b_rows && b_rows <= 256 && G.top > 0, "gemm_tc: bad groups");
         WICK_REQUIRE(total * G.n < (1ll << 30) && splits <= 65535 && p.grid_n <= 65535, "gemm_tc: too many tiles");
         const dim3 grid(p.grid_m * G.n, p.grid_n, splits);
@@ -504,6 +577,7 @@ static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const
     const bool persistent = !transposed && p.total_tiles > resident;
     WICK_REQUIRE(persistent || (p.grid_n <= 65535 && splits <= 65535), "gemm_tc: grid limit");
     const dim3 grid = persistent ? dim3(resident) : dim3(p.grid_m, p.grid_n, splits);
+    if (joined) return launch_joined(dim3(p.grid_m, p.grid_n, splits), smem, map_a, map_b, p, (cudaStream_t)stream);
     // One instantiation per (persistent, pair mode, orientation, output type): a
     // block of a decode step runs for a few microseconds, so the kernel it loads
     // should hold nothing but its own path.

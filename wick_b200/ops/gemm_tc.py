@@ -205,6 +205,9 @@ class Plan:
         self.decode_splits = max(1, min(2 * self.sms // tiles, 8, k_blocks // 8))
         self.k_blocks = k_blocks
 
+        # A gated pair (64 outputs a tile): runs that a cluster joins, where the tiles alone leave SMs without a block, of
+        # at least four 64-wide steps.
+        self.joined_splits = even_splits(min(2 * self.sms // ((self.n_out + 63) // 64), 8, k_blocks // 4), k_blocks) if gated else 1
     def matrix(self) -> torch.Tensor:
         """The weight as it was given: [rows, k], row-major (a copy)."""
         return unpack(self.w, self.rows, self.k, self.gated)
@@ -283,6 +286,8 @@ class Plan:
             gemm_tc_pair(x, self.w, self.n_out, out=out, ldo=self.n_out, gated=self.gated, pair_offset=self.pair_offset,
                          b_packed=True, splits=splits, split_stride=t * self.n_out)
         else:
+            if self.gated and out.dtype == torch.bfloat16 and t <= 128:
+                splits = self.joined_splits
             bn = min(128 if self.gated else 256, _ceil16(self.n_out))
             if bn > 128:
                 bn = 256                               # two packed tiles of 128 rows
