@@ -152,3 +152,22 @@ def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
     if n <= 64:
         one = part.forward(x[:1].contiguous(), types.SimpleNamespace(tokens=tok[:1].contiguous(), host=None)).sum(0)
         assert torch.equal(one, got[:1]), "a token's bits do not depend on the others"
+
+
+@pytest.mark.parametrize("width", [4, 132, 4096, 4100, 5120, 5124, 6144, 6148])
+@pytest.mark.parametrize("splits", [0, 1, 7, 9])
+def test_norm_forms_give_the_same_bits(width, splits):
+    """A warp per row (600 rows, up to 5,120 numbers), a block with the row in registers, a block with the row in shared memory."""
+    g = torch.Generator().manual_seed(width + splits)
+    x, w = torch.randn(600, width, generator=g).to(DEV), (1 + 0.1 * torch.randn(width, generator=g)).to(DEV)
+    delta = torch.randn(splits, 600, width, generator=g).to(DEV) if splits else None
+    ref = x.double() + (delta.double().sum(0) if splits else 0)
+    ref = ref / torch.sqrt((ref * ref).mean(1, keepdim=True) + 1e-5) * w.double()
+    for dtype, tol in ((torch.float32, 2e-6), (torch.bfloat16, 2 ** -8)):
+        many = ops.rmsnorm(x.clone(), w, 1e-5, dtype, delta=delta)
+        assert (many.double() - ref).abs().max() < tol * float(ref.abs().max())
+        few_x = x[:9].clone()
+        few = ops.rmsnorm(few_x, w, 1e-5, dtype, delta=delta[:, :9].contiguous() if splits else None)
+        assert torch.equal(few, many[:9])
+        if splits:
+            assert (few_x.double() - (x[:9].double() + delta[:, :9].double().sum(0))).abs().max() < 1e-5

@@ -147,10 +147,10 @@ __global__ void __launch_bounds__(1024, 1) rmsnorm_kernel(float* __restrict__ x,
     }
 }
 
-// One warp per output row, for rows that are a multiple of 4 wide and at most 4096:
+// One warp per output row, for rows that are a multiple of 4 wide and at most 128 QMAX:
 // the row stays in registers (lane l holds quads l, l + 32, ...: one class of the sum),
-// nothing is synchronised but the warp.
-template <typename TOut>
+// nothing is synchronised but the warp.  Built for rows of up to 4,096 and of up to 5,120 numbers.
+template <typename TOut, int QMAX>
 __global__ void __launch_bounds__(128) rmsnorm_rows_kernel(float* __restrict__ x, const float* __restrict__ delta, int splits,
                                                            int64_t split_stride, const float* __restrict__ w, float eps,
                                                            const int* __restrict__ rows, TOut* __restrict__ out, int n_out,
@@ -159,7 +159,6 @@ __global__ void __launch_bounds__(128) rmsnorm_rows_kernel(float* __restrict__ x
     pdl_wait();
     x = fresh(x);
     delta = fresh(delta);
-    constexpr int QMAX = 4096 / 4 / 32;                 // quads of a lane
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (i >= n_out) return;
@@ -504,13 +503,16 @@ int rmsnorm(float* x, const float* delta, int splits, int64_t n_rows_x, const fl
         raised = true;
     }
     const int threads = width >= 4096 ? 1024 : (width >= 2048 ? 512 : (width >= 512 ? 256 : 128));
-    if (n_out >= 512 && width % 4 == 0 && width <= 4096) {
+    if (n_out >= 512 && width % 4 == 0 && width <= 5120) {
         // Enough rows to give every SM its warps: a warp per row (same bits as the block per row).
+        // (17,600 rows of 5,120 numbers: 81 to 99 us, a block per row 405: its threads all wait for the first warp to add up the
+        // classes, and a block of 1,024 threads is all that an SM holds.)
         // With fewer rows (a decode step of 64 sequences) a warp per row leaves most of the part
         // idle and each warp walks its row's partial sums alone: the block per row is 3x faster there.
         const dim3 grid(ceil_div(n_out, 4)), block(128);
         const int64_t stride = n_rows_x * width;
-        WICK_CUDA(launch(rmsnorm_rows_kernel<TOut>, grid, block, 0, s, x, delta, splits, stride, w, eps, rows, (TOut*)out, n_out, width));
+        if (width <= 4096) WICK_CUDA(launch(rmsnorm_rows_kernel<TOut, 32>, grid, block, 0, s, x, delta, splits, stride, w, eps, rows, (TOut*)out, n_out, width));
+        else WICK_CUDA(launch(rmsnorm_rows_kernel<TOut, 40>, grid, block, 0, s, x, delta, splits, stride, w, eps, rows, (TOut*)out, n_out, width));
         return check_launch("rmsnorm");
     }
     WICK_CUDA(launch(rmsnorm_kernel<TOut>, dim3(n_out), dim3(threads), smem, s, x, delta, splits, n_rows_x * width, w,
