@@ -219,8 +219,14 @@ class Plan:
         fill the part."""
         if self.gated:
             return 1
-        tiles = ((t + 255) // 256) * ((self.n_out + 255) // 256)
-        return max(1, min(4, (self.sms // 2) // tiles, self.k_blocks // 32))
+        # In units of a 64-wide step of a tile (0.36 us): rounds of tiles over the pairs of SMs, the end of the last tile, and what
+        # writing and reading the runs' float32 results costs.  (1,110 tokens x 4,096 outputs of 12,288 inputs:
+        # 80 tiles for 74 pairs are two rounds, 177 us; three runs make four rounds of a third of the length, about 105 us, and
+        # the norm that adds them up takes 18 us instead of 12.)
+        tiles, pairs = ((t + 255) // 256) * ((self.n_out + 255) // 256), max(1, self.sms // 2)
+        def cost(s):
+            return -(-tiles * s // pairs) * -(-self.k_blocks // s) + 16 + (t * self.n_out * 8 * s / 1.6e6 if s > 1 else 0)
+        return min((s for s in range(1, 5) if s == 1 or self.k_blocks // s >= 32), key=cost)
 
     def short_prompt_splits(self) -> int:
         """Runs of the inner dimension for SMALL < tokens <= SWAP_MAX (weights as the 128-row
