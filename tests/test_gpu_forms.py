@@ -171,3 +171,18 @@ def test_norm_forms_give_the_same_bits(width, splits):
         assert torch.equal(few, many[:9])
         if splits:
             assert (few_x.double() - (x[:9].double() + delta[:, :9].double().sum(0))).abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("width", [4, 260, 2048, 4096, 4100, 8192, 8196])
+@pytest.mark.parametrize("n", [3, 65])
+@pytest.mark.parametrize("splits", [0, 1, 3, 9])
+def test_scaled_sum_and_norm_forms(width, n, splits):
+    g = torch.Generator().manual_seed(width + n)
+    x, w = torch.randn(n, width, generator=g).to(DEV), (1 + 0.1 * torch.randn(width, generator=g)).to(DEV)
+    delta = torch.randn(splits, n, width, generator=g).to(DEV) if splits else None
+    ref = 1.7 * x.double() + (delta.double().sum(0) if splits else 0)
+    ref = ref / torch.sqrt((ref * ref).mean(1, keepdim=True) + 1e-5) * w.double()
+    xd = x.clone()
+    out = ops.scaled_add_rmsnorm(xd, delta, 1.7, w, 1e-5, torch.bfloat16)
+    assert (xd.double() - ref).abs().max() < 2e-6 * float(ref.abs().max())
+    assert torch.equal(out, xd.bfloat16())
