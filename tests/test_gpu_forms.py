@@ -186,3 +186,35 @@ def test_scaled_sum_and_norm_forms(width, n, splits):
     out = ops.scaled_add_rmsnorm(xd, delta, 1.7, w, 1e-5, torch.bfloat16)
     assert (xd.double() - ref).abs().max() < 2e-6 * float(ref.abs().max())
     assert torch.equal(out, xd.bfloat16())
+
+
+@pytest.mark.parametrize("H, G, d, e, rot, n, splits", [(4, 2, 16, 24, 8, 3, 1), (32, 8, 128, 128, 128, 70, 1), (32, 8, 128, 128, 64, 8, 8),
+                                                        (10, 2, 20, 4, 20, 66, 3), (48, 8, 128, 64, 0, 65, 2), (1, 1, 4, 4, 4, 1, 9)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_projection_finish_in_registers_is_the_general_form(H, G, d, e, rot, n, splits, dtype, mode):
+    """The same call with a further column in every row of partial sums, so that rows are no multiple of four numbers, takes the
+    general form, element by element."""
+    g = torch.Generator().manual_seed(H * d + n)
+    W = (H + G) * d + G * e
+    parts = torch.randn(splits, n, W, generator=g).to(DEV)
+    odd = torch.cat([parts, torch.zeros(splits, n, 1, device=DEV)], 2).contiguous()
+    assert W % 4 == 0 and odd.shape[2] % 4 != 0
+    bias, qw, kw = ((s + 0.1 * torch.randn(m, generator=g)).to(DEV) for s, m in ((0.0, W), (1.0, H * d), (1.0, G * d)))
+    batch, pages, n_pages = batch_of([n], [37])
+    cos = sin = None
+    if rot:
+        inv = torch.tensor([100.0 ** (-2.0 * i / rot) for i in range(rot // 2)]).to(DEV)
+        cos, sin = ops.rope_table(batch.positions, inv)
+    keep0 = torch.randn(n, G * e, generator=g).to(DEV)
+    got = []
+    for p in (parts, odd):
+        keep = keep0.clone()
+        kv = torch.zeros((n_pages, G * PAGE * (d + e)), dtype=dtype, device=DEV)
+        q = ops.qkv_finish(p, H, G, d, e, dtype=dtype, bias=bias, q_weight=qw, k_weight=kw, eps=1e-5, cos=cos, sin=sin, rot_dims=rot,
+                           v_keep=keep if mode else None, v_mode=mode, blend=torch.tensor([0.3], device=DEV) if mode == 2 else None, kv=kv,
+                           page_table=batch.page_table, seq_of_token=batch.seq_of_token, positions=batch.positions)
+        got.append((q, kv, keep))
+    tol = 1e-5 if dtype == torch.float32 else 2 ** -7              # (the sums of squares run in another order: the last bit of 32, or one of bfloat16)
+    for a, b in zip(*got):
+        assert (a.double() - b.double()).abs().max() <= tol * max(1.0, float(b.double().abs().max()))

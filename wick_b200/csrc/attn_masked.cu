@@ -327,6 +327,114 @@ qkv_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_str
     }
 }
 
+// The form without the extras (no filter, no blocks, no gate, no norm of the values, one vector a head), for norms over the whole
+// projection and rotations of neighbouring pairs, rows of whole groups of four: a thread keeps VPT groups of four of the row in
+// registers, the loads of all of them on their way together, and writes each once, eight or sixteen bytes at a time.  (3,300 rows of
+// 6,144 numbers: 56 us where the form above takes 136, which writes element by element and divides to find each one's
+// place; eight rows of 3,072, eight partial sums: 5.5 us against 15.)
+template <typename T, int VPT>
+__global__ void __launch_bounds__(VPT <= 2 ? 1024 : 256)
+qkv_finish_regs_kernel(const float* __restrict__ parts, int splits, int64_t split_stride, const float* __restrict__ bias,
+                       int H, int G, int d, int e, const float* __restrict__ q_w, int q_span, const float* __restrict__ k_w,
+                       int k_span, float eps, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot_dims,
+                       float* __restrict__ v_keep, int v_mode, const float* __restrict__ lambda, T* __restrict__ q_out,
+                       T* __restrict__ kv, const int* __restrict__ page_table, int table_width,
+                       const int* __restrict__ seq_of_token, const int* __restrict__ positions, int write_kv, int cols) {
+    constexpr int SU = VPT == 1 ? 8 : (VPT == 2 ? 4 : 1);             // partial sums whose loads go out together
+    constexpr bool AHEAD = VPT <= 2;                    // few tokens: weights and the step's description before the kernel before this one has finished
+    __shared__ float red[2 * 32];
+    pdl_trigger();
+    const int t = blockIdx.x;
+    const int Wq = H * d, Wk = G * d, Wv = G * e, W = Wq + Wk + Wv;
+    const int pos = positions[t], half = cos_t ? rot_dims >> 1 : 0, r = pos % kPage;
+    T* page = nullptr;
+    if (write_kv) page = kv + (int64_t)page_table[(int64_t)seq_of_token[t] * table_width + pos / kPage] * G * kPage * (d + e);
+    const float lam = v_mode == 2 ? *lambda : 0.f;
+    float4 b4[VPT], w4[VPT];
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) {
+        const int j = (u * (int)blockDim.x + (int)threadIdx.x) * 4;
+        if (!AHEAD || j >= W) continue;
+        if (bias) b4[u] = ld4(bias + j);
+        if (j < Wq ? q_w != nullptr : (j < Wq + Wk && k_w)) w4[u] = ld4(j < Wq ? q_w + j : k_w + j - Wq);
+    }
+    pdl_wait();
+    parts = fresh(parts);
+    v_keep = fresh(v_keep);
+    cos_t = fresh(cos_t);
+    sin_t = fresh(sin_t);
+    const float* mine = parts + (int64_t)t * cols;
+    float4 v[VPT];
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < splits; s0 += SU) {
+        float4 p[SU][VPT];
+#pragma unroll
+        for (int k = 0; k < SU; ++k)
+#pragma unroll
+            for (int u = 0; u < VPT; ++u) {
+                const int j = (u * (int)blockDim.x + (int)threadIdx.x) * 4;
+                p[k][u] = s0 + k < splits && j < W ? ld4(mine + (s0 + k) * split_stride + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+        for (int k = 0; k < SU; ++k)
+#pragma unroll
+            for (int u = 0; u < VPT; ++u) {
+                v[u].x += p[k][u].x; v[u].y += p[k][u].y; v[u].z += p[k][u].z; v[u].w += p[k][u].w;
+            }
+    }
+    float ss[2] = {0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) {
+        const int j = (u * (int)blockDim.x + (int)threadIdx.x) * 4;
+        if (j >= W) continue;
+        if (bias) {
+            const float4 b = AHEAD ? b4[u] : ld4(bias + j);
+            v[u].x += b.x; v[u].y += b.y; v[u].z += b.z; v[u].w += b.w;
+        }
+        const float sq = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, v[u].w * v[u].w)));
+        if (j < Wq) ss[0] += sq;
+        else if (j < Wq + Wk) ss[1] += sq;
+    }
+    if (q_span > 0 || k_span > 0) block_sums(ss, red);
+    const float fq = q_span > 0 ? 1.0f / sqrtf(ss[0] / (float)Wq + eps) : 1.f, fk = k_span > 0 ? 1.0f / sqrtf(ss[1] / (float)Wk + eps) : 1.f;
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) {
+        const int j = (u * (int)blockDim.x + (int)threadIdx.x) * 4;
+        if (j >= W) continue;
+        float4 y = v[u];
+        if (j >= Wq + Wk) {
+            const int at = j - Wq - Wk, g = at / e, x = at - g * e;
+            float* keep = v_keep + (int64_t)t * Wv + at;
+            if (v_mode == 1) st4(keep, y.x, y.y, y.z, y.w);
+            if (v_mode == 2) {
+                const float4 k = ld4(keep);
+                y = make_float4((1.0f - lam) * y.x + lam * k.x, (1.0f - lam) * y.y + lam * k.y, (1.0f - lam) * y.z + lam * k.z,
+                                (1.0f - lam) * y.w + lam * k.w);
+            }
+            if (write_kv) st4(page + (int64_t)G * kPage * d + ((int64_t)g * kPage + r) * e + x, y.x, y.y, y.z, y.w);
+            continue;
+        }
+        const bool is_q = j < Wq;
+        const int at = is_q ? j : j - Wq, h = at / d, x = at - h * d;
+        if ((is_q ? q_span : k_span) > 0) {
+            const float f = is_q ? fq : fk;
+            y.x *= f; y.y *= f; y.z *= f; y.w *= f;
+            const float* w = is_q ? q_w : k_w;
+            if (w) {
+                const float4 g = AHEAD ? w4[u] : ld4(w + at);
+                y.x *= g.x; y.y *= g.y; y.z *= g.z; y.w *= g.w;
+            }
+        }
+        if (x < 2 * half) {
+            const float2 c = ld2(cos_t + (int64_t)t * half + (x >> 1)), s = ld2(sin_t + (int64_t)t * half + (x >> 1));
+            y = make_float4(y.x * c.x - y.y * s.x, y.y * c.x + y.x * s.x, y.z * c.y - y.w * s.y, y.w * c.y + y.z * s.y);
+        }
+        if (is_q) st4(q_out + (int64_t)t * Wq + j, y.x, y.y, y.z, y.w);
+        else if (write_kv) st4(page + ((int64_t)h * kPage + r) * d + x, y.x, y.y, y.z, y.w);
+    }
+}
+
 // The blocks of `block` positions that a step completes: their mean keys and values go to the store (as above), and, with
 // `flat`, so do all blocks the sequences' tokens can see to arrays whose tiles of 64 blocks lie like cache pages: tile i of sequence b is
 // page b * flat_tiles + i of [G][64][d] keys, then [G][64][e] values (places beyond a sequence's whole blocks hold zeros).
@@ -742,6 +850,25 @@ int qkv_finish(const float* parts, int splits, int n, const float* bias, int H, 
     WICK_REQUIRE(!X.pool || (write_kv && X.block > 0 && X.rows == (kPage + X.block - 1) / X.block && X.pool_page == (int64_t)G * X.rows * (d + e)),
                  "qkv_finish: bad blocks");
     if (n == 0) return 0;
+    // (the extras and the other norms and rotations: the form below; a block's size changes with n beyond the sizes of decode steps only)
+    const int W = Wq + Wk + G * e;
+    if (!X.conv_w && !X.v_norm && !X.pool && X.gate_heads == 0 && flags == 0 && maps == 1 && (q_span == 0 || q_span == Wq) &&
+        (k_span == 0 || k_span == Wk) && (!cos_t || rot_dims == 0 || (pairing == 0 && rot_dims % 4 == 0)) && d % 4 == 0 && e % 4 == 0 && cols % 4 == 0 &&
+        W <= 8192 && (((uintptr_t)parts | (uintptr_t)bias | (uintptr_t)q_w | (uintptr_t)k_w | (uintptr_t)cos_t | (uintptr_t)sin_t |
+                        (uintptr_t)v_keep | (uintptr_t)q_out | (uintptr_t)kv) & 15) == 0) {
+        const int groups = W / 4, most = n > 64 ? 256 : 1024;
+        const int threads = min(most, (groups + 31) / 32 * 32), vpt = ceil_div(groups, threads);
+#define WICK_FINISH(V) WICK_CUDA(launch(qkv_finish_regs_kernel<T, V>, dim3(n), dim3(threads), 0, s, parts, splits, (int64_t)n * cols, bias, H, G, d, e, \
+                                        q_w, q_span, k_w, k_span, eps, cos_t, sin_t, rot_dims, v_keep, v_mode, lambda, (T*)q_out, (T*)kv, page_table,   \
+                                        table_width, seq_of_token, positions, write_kv, cols))
+        if (vpt == 1) WICK_FINISH(1);
+        else if (vpt == 2) WICK_FINISH(2);
+        else if (vpt <= 4) WICK_FINISH(4);
+        else if (vpt <= 6) WICK_FINISH(6);
+        else WICK_FINISH(8);
+#undef WICK_FINISH
+        return check_launch("qkv_finish");
+    }
     const size_t smem = (size_t)(Wq + Wk + G * e) * sizeof(float);
     WICK_REQUIRE(smem <= 200 * 1024, "qkv_finish: a row of %d numbers is beyond one block's shared memory", Wq + Wk + G * e);
     static bool raised = false;
