@@ -204,10 +204,10 @@ class Plan:
         # split keeps at least eight 64-wide steps of the inner dimension.
         self.decode_splits = max(1, min(2 * self.sms // tiles, 8, k_blocks // 8))
         self.k_blocks = k_blocks
-
         # A gated pair (64 outputs a tile): runs that a cluster joins, where the tiles alone leave SMs without a block, of
         # at least four 64-wide steps.
         self.joined_splits = even_splits(min(2 * self.sms // ((self.n_out + 63) // 64), 8, k_blocks // 4), k_blocks) if gated else 1
+
     def matrix(self) -> torch.Tensor:
         """The weight as it was given: [rows, k], row-major (a copy)."""
         return unpack(self.w, self.rows, self.k, self.gated)
@@ -284,6 +284,8 @@ class Plan:
             # other's streaming.  A gated pair shares one 128-row tile (64 gate rows,
             # 64 up rows), which doubles the number of blocks.  (More than 128 tokens make
             # stages of 48 KB: one block of 200 KB per SM then.)
+            if self.gated and out.dtype == torch.bfloat16 and t <= 128:
+                splits = self.joined_splits
             gemm_tc(self.w, self.n_out, x, t, bn=_ceil16(t), out=out, ldo=self.n_out,
                     gated=3 if self.gated else 0, pair_offset=self.pair_offset, transposed=True, splits=splits,
                     split_stride=t * self.n_out, max_smem=(100 if t <= 128 else 200) * 1024, a_static=True,
@@ -292,14 +294,20 @@ class Plan:
             gemm_tc_pair(x, self.w, self.n_out, out=out, ldo=self.n_out, gated=self.gated, pair_offset=self.pair_offset,
                          b_packed=True, splits=splits, split_stride=t * self.n_out)
         else:
-            if self.gated and out.dtype == torch.bfloat16 and t <= 128:
-                splits = self.joined_splits
             bn = min(128 if self.gated else 256, _ceil16(self.n_out))
             if bn > 128:
                 bn = 256                               # two packed tiles of 128 rows
             gemm_tc(x, t, self.w, self.n_out, bn=bn, out=out, ldo=self.n_out, gated=2 if self.gated else 0,
                     pair_offset=self.pair_offset, transposed=False, splits=splits, split_stride=t * self.n_out,
                     max_smem=200 * 1024, b_static=True, b_packed=True, k=self.k)
+
+
+def even_splits(wanted: int, k_blocks: int) -> int:
+    """At most ``wanted`` runs of ``k_blocks`` steps, none of them empty."""
+    s = max(1, wanted)
+    while s > 1 and (s - 1) * -(-k_blocks // s) >= k_blocks:
+        s -= 1
+    return s
 
 
 def plan_for(weight: torch.Tensor, gated: bool = False) -> Optional[Plan]:
@@ -311,11 +319,3 @@ def plan_for(weight: torch.Tensor, gated: bool = False) -> Optional[Plan]:
     if gated and weight.shape[0] % 2 != 0:
         return None
     return Plan(weight, gated)
-def even_splits(wanted: int, k_blocks: int) -> int:
-    """At most ``wanted`` runs of ``k_blocks`` steps, none of them empty."""
-    s = max(1, wanted)
-    while s > 1 and (s - 1) * -(-k_blocks // s) >= k_blocks:
-        s -= 1
-    return s
-
-
