@@ -9,8 +9,8 @@ which way round the kernel runs:
   several blocks, so that enough of them stream weights at once; the float32
   partial sums are added by the consumer in index order.  Up to 64 tokens (a
   decode step) the number of splits depends on the matrix alone, never on the
-  batch, and two blocks of 100 KB share an SM; short prompts of 65 to 255 tokens
-  take fewer splits (and one 200 KB block per SM beyond 128 tokens).
+  batch, and two blocks of 100 KB share an SM, as they do up to 128 tokens; short prompts of 129
+  to 255 tokens take fewer splits and one 200 KB block per SM.
 * 256 tokens and more: the kernel of ``csrc/gemm_tc2.cu``, in which two thread
   blocks on neighbouring SMs share one 256 x 256 tile (few tiles: the inner
   dimension in 2 to 4 runs).
@@ -201,8 +201,9 @@ class Plan:
         k_blocks = (self.k + 63) // 64
         tiles = (self.n_out + 127) // 128
         # Decode: about two blocks per SM (just under two per SM) stream best; every
-        # split keeps at least eight 64-wide steps of the inner dimension.
-        self.decode_splits = max(1, min(2 * self.sms // tiles, 8, k_blocks // 8))
+        # split keeps at least four 64-wide steps of the inner dimension.  (At least eight, for 2,048 inputs:
+        # four runs of 3,072 / 2,048 outputs took 5.1 / 5.0 us, eight take 4.1 / 3.6.)
+        self.decode_splits = even_splits(min(2 * self.sms // tiles, 8, k_blocks // 4), k_blocks)
         self.k_blocks = k_blocks
         # A gated pair (64 outputs a tile): runs that a cluster joins, where the tiles alone leave SMs without a block, of
         # at least four 64-wide steps.
@@ -230,7 +231,7 @@ class Plan:
 
     def short_prompt_splits(self) -> int:
         """Runs of the inner dimension for SMALL < tokens <= SWAP_MAX (weights as the 128-row
-        operand, at most one block per SM)."""
+        operand) beyond 128, at most one block per SM."""
         return max(1, min(self.sms // ((self.n_out + 127) // 128), 8, self.k_blocks // 8))
 
     def mid_splits(self, t: int) -> int:
@@ -256,7 +257,9 @@ class Plan:
         t = x.shape[0]
         if self.gated:
             raise KernelError("gemm_tc: a gated pair has no partial sums")
-        if t <= SMALL:
+        if t <= 128:
+            # (65 to 128 tokens as in decode, two blocks of 100 KB per SM.  100 tokens, 4,096 outputs of 4,096 / 12,288 inputs:
+            # 9.3 / 21.9 us; with the runs of longer prompts, at most one block per SM, 11.2 / 27.)
             splits = self.decode_splits
         elif t <= SWAP_MAX:
             splits = self.short_prompt_splits()
