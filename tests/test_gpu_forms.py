@@ -115,7 +115,7 @@ def test_gated_products_of_few_tokens_joined_over_a_cluster(ff, width, t):
         assert torch.equal(plan.forward(x[:1].contiguous(), torch.bfloat16), got[:1])
 
 
-@pytest.mark.parametrize("E, top, ff, width, shared", [(5, 3, 136, 264, False), (8, 2, 192, 1024, True), (1, 1, 64, 128, False), (16, 2, 72, 512, False)])
+@pytest.mark.parametrize("E, top, ff, width, shared", [(5, 3, 136, 264, 0), (8, 2, 192, 1024, 64), (1, 1, 64, 128, 0), (16, 2, 72, 512, 0), (5, 2, 520, 264, 1000)])
 @pytest.mark.parametrize("n", [1, 2, 17, 64, 65, 128, 129])
 def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
     """Experts that no token uses are left alone; results beyond a token's own experts are never read (they hold NaN before)."""
@@ -124,7 +124,7 @@ def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
     from wick_b200.parts import feedforward  # noqa: F401
     g = torch.Generator().manual_seed(E + n)
     part = build_part("ffn", PartSpec("table_moe", dict(width=width, vocab=50, experts=E, top=top, intermediate=ff,
-                                                        shared=PartSpec("gated_mlp", dict(width=width, intermediate=64, activation="silu",
+                                                        shared=PartSpec("gated_mlp", dict(width=width, intermediate=shared, activation="silu",
                                                                                           names=dict(gate="gate_proj.weight", up="up_proj.weight", down="down_proj.weight"))) if shared else None)),
                       BuildContext(dtype=torch.bfloat16, device=torch.device(DEV)))
     tensors = {}
@@ -132,7 +132,8 @@ def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
     def get(name):
         if name == "table":
             return torch.rand(50, E, generator=g).argsort(1)[:, :top].int()
-        rows, cols = (width, 64 if "shared" in name else ff) if "down" in name else (64 if "shared" in name else ff, width)
+        inner = shared if "shared" in name else ff
+        rows, cols = (width, inner) if "down" in name else (inner, width)
         return tensors.setdefault(name, (torch.randn(rows, cols, generator=g) / math.sqrt(cols)).bfloat16().to(DEV))
     part.load(get)
     x = torch.randn(n, width, generator=g).bfloat16().to(DEV)

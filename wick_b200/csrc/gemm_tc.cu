@@ -69,6 +69,11 @@ struct GroupedParams : GemmParams {
     int group_tiles, group_rows, group_b_rows, top, n_tokens;
     long long group_out;
     const int *tokens, *table;
+    // A matrix that every token uses besides (the shared expert's; its m tiles follow the groups'), multiplied with rows of its own:
+    // operands, sizes and result as for the groups.  shared_tiles 0: there is none.
+    int groups_end, shared_tiles, shared_rows, shared_pair_offset, shared_k_blocks, shared_k_blocks_per_split;
+    long long shared_split_stride;
+    void* shared_out;
 };
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -89,10 +94,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // tokens each, adding the runs' sums in index order over distributed shared memory.  A pair cannot be left as partial sums, and
 // without runs a narrow matrix fills a part of the device only: 5,120 + 5,120 rows of 2,048 at one token are 80 blocks,
 // 16.5 us; as 240 blocks 11.7 us.
-template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool GROUPED = false, bool JOINED = false>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const std::conditional_t<GROUPED, GroupedParams, GemmParams> p) {
+template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool GROUPED, bool JOINED>
+__device__ __forceinline__ void
+gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap* shared_a, const CUtensorMap* shared_b,
+              const std::conditional_t<GROUPED, GroupedParams, GemmParams>& p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full_bar[MAX_STAGES];
     __shared__ uint64_t empty_bar[MAX_STAGES];
@@ -108,13 +113,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int group = 0, bx = blockIdx.x;                          // this block's matrix, its m tile there
     if constexpr (GROUPED) {
-        group = bx / p.group_tiles;
-        bx -= group * p.group_tiles;
+        group = bx < p.groups_end ? bx / p.group_tiles : -1;       // (-1: the shared matrix)
+        bx -= group < 0 ? p.groups_end : group * p.group_tiles;
         // (the step's description is the host's or step_prepare's: it may be read before griddepcontrol.wait)
-        if (threadIdx.x < 8) uses[threadIdx.x] = 0;
+        if (threadIdx.x < 8) uses[threadIdx.x] = group < 0 ? ~0u : 0u;
         __syncthreads();
-        bool mine = false;
-        for (int i = threadIdx.x; i < p.n_tokens * p.top; i += NUM_THREADS) {
+        bool mine = group < 0;
+        for (int i = threadIdx.x; i < (group < 0 ? 0 : p.n_tokens * p.top); i += NUM_THREADS) {
             const int t = i / p.top;
             if (p.table[(long long)p.tokens[t] * p.top + (i - t * p.top)] == group) {
                 mine = true;
@@ -151,9 +156,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         m0 = x * tile_m;
         n0 = y * p.bn;
-        kb_begin = z * p.k_blocks_per_split;
-        n_kb = min(p.k_blocks, kb_begin + p.k_blocks_per_split) - kb_begin;
+        if constexpr (GROUPED) {
+            const int per = group < 0 ? p.shared_k_blocks_per_split : p.k_blocks_per_split;
+            kb_begin = z * per;
+            n_kb = min(group < 0 ? p.shared_k_blocks : p.k_blocks, kb_begin + per) - kb_begin;
+        } else {
+            kb_begin = z * p.k_blocks_per_split;
+            n_kb = min(p.k_blocks, kb_begin + p.k_blocks_per_split) - kb_begin;
+        }
     };
+    // this block's operands and result
+    const CUtensorMap *ma = &map_a, *mb = &map_b;
+    int k_blocks = p.k_blocks, pair_offset = p.pair_offset, a_rows = p.a_rows;
+    long long ldo = p.ldo;
+    if constexpr (GROUPED) {
+        if (group < 0) {
+            ma = shared_a;
+            mb = shared_b;
+            k_blocks = p.shared_k_blocks;
+            pair_offset = p.shared_pair_offset;
+            ldo = a_rows = p.shared_rows;
+        }
+    }
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -186,29 +210,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 int m0, n0, kb_begin, n_kb, z;
                 tile_coords(w, m0, n0, kb_begin, n_kb, z);
                 if constexpr (GROUPED) {                     // (from here on rows of the operands, not of the result)
-                    m0 += group * p.group_rows;
-                    n0 += group * p.group_b_rows;
+                    m0 += max(group, 0) * p.group_rows;
+                    n0 += max(group, 0) * p.group_b_rows;
                 }
                 // Coordinates of the box that holds rows row.. of k-block kb: in a row-major
                 // operand (kb * 64, row); in a packed one the tile (row / 128, kb) lies as
                 // 128 contiguous lines of 128 bytes.
                 auto load = [&](const CUtensorMap* map, int packed, int s, void* dst, int kb, int row) {
-                    if (packed) tma_load_2d(map, &full_bar[s], dst, 0, ((row >> 7) * p.k_blocks + kb) * 128 + (row & 127));
+                    if (packed) tma_load_2d(map, &full_bar[s], dst, 0, ((row >> 7) * k_blocks + kb) * 128 + (row & 127));
                     else tma_load_2d(map, &full_bar[s], dst, kb * BK, row);
                 };
                 auto load_a = [&](int i, int s) {
                     uint8_t* st = tiles + (size_t)s * stage_bytes;
                     const int kb = kb_begin + i;
-                    load(&map_a, p.a_packed, s, st, kb, m0);
-                    if (a_tiles == 2) load(&map_a, p.a_packed, s, st + a_bytes, kb, m0 + p.pair_offset);
-                    if (GATED == 3) load(&map_a, p.a_packed, s, st + a_bytes / 2, kb, m0 + p.pair_offset);   // 64-row boxes
+                    load(ma, p.a_packed, s, st, kb, m0);
+                    if (a_tiles == 2) load(ma, p.a_packed, s, st + a_bytes, kb, m0 + pair_offset);
+                    if (GATED == 3) load(ma, p.a_packed, s, st + a_bytes / 2, kb, m0 + pair_offset);   // 64-row boxes
                 };
                 auto load_b = [&](int i, int s) {
                     uint8_t* sb = tiles + (size_t)s * stage_bytes + a_tiles * a_bytes;
                     const int kb = kb_begin + i;
-                    load(&map_b, p.b_packed, s, sb, kb, n0);
-                    if (p.b_packed && p.bn > 128) load(&map_b, p.b_packed, s, sb + 128 * BK * 2, kb, n0 + 128);   // 256 rows: two tiles
-                    if (b_tiles == 2) load(&map_b, p.b_packed, s, sb + b_bytes, kb, n0 + p.pair_offset);
+                    load(mb, p.b_packed, s, sb, kb, n0);
+                    if (p.b_packed && p.bn > 128) load(mb, p.b_packed, s, sb + 128 * BK * 2, kb, n0 + 128);   // 256 rows: two tiles
+                    if (b_tiles == 2) load(mb, p.b_packed, s, sb + b_bytes, kb, n0 + pair_offset);
                 };
                 int i = 0;
                 if (it == 0) {
@@ -292,7 +316,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int m = m0 + q * 32 + lane;
             const uint32_t lane_addr = tmem_base + buf * acc_cols + ((uint32_t)(q * 32) << 16);
             char* out_base = (char*)p.out + (size_t)z * p.split_stride * (OUT_F32 ? 4 : 2);
-            if constexpr (GROUPED) out_base += (size_t)group * p.group_out * (OUT_F32 ? 4 : 2);
+            if constexpr (GROUPED) {
+                if (group >= 0) out_base += (size_t)group * p.group_out * (OUT_F32 ? 4 : 2);
+                else out_base = (char*)p.shared_out + (size_t)z * p.shared_split_stride * (OUT_F32 ? 4 : 2);
+            }
             // One answer for the four epilogue warps, so that they leave the loop together.
             const bool ok_warp = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1, &abort_flag, p.status, 3));
             bool ok = ok_warp;
@@ -328,7 +355,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                     for (int j = 0; j < 8; ++j) xb[xrow][upper ? j : 8 + j] = upper ? v[j] : v[8 + j];
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (ok && n_kb > 0 && mg < p.a_rows) {
+                    if (ok && n_kb > 0 && mg < a_rows) {
 #pragma unroll
                         for (int jj = 0; jj < 8; ++jj) {
                             const int j = upper ? 8 + jj : jj;
@@ -339,7 +366,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                 const float mine = upper ? v[8 + jj] : v[jj], other = xb[xrow][j];
                                 const float g = upper ? other : mine, u = upper ? mine : other;
                                 const float r = g / (1.0f + expf(-g)) * u;
-                                const long long off = (long long)n * p.ldo + mg;
+                                const long long off = (long long)n * ldo + mg;
                                 if (OUT_F32) ((float*)out_base)[off] = r;
                                 else ((__nv_bfloat16*)out_base)[off] = __float2bfloat16_rn(r);
                             }
@@ -357,10 +384,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                         for (int j = 0; j < 16; ++j) v[j] = v[j] / (1.0f + expf(-v[j])) * u[j];
                     }
-                    if (m < p.a_rows) {
+                    if (m < a_rows) {
                         if (!TRANSPOSED) {
                             const int n_left = p.b_rows - (n0 + c0);
-                            const long long off = (long long)m * p.ldo + n0 + c0;
+                            const long long off = (long long)m * ldo + n0 + c0;
                             if (OUT_F32) {
                                 float* o = (float*)out_base + off;
                                 if (n_left >= 16 && (off & 3) == 0) {
@@ -389,7 +416,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                 bool wanted = n < p.b_rows;
                                 if constexpr (GROUPED) wanted = wanted && (uses[n >> 5] >> (n & 31) & 1u);
                                 if (wanted) {
-                                    const long long off = (long long)n * p.ldo + m;
+                                    const long long off = (long long)n * ldo + m;
                                     if (OUT_F32) ((float*)out_base)[off] = v[j];
                                     else ((__nv_bfloat16*)out_base)[off] = __float2bfloat16_rn(v[j]);
                                 }
@@ -451,6 +478,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
 }
 
+template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool JOINED = false>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+    gemm_tc_block<PERSIST, GATED, TRANSPOSED, OUT_F32, false, JOINED>(map_a, map_b, nullptr, nullptr, p);
+}
+
+template <int GATED, bool OUT_F32>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                       const __grid_constant__ CUtensorMap shared_a, const __grid_constant__ CUtensorMap shared_b, const GroupedParams p) {
+    gemm_tc_block<false, GATED, true, OUT_F32, true, false>(map_a, map_b, &shared_a, &shared_b, p);
+}
+
 // ---- host side ---------------------------------------------------------------
 // A [rows, k] bfloat16 matrix, row-major, as a TMA descriptor with boxes of box_rows x 64.
 static int make_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t k, int box_rows) {
@@ -478,13 +518,18 @@ struct Groups {
     int n, rows, b_rows, top, n_tokens;            // n: 0 where A is one matrix
     long long out;
     const int *tokens, *table;
+    // the shared matrix (null: none): packed, with k_shared inner numbers; its rows of B; its result
+    const void *shared_a, *shared_b;
+    long long shared_a_rows, shared_b_rows;
+    int shared_rows, shared_k, shared_pair_offset;
+    void* shared_out;
 };
 
 // The blocks along z are a cluster.
 static int launch_joined(dim3 grid, int smem, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, cudaStream_t s) {
     static bool raised = false;
     if (!raised) {
-        WICK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false, 3, true, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+        WICK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false, 3, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
         raised = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -500,7 +545,7 @@ static int launch_joined(dim3 grid, int smem, const CUtensorMap& map_a, const CU
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    WICK_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false, 3, true, false, false, true>, map_a, map_b, p));
+    WICK_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false, 3, true, false, true>, map_a, map_b, p));
     return check_launch("gemm_tc_joined");
 }
 
@@ -555,18 +600,32 @@ static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const
         static_cast<GemmParams&>(g) = p;
         g.group_tiles = p.grid_m; g.group_rows = G.rows; g.group_b_rows = G.b_rows; g.group_out = G.out;
         g.top = G.top; g.n_tokens = G.n_tokens; g.tokens = G.tokens; g.table = G.table;
+        g.groups_end = p.grid_m * G.n;
+        CUtensorMap shared_a = map_a, shared_b = map_b;
+        g.shared_tiles = 0;
+        if (G.shared_a) {
+            g.shared_k_blocks = ceil_div(G.shared_k, BK);
+            g.shared_k_blocks_per_split = ceil_div(g.shared_k_blocks, splits);
+            WICK_REQUIRE(G.shared_rows > 0 && G.shared_out && G.shared_a_rows % 128 == 0 && G.shared_b_rows >= G.n_tokens &&
+                         (long long)(splits - 1) * g.shared_k_blocks_per_split < g.shared_k_blocks, "gemm_tc: bad shared matrix");
+            g.shared_tiles = ceil_div(G.shared_rows, gated == 3 ? BM / 2 : BM);
+            g.shared_rows = G.shared_rows; g.shared_pair_offset = G.shared_pair_offset; g.shared_out = G.shared_out;
+            g.shared_split_stride = (long long)G.n_tokens * G.shared_rows;
+            if (int e = make_map(&shared_a, G.shared_a, G.shared_a_rows * g.shared_k_blocks, 64, gated == 3 ? BM / 2 : BM)) return e;
+            if (int e = make_map(&shared_b, G.shared_b, G.shared_b_rows, G.shared_k, bn)) return e;
+        }
         WICK_REQUIRE(a_packed && transposed && (gated == 0 || gated == 3) && (out_f32 != 0) == (gated == 0) && !joined, "gemm_tc: grouped products are built for packed matrices, transposed results");
         WICK_REQUIRE((long long)G.n * G.rows <= a_total_rows && G.rows % 128 == 0 && G.n_tokens == b_rows && b_rows <= 256 && G.top > 0, "gemm_tc: bad groups");
         WICK_REQUIRE(total * G.n < (1ll << 30) && splits <= 65535 && p.grid_n <= 65535, "gemm_tc: too many tiles");
-        const dim3 grid(p.grid_m * G.n, p.grid_n, splits);
+        const dim3 grid(g.groups_end + g.shared_tiles, p.grid_n, splits);
         static bool raised = false;
         if (!raised) {
-            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false, 3, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
-            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false, 0, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_grouped_kernel<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_grouped_kernel<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
             raised = true;
         }
-        if (gated) WICK_CUDA(launch(gemm_tc_kernel<false, 3, true, false, true>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, g));
-        else WICK_CUDA(launch(gemm_tc_kernel<false, 0, true, true, true>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, g));
+        if (gated) WICK_CUDA(launch(gemm_tc_grouped_kernel<3, false>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, shared_a, shared_b, g));
+        else WICK_CUDA(launch(gemm_tc_grouped_kernel<0, true>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, shared_a, shared_b, g));
         return check_launch("gemm_tc_grouped");
     }
     // persistent blocks: as many as can be resident at once (one or two per SM by shared memory)
@@ -617,13 +676,18 @@ WICK_API int wick_gemm_tc(const void* a, long long a_total_rows, int a_rows, con
 // of group_rows padded rows one after the other; a gated pair (silu(g) * u, bfloat16 out) or plain (float32 out).  Matrix e's
 // results lie at out + e * n_tokens * a_rows, token by token; only those of tokens whose id names e are written.  splits: runs of the
 // inner dimension, left as partial sums n_groups * n_tokens * a_rows apart (not for gated pairs).
+// shared_a (or null): a packed matrix (of a pair, the second half shared_pair_offset rows on) that every token uses, times the n_tokens rows
+// of shared_b, in the same launch; result as for one group, at shared_out.
 // per_group_b: matrix e is multiplied with rows e * n_tokens .. of b, otherwise all of them with the first n_tokens rows.
 WICK_API int wick_gemm_tc_grouped(const void* a, int n_groups, int group_rows, int a_rows, const void* b, long long b_total_rows,
                                   int per_group_b, int n_tokens, int k, int bn, int gated, int pair_offset, void* out,
-                                  const int* tokens, const int* table, int top, int splits, int max_smem_bytes, int* status, void* stream) {
+                                  const int* tokens, const int* table, int top, int splits, const void* shared_a, long long shared_a_rows,
+                                  const void* shared_b, int shared_rows, int shared_k, int shared_pair_offset, void* shared_out,
+                                  int max_smem_bytes, int* status, void* stream) {
     WICK_REQUIRE(n_groups > 0 && tokens && table, "gemm_tc: bad groups");
     WICK_REQUIRE(bn >= n_tokens, "gemm_tc: a grouped product takes its tokens in one tile");
-    const Groups G = {n_groups, group_rows, per_group_b ? n_tokens : 0, top, n_tokens, (long long)n_tokens * a_rows, tokens, table};
+    const Groups G = {n_groups, group_rows, per_group_b ? n_tokens : 0, top, n_tokens, (long long)n_tokens * a_rows, tokens, table,
+                      shared_a, shared_b, shared_a_rows, n_tokens, shared_rows, shared_k, shared_pair_offset, shared_out};
     return gemm_tc_host(a, (long long)n_groups * group_rows, a_rows, b, b_total_rows, n_tokens, k, bn, gated ? 3 : 0, pair_offset, 1, gated ? 0 : 1,
                         1, 0, 1, 0, out, a_rows, splits, gated ? 0 : (long long)n_groups * n_tokens * a_rows, max_smem_bytes, status, G, stream);
 }

@@ -22,7 +22,7 @@ cannot be fetched by TMA) have no plan; the caller then uses the CUDA-core kerne
 """
 from __future__ import annotations
 
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 
@@ -151,13 +151,15 @@ def gemm_tc_pair(a: torch.Tensor, b: torch.Tensor, b_rows: int, *, out: torch.Te
 
 
 def gemm_tc_experts(a: torch.Tensor, n_experts: int, rows: int, b: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, *,
-                    gated: bool, per_expert_b: bool, k: int, splits: int = 1) -> torch.Tensor:
+                    gated: bool, per_expert_b: bool, k: int, splits: int = 1,
+                    shared: Optional[Tuple["Plan", torch.Tensor]] = None):
     """Few tokens times the matrices of the experts that ``table`` (int32 [vocab, top]) names for their ids ``tokens`` (int32 [n]):
     ``a`` holds the experts' packed matrices (:func:`pack`) of ``rows`` outputs one after the other.  b: [n, k], or with
     ``per_expert_b`` [n_experts * n, k] (an expert's rows by token).  ``splits`` (plain matrices):
     runs of the inner dimension.  Returns bfloat16
     [n_experts, n, rows], silu(g) * u, for gated pairs, otherwise float32 partial sums [splits, n_experts, n, rows]; only the
-    places of tokens whose id names the expert hold numbers."""
+    places of tokens whose id names the expert hold numbers.  ``shared`` = (the plan of a matrix that every token uses, its rows
+    [n, its k]): multiplied in the same launch; returns (as above, bfloat16 [n, its outputs] or float32 [splits, n, its outputs])."""
     for nm, t in (("a", a), ("b", b)):
         if not (t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()):
             raise KernelError(f"gemm_tc_experts: {nm} must be a contiguous bfloat16 CUDA tensor")
@@ -171,13 +173,21 @@ def gemm_tc_experts(a: torch.Tensor, n_experts: int, rows: int, b: torch.Tensor,
     group_rows = a.shape[0] // n_experts * 128
     out = torch.empty((n_experts, n, rows) if gated else (splits, n_experts, n, rows),
                       dtype=torch.bfloat16 if gated else torch.float32, device=b.device)
+    plan = beside = None
+    if shared is not None:
+        plan, x = shared
+        if not (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and tuple(x.shape) == (n, plan.k) and plan.gated == gated):
+            raise KernelError("gemm_tc_experts: the shared matrix and its rows do not go together")
+        beside = torch.empty((n, plan.n_out) if gated else (splits, n, plan.n_out), dtype=out.dtype, device=b.device)
     if n == 0:
-        return out
+        return out if shared is None else (out, beside)
     st = status_tensor(a.device)
-    _lib().call("wick_gemm_tc_grouped", "piiipliiiiiipppiiipp", _p(a), n_experts, group_rows, rows, _p(b), b.shape[0], 1 if per_expert_b else 0,
+    _lib().call("wick_gemm_tc_grouped", "piiipliiiiiipppiiplpiiipipp", _p(a), n_experts, group_rows, rows, _p(b), b.shape[0], 1 if per_expert_b else 0,
                 n, k, _ceil16(n), 1 if gated else 0, (rows + 127) // 128 * 128, _p(out), _p(tokens), _p(table), table.shape[1],
-                splits, (100 if n <= 128 else 200) * 1024, _p(st), _stream())
-    return out
+                splits, _p(plan.w) if plan else None, plan.w.shape[0] * 128 if plan else 0, _p(shared[1]) if plan else None,
+                plan.n_out if plan else 0, plan.k if plan else 0, plan.pair_offset if plan else 0, _p(beside),
+                (100 if n <= 128 else 200) * 1024, _p(st), _stream())
+    return out if shared is None else (out, beside)
 
 
 FEW_MAX = 128               # tokens of gemm_tc_experts at most

@@ -35,6 +35,7 @@ import torch
 from .. import ops
 from .base import FeedForward, TensorSpec, build_part, register_part
 from .linear import Linear
+from .standard import GatedMLP
 
 
 class NoFeedForward(FeedForward):
@@ -180,38 +181,58 @@ class TableMoE(FeedForward):
         return n + (self.shared.weight_bytes() if self.shared is not None else 0)
 
     def forward(self, x, batch):
-        base = None
-        if self.shared is not None:
-            base = self.shared.forward(x, batch)
-            if base.dim() == 2:
-                base = base.unsqueeze(0)
         n = x.shape[0]
-        if self.up_tiles is not None and n > self.FEW_MAX:
-            return self._forward_sorted(x, batch, base)
+        if self.up_tiles is not None and n <= self.FEW_MAX:
+            return self._forward_few(x, batch)
+        base = self._forward_shared(x, batch)
         if self.up_tiles is not None:
-            return self._forward_few(x, batch, base)
+            return self._forward_sorted(x, batch, base)
         hidden = ops.moe_table_up(x, batch.tokens, self.table, self.gate_up)
         return ops.moe_table_down(hidden, batch.tokens, self.table, self.down, 1.0 / self.top, base).unsqueeze(0)
+
+    def _forward_shared(self, x, batch):
+        """float32 [splits, n, width] of the expert that every token uses, or None."""
+        if self.shared is None:
+            return None
+        base = self.shared.forward(x, batch)
+        return base.unsqueeze(0) if base.dim() == 2 else base
 
     # Up to this many tokens every expert that the step uses is multiplied with all of them, in the orientation of the dense
     # products of few tokens (the matrices stream through the 128-row side once; what other tokens make of an expert is not
     # written).  The runs of the inner dimension depend on the matrices alone, so that a token's bits do not depend on the step.
     FEW_MAX = 128
 
-    def _few_splits(self, n):
+    def _few_splits(self, n, shared):
         """Runs of the down product's inner dimension: two, where its tiles alone leave SMs without a block, fixed for the sizes of
         decode steps so that a token's bits do not depend on the step.  (Experts of 1,536 x 2,048, 8 tokens: 36.5 us in one run,
         33.7 in two, 38.2 in four; the gated product in two runs is faster up to four tokens only.)"""
         from ..ops import gemm_tc
-        k_blocks = (self.intermediate + 63) // 64
-        return gemm_tc.even_splits(min(2, k_blocks // 4), k_blocks) if n <= gemm_tc.SMALL else 1
+        ks = [(self.intermediate + 63) // 64] + ([shared[1].k_blocks] if shared else [])
+        return min(gemm_tc.even_splits(min(2, k // 4), k) for k in ks) if n <= gemm_tc.SMALL else 1
 
-    def _forward_few(self, x, batch, base):
+    def _shared_plans(self):
+        """The plans of the shared expert's two matrices, where its products can join the experts' (a gated feed-forward on the
+        tensor cores), else None.  Two launches less, and its tiles fill SMs that the experts' leave: with eight experts and a
+        shared one, 2,048 wide, 8 tokens, a layer of 81 us takes 8 us less."""
+        if type(self.shared) is not GatedMLP:
+            return None
+        plans = (self.shared.gate_up._tensor_core(), self.shared.down._tensor_core())
+        return plans if all(plans) else None
+
+    def _forward_few(self, x, batch):
         from ..ops import gemm_tc
         f, w = self.intermediate, self.width
-        hidden = gemm_tc.gemm_tc_experts(self.up_tiles, self.experts, f, x, batch.tokens, self.table, gated=True, per_expert_b=False, k=w)
-        y = gemm_tc.gemm_tc_experts(self.down_tiles, self.experts, w, hidden.view(-1, f), batch.tokens, self.table, gated=False,
-                                    per_expert_b=True, k=f, splits=self._few_splits(x.shape[0]))
+        plans = self._shared_plans()
+        up = dict(gated=True, per_expert_b=False, k=w)
+        down = dict(gated=False, per_expert_b=True, k=f, splits=self._few_splits(x.shape[0], plans))
+        if plans:
+            hidden, beside = gemm_tc.gemm_tc_experts(self.up_tiles, self.experts, f, x, batch.tokens, self.table, shared=(plans[0], x), **up)
+            y, base = gemm_tc.gemm_tc_experts(self.down_tiles, self.experts, w, hidden.view(-1, f), batch.tokens, self.table,
+                                              shared=(plans[1], beside), **down)
+        else:
+            base = self._forward_shared(x, batch)
+            hidden = gemm_tc.gemm_tc_experts(self.up_tiles, self.experts, f, x, batch.tokens, self.table, **up)
+            y = gemm_tc.gemm_tc_experts(self.down_tiles, self.experts, w, hidden.view(-1, f), batch.tokens, self.table, **down)
         return ops.moe_combine_table(y, batch.tokens, self.table, 1.0 / self.top, base).unsqueeze(0)
 
     # With more tokens a step sorts its rows by expert, every expert's rows starting at a
