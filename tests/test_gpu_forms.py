@@ -219,3 +219,17 @@ def test_projection_finish_in_registers_is_the_general_form(H, G, d, e, rot, n, 
     tol = 1e-5 if dtype == torch.float32 else 2 ** -7              # (the sums of squares run in another order: the last bit of 32, or one of bfloat16)
     for a, b in zip(*got):
         assert (a.double() - b.double()).abs().max() <= tol * max(1.0, float(b.double().abs().max()))
+
+
+@pytest.mark.parametrize("t, k, out, pair", [(4357, 7400, 300, False), (2305, 14000, 513, True), (4096, 7688, 257, False)])
+def test_prompt_products_in_slabs_of_rows_are_those_of_fewer_rows(t, k, out, pair):
+    """More than 60 MB of activations: the tiles come in slabs of rows, every tile computed as it is in a product of fewer rows."""
+    from wick_b200.ops import gemm_tc
+    g = torch.Generator().manual_seed(t)
+    plan = gemm_tc.plan_for((torch.randn(2 * out if pair else out, k, generator=g) / math.sqrt(k)).bfloat16().to(DEV), gated=pair)
+    x = torch.randn(t, k, generator=g).bfloat16().to(DEV)
+    assert x.numel() * 2 > 60 << 20
+    got = plan.forward(x, torch.bfloat16)
+    for a in (0, 1024, t - 700):
+        assert torch.equal(got[a:a + 700], plan.forward(x[a:a + 700].contiguous(), torch.bfloat16))
+    ops.check_status()

@@ -50,6 +50,7 @@ struct Params {
     int pair_offset;               // row offset of the up half inside B
     int out_f32;
     int grid_m, grid_n, total_tiles;
+    int slab_m;                    // tiles of a slab of rows: slabs come one after the other, a slab's tiles column by column
     int splits;                    // runs of the inner dimension (1: whole)
     long long split_stride;        // elements between the outputs of two runs
     long long ldo;
@@ -146,7 +147,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int total_units = p.total_tiles * p.splits;
     auto tile_coords = [&](int w, int& m0, int& n0) {
         const int tile = w % p.total_tiles;
-        const int x = tile % p.grid_m, y = tile / p.grid_m;
+        const int slab = tile / (p.slab_m * p.grid_n), in = tile - slab * p.slab_m * p.grid_n;
+        const int rows = min(p.slab_m, p.grid_m - slab * p.slab_m), y = in / rows;
+        const int x = slab * p.slab_m + in - y * rows;
         m0 = x * 2 * BM;
         n0 = y * (GATED ? BNH : BN);
     };
@@ -371,6 +374,13 @@ WICK_API int wick_gemm_tc2_grouped(const void* a, int a_rows, const void* b, lon
     const long long total = (long long)p.grid_m * p.grid_n;
     WICK_REQUIRE(total < (1ll << 30), "gemm_tc2: too many tiles");
     p.total_tiles = (int)total;
+    // One slab of all rows reads every weight once and all of A for every round of tiles, which is right while A stays in the L2 cache
+    // (126 MB, of which half is left for it): 4,096 x 4,096 in slabs of 8 tiles took 635 us instead of 631.  A larger A came from memory
+    // in every round (66 tiles of rows for 74 pairs: 172 MB of it).  In even slabs of up to 8 tiles a round reads
+    // about 8 + 9 strips of 256 rows: 16,800 tokens, 5,120 inputs, 7,168 outputs 1,245 -> 1,160 us, 5,120 outputs 909 -> 855, of 17,408
+    // inputs 2,691 -> 2,604; slabs of 4 or 16 tiles the same.
+    const int slab_max = (long long)a_rows * k * 2 > (60ll << 20) ? 8 : p.grid_m;
+    p.slab_m = ceil_div(p.grid_m, ceil_div(p.grid_m, slab_max));
     p.splits = splits;
     p.split_stride = split_stride;
     WICK_REQUIRE(total * splits < (1ll << 30), "gemm_tc2: too many units");
