@@ -541,22 +541,29 @@ attn_multi_merge_kernel(const float* __restrict__ partial, TO* __restrict__ out,
         const float sum = warp_sum(mine) + (sink ? expf(sink[h] - big) : 0.f);
 #pragma unroll
         for (int c = 0; c < 4 * CPW; ++c) y[a][c] = 0.f;
-        auto fold = [&](int r, float fr) {
-            const float* rec = recs + (int64_t)r * (4 + e_pad) + 4;
+        // RU runs' values are on their way together (4 tokens, 32 heads, values of 512 numbers: 5.8 us; one run's at a time 8.4)
+        constexpr int RU = CPW == 1 ? 8 : 2;
+        for (int r0 = 0; r0 < runs; r0 += RU) {
+            float fr[RU];
+            float4 v[RU][CPW];
 #pragma unroll
-            for (int c = 0; c < CPW; ++c)
-                if (128 * (c0 + c) < e_pad) {
-                    const float4 v = *reinterpret_cast<const float4*>(rec + 128 * (c0 + c) + 4 * lane);
-                    y[a][4 * c] = fmaf(v.x, fr, y[a][4 * c]);
-                    y[a][4 * c + 1] = fmaf(v.y, fr, y[a][4 * c + 1]);
-                    y[a][4 * c + 2] = fmaf(v.z, fr, y[a][4 * c + 2]);
-                    y[a][4 * c + 3] = fmaf(v.w, fr, y[a][4 * c + 3]);
-                }
-        };
-#pragma unroll 4
-        for (int r = 0; r < runs; ++r) {
-            const float fr = __shfl_sync(ALL, r < 32 ? f[0] : f[1], r & 31);
-            if (fr != 0.f) fold(r, fr);               // (a run without a key left no values)
+            for (int k = 0; k < RU; ++k) {
+                const int r = r0 + k;
+                fr[k] = __shfl_sync(ALL, r < 32 ? f[0] : f[1], r & 31);       // (a run without a key, or beyond the last: 0, it left no values)
+#pragma unroll
+                for (int c = 0; c < CPW; ++c)
+                    if (fr[k] != 0.f && 128 * (c0 + c) < e_pad) v[k][c] = ld4(recs + (int64_t)r * (4 + e_pad) + 4 + 128 * (c0 + c) + 4 * lane);
+            }
+#pragma unroll
+            for (int k = 0; k < RU; ++k)
+#pragma unroll
+                for (int c = 0; c < CPW; ++c)
+                    if (fr[k] != 0.f && 128 * (c0 + c) < e_pad) {
+                        y[a][4 * c] = fmaf(v[k][c].x, fr[k], y[a][4 * c]);
+                        y[a][4 * c + 1] = fmaf(v[k][c].y, fr[k], y[a][4 * c + 1]);
+                        y[a][4 * c + 2] = fmaf(v[k][c].z, fr[k], y[a][4 * c + 2]);
+                        y[a][4 * c + 3] = fmaf(v[k][c].w, fr[k], y[a][4 * c + 3]);
+                    }
         }
         float inv = 1.0f / sum;
         if (gate) inv *= gate[th];
