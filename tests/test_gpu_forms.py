@@ -233,3 +233,17 @@ def test_prompt_products_in_slabs_of_rows_are_those_of_fewer_rows(t, k, out, pai
     for a in (0, 1024, t - 700):
         assert torch.equal(got[a:a + 700], plan.forward(x[a:a + 700].contiguous(), torch.bfloat16))
     ops.check_status()
+
+
+@pytest.mark.parametrize("ff", [8192, 8196, 16384, 16388])
+@pytest.mark.parametrize("n", [1, 148, 149])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_poly_norm_forms(ff, n, splits):
+    g = torch.Generator().manual_seed(ff + n)
+    parts = (0.7 * torch.randn(splits, n, ff, generator=g)).to(DEV)
+    z = parts.double().sum(0)
+    co = torch.tensor([0.5, -1.2, 0.8, 0.3], device=DEV)
+    ref = sum(c * z ** (i + 1) / torch.sqrt((z ** (2 * i + 2)).mean(1, keepdim=True) + 1e-5) for i, c in enumerate(co.tolist()[:3])) + 0.3
+    got = ops.poly_norm(parts, co, 1e-5, torch.float32)
+    assert (got.double() - ref).abs().max() < 5e-6 * float(ref.abs().max())
+    assert torch.equal(ops.poly_norm(parts, co, 1e-5, torch.bfloat16), got.bfloat16())
