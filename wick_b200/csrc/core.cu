@@ -149,11 +149,12 @@ __global__ void __launch_bounds__(1024, 1) rmsnorm_kernel(float* __restrict__ x,
 
 // The same for rows of whole groups of four that fit a block's registers (VPT groups a thread): the weights are fetched before the
 // kernel before this one has finished, the row's and all partial sums' loads go out together, and the row stays in registers.  A
-// decode step waits for two of these a layer and they move next to nothing: what counts is the chain of trips to memory.  (Eight
-// rows of 4,096 numbers, eight partial sums: 4.1 us against 4.3 with the row in shared memory and the loads in a loop; five
-// rows of 5,120, seven partial sums: 6.6 us against 8.3.)  The same bits as the other forms.
+// decode step waits for two of these a layer and they move next to nothing: what counts is the chain of trips to memory.  (In a chain of
+// norms, eight rows of 4,096 numbers, eight partial sums: 3.1 us against 3.3 with the row in shared memory and the loads in a loop; of
+// 5,120: 3.5 against 4.2.  64 registers where a thread has one group, so that an SM holds two rows of 2,048: 300 of them 3.4 us against
+// 3.9, with 80 registers and one row an SM a prompt of a few hundred tokens took 5 % longer.)  The same bits as the other forms.
 template <typename TOut, int VPT>
-__global__ void __launch_bounds__(VPT == 1 ? 512 : 768, 1)
+__global__ void __launch_bounds__(VPT == 1 ? 1024 : 768, 1)
 rmsnorm_regs_kernel(float* __restrict__ x, const float* __restrict__ delta, int splits, int64_t split_stride, const float* __restrict__ w,
                     float eps, const int* __restrict__ rows, TOut* __restrict__ out, int width) {
     extern __shared__ float smem[];                     // [width / 4] sums of four neighbouring squares
