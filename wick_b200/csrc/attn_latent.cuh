@@ -15,7 +15,7 @@
 //
 // What bounds it: with few tokens the chain of a block's start, one or two tiles and its record; with many the tensor cores.  The form
 // for other sizes (a key row per warp on the CUDA cores, four heads a block) reads rows and queries from shared memory once per four
-// heads.  32 heads, rows of 576 numbers, values of 512, merge included, before -> now: 4 tokens of 700 to 1,500 positions 60 -> 24 us,
+// heads.  32 heads, rows of 576 numbers, values of 512, merge included, before -> now: 4 tokens of 700 to 1,500 positions 60 -> 22 us,
 // 8 of 1,500 147 -> 25, 64 of 1,000 615 -> 71; prompts of 60 + 100 + 40 tokens 166 -> 29, of 2 x 200 688 -> 69.  Error against 64 bits
 // 0.6 to 1.5e-7 of the result's norm (before 1.3 to 2.1e-7).
 #pragma once
