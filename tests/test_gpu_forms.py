@@ -54,6 +54,20 @@ def test_float32_products_of_every_form_give_the_same_bits(n, k, pair):
         assert torch.equal(ops.gemm_simt(x[:m].contiguous(), w, torch.float32, gated=pair, w_static=m % 2 == 0), got[:m]), m
 
 
+@pytest.mark.parametrize("m", [1, 32, 33, 300])
+def test_float32_products_read_a_matrix_that_the_kernel_before_wrote(m):
+    """Without ``w_static`` the second operand may be the result of the kernel launched just before, which need not have finished
+    when the product's blocks start: nothing of it may be read early."""
+    x, src = torch.randn(m, 2048).to(DEV), torch.randn(2048, 2048).to(DEV)
+    delta, one = torch.randn(8, 2048, 2048).to(DEV), torch.ones(2048, device=DEV)
+    for _ in range(5):
+        w = torch.full((2048, 2048), float("nan"), device=DEV)        # (what an early load would find)
+        ops.rmsnorm(src.clone(), one, 1e-5, torch.float32, delta=delta, out=w)
+        got = ops.gemm_simt(x, w, torch.float32)
+        torch.cuda.synchronize()
+        assert torch.equal(got, ops.gemm_simt(x, w, torch.float32))
+
+
 def test_float32_products_of_misaligned_rows_take_the_general_form():
     x, w = torch.randn(5 * 64 + 1).to(DEV)[1:].view(5, 64), torch.randn(24, 64).to(DEV)
     assert x.data_ptr() % 16 != 0

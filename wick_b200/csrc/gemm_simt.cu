@@ -181,6 +181,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     pdl_trigger();
     pdl_wait();
     A = fresh(A);
+    W = fresh(W);                                        // (an earlier kernel may have made it: this form does not ask w_static)
     const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * NB;
     const float* arow[LA];
