@@ -203,6 +203,21 @@ def test_scaled_sum_and_norm_forms(width, n, splits):
     assert torch.equal(out, xd.bfloat16())
 
 
+@pytest.mark.parametrize("width", [4, 132, 2048, 2052, 4096, 4100, 8192])
+@pytest.mark.parametrize("splits", [0, 1, 3, 9])
+def test_a_row_of_the_scaled_sum_and_norm_does_not_depend_on_the_number_of_rows(width, splits):
+    """The block's size follows the number of rows (64 and 65), the order of a row's sum of squares does not."""
+    g = torch.Generator().manual_seed(width + splits)
+    x, w = torch.randn(300, width, generator=g).to(DEV), (1 + 0.1 * torch.randn(width, generator=g)).to(DEV)
+    delta = torch.randn(splits, 300, width, generator=g).to(DEV) if splits else None
+    many = x.clone()
+    ops.scaled_add_rmsnorm(many, delta, 1.7, w, 1e-5, torch.float32)
+    for n in (1, 3, 64, 65):
+        few = x[:n].clone()
+        ops.scaled_add_rmsnorm(few, delta[:, :n].contiguous() if splits else None, 1.7, w, 1e-5, torch.float32)
+        assert torch.equal(few, many[:n]), n
+
+
 @pytest.mark.parametrize("H, G, d, e, rot, n, splits", [(4, 2, 16, 24, 8, 3, 1), (32, 8, 128, 128, 128, 70, 1), (32, 8, 128, 128, 64, 8, 8),
                                                         (10, 2, 20, 4, 20, 66, 3), (48, 8, 128, 64, 0, 65, 2), (1, 1, 4, 4, 4, 1, 9)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -163,6 +163,53 @@ __device__ __forceinline__ void block_sums(float (&v)[K], float* scratch) {
     for (int k = 0; k < K; ++k) v[k] = warp_sum(lane < nw ? scratch[k * 32 + lane] : 0.f);
 }
 
+// The sums over the warp of N numbers a lane (N a power of two): lane l gets that of v[l N / 32].  Each is what warp_sum gives, bit for
+// bit (the same pairs at the same distances), with N - 1 + 5 - log2(N) exchanges instead of 5 N.
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = N / 2; n >= 1; n /= 2, o /= 2) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float keep = upper ? v[i + n] : v[i], give = upper ? v[i] : v[i + n];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    float r = v[0];
+#pragma unroll
+    for (; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
+}
+
+// K sums over a row of groups, thread t of the block holding the groups t, t + blockDim, ...: v[k][u] is what group u blockDim + t adds
+// to sum k (0 beyond the row's end).  ONE order for every size of block, so that the size may follow the number of rows and a row's bits do
+// not: 32 neighbouring groups by the butterfly; those sums, 32 apart, in index order; the last 32 by the butterfly.  Every thread
+// gets the sums.  scratch: 32 K N floats of shared memory that nobody has read or written since the block's last barrier (or since
+// the kernel began).
+template <int K, int N>
+__device__ __forceinline__ void row_sums(float (&v)[K][N], float (&sums)[K], float* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const float s = warp_sums(v[k]);
+        if (lane % (32 / N) == 0) scratch[k * 32 * N + lane * N / 32 * nw + warp] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        float p = 0.f;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int c = 32 * i + lane;
+            if (c < N * nw) p += scratch[k * 32 * N + c];
+        }
+        sums[k] = warp_sum(p);
+    }
+}
+
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 // Positions per cache page.  The Python side carries the same number (wick_b200/layout.py);

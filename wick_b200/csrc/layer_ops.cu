@@ -59,7 +59,8 @@ __device__ __forceinline__ void row_partials(float4 (&v)[VPT], const float* __re
 // One block per row; the row waits in shared memory between the two passes.  First pass:
 // v = alpha x + the partial sums (index order) and the sum of its squares (a thread's elements in
 // index order, then the block's sum in thread order); second pass: y = v * scale * w to x and out.
-// The block's size depends on the width alone, so a row's bits do not depend on the batch.
+// The block's size depends on the width alone, so a row's bits do not depend on the batch.  (Rows that are no whole groups of four, longer
+// than 8,192 numbers or misaligned.)
 template <typename TOut>
 __global__ void __launch_bounds__(1024)
 scaled_add_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta, int splits, int64_t split_stride,
@@ -101,21 +102,26 @@ scaled_add_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta
     }
 }
 
-// The same for rows of whole groups of four: a thread keeps VPT groups of the row in registers, the loads of all of them on their
-// way together, and everything is written once.  (3,300 rows of 4,096 numbers, one partial sum: 32 us, with the row in shared
-// memory and element-wise stores 68; eight rows of 2,048, eight partial sums: 2.9 us against 4.3.)
+// The same for rows of whole groups of four up to 8,192 numbers: a thread keeps VPT groups of the row in registers, the loads of all of
+// them on their way together, and everything is written once.  Bound by the trips to memory in steps of few rows, by memory in long ones.
+// One group a thread, four partial sums' loads together, is the faster form for few rows, four groups and one partial sum at a time (several
+// blocks an SM, which hide each other's sums) for many; with 256 threads of two groups, or 1,024 of two groups for the longer rows, eight
+// partial sums and many rows took longer than the form above.  us, the form above -> here: 8 rows of 2,048, eight partial sums 3.5 -> 2.8;
+// 65 of them 3.7 -> 3.1; 8 rows of 4,096 3.9 -> 3.3; 1,000 rows of 5,120, four partial sums 37 -> 26; 4,000 rows of 4,096, one partial
+// sum 85 -> 37.  The order of the sum of squares is row_sums' and every product that is added to something is rounded or fused as written,
+// so a row's bits depend neither on VPT nor on the block's size.
 template <typename TOut, int VPT>
-__global__ void __launch_bounds__(VPT <= 2 ? 1024 : 256)
+__global__ void __launch_bounds__(VPT == 1 ? 1024 : 512)
 scaled_add_rmsnorm_regs_kernel(float* __restrict__ x, const float* __restrict__ delta, int splits, int64_t split_stride,
                                float alpha, const float* __restrict__ w, float eps, TOut* __restrict__ out, int width) {
-    constexpr int SU = VPT == 1 ? 8 : (VPT == 2 ? 4 : 1);             // partial sums whose loads go out together
-    __shared__ float red[32];
+    constexpr int SU = VPT == 1 ? 4 : 1;                // partial sums whose loads go out together
+    __shared__ float red[32 * VPT];
     pdl_trigger();
-    float4 g[VPT];                                      // (weights: fetched before the kernel before this one has finished)
+    float4 g[VPT];                                      // (weights: in steps of few rows fetched before the kernel before this one has finished)
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
         const int j = (u * (int)blockDim.x + (int)threadIdx.x) * 4;
-        if (VPT <= 2) g[u] = j < width ? ld4(w + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (VPT == 1) g[u] = j < width ? ld4(w + j) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     pdl_wait();
     x = fresh(x);
@@ -128,7 +134,7 @@ scaled_add_rmsnorm_regs_kernel(float* __restrict__ x, const float* __restrict__ 
     for (int u = 0; u < VPT; ++u) {
         const int j = (u * (int)blockDim.x + (int)threadIdx.x) * 4;
         v[u] = j < width ? ld4(xr + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        v[u].x *= alpha; v[u].y *= alpha; v[u].z *= alpha; v[u].w *= alpha;
+        v[u] = make_float4(__fmul_rn(v[u].x, alpha), __fmul_rn(v[u].y, alpha), __fmul_rn(v[u].z, alpha), __fmul_rn(v[u].w, alpha));
     }
     for (int s0 = 0; s0 < splits; s0 += SU) {
         float4 d[SU][VPT];
@@ -146,17 +152,17 @@ scaled_add_rmsnorm_regs_kernel(float* __restrict__ x, const float* __restrict__ 
                 v[u].x += d[k][u].x; v[u].y += d[k][u].y; v[u].z += d[k][u].z; v[u].w += d[k][u].w;
             }
     }
-    float ss[1] = {0.f};
+    float sq[1][VPT], ss[1];
 #pragma unroll
     for (int u = 0; u < VPT; ++u)
-        ss[0] = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, fmaf(v[u].w, v[u].w, ss[0]))));
-    block_sums(ss, red);
+        sq[0][u] = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, __fmul_rn(v[u].w, v[u].w))));
+    row_sums(sq, ss, red);
     const float scale = 1.0f / sqrtf(ss[0] / (float)width + eps);
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
         const int j = (u * (int)blockDim.x + (int)threadIdx.x) * 4;
         if (j >= width) continue;
-        if (VPT > 2) g[u] = ld4(w + j);
+        if (VPT > 1) g[u] = ld4(w + j);
         const float4 y = make_float4((v[u].x * scale) * g[u].x, (v[u].y * scale) * g[u].y, (v[u].z * scale) * g[u].z, (v[u].w * scale) * g[u].w);
         st4(xr + j, y.x, y.y, y.z, y.w);
         if (out) st4(out + r * width + j, y.x, y.y, y.z, y.w);
@@ -671,16 +677,14 @@ int scaled_add_rmsnorm(float* x, const float* delta, int splits, float alpha, co
                        int width, cudaStream_t s) {
     WICK_REQUIRE(width > 0 && n >= 0 && splits >= 0, "scaled_add_rmsnorm: bad sizes");
     if (n == 0) return 0;
-    // Rows of whole groups of four numbers: in registers.  Many rows: blocks of 256 threads with up to four groups each (several blocks an SM
-    // hide each other's sums); few rows, or long ones: up to 1,024 threads.  (The block's size decides the order of a row's sum of squares: it
-    // changes with n beyond the sizes of decode steps only.)
+    // Rows of whole groups of four numbers: in registers.  Up to 512 threads' worth of groups for every SM's two blocks, a thread a group;
+    // more, or longer rows: four groups a thread.
     if (width % 4 == 0 && width <= 8192 && (((uintptr_t)x | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
-        const int groups = width / 4, most = n > 64 && groups <= 1024 ? 256 : (groups <= 1024 ? 512 : 1024);
-        const int threads = min(most, (groups + 31) / 32 * 32), vpt = ceil_div(groups, threads);
+        const int groups = width / 4, vpt = groups <= 1024 && (int64_t)n * groups <= (int64_t)2 * sm_count() * 512 ? 1 : 4;
+        const int threads = (ceil_div(groups, vpt) + 31) / 32 * 32;
 #define WICK_SARMS(V) WICK_CUDA(launch(scaled_add_rmsnorm_regs_kernel<TOut, V>, dim3(n), dim3(threads), 0, s, x, delta, splits, (int64_t)n * width, alpha, \
                                        w, eps, (TOut*)out, width))
         if (vpt == 1) WICK_SARMS(1);
-        else if (vpt == 2) WICK_SARMS(2);
         else WICK_SARMS(4);
 #undef WICK_SARMS
         return check_launch("scaled_add_rmsnorm");
