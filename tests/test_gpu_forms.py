@@ -250,6 +250,31 @@ def test_projection_finish_in_registers_is_the_general_form(H, G, d, e, rot, n, 
         assert (a.double() - b.double()).abs().max() <= tol * max(1.0, float(b.double().abs().max()))
 
 
+@pytest.mark.parametrize("H, G, d, e, rot, splits", [(4, 2, 16, 24, 8, 1), (16, 4, 128, 128, 128, 8), (32, 8, 128, 128, 64, 3), (48, 8, 128, 128, 128, 2), (1, 1, 4, 4, 4, 9)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_row_of_the_projections_finish_does_not_depend_on_the_number_of_rows(H, G, d, e, rot, splits, dtype):
+    """The block's size follows the number of rows (64 and 65), a row's bits do not."""
+    g = torch.Generator().manual_seed(H * d)
+    W, start = (H + G) * d + G * e, 37
+    parts, keep0 = torch.randn(splits, 200, W, generator=g).to(DEV), torch.randn(200, G * e, generator=g).to(DEV)
+    bias, qw, kw = ((s + 0.1 * torch.randn(m, generator=g)).to(DEV) for s, m in ((0.0, W), (1.0, H * d), (1.0, G * d)))
+    inv = torch.tensor([100.0 ** (-2.0 * i / rot) for i in range(rot // 2)]).to(DEV)
+    got = {}
+    for n in (200, 65, 64, 3, 1):
+        batch, pages, n_pages = batch_of([n], [start])
+        cos, sin = ops.rope_table(batch.positions, inv)
+        kv = torch.zeros((n_pages, G * PAGE * (d + e)), dtype=dtype, device=DEV)
+        q = ops.qkv_finish(parts[:, :n].contiguous(), H, G, d, e, dtype=dtype, bias=bias, q_weight=qw, k_weight=kw, eps=1e-5, cos=cos, sin=sin,
+                           rot_dims=rot, v_keep=keep0[:n].contiguous(), v_mode=2, blend=torch.tensor([0.3], device=DEV), kv=kv,
+                           page_table=batch.page_table, seq_of_token=batch.seq_of_token, positions=batch.positions)
+        k = kv[:, :G * PAGE * d].view(n_pages, G, PAGE, d)
+        v = kv[:, G * PAGE * d:].view(n_pages, G, PAGE, e)
+        at = [(pages[0][p // PAGE], p % PAGE) for p in range(start, start + n)]
+        got[n] = (q, torch.stack([k[a, :, r] for a, r in at]), torch.stack([v[a, :, r] for a, r in at]))
+        for one, many in zip(got[n], got[200]):
+            assert torch.equal(one, many[:n]), n
+
+
 @pytest.mark.parametrize("t, k, out, pair", [(4357, 7400, 300, False), (2305, 14000, 513, True), (4096, 7688, 257, False)])
 def test_prompt_products_in_slabs_of_rows_are_those_of_fewer_rows(t, k, out, pair):
     """More than 60 MB of activations: the tiles come in slabs of rows, every tile computed as it is in a product of fewer rows."""

@@ -331,7 +331,9 @@ qkv_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_str
 // projection and rotations of neighbouring pairs, rows of whole groups of four: a thread keeps VPT groups of four of the row in
 // registers, the loads of all of them on their way together, and writes each once, eight or sixteen bytes at a time.  (3,300 rows of
 // 6,144 numbers: 56 us where the form above takes 136, which writes element by element and divides to find each one's
-// place; eight rows of 3,072, eight partial sums: 5.5 us against 15.)
+// place; eight rows of 3,072, eight partial sums: 3.6 us against 9.4.)  A row's bits depend neither on VPT nor on the block's size: a sum of
+// squares is that of 256 threads, thread t adding groups t, t + 256, ... in index order (larger blocks leave the groups' sums in shared
+// memory for the first 256), and every product that is added to something is rounded or fused as written.
 template <typename T, int VPT>
 __global__ void __launch_bounds__(VPT <= 2 ? 1024 : 256)
 qkv_finish_regs_kernel(const float* __restrict__ parts, int splits, int64_t split_stride, const float* __restrict__ bias,
@@ -343,6 +345,7 @@ qkv_finish_regs_kernel(const float* __restrict__ parts, int splits, int64_t spli
     constexpr int SU = VPT == 1 ? 8 : (VPT == 2 ? 4 : 1);             // partial sums whose loads go out together
     constexpr bool AHEAD = VPT <= 2;                    // few tokens: weights and the step's description before the kernel before this one has finished
     __shared__ float red[2 * 32];
+    __shared__ float quads[AHEAD ? 1024 * VPT : 1];
     pdl_trigger();
     const int t = blockIdx.x;
     const int Wq = H * d, Wk = G * d, Wv = G * e, W = Wq + Wk + Wv;
@@ -392,9 +395,24 @@ qkv_finish_regs_kernel(const float* __restrict__ parts, int splits, int64_t spli
             const float4 b = AHEAD ? b4[u] : ld4(bias + j);
             v[u].x += b.x; v[u].y += b.y; v[u].z += b.z; v[u].w += b.w;
         }
-        const float sq = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, v[u].w * v[u].w)));
-        if (j < Wq) ss[0] += sq;
+        const float sq = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, __fmul_rn(v[u].w, v[u].w))));
+        if (AHEAD && blockDim.x > 256) quads[j >> 2] = sq;
+        else if (j < Wq) ss[0] += sq;
         else if (j < Wq + Wk) ss[1] += sq;
+    }
+    if (AHEAD && blockDim.x > 256) {
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            float sq[4 * VPT];
+#pragma unroll
+            for (int i = 0; i < 4 * VPT; ++i) sq[i] = quads[256 * i + threadIdx.x];     // (what lies behind the row is not used)
+#pragma unroll
+            for (int i = 0; i < 4 * VPT; ++i) {
+                const int j = 4 * (256 * i + (int)threadIdx.x);
+                if (j < Wq) ss[0] += sq[i];
+                else if (j < Wq + Wk) ss[1] += sq[i];
+            }
+        }
     }
     if (q_span > 0 || k_span > 0) block_sums(ss, red);
     const float fq = q_span > 0 ? 1.0f / sqrtf(ss[0] / (float)Wq + eps) : 1.f, fk = k_span > 0 ? 1.0f / sqrtf(ss[1] / (float)Wk + eps) : 1.f;
@@ -409,8 +427,9 @@ qkv_finish_regs_kernel(const float* __restrict__ parts, int splits, int64_t spli
             if (v_mode == 1) st4(keep, y.x, y.y, y.z, y.w);
             if (v_mode == 2) {
                 const float4 k = ld4(keep);
-                y = make_float4((1.0f - lam) * y.x + lam * k.x, (1.0f - lam) * y.y + lam * k.y, (1.0f - lam) * y.z + lam * k.z,
-                                (1.0f - lam) * y.w + lam * k.w);
+                const float own = 1.0f - lam;
+                y = make_float4(fmaf(own, y.x, __fmul_rn(lam, k.x)), fmaf(own, y.y, __fmul_rn(lam, k.y)), fmaf(own, y.z, __fmul_rn(lam, k.z)),
+                                fmaf(own, y.w, __fmul_rn(lam, k.w)));
             }
             if (write_kv) st4(page + (int64_t)G * kPage * d + ((int64_t)g * kPage + r) * e + x, y.x, y.y, y.z, y.w);
             continue;
@@ -428,7 +447,8 @@ qkv_finish_regs_kernel(const float* __restrict__ parts, int splits, int64_t spli
         }
         if (x < 2 * half) {
             const float2 c = ld2(cos_t + (int64_t)t * half + (x >> 1)), s = ld2(sin_t + (int64_t)t * half + (x >> 1));
-            y = make_float4(y.x * c.x - y.y * s.x, y.y * c.x + y.x * s.x, y.z * c.y - y.w * s.y, y.w * c.y + y.z * s.y);
+            y = make_float4(fmaf(y.x, c.x, -__fmul_rn(y.y, s.x)), fmaf(y.y, c.x, __fmul_rn(y.x, s.x)), fmaf(y.z, c.y, -__fmul_rn(y.w, s.y)),
+                            fmaf(y.w, c.y, __fmul_rn(y.z, s.y)));
         }
         if (is_q) st4(q_out + (int64_t)t * Wq + j, y.x, y.y, y.z, y.w);
         else if (write_kv) st4(page + ((int64_t)h * kPage + r) * d + x, y.x, y.y, y.z, y.w);
@@ -850,7 +870,7 @@ int qkv_finish(const float* parts, int splits, int n, const float* bias, int H, 
     WICK_REQUIRE(!X.pool || (write_kv && X.block > 0 && X.rows == (kPage + X.block - 1) / X.block && X.pool_page == (int64_t)G * X.rows * (d + e)),
                  "qkv_finish: bad blocks");
     if (n == 0) return 0;
-    // (the extras and the other norms and rotations: the form below; a block's size changes with n beyond the sizes of decode steps only)
+    // (the extras and the other norms and rotations: the form below)
     const int W = Wq + Wk + G * e;
     if (!X.conv_w && !X.v_norm && !X.pool && X.gate_heads == 0 && flags == 0 && maps == 1 && (q_span == 0 || q_span == Wq) &&
         (k_span == 0 || k_span == Wk) && (!cos_t || rot_dims == 0 || (pairing == 0 && rot_dims % 4 == 0)) && d % 4 == 0 && e % 4 == 0 && cols % 4 == 0 &&
