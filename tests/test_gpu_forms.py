@@ -275,6 +275,33 @@ def test_a_row_of_the_projections_finish_does_not_depend_on_the_number_of_rows(H
             assert torch.equal(one, many[:n]), n
 
 
+@pytest.mark.parametrize("qr, r, dr, gates", [(24, 40, 8, 3), (96, 300, 64, 0), (1536, 512, 64, 0), (512, 256, 32, 5), (3840, 512, 64, 0), (23, 41, 8, 2)])
+@pytest.mark.parametrize("splits", [1, 3, 8, 12])
+def test_a_latents_finish_does_not_depend_on_the_number_of_rows(qr, r, dr, gates, splits):
+    """Few rows take larger blocks and their partial sums' loads together; a row's bits are the same.  The last sizes cannot be read four
+    numbers at a time."""
+    g = torch.Generator().manual_seed(qr)
+    W, start, n_all = qr + r + dr + gates, 50, 200
+    parts = torch.randn(splits, n_all, W + (-W % 4 if qr % 4 == 0 else 0), generator=g).to(DEV)
+    wq, wkv = torch.randn(qr, generator=g).to(DEV), torch.randn(r, generator=g).to(DEV)
+    s = parts.double().sum(0)
+    unit = lambda x: x / torch.sqrt((x * x).mean(1, keepdim=True) + 1e-5)  # noqa: E731
+    got = {}
+    for n in (n_all, 65, 64, 1):
+        batch, pages, n_pages = batch_of([n], [start])
+        cos, sin = ops.rope_table(batch.positions, torch.tensor([100.0 ** (-2.0 * i / dr) for i in range(dr // 2)]).to(DEV))
+        rows = torch.zeros(n_pages, PAGE, r + dr, device=DEV)
+        cq, gate = ops.latent_finish(parts[:, :n].contiguous(), qr, r, dr, gates, dtype=torch.float32, q_weight=wq, kv_weight=wkv, eps=1e-5, cos=cos,
+                                     sin=sin, rows=rows, page_table=batch.page_table, seq_of_token=batch.seq_of_token, positions=batch.positions)
+        own = torch.stack([rows[pages[0][p // PAGE], p % PAGE] for p in range(start, start + n)])
+        got[n] = [cq, own] + ([gate] if gates else [])
+        for one, many in zip(got[n], got[n_all]):
+            assert torch.equal(one, many[:n]), n
+    # (a float32 sum of a few numbers of order one, a norm and a product: a few 2^-24 of the largest, below 3e-6 of it)
+    for a, ref in ((got[n_all][0], unit(s[:, :qr]) * wq.double()), (got[n_all][1][:, :r], unit(s[:, qr:qr + r]) * wkv.double())):
+        assert (a.double() - ref).abs().max() < 3e-6 * float(ref.abs().max())
+
+
 @pytest.mark.parametrize("t, k, out, pair", [(4357, 7400, 300, False), (2305, 14000, 513, True), (4096, 7688, 257, False)])
 def test_prompt_products_in_slabs_of_rows_are_those_of_fewer_rows(t, k, out, pair):
     """More than 60 MB of activations: the tiles come in slabs of rows, every tile computed as it is in a product of fewer rows."""

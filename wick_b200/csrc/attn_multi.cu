@@ -582,8 +582,8 @@ attn_multi_merge_kernel(const float* __restrict__ partial, TO* __restrict__ out,
 }
 
 // Four neighbours' partial sums, added in index order; up to eight sums' loads go out together: a step of few tokens waits for
-// each trip to memory (4 tokens, 32 heads, latents of 1,536 and 512 numbers: the row's finish 8.4 us before, 7.3 now, the queries
-// through the key matrix 8.4 and 8.2, the latents through the value matrix 8.1 and 7.3).
+// each trip to memory (4 tokens, 32 heads, latents of 1,536 and 512 numbers: the queries through the key matrix 8.4 -> 8.2 us, the
+// latents through the value matrix 8.1 -> 7.3).
 __device__ __forceinline__ float4 sum_parts4(const float* __restrict__ p, int splits, int64_t split_stride) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int s0 = 0; s0 < splits; s0 += 8) {
@@ -605,8 +605,13 @@ __device__ __forceinline__ float4 sum_parts4(const float* __restrict__ p, int sp
 // cache ([page][64][r + dr]), and sigmoid(gate) goes out in float32.  A row of the sums has `cols` numbers; what lies
 // behind the gates of the heads is somebody else's.
 //   pairing 0: (2i, 2i + 1) turn together; 1: (i, i + dr / 2).
-template <typename T>
-__global__ void __launch_bounds__(1024)
+// TOGETHER (few tokens, four partial sums and more, rows of more than a group of four numbers for each of 256 threads): up to 1,024 threads
+// whose partial sums' loads go out together; the squares are added by the first 256 threads in the order of the other form, so that a
+// row's bits do not depend on the form.  (Row of 2,112 numbers, us, one row after the other / together: 8 tokens, 3, 4 and 8 partial sums
+// 3.8 / 3.9, 4.3 / 3.9, 5.4 / 4.0; 148 tokens, 4 and 8 4.6 / 4.1, 5.8 / 4.3; 300 tokens 5.1 / 6.7, 6.9 / 7.7.  Together for every number of
+// partial sums and tokens, as it was, one or two of them took 1.2 to 1.8 times as long in prompts: 2,000 tokens 18.6 against 10.5.)
+template <typename T, bool TOGETHER>
+__global__ void __launch_bounds__(TOGETHER ? 1024 : 256)
 latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_stride, int cols, int qr, int r, int dr, int Hg,
                      const float* __restrict__ q_w, const float* __restrict__ kv_w, float eps,
                      const float* __restrict__ cos_t, const float* __restrict__ sin_t, int pairing, T* __restrict__ cq_out,
@@ -624,13 +629,27 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
     const int W = qr + r + dr + Hg;
     const float* mine = parts + (int64_t)t * cols;
     float ss[2] = {0.f, 0.f};                       // of the query latent, of the latent
-    if (((qr | r | cols) & 3) == 0 && (reinterpret_cast<size_t>(parts) & 15) == 0) {
+    auto squares = [&](int j, float4 v) {           // of the group at j, to the sum it belongs to
+        const float sq = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, __fmul_rn(v.w, v.w))));
+        if (j < qr) ss[0] += sq;
+        else if (j < qr + r) ss[1] += sq;
+    };
+    if (TOGETHER) {
+        for (int j = tid * 4; j < W; j += blockDim.x * 4)                  // (the last group may reach behind W: the row has cols numbers)
+            *reinterpret_cast<float4*>(row + j) = sum_parts4(mine + j, splits, split_stride);
+        __syncthreads();
+        if (tid < 256)
+            for (int j = tid * 4; j < qr + r; j += 1024) squares(j, *reinterpret_cast<const float4*>(row + j));
+    } else if (((qr | r | cols) & 3) == 0 && (reinterpret_cast<size_t>(parts) & 15) == 0) {
+#pragma unroll 2
         for (int j = tid * 4; j < W; j += blockDim.x * 4) {
-            const float4 v = sum_parts4(mine + j, splits, split_stride);   // (the last group may reach behind W: the row has cols numbers)
+            float4 v = ld4(mine + j);               // (the last group may reach behind W: the row has cols numbers)
+            for (int s = 1; s < splits; ++s) {
+                const float4 d = ld4(mine + s * split_stride + j);
+                v.x += d.x; v.y += d.y; v.z += d.z; v.w += d.w;
+            }
             *reinterpret_cast<float4*>(row + j) = v;
-            const float sq = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
-            if (j < qr) ss[0] += sq;
-            else if (j < qr + r) ss[1] += sq;
+            squares(j, v);
         }
     } else {
         for (int j = tid; j < W; j += blockDim.x) {
@@ -641,7 +660,7 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
             else if (j < qr + r) ss[1] = fmaf(v, v, ss[1]);
         }
     }
-    block_sums(ss, red);                            // (its barrier also makes the row whole)
+    block_sums(ss, red);                            // (its barrier also makes the row whole; TOGETHER's further warps add zeros)
     const float fq = 1.0f / sqrtf(ss[0] / (float)qr + eps);
     if ((qr & 3) == 0) {
         for (int j = tid * 4; j < qr; j += blockDim.x * 4)
@@ -1190,11 +1209,14 @@ int latent_finish(const float* parts, int splits, int n, int cols, int qr, int r
     const size_t smem = (size_t)((W + 3) & ~3) * sizeof(float);
     WICK_REQUIRE(W <= cols, "latent_finish: rows of %d numbers, %d expected", cols, W);
     WICK_REQUIRE(smem <= 48 * 1024, "latent_finish: a row of %d numbers is beyond one block's shared memory", W);
-    // (few tokens: a thread per group of four, so that a row is one trip to memory)
-    const int threads = n <= 64 ? min(1024, max(256, (W / 4 + 31) / 32 * 32)) : 256;
-    WICK_CUDA(launch(latent_finish_kernel<T>, dim3(n), dim3(threads), smem, s, parts, splits, (int64_t)n * cols, cols, qr, r, dr, Hg, q_w, kv_w, eps,
-                     cos_t, sin_t, pairing, (T*)cq_out, gate_out, (T*)rows, (T*)flat_c, (T*)flat_kr, page_table, table_width, seq_of_token,
-                     positions));
+    const bool together = n <= sm_count() && splits > 3 && W > 1024 && ((qr | r | cols) & 3) == 0 && ((uintptr_t)parts & 15) == 0;
+    const int threads = together ? min(1024, (W / 4 + 31) / 32 * 32) : 256;
+#define WICK_LATENT_FINISH(F) WICK_CUDA(launch(latent_finish_kernel<T, F>, dim3(n), dim3(threads), smem, s, parts, splits, (int64_t)n * cols, cols, qr, r, \
+                                               dr, Hg, q_w, kv_w, eps, cos_t, sin_t, pairing, (T*)cq_out, gate_out, (T*)rows, (T*)flat_c, (T*)flat_kr,     \
+                                               page_table, table_width, seq_of_token, positions))
+    if (together) WICK_LATENT_FINISH(true);
+    else WICK_LATENT_FINISH(false);
+#undef WICK_LATENT_FINISH
     return check_launch("latent_finish");
 }
 
