@@ -302,6 +302,16 @@ def test_a_latents_finish_does_not_depend_on_the_number_of_rows(qr, r, dr, gates
         assert (a.double() - ref).abs().max() < 3e-6 * float(ref.abs().max())
 
 
+@pytest.mark.parametrize("ff", [8196, 15360, 16384])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_a_long_row_of_poly_norm_does_not_depend_on_the_number_of_rows(ff, splits):
+    parts = (0.7 * torch.randn(splits, 300, ff, generator=torch.Generator().manual_seed(ff))).to(DEV)
+    co = torch.tensor([0.5, -1.2, 0.8, 0.3], device=DEV)
+    many = ops.poly_norm(parts, co, 1e-5, torch.float32)
+    for n in (1, 148, 149, 296, 297):
+        assert torch.equal(ops.poly_norm(parts[:, :n].contiguous(), co, 1e-5, torch.float32), many[:n]), n
+
+
 @pytest.mark.parametrize("t, k, out, pair", [(4357, 7400, 300, False), (2305, 14000, 513, True), (4096, 7688, 257, False)])
 def test_prompt_products_in_slabs_of_rows_are_those_of_fewer_rows(t, k, out, pair):
     """More than 60 MB of activations: the tiles come in slabs of rows, every tile computed as it is in a product of fewer rows."""
