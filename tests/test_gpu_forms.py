@@ -188,6 +188,19 @@ def test_norm_forms_give_the_same_bits(width, splits):
             assert (few_x.double() - (x[:9].double() + delta[:, :9].double().sum(0))).abs().max() < 1e-5
 
 
+@pytest.mark.parametrize("width", [4096, 4100, 5120])
+def test_norms_of_long_rows_among_many_give_the_same_bits(width):
+    """Up to two partial sums of long rows take a warp a row from 512 rows on, more a block a row."""
+    g = torch.Generator().manual_seed(width)
+    w = (1 + 0.1 * torch.randn(width, generator=g)).to(DEV)
+    for splits in (1, 2, 3, 8):
+        x, delta = torch.randn(513, width, generator=g).to(DEV), torch.randn(splits, 513, width, generator=g).to(DEV)
+        many_x, few_x = x.clone(), x[:511].clone()
+        many = ops.rmsnorm(many_x, w, 1e-5, torch.float32, delta=delta)
+        few = ops.rmsnorm(few_x, w, 1e-5, torch.float32, delta=delta[:, :511].contiguous())
+        assert torch.equal(few, many[:511]) and torch.equal(few_x, many_x[:511])
+
+
 @pytest.mark.parametrize("width", [4, 260, 2048, 4096, 4100, 8192, 8196])
 @pytest.mark.parametrize("n", [3, 65])
 @pytest.mark.parametrize("splits", [0, 1, 3, 9])

@@ -581,10 +581,13 @@ int rmsnorm(float* x, const float* delta, int splits, int64_t n_rows_x, const fl
         raised = true;
     }
     const int threads = width >= 4096 ? 1024 : (width >= 2048 ? 512 : (width >= 512 ? 256 : 128));
-    if (n_out >= 512 && width % 4 == 0 && width <= 5120) {
+    if (n_out >= 512 && width % 4 == 0 && (width <= 4096 || (width <= 5120 && splits <= 2))) {
         // Enough rows to give every SM its warps: a warp per row (same bits as the block per row).
         // (17,600 rows of 5,120 numbers: 81 to 99 us, a block per row 405: its threads all wait for the first warp to add up the
-        // classes, and a block of 1,024 threads is all that an SM holds.)
+        // classes, and a block of 1,024 threads is all that an SM holds.  Beyond 4,096 numbers a warp holds so much of a row that it
+        // does not pay for more than two partial sums: 5,120 numbers, us a warp / a block with the row in registers, two partial sums
+        // 512 rows 12.6 / 12.6, 1,000 18.8 / 24.1; four 20.4 / 16.2, 27.4 / 28.0; eight 31.9 / 22.6, 42.4 / 39.3.  Beyond 5,120 its
+        // registers would: 40 groups of four a lane are 160 of them.)
         // With fewer rows (a decode step of 64 sequences) a warp per row leaves most of the part
         // idle and each warp walks its row's partial sums alone: the block per row is 3x faster there.
         const dim3 grid(ceil_div(n_out, 4)), block(128);
