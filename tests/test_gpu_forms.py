@@ -325,6 +325,41 @@ def test_a_long_row_of_poly_norm_does_not_depend_on_the_number_of_rows(ff, split
         assert torch.equal(ops.poly_norm(parts[:, :n].contiguous(), co, 1e-5, torch.float32), many[:n]), n
 
 
+@pytest.mark.parametrize("hd", [16, 48, 64, 128])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H, G", [(4, 4), (10, 2), (12, 4), (34, 2)])
+def test_short_form_of_the_decode_attention_among_few_and_many(hd, dtype, H, G):
+    """Few blocks have a warp per page and head, many a warp per page for four heads: the same bits."""
+    g = torch.Generator().manual_seed(hd + H)
+    lens = [1, 63, 64, 65, 300, 777, 1025] + [130] * 60
+    store, n_pages = torch.randn(160, 2, G, PAGE, hd, generator=g).to(dtype).to(DEV), 160
+    q = torch.randn(len(lens), H, hd, generator=g).to(dtype).to(DEV)
+
+    def run(which):
+        pages, at = [], 1
+        for i, n in enumerate(lens):
+            k = (n + PAGE - 1) // PAGE
+            pages.append([1 + (at + j) % (n_pages - 1) for j in range(k)])
+            at += k
+        ls = [lens[i] for i in which]
+        layout = BatchLayout(len(ls), len(ls), max(len(pages[i]) for i in which), len(ls))
+        host = np.zeros(layout.size, dtype=np.int32)
+        fill_host(layout, host, tokens=[[0]] * len(ls), starts=[n - 1 for n in ls], slots=[1 + i for i in range(len(ls))],
+                  pages=[pages[i] for i in which], want=[[0]] * len(ls))
+        batch = StepBatch(layout, torch.from_numpy(host).to(DEV), q_lens=[1] * len(ls), starts=[n - 1 for n in ls])
+        scratch = torch.empty(ops.attention_decode_scratch_floats(len(ls), H, hd, max(ls), dtype), device=DEV)
+        return ops.attention_decode(q[which].contiguous(), store, batch, hd ** -0.5, scratch), pages
+    many, pages = run(list(range(len(lens))))
+    for i in range(8):
+        assert torch.equal(run([i])[0][0], many[i]), lens[i]
+        k, v = (torch.cat([store[p, a] for p in pages[i]], 1)[:, :lens[i]].double() for a in (0, 1))
+        z = torch.softmax(torch.einsum("ghd,gkd->ghk", q[i].double().view(G, H // G, hd), k) * hd ** -0.5, -1)
+        ref = (z @ v).reshape(H, hd)
+        # (float32 sums of at most 1,025 terms: below 1e-5; the result's own rounding to bfloat16 2^-9)
+        assert (many[i].double() - ref).abs().max() < (1e-5 if dtype == torch.float32 else 2 ** -8) * max(1.0, float(ref.abs().max()))
+    ops.check_status()
+
+
 @pytest.mark.parametrize("t, k, out, pair", [(4357, 7400, 300, False), (2305, 14000, 513, True), (4096, 7688, 257, False)])
 def test_prompt_products_in_slabs_of_rows_are_those_of_fewer_rows(t, k, out, pair):
     """More than 60 MB of activations: the tiles come in slabs of rows, every tile computed as it is in a product of fewer rows."""

@@ -1,11 +1,15 @@
 // Decode attention (one new token per sequence) over the paged cache, fast form.
 //
-// grid = (splits, kv_heads, sequences).  A block of W * 4 warps handles W pages
-// (64 positions each) of one sequence and kv head, for all query heads of that
-// kv head, four at a time: a warp takes one page for one head.  (With one warp for a
-// page's four heads a block of the 32-bit path was a single warp that walked 64 KB of
-// shared memory alone: 4 sequences of 100 positions, 4 kv heads of 128, 14.6 us, now
-// 6.2 us; bfloat16, 8 sequences of 500, 4 kv heads, 13.4 us, now 11.9 us.)
+// grid = (splits, kv_heads, sequences).  A block handles W pages (64 positions each) of one
+// sequence and kv head, for all query heads of that kv head, four at a time: a warp takes one
+// page for one head, or for all four.  With one warp for a page's four heads a block of one
+// or two pages was one or two warps that walked 64 KB of shared memory alone (4 sequences of 100
+// positions, 4 kv heads of 128, float32 14.6 us, now 6.2; bfloat16, 8 sequences of 500, 13.4 us,
+// now 11.9).  A block of four pages (heads of up to 64 numbers in bfloat16, 32 in float32) has
+// four warps anyway: there a warp per head is better only while few blocks run, since a
+// page is read from shared memory once per warp (64 sequences of 3,000 positions, 8 kv heads
+// of 32, bfloat16, 32 heads: 122 us, a warp for four heads 70; heads of 64, 16 sequences of 250: 8.3 us and 9.9).
+// Both give the same bits.
 // One thread starts bulk copies (cp.async.bulk, completion on an mbarrier) of the pages'
 // key and value tiles — each tile is one contiguous [64][head_dim] block of the cache —
 // so that everything the block needs is in flight at once; scores, softmax statistics
@@ -42,7 +46,6 @@ template <typename T> struct Shape {
     static constexpr int W_RAW = 65536 / (2 * TILE_BYTES);
     static constexpr int WARPS = W_RAW >= 4 ? 4 : (W_RAW >= 2 ? 2 : 1);
     static constexpr int SPLIT = WARPS * kPage;
-    static constexpr int THREADS = WARPS * GT * 32;                     // WARPS pages, GT heads each
     static constexpr int pow2ceil(int v) { int p = 1; while (p < v) p <<= 1; return p; }
     static constexpr int TS = CHUNKS >= 32 ? 32 : pow2ceil(CHUNKS);   // lanes that share a key in the value pass
     static constexpr int CPL = (CHUNKS + TS - 1) / TS;
@@ -51,14 +54,15 @@ template <typename T> struct Shape {
     static constexpr size_t SMEM = (size_t)2 * WARPS * TILE_BYTES + (size_t)(GT * HD + GT * SPLIT + WARPS * GT * HD) * sizeof(float);
 };
 
-template <typename T>
-__global__ void __launch_bounds__(Shape<T>::THREADS)
+// HPW: heads that a warp takes of its page.
+template <typename T, int HPW>
+__global__ void __launch_bounds__(Shape<T>::WARPS * (GT / HPW) * 32)
 attn_decode_fast_kernel(const T* __restrict__ q, const T* __restrict__ kv, float* __restrict__ part_o,
                         float* __restrict__ part_ml, const int* __restrict__ kv_len_arr,
                         const int* __restrict__ page_table, int table_width, int n_heads, int n_kv, int max_splits,
                         float scale, int* status, int mask, int mask_size) {
     using S = Shape<T>;
-    constexpr int EPC = S::EPC, CHUNKS = S::CHUNKS, WARPS = S::WARPS, SPLIT = S::SPLIT, THREADS = S::THREADS;
+    constexpr int EPC = S::EPC, CHUNKS = S::CHUNKS, WARPS = S::WARPS, SPLIT = S::SPLIT, PER_PAGE = GT / HPW, THREADS = WARPS * PER_PAGE * 32;
     constexpr int TS = S::TS, CPL = S::CPL, KPI = S::KPI;
     pdl_trigger();
     pdl_wait();
@@ -108,15 +112,15 @@ attn_decode_fast_kernel(const T* __restrict__ q, const T* __restrict__ kv, float
             bulk_load(v_s + (size_t)i * kPage * HD, kp + (int64_t)n_kv * kPage * HD, S::TILE_BYTES, &bar);
         }
     }
-    const int w = warp / GT, hh = warp % GT;                     // this warp's page and head
-    const bool warp_live = w < n_pages;
+    const int w = warp / PER_PAGE, hh = warp % PER_PAGE * HPW;   // this warp's page and (first) head
     const T* kw = k_s + (size_t)w * kPage * HD;
     const T* vw = v_s + (size_t)w * kPage * HD;
-    float* mine = sc + hh * SPLIT + w * kPage;                   // the warp's weights
+    float* mine = sc + hh * SPLIT + w * kPage;                   // the warp's weights (its next head's SPLIT on)
     bool waited = false;
 
     for (int h0 = 0; h0 < group; h0 += GT) {
         const int nh = min(GT, group - h0);
+        const bool warp_live = w < n_pages && hh < nh;
         __syncthreads();
         for (int i = tid; i < GT * HD; i += THREADS) {
             const int h = i / HD, d = i % HD;
@@ -131,55 +135,70 @@ attn_decode_fast_kernel(const T* __restrict__ q, const T* __restrict__ kv, float
         }
 
         // ---- scores: lane = key (two keys per lane), chunks of the row in turn ----
-        float s0 = 0.f, s1 = 0.f;
+        float s0[HPW], s1[HPW];
+#pragma unroll
+        for (int h = 0; h < HPW; ++h) s0[h] = s1[h] = 0.f;
         if (warp_live) {
-#pragma unroll 4
+#pragma unroll (HPW == 1 ? 4 : 2)
             for (int c = 0; c < CHUNKS; ++c) {
                 const int cc = S::SWZ ? (c ^ (lane & 7)) : c;
                 Vec16<T> k0, k1;
                 k0.load(kw + (size_t)lane * HD + cc * EPC);
                 k1.load(kw + (size_t)(lane + 32) * HD + cc * EPC);
-                const float* qh = q_s + hh * HD + cc * EPC;
 #pragma unroll
-                for (int e = 0; e < EPC; e += 4) {
-                    const float4 q4 = *reinterpret_cast<const float4*>(qh + e);
-                    s0 = fmaf(q4.x, k0.v[e], s0); s0 = fmaf(q4.y, k0.v[e + 1], s0); s0 = fmaf(q4.z, k0.v[e + 2], s0); s0 = fmaf(q4.w, k0.v[e + 3], s0);
-                    s1 = fmaf(q4.x, k1.v[e], s1); s1 = fmaf(q4.y, k1.v[e + 1], s1); s1 = fmaf(q4.z, k1.v[e + 2], s1); s1 = fmaf(q4.w, k1.v[e + 3], s1);
+                for (int h = 0; h < HPW; ++h) {
+                    const float* qh = q_s + (hh + h) * HD + cc * EPC;
+#pragma unroll
+                    for (int e = 0; e < EPC; e += 4) {
+                        const float4 q4 = *reinterpret_cast<const float4*>(qh + e);
+                        s0[h] = fmaf(q4.x, k0.v[e], s0[h]); s0[h] = fmaf(q4.y, k0.v[e + 1], s0[h]);
+                        s0[h] = fmaf(q4.z, k0.v[e + 2], s0[h]); s0[h] = fmaf(q4.w, k0.v[e + 3], s0[h]);
+                        s1[h] = fmaf(q4.x, k1.v[e], s1[h]); s1[h] = fmaf(q4.y, k1.v[e + 1], s1[h]);
+                        s1[h] = fmaf(q4.z, k1.v[e + 2], s1[h]); s1[h] = fmaf(q4.w, k1.v[e + 3], s1[h]);
+                    }
                 }
             }
         }
         const int at = key_begin + w * kPage + lane;
-        s0 = warp_live && at < kv_len && at >= key_lo ? s0 * scale : -INFINITY;
-        s1 = warp_live && at + 32 < kv_len && at + 32 >= key_lo ? s1 * scale : -INFINITY;
+        const bool sees0 = warp_live && at < kv_len && at >= key_lo, sees1 = warp_live && at + 32 < kv_len && at + 32 >= key_lo;
 
         // ---- softmax statistics of the split, per head ----
-        float m = warp_max(fmaxf(s0, s1));
-        if (lane == 0) stat[0][hh][w] = m;
-        __syncthreads();
-        m = stat[0][hh][0];
 #pragma unroll
-        for (int i = 1; i < WARPS; ++i) m = fmaxf(m, stat[0][hh][i]);            // (finite: the split holds a visible key)
-        const float p0 = expf(s0 - m), p1 = expf(s1 - m);
-        mine[lane] = p0;
-        mine[lane + 32] = p1;
-        const float l = warp_sum(p0 + p1);
-        if (lane == 0) stat[1][hh][w] = l;
+        for (int h = 0; h < HPW; ++h) {
+            s0[h] = sees0 ? __fmul_rn(s0[h], scale) : -INFINITY;
+            s1[h] = sees1 ? __fmul_rn(s1[h], scale) : -INFINITY;
+            const float m = warp_max(fmaxf(s0[h], s1[h]));
+            if (lane == 0) stat[0][hh + h][w] = m;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < HPW; ++h) {
+            float m = stat[0][hh + h][0];
+#pragma unroll
+            for (int i = 1; i < WARPS; ++i) m = fmaxf(m, stat[0][hh + h][i]);    // (finite: the split holds a visible key)
+            const float p0 = expf(s0[h] - m), p1 = expf(s1[h] - m);
+            mine[h * SPLIT + lane] = p0;
+            mine[h * SPLIT + lane + 32] = p1;
+            const float l = warp_sum(p0 + p1);
+            if (lane == 0) stat[1][hh + h][w] = l;
+        }
         __syncwarp();
 
         // ---- weighted sum of values: TS lanes share a key, each owns 16-byte chunks of the row ----
         const int tl = lane % TS, team = lane / TS;
-        float acc[CPL][EPC];
+        float acc[HPW][CPL][EPC];
 #pragma unroll
-        for (int c = 0; c < CPL; ++c)
+        for (int h = 0; h < HPW; ++h)
 #pragma unroll
-            for (int e = 0; e < EPC; ++e) acc[c][e] = 0.f;
+            for (int c = 0; c < CPL; ++c)
+#pragma unroll
+                for (int e = 0; e < EPC; ++e) acc[h][c][e] = 0.f;
         if (warp_live) {
             const int keys_here = min(kPage, kv_len - key_begin - w * kPage);
-#pragma unroll 8
+#pragma unroll (HPW == 1 ? 8 : 4)
             for (int it = 0; it < kPage / KPI; ++it) {
                 const int key = it * KPI + team;
                 if (key < keys_here) {
-                    const float p = mine[key];
 #pragma unroll
                     for (int c = 0; c < CPL; ++c) {
                         const int chunk = tl + c * TS;
@@ -187,22 +206,28 @@ attn_decode_fast_kernel(const T* __restrict__ q, const T* __restrict__ kv, float
                             Vec16<T> vv;
                             vv.load(vw + (size_t)key * HD + chunk * EPC);
 #pragma unroll
-                            for (int e = 0; e < EPC; ++e) acc[c][e] = fmaf(p, vv.v[e], acc[c][e]);
+                            for (int h = 0; h < HPW; ++h) {
+                                const float p = mine[h * SPLIT + key];
+#pragma unroll
+                                for (int e = 0; e < EPC; ++e) acc[h][c][e] = fmaf(p, vv.v[e], acc[h][c][e]);
+                            }
                         }
                     }
                 }
             }
         }
 #pragma unroll
-        for (int c = 0; c < CPL; ++c)
+        for (int h = 0; h < HPW; ++h)
 #pragma unroll
-            for (int e = 0; e < EPC; ++e) {
-                float v = acc[c][e];
+            for (int c = 0; c < CPL; ++c)
 #pragma unroll
-                for (int o = TS; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                const int chunk = tl + c * TS;
-                if (team == 0 && chunk < CHUNKS) red[(w * GT + hh) * HD + chunk * EPC + e] = v;
-            }
+                for (int e = 0; e < EPC; ++e) {
+                    float v = acc[h][c][e];
+#pragma unroll
+                    for (int o = TS; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    const int chunk = tl + c * TS;
+                    if (team == 0 && chunk < CHUNKS) red[(w * GT + hh + h) * HD + chunk * EPC + e] = v;
+                }
         __syncthreads();
         for (int i = tid; i < nh * HD; i += THREADS) {
             const int h = i / HD, d = i % HD;
@@ -270,14 +295,28 @@ int run(const void* q, const void* kv, void* out, float* scratch, int64_t scratc
     WICK_REQUIRE(scratch_floats >= need, "attention decode: scratch of %lld floats, %lld needed",
                  (long long)scratch_floats, (long long)need);
     float* ml = scratch + (int64_t)n_seqs * n_heads * max_splits * HD;
-    static bool raised = false;
-    if (!raised) {
-        WICK_CUDA(cudaFuncSetAttribute(attn_decode_fast_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
-        raised = true;
+#define WICK_DECODE(HPW)                                                                                                                                  \
+    do {                                                                                                                                                  \
+        static bool raised = false;                                                                                                                       \
+        if (!raised) {                                                                                                                                    \
+            WICK_CUDA(cudaFuncSetAttribute(attn_decode_fast_kernel<T, HPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));                  \
+            raised = true;                                                                                                                                \
+        }                                                                                                                                                 \
+        WICK_CUDA(launch(attn_decode_fast_kernel<T, HPW>, dim3(max_splits, n_kv, n_seqs), dim3(S::WARPS * (GT / HPW) * 32), S::SMEM, s, (const T*)q,        \
+                         (const T*)kv, scratch, ml, kv_len, page_table, table_width, n_heads, n_kv, max_splits, scale, status, mask, mask_size));          \
+    } while (0)
+    // (a warp takes one head up to a block for every SM, or every other one where pages are small, 16 or 32 numbers a head in bfloat16 and
+    // 16 in float32: of 1,225 sizes measured none was slower by more than runs differ than the form before, a warp for four heads and
+    // barriers for every head and sum)
+    bool done = false;
+    if constexpr (S::WARPS == 4) {
+        if ((int64_t)max_splits * n_kv * n_seqs * (S::TILE_BYTES < 8192 ? 2 : 1) > sm_count()) {
+            WICK_DECODE(GT);
+            done = true;
+        }
     }
-    WICK_CUDA(launch(attn_decode_fast_kernel<T>, dim3(max_splits, n_kv, n_seqs), dim3(S::THREADS), S::SMEM, s, (const T*)q,
-                     (const T*)kv, scratch, ml, kv_len, page_table, table_width, n_heads, n_kv, max_splits, scale, status, mask,
-                     mask_size));
+    if (!done) WICK_DECODE(1);
+#undef WICK_DECODE
     if (int e = check_launch("attn_decode")) return e;
     WICK_CUDA(launch(attn_decode_fast_merge_kernel<T>, dim3(n_heads, n_seqs), dim3(HD >= 128 ? 128 : 64), 0, s,
                      (const float*)scratch, (const float*)ml, kv_len, (T*)out, n_heads, max_splits, mask, mask_size, sink));
