@@ -112,6 +112,21 @@ def test_attention_over_rows_on_the_tensor_cores(H, R, r, q_lens, starts, window
             t += 1
 
 
+@pytest.mark.parametrize("H, R, tensor_cores", [(1, 80, False), (1, 192, False), (2, 80, False), (2, 128, True), (3, 80, True)])
+def test_attention_over_rows_of_few_heads_stays_on_the_cuda_cores(H, R, tensor_cores, monkeypatch):
+    batch, pages, n_pages = batch_of([150], [30])
+    store = torch.randn(n_pages, PAGE, R, generator=torch.Generator().manual_seed(H)).bfloat16()
+    q = torch.randn(150, H, R, generator=torch.Generator().manual_seed(9))
+    form, taken = ops._attention_latent, []
+    monkeypatch.setattr(ops, "_attention_latent", lambda *a: taken.append(1) or form(*a))
+    out = ops.attention_multi(q.to(DEV), store.to(DEV), batch, 0.1, maps=1, kv_heads=1, v_dim=64, rows_of=R, out_dtype=torch.float32)
+    assert bool(taken) == tensor_cores
+    k = torch.cat([store[p] for p in pages[0]])[:180].double()
+    for t in (0, 77, 149):
+        ref = torch.softmax(q[t].double() @ k[:31 + t].T * 0.1, -1) @ k[:31 + t, :64]
+        assert (out[t].double().cpu() - ref).abs().max() < 1e-5 * float(ref.abs().max())
+
+
 @pytest.mark.parametrize("ff, width, t", [(64, 512, 1), (200, 1024, 16), (320, 2048, 17), (65, 576, 128), (1000, 264, 5)])
 def test_gated_products_of_few_tokens_joined_over_a_cluster(ff, width, t):
     """Few tiles of a gated pair: runs of the inner dimension meet inside the kernel; a token's bits do not depend on the others."""

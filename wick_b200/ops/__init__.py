@@ -744,8 +744,11 @@ def attention_multi(q: torch.Tensor, store: torch.Tensor, batch, scale: float, *
     if gate is not None:
         _cuda("gate", gate, torch.float32, (n, H))
         _need(maps == 1, "the factor per head belongs to one map")
+    # (One head, or two with short rows, leave too many of the 16 rows of a tensor-core tile empty.  1,000 tokens behind 2,000, us on the
+    # CUDA cores / there: one head, rows of 64 381 / 664, of 576 941 / 1,349; two heads, rows of 64 492 / 664, of 320 1,621 / 991; three
+    # heads, rows of 64 789 / 664.)
     if (rows_of is not None and maps == 1 and T == torch.bfloat16 and q.dtype == torch.float32 and not soft_cap and gate is None
-            and attention_latent_supported(d, v_dim) and (q.data_ptr() | store.data_ptr()) % 16 == 0 and not plain_kernels()):
+            and (H > 2 or (H == 2 and d >= 128)) and attention_latent_supported(d, v_dim) and (q.data_ptr() | store.data_ptr()) % 16 == 0 and not plain_kernels()):
         return _attention_latent(q, store, batch, scale, v_dim, window, keep_first, sink)
     out = torch.empty((n, H, v_dim), dtype=out_dtype, device=q.device)
     # A step of few tokens: eight warps a block, heads that read the same rows together, and the visible keys cut into
