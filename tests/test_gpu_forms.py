@@ -68,6 +68,22 @@ def test_float32_products_read_a_matrix_that_the_kernel_before_wrote(m):
         assert torch.equal(got, ops.gemm_simt(x, w, torch.float32))
 
 
+@pytest.mark.parametrize("n, k, pair", [(2049, 64, False), (16385, 100, False), (4097, 128, True), (12300, 128, True), (4096, 132, False), (4100, 256, True), (300, 64, True),
+                                        (37900, 64, False), (18950, 260, True)])
+def test_float32_products_of_wide_matrices_give_the_same_bits(n, k, pair):
+    """Wide matrices of few inputs: the general form (a single slice), tiles instead of streamed weights, tiles of 64 rows where the
+    large ones would be half empty."""
+    g = torch.Generator().manual_seed(n + k)
+    x = torch.randn(300, k, generator=g).to(DEV)
+    w = (torch.randn(2 * n if pair else n, k, generator=g) / math.sqrt(k)).to(DEV)
+    got = ops.gemm_simt(x, w, torch.float32, gated=pair, w_static=True)
+    ref = x.double() @ w.double().T
+    ref = gated(ref) if pair else ref
+    assert (got.double() - ref).abs().max() < 1e-5 * max(1.0, float(ref.abs().max()))
+    for m in (1, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129):
+        assert torch.equal(ops.gemm_simt(x[:m].contiguous(), w, torch.float32, gated=pair, w_static=True), got[:m]), m
+
+
 def test_float32_products_of_misaligned_rows_take_the_general_form():
     x, w = torch.randn(5 * 64 + 1).to(DEV)[1:].view(5, 64), torch.randn(24, 64).to(DEV)
     assert x.data_ptr() % 16 != 0

@@ -10,9 +10,10 @@
 // eight slices of slice_len(K) numbers; an output is the sum, in slice order, of the slices' dot
 // products, each accumulated along k in index order.  That order depends on K alone, and all forms
 // below follow it, so a row's result depends neither on the other rows nor on M:
-//   * gemm_f32_few_kernel, up to 32 rows of A: the weights stream through shared memory once;
-//   * gemm_f32_tile_kernel, more rows: tiles of 128 x 128, 64 x 128 or 64 x 64 outputs.
-// Everything else goes through gemm_nt_kernel (one dot product along K in index order).
+//   * gemm_f32_few_kernel, up to 32 rows of A: the weights stream through shared memory, once per 16 rows;
+//   * gemm_f32_tile_kernel, more rows: tiles of 128 x 128, 64 x 128 or 64 x 64 outputs;
+//   * gemm_nt_kernel (one dot product along K in index order), where a single slice holds all of K: some sizes, see gemm_f32.
+// Everything else goes through gemm_nt_kernel.
 #include <type_traits>
 
 #include "common.cuh"
@@ -168,7 +169,7 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
 // in tiles of 128 x 128 5,290 -> 2,950 (47).
 constexpr int TILE_BK = 16;
 
-template <int BM, int BN, int TN, bool GATED, bool SLICED>
+template <int BM, int BN, int TN, bool GATED, bool SLICED, bool W_STATIC>
 __global__ void __launch_bounds__((BM / 8) * (BN / TN))
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K) {
     constexpr int THREADS = (BM / 8) * (BN / TN), TX = BN / TN, NB = GATED ? BN / 2 : BN;
@@ -181,7 +182,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     pdl_trigger();
     pdl_wait();
     A = fresh(A);
-    W = fresh(W);                                        // (an earlier kernel may have made it: this form does not ask w_static)
+    if (!W_STATIC) W = fresh(W);                         // (300 rows, gated 2 x 2,048 x 512: 47.6 us with it, 43.6 without)
     const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * NB;
     const float* arow[LA];
@@ -324,7 +325,7 @@ int gemm_f32_few(const float* A, const float* W, float* C, int M, int N, int K, 
 }
 
 template <int BM, int BN, int TN, bool GATED, bool SLICED>
-int gemm_f32_tiles(const float* A, const float* W, float* C, int M, int N, int K, cudaStream_t s) {
+int gemm_f32_tiles(const float* A, const float* W, float* C, int M, int N, int K, int w_static, cudaStream_t s) {
     const int slices = SLICED ? ceil_div(K, slice_len(K)) : 1;                // at most eight: a cluster
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ceil_div(N, GATED ? BN / 2 : BN), ceil_div(M, BM), slices);
@@ -338,13 +339,28 @@ int gemm_f32_tiles(const float* A, const float* W, float* C, int M, int N, int K
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    WICK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM, BN, TN, GATED, SLICED>, A, W, C, M, N, K));
+    if (w_static) WICK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM, BN, TN, GATED, SLICED, true>, A, W, C, M, N, K));
+    else WICK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM, BN, TN, GATED, SLICED, false>, A, W, C, M, N, K));
     return check_launch("gemm_f32_tile");
+}
+
+// A single slice (K up to 128): one warp in eight of the streaming form works, and the tiles' loop over K is short.  The general form,
+// which adds in the same order, is then faster on wide matrices of 9 to 32 rows and for gated products of many outputs.  (us, streamed or
+// tiles / general form: K = 64 16 rows x 32,768 16.4 / 13.4, x 8,192 6.1 / 6.5, 17 rows x 8,192 9.5 / 6.1, x 2,048 4.1 / 6.1; K = 128 17 rows x
+// 8,192 15.0 / 10.6, x 4,096 9.3 / 10.3.  Gated, K = 64 100 rows x 8,192 17.2 / 13.9, x 2,048 10.2 / 9.9; K = 128 100 rows x 8,192 27.4 /
+// 23.6, x 2,048 14.1 / 16.9, x 32,768, in tiles of 128 x 128, 69 / 74.)
+inline bool one_slice_general(int M, int N, int K, bool gated) {
+    if (K > slice_len(K) || M <= 8) return false;
+    if (M <= FEW_MAX) return N > (M <= 16 ? 16384 : (K <= 100 ? 2048 : 4096));
+    return gated && (int64_t)M * N >= 400000 && (K <= 100 || (int64_t)ceil_div(M, 128) * ceil_div(N, 64) < 2 * sm_count());
 }
 
 template <bool GATED>
 int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int w_static, cudaStream_t s) {
-    if (M <= FEW_MAX) {
+    // (few slices leave most warps of the streaming form without work: then tiles, which bring the weights once, from 17 rows on.
+    // us streamed / as tiles, 17 rows, K = 256 x 4,096 10.4 / 9.0, x 32,768 70 / 33, gated x 4,096 17.2 / 14.7; K = 384 x 8,192 18.1 / 20.5)
+    const bool wide = M > 16 && K <= 256 && N >= 4096;
+    if (M <= FEW_MAX && !wide) {
         // (16 outputs a block halve the trips of A's rows; with few outputs 8 a block fill the device)
         if (M <= 2) return gemm_f32_few<2, 1, GATED>(A, W, C, M, N, K, w_static, s);
         if (M <= 4) return gemm_f32_few<4, 1, GATED>(A, W, C, M, N, K, w_static, s);
@@ -352,9 +368,13 @@ int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int 
         if (M <= 8) return gemm_f32_few<8, 2, GATED>(A, W, C, M, N, K, w_static, s);
         return gemm_f32_few<16, 2, GATED>(A, W, C, M, N, K, w_static, s);
     }
-    if ((int64_t)ceil_div(M, 128) * ceil_div(N, GATED ? 64 : 128) >= 2 * sm_count()) return gemm_f32_tiles<128, 128, 8, GATED, false>(A, W, C, M, N, K, s);
-    if constexpr (GATED) return gemm_f32_tiles<64, 128, 8, true, true>(A, W, C, M, N, K, s);
-    else return gemm_f32_tiles<64, 64, 4, false, true>(A, W, C, M, N, K, s);
+    // (up to 64 rows of a gated product: half of a tile of 128 rows would be empty.  33 rows, gated 2 x 32,768 x 1,024: 439 us in tiles of
+    // 128 x 128, 224 in tiles of 64 x 128.)
+    if constexpr (GATED)
+        if (M <= 64 && ceil_div(N, 64) >= 2 * sm_count()) return gemm_f32_tiles<64, 128, 8, true, false>(A, W, C, M, N, K, w_static, s);
+    if ((int64_t)ceil_div(M, 128) * ceil_div(N, GATED ? 64 : 128) >= 2 * sm_count()) return gemm_f32_tiles<128, 128, 8, GATED, false>(A, W, C, M, N, K, w_static, s);
+    if constexpr (GATED) return gemm_f32_tiles<64, 128, 8, true, true>(A, W, C, M, N, K, w_static, s);
+    else return gemm_f32_tiles<64, 64, 4, false, true>(A, W, C, M, N, K, w_static, s);
 }
 
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
@@ -424,7 +444,7 @@ int gemm_nt(const void* A, const void* W, void* C, int M, int N, int K, int w_st
     WICK_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm: bad sizes M=%d N=%d K=%d", M, N, K);
     if (M == 0) return 0;
     if constexpr (std::is_same<T, float>::value && std::is_same<TOut, float>::value) {
-        if (K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && M <= 65535 * 64)
+        if (K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && M <= 65535 * 64 && !one_slice_general(M, N, K, GATED))
             return gemm_f32<GATED>((const float*)A, (const float*)W, (float*)C, M, N, K, w_static, s);
     }
     dim3 grid(ceil_div(N, BN), ceil_div(M, BM));
