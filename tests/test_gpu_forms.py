@@ -160,6 +160,21 @@ def test_gated_products_of_few_tokens_joined_over_a_cluster(ff, width, t):
         assert torch.equal(plan.forward(x[:1].contiguous(), torch.bfloat16), got[:1])
 
 
+@pytest.mark.parametrize("ff, width, runs", [(66, 768, 3), (130, 640, 2), (257, 1280, 5), (70, 1536, 6)])
+@pytest.mark.parametrize("t", [1, 31, 128])
+def test_gated_products_joined_with_rows_that_are_no_whole_groups(ff, width, runs, t):
+    """Up to four runs four neighbours a thread are finished at once, or one by one at a row's end."""
+    from wick_b200.ops import gemm_tc as G
+    g = torch.Generator().manual_seed(ff)
+    w = (torch.randn(2 * ff, width, generator=g) / math.sqrt(width)).bfloat16().to(DEV)
+    x = torch.randn(t, width, generator=g).bfloat16().to(DEV)
+    plan = G.plan_for(w, gated=True)
+    assert plan.joined_splits == runs
+    got, ref = plan.forward(x, torch.bfloat16), gated(x.double() @ w.double().T)
+    G.check_status()
+    assert (got.double() - ref).abs().max() < 2 ** -8 * max(1.0, float(ref.abs().max()))
+
+
 @pytest.mark.parametrize("E, top, ff, width, shared", [(5, 3, 136, 264, 0), (8, 2, 192, 1024, 64), (1, 1, 64, 128, 0), (16, 2, 72, 512, 0), (5, 2, 520, 264, 1000)])
 @pytest.mark.parametrize("n", [1, 2, 17, 64, 65, 128, 129])
 def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
