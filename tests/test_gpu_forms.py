@@ -215,6 +215,28 @@ def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
         assert torch.equal(one, got[:1]), "a token's bits do not depend on the others"
 
 
+@pytest.mark.parametrize("E, top", [(40, 3), (300, 2), (320, 5), (1024, 1), (1025, 1)])
+@pytest.mark.parametrize("n", [1, 25, 26, 60, 61, 128])
+def test_table_experts_of_which_a_step_names_a_few(E, top, n):
+    """Blocks for as many experts as the step can name where those are few of many (up to 1,024 experts), the i-th slot's expert being the
+    i-th that it names; otherwise blocks for all."""
+    from wick_b200.ops import gemm_tc as G
+    g, f, w = torch.Generator().manual_seed(E + n), 72, 64
+    mats = (torch.randn(E, f, w, generator=g) / math.sqrt(w)).bfloat16()
+    table = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(50)]).int()
+    table[7], table[8] = torch.arange(top), torch.arange(E - top, E)        # (the first and the last)
+    tiles = torch.cat([G.pack(m.to(DEV)) for m in mats], 0)
+    x = torch.randn(n, w, generator=g).bfloat16()
+    tok = torch.randint(0, 50, (n,), generator=g).int()
+    tok[0], tok[-1] = 7, 8
+    y = G.gemm_tc_experts(tiles, E, f, x.to(DEV), tok.to(DEV), table.to(DEV), gated=False, per_expert_b=False, k=w)[0].cpu()
+    G.check_status()
+    for t in range(n):
+        for e in table[int(tok[t])].tolist():
+            ref = mats[e].double() @ x[t].double()
+            assert (y[e, t].double() - ref).abs().max() < 1e-5, (t, e)
+
+
 @pytest.mark.parametrize("width", [4, 132, 4096, 4100, 5120, 5124, 6144, 6148])
 @pytest.mark.parametrize("splits", [0, 1, 7, 9])
 def test_norm_forms_give_the_same_bits(width, splits):

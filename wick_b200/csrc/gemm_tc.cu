@@ -62,11 +62,13 @@ struct GemmParams {
 
 // (A struct of its own: with these fields in GemmParams the kernels that do not use them came out with up to half as many registers
 // again, and the decode products were 1 to 3 % slower.)
+constexpr int NAMED_WORDS = 32;
 struct GroupedParams : GemmParams {
     // Grouped (several matrices of A one after the other, see wick_gemm_tc_grouped): the m tiles of one matrix, its padded
     // rows, the rows of B it is multiplied with (0: all matrices with the same rows), elements of out between two matrices'
     // results; the step's token ids and the table that names each id's `top` matrices.
     int group_tiles, group_rows, group_b_rows, top, n_tokens;
+    int n_groups;                                   // of matrices (ranked; at most 32 NAMED_WORDS)
     long long group_out;
     const int *tokens, *table;
     // A matrix that every token uses besides (the shared expert's; its m tiles follow the groups'), multiplied with rows of its own:
@@ -89,6 +91,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // its own.  A block whose matrix no token of the step uses leaves at once, and of the others' results only those of tokens
 // that use the matrix are written.
 //
+// Ranked: there are blocks for as many matrices as the step can name, the blocks of slot i taking the i-th that it names.  (With blocks
+// for all of 256 experts of 512 x 1,024, eight a token, a layer of one token took 48 us, with the kernels that walk the rows 40; ranked 18.
+// It costs half a microsecond, and the blocks of experts that are named late start late.)
+//
 // Joined (a gated pair that shares a tile, transposed bfloat16 result): the runs of the inner dimension along blockIdx.z are a
 // cluster; every block leaves its accumulator in its shared memory (the ring is idle by then), and the blocks finish a share of the
 // tokens each, adding the runs' sums in index order over distributed shared memory.  A pair cannot be left as partial sums, and
@@ -96,7 +102,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // 16.5 us; as 240 blocks 11.7 us.  With up to four runs a block finishes many results: four neighbours a thread (one at a time, 128 tokens
 // x 512 inputs, two runs took 15.9 us, 12.8 without runs; now 8.3); with more, one at a time (2,048 inputs, eight runs, 24 tokens 6.8 us
 // against 7.7).
-template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool GROUPED, bool JOINED>
+template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool GROUPED, bool JOINED, bool RANKED = false>
 __device__ __forceinline__ void
 gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap* shared_a, const CUtensorMap* shared_b,
               const std::conditional_t<GROUPED, GroupedParams, GemmParams>& p) {
@@ -111,6 +117,7 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
     __shared__ float xch[2][64][17];           // gated == 3: up values on their way to the warps that hold the gate values
 
     __shared__ unsigned uses[GROUPED ? 8 : 1];   // grouped: a bit per token that uses this block's matrix
+    __shared__ unsigned named[RANKED ? NAMED_WORDS : 1];               // ranked: a bit per matrix that the step names
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int group = 0, bx = blockIdx.x;                          // this block's matrix, its m tile there
@@ -119,6 +126,22 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
         bx -= group < 0 ? p.groups_end : group * p.group_tiles;
         // (the step's description is the host's or step_prepare's: it may be read before griddepcontrol.wait)
         if (threadIdx.x < 8) uses[threadIdx.x] = group < 0 ? ~0u : 0u;
+        if (RANKED && group >= 0) {
+            const int words = (p.n_groups + 31) / 32;
+            for (int i = threadIdx.x; i < words; i += NUM_THREADS) named[i] = 0u;
+            __syncthreads();
+            for (int i = threadIdx.x; i < p.n_tokens * p.top; i += NUM_THREADS) {
+                const int e = p.table[(long long)p.tokens[i / p.top] * p.top + i % p.top];
+                if (e >= 0 && e < p.n_groups) atomicOr(&named[e >> 5], 1u << (e & 31));
+            }
+            __syncthreads();
+            int word = 0, rank = group;                      // (every thread finds the same one)
+            while (word < words && rank >= __popc(named[word])) rank -= __popc(named[word++]);
+            if (word == words) return;
+            unsigned left = named[word];
+            while (rank-- > 0) left &= left - 1;
+            group = 32 * word + __ffs(left) - 1;
+        }
         __syncthreads();
         bool mine = group < 0;
         for (int i = threadIdx.x; i < (group < 0 ? 0 : p.n_tokens * p.top); i += NUM_THREADS) {
@@ -506,11 +529,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     gemm_tc_block<PERSIST, GATED, TRANSPOSED, OUT_F32, false, JOINED>(map_a, map_b, nullptr, nullptr, p);
 }
 
-template <int GATED, bool OUT_F32>
+template <int GATED, bool OUT_F32, bool RANKED>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap shared_a, const __grid_constant__ CUtensorMap shared_b, const GroupedParams p) {
-    gemm_tc_block<false, GATED, true, OUT_F32, true, false>(map_a, map_b, &shared_a, &shared_b, p);
+    gemm_tc_block<false, GATED, true, OUT_F32, true, false, RANKED>(map_a, map_b, &shared_a, &shared_b, p);
 }
 
 // ---- host side ---------------------------------------------------------------
@@ -622,7 +645,12 @@ static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const
         static_cast<GemmParams&>(g) = p;
         g.group_tiles = p.grid_m; g.group_rows = G.rows; g.group_b_rows = G.b_rows; g.group_out = G.out;
         g.top = G.top; g.n_tokens = G.n_tokens; g.tokens = G.tokens; g.table = G.table;
-        g.groups_end = p.grid_m * G.n;
+        // Ranked where the blocks of all matrices are more than run at once and the step can name two in five of them at most.  (Layers of
+        // 64 experts of 768 x 2,048, eight a token, us as all / ranked: 1 token 33 / 28, 3 52 / 50, 4 67 / 69; 128 experts 1 token
+        // 49 / 29, 6 93 / 89, 8 113 / 115, 15 157 / 175; 8 experts of 1,536 x 2,048, two a token, 1 token 24.7 / 25.0.)
+        const bool ranked = 5ll * G.n_tokens * G.top <= 2ll * G.n && G.n <= 32 * NAMED_WORDS && (long long)p.grid_m * G.n > 2 * sm_count();
+        g.n_groups = G.n;
+        g.groups_end = p.grid_m * (ranked ? G.n_tokens * G.top : G.n);
         CUtensorMap shared_a = map_a, shared_b = map_b;
         g.shared_tiles = 0;
         if (G.shared_a) {
@@ -642,12 +670,18 @@ static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const
         const dim3 grid(g.groups_end + g.shared_tiles, p.grid_n, splits);
         static bool raised = false;
         if (!raised) {
-            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_grouped_kernel<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
-            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_grouped_kernel<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_grouped_kernel<3, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_grouped_kernel<0, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_grouped_kernel<3, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+            WICK_CUDA(cudaFuncSetAttribute(gemm_tc_grouped_kernel<0, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
             raised = true;
         }
-        if (gated) WICK_CUDA(launch(gemm_tc_grouped_kernel<3, false>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, shared_a, shared_b, g));
-        else WICK_CUDA(launch(gemm_tc_grouped_kernel<0, true>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, shared_a, shared_b, g));
+#define WICK_GROUPED(P, F, R) WICK_CUDA(launch(gemm_tc_grouped_kernel<P, F, R>, grid, dim3(NUM_THREADS), (size_t)smem, (cudaStream_t)stream, map_a, map_b, shared_a, shared_b, g))
+        if (gated && ranked) WICK_GROUPED(3, false, true);
+        else if (gated) WICK_GROUPED(3, false, false);
+        else if (ranked) WICK_GROUPED(0, true, true);
+        else WICK_GROUPED(0, true, false);
+#undef WICK_GROUPED
         return check_launch("gemm_tc_grouped");
     }
     // persistent blocks: as many as can be resident at once (one or two per SM by shared memory)
