@@ -128,6 +128,20 @@ def test_attention_over_rows_on_the_tensor_cores(H, R, r, q_lens, starts, window
             t += 1
 
 
+def test_attention_over_rows_of_queries_near_the_largest_float():
+    """Queries beyond bfloat16's largest number are still the sum of their three parts."""
+    batch, pages, n_pages = batch_of([1, 1], [40, 3])
+    store = torch.randn(n_pages, PAGE, 80, generator=torch.Generator().manual_seed(1)).bfloat16()
+    store[:, :, 79] = ((1 + torch.arange(PAGE) / 64) * 2.0 ** -126).bfloat16()
+    q = torch.randn(2, 5, 80, generator=torch.Generator().manual_seed(2))
+    q[0, 1, 79], q[0, 3, 79] = 3.4e38, -torch.finfo(torch.float32).max
+    out = ops.attention_multi(q.to(DEV), store.to(DEV), batch, 0.3, maps=1, kv_heads=1, v_dim=64, rows_of=80, out_dtype=torch.float32).double().cpu()
+    for t, n in ((0, 41), (1, 4)):
+        k = torch.cat([store[p] for p in pages[t]])[:n].double()
+        ref = torch.softmax(q[t].double() @ k.T * 0.3, -1) @ k[:, :64]
+        assert (out[t] - ref).abs().max() < 1e-5 * float(ref.abs().max())
+
+
 @pytest.mark.parametrize("H, R, tensor_cores", [(1, 80, False), (1, 192, False), (2, 80, False), (2, 128, True), (3, 80, True)])
 def test_attention_over_rows_of_few_heads_stays_on_the_cuda_cores(H, R, tensor_cores, monkeypatch):
     batch, pages, n_pages = batch_of([150], [30])

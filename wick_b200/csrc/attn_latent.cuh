@@ -11,6 +11,8 @@
 //   * values: warp w adds the tile's weighted rows into columns w * r / 8 .. of all heads' results.
 // Tiles come by cp.async, two ahead (those of rows that no kernel of this step writes before the kernel before this one has
 // finished).  A row lies on an odd number of 16-byte pieces in shared memory, so that ldmatrix meets no bank twice.
+// A cached row that holds an infinity makes NaN of its tokens' results, also where float32 products would have left an infinity: the
+// parts of a number have either sign.
 // With `partial` a run's result goes there as a record (maximum, sum, two unused numbers, unnormalised values) for the merge.
 //
 // What bounds it: with few tokens the chain of a block's start, one or two tiles and its record; with many the tensor cores.  The form
@@ -57,13 +59,20 @@ __device__ __forceinline__ void mma(float* c, const uint32_t* a, uint32_t b0, ui
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// x = t[0] + t[1] + t[2], each a bfloat16 number (the differences are exact)
+// x = t[0] + t[1] + t[2], each a bfloat16 number (the differences are exact).  For x in [0, 1].
 __device__ __forceinline__ void split3(float x, bf16* t) {
     t[0] = __float2bfloat16_rn(x);
     x -= __bfloat162float(t[0]);
     t[1] = __float2bfloat16_rn(x);
     x -= __bfloat162float(t[1]);
     t[2] = __float2bfloat16_rn(x);
+}
+// The same for any x: a number that would be rounded beyond bfloat16's largest is cut instead; an infinity and a NaN are their own first part.
+__device__ __forceinline__ void split3_any(float x, bf16* t) {
+    t[0] = fabsf(x) < 3.3895e38f ? __float2bfloat16_rn(x) : __float2bfloat16_rz(x);
+    const float rest = isfinite(x) ? x - __bfloat162float(t[0]) : 0.f;
+    t[1] = __float2bfloat16_rn(rest);
+    t[2] = __float2bfloat16_rn(rest - __bfloat162float(t[1]));
 }
 __device__ __forceinline__ uint32_t pair(bf16 a, bf16 b) {
     __nv_bfloat162 v = __halves2bfloat162(a, b);
@@ -142,8 +151,8 @@ attn_latent_kernel(const Params P) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 bf16 a[3], b[3];
-                split3(x[i].x, a);
-                split3(x[i].y, b);
+                split3_any(x[i].x, a);
+                split3_any(x[i].y, b);
 #pragma unroll
                 for (int j = 0; j < 3; ++j) qf[k][j][i] = pair(a[j], b[j]);
             }
