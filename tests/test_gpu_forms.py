@@ -31,6 +31,16 @@ def batch_of(q_lens, starts):
     return StepBatch(layout, torch.from_numpy(host).to(DEV), q_lens=q_lens, starts=starts), pages, n_pages + 1
 
 
+def unwritten_as_nan(monkeypatch):
+    """What torch.empty gives on the device holds NaN until a kernel writes it."""
+    real = torch.empty
+
+    def empty(*a, **k):
+        t = real(*a, **k)
+        return t.fill_(float("nan")) if t.is_cuda and t.is_floating_point() else t
+    monkeypatch.setattr(torch, "empty", empty)
+
+
 def gated(y):
     g, u = y.chunk(2, dim=1)
     return g / (1 + torch.exp(-g)) * u
@@ -142,6 +152,48 @@ def test_attention_over_rows_of_queries_near_the_largest_float():
         assert (out[t] - ref).abs().max() < 1e-5 * float(ref.abs().max())
 
 
+@pytest.mark.parametrize("H, R, r, q_lens, starts, window, keep", [
+    (16, 80, 64, [1, 1], [500, 90], 64, 10),                        # kept keys end inside a tile, runs of keys
+    (4, 80, 64, [70], [300], 100, 40),                              # beyond one tile, few runs
+    (5, 80, 64, [200], [5], 50, 7),                                 # many tokens: one run each, some before the window's start
+    (32, 576, 512, [1, 2], [2000, 31], 512, 33),
+])
+def test_attention_over_rows_with_kept_first_keys_on_the_tensor_cores(H, R, r, q_lens, starts, window, keep):
+    g = torch.Generator().manual_seed(H)
+    batch, pages, n_pages = batch_of(q_lens, starts)
+    store = torch.randn(n_pages, PAGE, R, generator=g).bfloat16()
+    q = torch.randn(sum(q_lens), H, R, generator=g)
+    out = ops.attention_multi(q.to(DEV), store.to(DEV), batch, R ** -0.5, maps=1, kv_heads=1, v_dim=r, window=window, keep_first=keep, rows_of=R,
+                              out_dtype=torch.float32).double().cpu()
+    t = 0
+    for b, (ql, s) in enumerate(zip(q_lens, starts)):
+        k = torch.cat([store[p] for p in pages[b]])[:s + ql].double()
+        for p in range(s, s + ql):
+            j = torch.arange(p + 1)
+            seen = k[:p + 1][(p - j < window) | (j < keep)]
+            ref = torch.softmax(q[t].double() @ seen.T * R ** -0.5, -1) @ seen[:, :r]
+            assert (out[t] - ref).abs().max() < 1e-5 * float(ref.abs().max()), (b, p)
+            t += 1
+
+
+def test_attention_over_rows_of_a_token_alone_and_among_others():
+    """How many runs a token's keys are cut into follows the number of tokens and the step's bound: what differs is the order of float32
+    sums, a few 2^-24 of a result that is an average of its values."""
+    g = torch.Generator().manual_seed(8)
+    starts = [700, 33, 1500, 64] * 6
+    batch, pages, n_pages = batch_of([1] * 24, starts)
+    store, q = torch.randn(n_pages, PAGE, 144, generator=g).bfloat16().to(DEV), torch.randn(24, 20, 144, generator=g).to(DEV)
+    args = dict(maps=1, kv_heads=1, v_dim=128, rows_of=144, out_dtype=torch.float32)
+    many = ops.attention_multi(q, store, batch, 0.08, **args)
+    for i in range(4):
+        layout = BatchLayout(1, 1, len(pages[i]), 1)
+        host = np.zeros(layout.size, dtype=np.int32)
+        fill_host(layout, host, tokens=[[0]], starts=starts[i:i + 1], slots=[1], pages=pages[i:i + 1], want=[[0]])
+        one = StepBatch(layout, torch.from_numpy(host).to(DEV), q_lens=[1], starts=starts[i:i + 1])
+        alone = ops.attention_multi(q[i:i + 1].contiguous(), store, one, 0.08, **args)[0]
+        assert (alone - many[i]).abs().max() < 2e-6 * float(many[i].abs().max())
+
+
 @pytest.mark.parametrize("H, R, tensor_cores", [(1, 80, False), (1, 192, False), (2, 80, False), (2, 128, True), (3, 80, True)])
 def test_attention_over_rows_of_few_heads_stays_on_the_cuda_cores(H, R, tensor_cores, monkeypatch):
     batch, pages, n_pages = batch_of([150], [30])
@@ -191,8 +243,10 @@ def test_gated_products_joined_with_rows_that_are_no_whole_groups(ff, width, run
 
 @pytest.mark.parametrize("E, top, ff, width, shared", [(5, 3, 136, 264, 0), (8, 2, 192, 1024, 64), (1, 1, 64, 128, 0), (16, 2, 72, 512, 0), (5, 2, 520, 264, 1000)])
 @pytest.mark.parametrize("n", [1, 2, 17, 64, 65, 128, 129])
-def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
-    """Experts that no token uses are left alone; results beyond a token's own experts are never read (they hold NaN before)."""
+def test_table_experts_of_few_tokens(E, top, ff, width, shared, n, monkeypatch):
+    """Experts that no token uses are left alone; results beyond a token's own experts are never read (they hold NaN before), nor, beyond
+    128 tokens, rows between the sorted experts' and tiles beyond the last one's (without the host's token ids there are the most rows
+    that there can be)."""
     from wick_b200.models.spec import PartSpec
     from wick_b200.parts.base import BuildContext, build_part
     from wick_b200.parts import feedforward  # noqa: F401
@@ -212,7 +266,7 @@ def test_table_experts_of_few_tokens(E, top, ff, width, shared, n):
     part.load(get)
     x = torch.randn(n, width, generator=g).bfloat16().to(DEV)
     tok = torch.randint(0, 50, (n,), generator=g).int().to(DEV)
-    torch.full((1 << 22,), float("nan"), device=DEV)                   # (scratch that the step may be given again)
+    unwritten_as_nan(monkeypatch)
     got = part.forward(x, types.SimpleNamespace(tokens=tok, host=None)).sum(0)
     ops.check_status()
 
@@ -440,6 +494,19 @@ def test_short_form_of_the_decode_attention_among_few_and_many(hd, dtype, H, G):
         # (float32 sums of at most 1,025 terms: below 1e-5; the result's own rounding to bfloat16 2^-9)
         assert (many[i].double() - ref).abs().max() < (1e-5 if dtype == torch.float32 else 2 ** -8) * max(1.0, float(ref.abs().max()))
     ops.check_status()
+
+
+def test_a_prompt_product_in_three_runs():
+    """Few tiles for the pairs of SMs, an inner dimension of three runs of 32 steps at most."""
+    from wick_b200.ops import gemm_tc as G
+    g = torch.Generator().manual_seed(3)
+    w, x = (torch.randn(1000, 6144, generator=g) / 78).bfloat16().to(DEV), torch.randn(300, 6144, generator=g).bfloat16().to(DEV)
+    plan = G.plan_for(w)
+    assert plan.prompt_splits(300) == 3
+    parts = plan.forward_delta(x)
+    G.check_status()
+    assert parts.shape == (3, 300, 1000)
+    assert (parts.sum(0).double() - x.double() @ w.double().T).abs().max() < 1e-5 * 5
 
 
 @pytest.mark.parametrize("t, k, out, pair", [(4357, 7400, 300, False), (2305, 14000, 513, True), (4096, 7688, 257, False)])
