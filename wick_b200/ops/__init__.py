@@ -926,17 +926,16 @@ def attention_latent_supported(row: int, v_dim: int) -> bool:
     return row % 16 == 0 and row <= 576 and v_dim % 64 == 0 and 0 < v_dim <= min(512, row)
 
 
-LATENT_BLOCKS = 148         # blocks of a step of few tokens
-
-
 def _attention_latent(q, store, batch, scale, v_dim, window, keep_first, sink) -> torch.Tensor:
+    from .gemm_tc import sm_count
     n, H, R = q.shape
     out = torch.empty((n, H, v_dim), dtype=torch.float32, device=q.device)
-    # A block takes a token's up to 32 heads and fills an SM; the visible keys are cut into runs until every SM has one.  (8 tokens of
+    # A block takes a token's up to 32 heads and fills an SM; the visible keys are cut into runs until every SM has one, so that the order in
+    # which a token's keys are added up follows the number of tokens and the step's bound.  (148 SMs: 8 tokens of
     # 1,500 positions: 74 blocks 32.8 us, 148 25.7, 296 38.3; 4 of 700 to 1,500: 22.8, 24.8, 31.0.)
     bound = getattr(batch, "kv_bound", None) or batch.max_kv_len
     keys = min(bound, window + keep_first) if window > 0 else bound
-    runs = max(1, min(LATENT_BLOCKS // (n * ((H + 31) // 32)), (max(1, keys) + 31) // 32, 64))
+    runs = max(1, min(sm_count(q.device) // (n * ((H + 31) // 32)), (max(1, keys) + 31) // 32, 64))
     partial = None
     if runs > 1:
         need = n * H * runs * (4 + (v_dim + 127) // 128 * 128)
