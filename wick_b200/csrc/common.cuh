@@ -252,8 +252,12 @@ __device__ __forceinline__ void find_work_item(const int* __restrict__ cu_seqlen
 // while this one still runs.  A kernel therefore (1) lets its successor start
 // (pdl_trigger) and (2) waits until its predecessor has completed and its writes
 // are visible (pdl_wait) before it touches anything another kernel produced or
-// may still read.  Only loads of data that no kernel ever writes (weights) may
-// come before pdl_wait.  Both are no-ops for a kernel launched the ordinary way.
+// may still read.  Only loads of data that no kernel in flight can be writing may
+// come before pdl_wait: weights, which no kernel ever writes; the step's description
+// (tokens, positions, lengths, page tables) and rows of the cache that earlier steps
+// wrote.  A step begins with the host's copy of its description or with step_prepare,
+// which never lets its successor start early, so all of its kernels run behind those of
+// the step before.  Both are no-ops for a kernel launched the ordinary way.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A pointer to data that the kernel before this one produces, as the compiler must

@@ -199,13 +199,17 @@ class TableMoE(FeedForward):
 
     # Up to this many tokens every expert that the step uses is multiplied with all of them, in the orientation of the dense
     # products of few tokens (the matrices stream through the 128-row side once; what other tokens make of an expert is not
-    # written).  The runs of the inner dimension depend on the matrices alone, so that a token's bits do not depend on the step.
+    # written).  Up to 64 tokens the runs of the inner dimension depend on the matrices alone, so that a token's bits do not depend on the
+    # step.  Measured from 8 experts of 1,536 x 2,048 to 256 of 512 x 1,024, one to eight a token, us a layer with the kernels that
+    # walk the experts' rows or the sorted rows / so: 8 experts, 1, 8, 16, 128 tokens 28 / 25, 55 / 30, 100 / 32, 102 / 54; 64 experts of
+    # 768, eight a token 37 / 28, 101 / 85, 308 / 116, 331 / 183; 256 experts 40 / 18, 61 / 51, 325 / 82, 680 / 267; slower only where
+    # matrices are tiny (16 experts of 256 x 512, up to four tokens 9.2 / 10.6).
     FEW_MAX = 128
 
     def _few_splits(self, n, shared):
-        """Runs of the down product's inner dimension: two, where its tiles alone leave SMs without a block, fixed for the sizes of
-        decode steps so that a token's bits do not depend on the step.  (Experts of 1,536 x 2,048, 8 tokens: 36.5 us in one run,
-        33.7 in two, 38.2 in four; the gated product in two runs is faster up to four tokens only.)"""
+        """Runs of the down product's inner dimension: two up to 64 tokens, whatever the number of tiles, so that a token's bits do not
+        depend on the step, one beyond.  (8 experts of 1,536 x 2,048, us a layer in one / two runs, 1 token 29.1 / 24.6, 64 tokens 42.2 /
+        40.4; 16 of 2,048 x 4,096 45.9 / 40.0, 144 / 157; 64 of 768 x 2,048, eight a token 27.9 / 28.5, 142 / 165.)"""
         from ..ops import gemm_tc
         ks = [(self.intermediate + 63) // 64] + ([shared[1].k_blocks] if shared else [])
         return min(gemm_tc.even_splits(min(2, k // 4), k) for k in ks) if n <= gemm_tc.SMALL else 1
@@ -240,8 +244,8 @@ class TableMoE(FeedForward):
     # multiplied with the matrices of the expert the tile belongs to.  How many rows that makes
     # depends on the step's tokens: the host counts them from the step's token ids where the step's
     # description has them (the table is a constant); otherwise (a captured step, whose tokens the
-    # host never sees) the product runs over the most rows there can be, and the tiles beyond the
-    # last expert's hold zeros.  The 32-bit path and sizes the tensor-core
+    # host never sees) the product runs over the most rows there can be.  The rows between the experts' and
+    # the tiles beyond the last expert's hold what nobody wrote, and nobody reads what becomes of them.  The 32-bit path and sizes the tensor-core
     # kernels do not take go through the kernels that walk the matrices by expert.
     ROW_TILE = 256
 
