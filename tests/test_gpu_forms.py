@@ -94,6 +94,22 @@ def test_float32_products_of_wide_matrices_give_the_same_bits(n, k, pair):
         assert torch.equal(ops.gemm_simt(x[:m].contiguous(), w, torch.float32, gated=pair, w_static=True), got[:m]), m
 
 
+@pytest.mark.parametrize("n, k, pair", [(8192, 132, True), (2100, 192, True), (1500, 256, True), (6200, 100, True), (16400, 48, True), (4100, 176, True),
+                                        (8192, 132, False), (4100, 160, False), (6200, 224, False), (6200, 100, False), (9500, 60, False), (2048, 132, False), (24600, 132, False), (32800, 384, False), (16400, 320, True)])
+def test_float32_products_of_few_inputs_give_the_same_bits(n, k, pair):
+    """One or two slices: the general form takes the slices as the others do, gated tiles of 64 rows both one after the other.  The rows
+    cross the sizes at which the forms change."""
+    g = torch.Generator().manual_seed(n + k)
+    x = torch.randn(600, k, generator=g).to(DEV)
+    w = (torch.randn(2 * n if pair else n, k, generator=g) / math.sqrt(k)).to(DEV)
+    got = ops.gemm_simt(x, w, torch.float32, gated=pair, w_static=True)
+    ref = x.double() @ w.double().T
+    ref = gated(ref) if pair else ref
+    assert (got.double() - ref).abs().max() < 1e-5 * max(1.0, float(ref.abs().max()))
+    for m in (1, 4, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 193, 257, 321):
+        assert torch.equal(ops.gemm_simt(x[:m].contiguous(), w, torch.float32, gated=pair, w_static=m % 2 == 0), got[:m]), m
+
+
 def test_float32_products_of_misaligned_rows_take_the_general_form():
     x, w = torch.randn(5 * 64 + 1).to(DEV)[1:].view(5, 64), torch.randn(24, 64).to(DEV)
     assert x.data_ptr() % 16 != 0

@@ -12,8 +12,8 @@
 // below follow it, so a row's result depends neither on the other rows nor on M:
 //   * gemm_f32_few_kernel, up to 32 rows of A: the weights stream through shared memory, once per 16 rows;
 //   * gemm_f32_tile_kernel, more rows: tiles of 128 x 128, 64 x 128 or 64 x 64 outputs;
-//   * gemm_nt_kernel (one dot product along K in index order), where a single slice holds all of K: some sizes, see gemm_f32.
-// Everything else goes through gemm_nt_kernel.
+//   * gemm_nt_kernel, some sizes of up to 256 inputs, see few_inputs_form.
+// Everything else goes through gemm_nt_kernel as well, one dot product along K in index order.
 #include <type_traits>
 
 #include "common.cuh"
@@ -344,22 +344,44 @@ int gemm_f32_tiles(const float* A, const float* W, float* C, int M, int N, int K
     return check_launch("gemm_f32_tile");
 }
 
-// A single slice (K up to 128): one warp in eight of the streaming form works, and the tiles' loop over K is short.  The general form,
-// which adds in the same order, is then faster on wide matrices of 9 to 32 rows and for gated products of many outputs.  (us, streamed or
-// tiles / general form: K = 64 16 rows x 32,768 16.4 / 13.4, x 8,192 6.1 / 6.5, 17 rows x 8,192 9.5 / 6.1, x 2,048 4.1 / 6.1; K = 128 17 rows x
-// 8,192 15.0 / 10.6, x 4,096 9.3 / 10.3.  Gated, K = 64 100 rows x 8,192 17.2 / 13.9, x 2,048 10.2 / 9.9; K = 128 100 rows x 8,192 27.4 /
-// 23.6, x 2,048 14.1 / 16.9, x 32,768, in tiles of 128 x 128, 69 / 74.)
-inline bool one_slice_general(int M, int N, int K, bool gated) {
-    if (K > slice_len(K) || M <= 8) return false;
-    if (M <= FEW_MAX) return N > (M <= 16 ? 16384 : (K <= 100 ? 2048 : 4096));
-    return gated && (int64_t)M * N >= 400000 && (K <= 100 || (int64_t)ceil_div(M, 128) * ceil_div(N, 64) < 2 * sm_count());
+// Few inputs (up to 256, one or two slices): only one or two of the streaming form's eight warps work, each through whole stages of 64 or 128
+// numbers whatever K is, and a second slice of a few numbers costs the tiles that a cluster joins as much as a full one.  Where
+// the general form's blocks of 64 x 64 outputs fill much of the device once and little more, it is the fastest then; with more blocks than
+// one or two an SM tiles of 64 rows that take both slices one after the other are.  All add in the same order.  us, the
+// streaming form or joined tiles / the general form / tiles of 64 rows: K = 132, gated x 8,192 24 rows 29.3 / 15.6 / 19.5, 64 rows 31.6 /
+// 16.0 / 19.7, 100 rows 33.8 / 25.5 / 20.7, 200 rows 58.4 / 49.4 / 39.8; x 2,048 200 rows 31.6 / 16.0 / 19.5; not gated x 8,192 64 rows
+// 18.6 / 11.3, 100 rows 23.0 / 16.0 / 18.6, x 32,768 24 rows 33.3 / 34.9 / 19.2; K = 192 gated x 8,192 64 rows 31.6 / 23.4 / 24.6, 100 rows 33.8 / 34.1 / 25.4; K = 100 not gated x 8,192 100
+// rows 16.8 / 12.2, gated x 8,192 12 rows 15.9 / 13.7; K = 48 gated x 32,768 4 rows 24.4 / 16.3.
+enum { AS_MANY_INPUTS = 0, GENERAL_FORM = 1, TILES_OF_64 = 2 };
+inline int few_inputs_form(int M, int N, int K, bool gated) {
+    const int64_t blocks = (int64_t)ceil_div(M, 64) * ceil_div(N, 64), sms = sm_count();
+    if (K > 256) return AS_MANY_INPUTS;
+    if (M <= 8) return K < 64 && blocks > sms ? GENERAL_FORM : AS_MANY_INPUTS;
+    if (M <= 16) {
+        const bool whole_stages = K % 64 == 0 || K % 64 > 40;           // (or nearly)
+        return K <= 144 && (blocks > sms || (blocks >= 128 && (K < 64 || !whole_stages))) ? GENERAL_FORM : AS_MANY_INPUTS;
+    }
+    if (K <= slice_len(K)) {
+        if (M <= FEW_MAX) return N > (K <= 100 ? 2048 : 4096) ? GENERAL_FORM : AS_MANY_INPUTS;
+        if (gated) return K < 64 || (blocks > 64 && (K <= 100 || (int64_t)ceil_div(M, 128) * ceil_div(N, 64) < 2 * sms)) ? GENERAL_FORM : AS_MANY_INPUTS;
+        return (blocks > 100 && blocks <= 3 * sms) || (K < 64 && blocks > 64 && blocks <= 4 * sms) ? GENERAL_FORM : AS_MANY_INPUTS;
+    }
+    if (blocks < 64 || (blocks == 64 && K > (gated ? 176 : 144)) || (blocks <= (K > 240 ? 100 : 90) && K > 200)) return AS_MANY_INPUTS;
+    if (gated) {
+        if (blocks <= sms) return GENERAL_FORM;
+        return blocks <= 2 * sms || (blocks < 4 * sms && (K <= 144 || (blocks > 3 * sms && K <= 192))) ? TILES_OF_64 : AS_MANY_INPUTS;
+    }
+    if (blocks <= (K <= 176 ? 2 : 1) * sms) return K <= 240 ? GENERAL_FORM : AS_MANY_INPUTS;
+    return K <= 176 && blocks <= 8 * sms ? TILES_OF_64 : AS_MANY_INPUTS;
 }
 
 template <bool GATED>
-int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int w_static, cudaStream_t s) {
+int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int w_static, int form, cudaStream_t s) {
+    if (form == TILES_OF_64) return gemm_f32_tiles<64, GATED ? 128 : 64, GATED ? 8 : 4, GATED, false>(A, W, C, M, N, K, w_static, s);
     // (few slices leave most warps of the streaming form without work: then tiles, which bring the weights once, from 17 rows on.
-    // us streamed / as tiles, 17 rows, K = 256 x 4,096 10.4 / 9.0, x 32,768 70 / 33, gated x 4,096 17.2 / 14.7; K = 384 x 8,192 18.1 / 20.5)
-    const bool wide = M > 16 && K <= 256 && N >= 4096;
+    // us streamed / as tiles, 17 rows, K = 256 x 4,096 10.4 / 9.0, x 32,768 70 / 33, gated x 4,096 17.2 / 14.7; K = 384 x 8,192 18.1 / 20.5,
+    // x 32,768 66 / 47, gated x 16,384 67 / 52, x 32,768 135 / 89)
+    const bool wide = M > 16 && ((K <= 256 && N >= 4096) || (K <= 384 && N >= (GATED ? 16384 : 32768)));
     if (M <= FEW_MAX && !wide) {
         // (16 outputs a block halve the trips of A's rows; with few outputs 8 a block fill the device)
         if (M <= 2) return gemm_f32_few<2, 1, GATED>(A, W, C, M, N, K, w_static, s);
@@ -379,7 +401,8 @@ int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int 
 
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
-template <typename T, typename TOut, bool GATED>
+// SLICED: the inner dimension's slices are added up as the forms above add them.
+template <typename T, typename TOut, bool GATED, bool SLICED>
 __global__ void __launch_bounds__(256)
 gemm_nt_kernel(const T* __restrict__ A, const T* __restrict__ W, TOut* __restrict__ C, int M, int N, int K) {
     __shared__ float As[BK][BM + 4];
@@ -392,6 +415,9 @@ gemm_nt_kernel(const T* __restrict__ A, const T* __restrict__ W, TOut* __restric
 
     float acc[TM][TN] = {};
     float accu[GATED ? TM : 1][TN] = {};
+    float total[SLICED ? TM : 1][TN], totalu[SLICED && GATED ? TM : 1][TN];
+    const int len = SLICED ? slice_len(K) : 0;
+    int until = len;                                     // where the slice at hand ends
 
     for (int k0 = 0; k0 < K; k0 += BK) {
 #pragma unroll
@@ -422,6 +448,22 @@ gemm_nt_kernel(const T* __restrict__ A, const T* __restrict__ W, TOut* __restric
                     if (GATED) accu[i][j] = fmaf(a[i], u[j], accu[i][j]);
                 }
         }
+        if constexpr (SLICED) {
+            if (k0 + BK == until || k0 + BK >= K) {
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        total[i][j] = until == len ? acc[i][j] : total[i][j] + acc[i][j];
+                        acc[i][j] = 0.f;
+                        if constexpr (GATED) {
+                            totalu[i][j] = until == len ? accu[i][j] : totalu[i][j] + accu[i][j];
+                            accu[i][j] = 0.f;
+                        }
+                    }
+                until += len;
+            }
+        }
         __syncthreads();
     }
 #pragma unroll
@@ -432,8 +474,8 @@ gemm_nt_kernel(const T* __restrict__ A, const T* __restrict__ W, TOut* __restric
         for (int j = 0; j < TN; ++j) {
             const int n = n0 + tx * TN + j;
             if (n >= N) continue;
-            float v = acc[i][j];
-            if (GATED) v = v / (1.0f + expf(-v)) * accu[i][j];
+            float v = SLICED ? total[SLICED ? i : 0][j] : acc[i][j];
+            if (GATED) v = v / (1.0f + expf(-v)) * (SLICED ? totalu[SLICED && GATED ? i : 0][j] : accu[GATED ? i : 0][j]);
             st(C + (int64_t)m * N + n, v);
         }
     }
@@ -444,12 +486,18 @@ int gemm_nt(const void* A, const void* W, void* C, int M, int N, int K, int w_st
     WICK_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm: bad sizes M=%d N=%d K=%d", M, N, K);
     if (M == 0) return 0;
     if constexpr (std::is_same<T, float>::value && std::is_same<TOut, float>::value) {
-        if (K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && M <= 65535 * 64 && !one_slice_general(M, N, K, GATED))
-            return gemm_f32<GATED>((const float*)A, (const float*)W, (float*)C, M, N, K, w_static, s);
+        if (K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && M <= 65535 * 64) {
+            const int form = few_inputs_form(M, N, K, GATED);
+            if (form != GENERAL_FORM) return gemm_f32<GATED>((const float*)A, (const float*)W, (float*)C, M, N, K, w_static, form, s);
+            const dim3 grid(ceil_div(N, BN), ceil_div(M, BM));
+            if (K <= slice_len(K)) gemm_nt_kernel<float, float, GATED, false><<<grid, 256, 0, s>>>((const float*)A, (const float*)W, (float*)C, M, N, K);
+            else gemm_nt_kernel<float, float, GATED, true><<<grid, 256, 0, s>>>((const float*)A, (const float*)W, (float*)C, M, N, K);
+            return check_launch("gemm_simt");
+        }
     }
     dim3 grid(ceil_div(N, BN), ceil_div(M, BM));
     WICK_REQUIRE(grid.y <= 65535, "gemm: M=%d is beyond the grid limit", M);
-    gemm_nt_kernel<T, TOut, GATED><<<grid, 256, 0, s>>>((const T*)A, (const T*)W, (TOut*)C, M, N, K);
+    gemm_nt_kernel<T, TOut, GATED, false><<<grid, 256, 0, s>>>((const T*)A, (const T*)W, (TOut*)C, M, N, K);
     return check_launch("gemm_simt");
 }
 
