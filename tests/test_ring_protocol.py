@@ -33,7 +33,8 @@ class Barrier:
 
 
 # ---------------------------------------------------------------------------
-# The ring of the tcgen05 prompt attention (csrc/attn_prompt_tc.cu): a producer (keys and
+# The ring that the tcgen05 prompt attention had before its blocks took two streams (kept for what it shows
+# about parities): a producer (keys and
 # values of block j into one of six tiles), an issuing thread (scores of up to three blocks
 # ahead, then P V block by block) and the softmax warps.  The producer may fetch the values of
 # block j only when the product of block j - 3 has read its tile.  If it learns that from the
@@ -138,3 +139,205 @@ def test_prompt_attention_ring_on_the_shared_product_barrier_can_stall_a_late_pr
         except AssertionError:
             stalled += 1
     assert stalled > 0
+
+
+# ---------------------------------------------------------------------------
+# The protocol of csrc/attn_prompt_tc.cu: a block works through its items one behind the other; five tiles, two streams of
+# scores, and for each item either two tiles of rows over all key blocks or (split) one tile whose even and odd key blocks are
+# a stream each, joined at the end.  Tensor-core instructions complete in order; copies complete in any order.
+def simulate_two_streams(items, seed):
+    """items: (key blocks, split) of each."""
+    rnd = random.Random(seed)
+    NSLOT, WARPS = 5, 2                                               # (two softmax warps a stream instead of four)
+    full, empty = [Barrier(1) for _ in range(NSLOT)], [Barrier(1) for _ in range(NSLOT)]
+    s_full, o_full = ([Barrier(1) for _ in range(2)] for _ in range(2))
+    p_first, p_full, o_empty = ([Barrier(WARPS) for _ in range(2)] for _ in range(3))
+    q_full, q_empty, join, joined = Barrier(1), Barrier(1), Barrier(2 * WARPS), Barrier(2 * WARPS)
+    tiles, mma, copies = [None] * NSLOT, [], []
+    state = dict(q=None)
+    scores, result = [None, None], [None, None]                       # what S and O of each stream hold: (item, step)
+    first, probs = [{}, {}], [{}, {}]                                 # (item, step) -> warps that have written P
+    read = [dict(), dict()]                                           # item -> warps that have read O
+
+    def place_k(n_blk, split, j):
+        return max(2 * j - 1, 0) if split else 2 * j
+
+    def place_v(n_blk, split, j):
+        return min(2 * j + 2, 2 * n_blk - 1) if split else 2 * j + 1
+
+    def block_of(split, s, t):
+        return 2 * t + s if split else t
+
+    def wait(bar, parity):
+        while not bar.done(parity):
+            yield
+
+    def producer():
+        base = 0
+        for k, (n_blk, split) in enumerate(items):
+            if k:
+                yield from wait(q_empty, (k - 1) & 1)
+            q_full.arrive(tx=1)
+            copies.append(lambda k=k: (state.update(q=k), q_full.complete_tx(1)))
+            for i in range(2 * n_blk):
+                last = split and i == 2 * n_blk - 1
+                is_v = (last or (i > 0 and not i & 1)) if split else bool(i & 1)
+                j = n_blk - 1 if last else (((i - 2) >> 1 if is_v else (i + 1) >> 1) if split else i >> 1)
+                assert i == (place_v if is_v else place_k)(n_blk, split, j)
+                n = base + i
+                if n >= NSLOT:
+                    yield from wait(empty[n % NSLOT], (n // NSLOT - 1) & 1)
+                full[n % NSLOT].arrive(tx=1)
+
+                def land(n=n, what=(k, j, is_v)):
+                    tiles[n % NSLOT] = what
+                    full[n % NSLOT].complete_tx(1)
+                copies.append(land)
+                yield
+            base += 2 * n_blk
+
+    def issuer():
+        base, steps, uses = 0, [0, 0], [0, 0]
+        for k, (n_blk, split) in enumerate(items):
+            def release(n, s):
+                if split or s == 1:
+                    mma.append(lambda: empty[n % NSLOT].arrive())
+
+            def keys_here(s, t):
+                j = block_of(split, s, t)
+                if (split or s == 0) and j < n_blk:
+                    n = base + place_k(n_blk, split, j)
+                    yield from wait(full[n % NSLOT], (n // NSLOT) & 1)
+
+            def issue_s(s, t):
+                j = block_of(split, s, t)
+                n = base + place_k(n_blk, split, j)
+                yield from keys_here(s, t)
+
+                def run():
+                    assert tiles[n % NSLOT] == (k, j, False) and state["q"] == k
+                    assert t == 0 or result[s] == (k, t - 1), "scores over probabilities that are not multiplied yet"
+                    scores[s] = (k, t)
+                    s_full[s].arrive()
+                mma.append(run)
+                release(n, s)
+                if j == n_blk - 1 and (split or s == 1):
+                    mma.append(lambda: q_empty.arrive())
+            yield from wait(q_full, k & 1)
+            for s in range(2):
+                if block_of(split, s, 0) < n_blk:
+                    yield from issue_s(s, 0)
+            t = 0
+            while block_of(split, 0, t) < n_blk:
+                for s in range(2):
+                    j = block_of(split, s, t)
+                    if j >= n_blk:
+                        break
+                    n = base + place_v(n_blk, split, j)
+                    if t == 0 and uses[s]:
+                        yield from wait(o_empty[s], (uses[s] - 1) & 1)
+                    if split or s == 0:
+                        yield from wait(full[n % NSLOT], (n // NSLOT) & 1)
+                    yield from wait(p_first[s], steps[s] & 1)
+
+                    def begin(n=n, j=j, s=s, t=t, k=k, split=split):  # the product of the first keys
+                        assert tiles[n % NSLOT] == (k, j, True) and first[s].get((k, t)) == WARPS
+                        if t == 0 and result[s] is not None:          # the result before has been read by all who read it
+                            kb = result[s][0]
+                            nb, sb = items[kb]
+                            assert read[s].get(kb) == (2 * WARPS if sb and nb > 1 else WARPS), "a result overwritten unread"
+                    mma.append(begin)
+                    yield from wait(p_full[s], steps[s] & 1)
+
+                    def run(n=n, j=j, s=s, t=t, k=k):
+                        assert tiles[n % NSLOT] == (k, j, True) and probs[s].get((k, t)) == WARPS
+                        result[s] = (k, t)
+                    mma.append(run)
+                    release(n, s)
+                    steps[s] += 1
+                    if block_of(split, s, t + 1) < n_blk:
+                        yield from issue_s(s, t + 1)
+                    else:
+                        mma.append(lambda s=s: o_full[s].arrive())
+                        uses[s] += 1
+                    yield
+                t += 1
+            base += 2 * n_blk
+
+    def softmax(s):
+        base, step, uses, joins = 0, 0, [0, 0], 0
+        for k, (n_blk, split) in enumerate(items):
+            ragged = k % 2 == 0
+            t = 0
+            while block_of(split, s, t) < n_blk:
+                yield from wait(s_full[s], step & 1)
+                step += 1
+                assert scores[s] == (k, t) and (t == 0 or result[s] == (k, t - 1))   # (the result may be rescaled here)
+                yield
+                if ragged and block_of(split, s, t) == n_blk - 1 and (split or s == 0):
+                    n = base + place_v(n_blk, split, n_blk - 1)       # the last values' rows beyond the end are zeroed
+                    yield from wait(full[n % NSLOT], (n // NSLOT) & 1)
+                    assert tiles[n % NSLOT] == (k, n_blk - 1, True)
+                first[s][k, t] = first[s].get((k, t), 0) + 1
+                p_first[s].arrive()
+                yield
+                probs[s][k, t] = probs[s].get((k, t), 0) + 1
+                p_full[s].arrive()
+                t += 1
+            base += 2 * n_blk
+            if not split or n_blk == 1:
+                if not split or s == 0:
+                    yield from wait(o_full[s], uses[s] & 1)
+                    assert result[s] == (k, t - 1)
+                    read[s][k] = read[s].get(k, 0) + 1
+                    o_empty[s].arrive()
+                uses[0] += 1
+                uses[1] += 0 if split else 1
+            else:
+                yield from wait(o_full[0], uses[0] & 1)
+                yield from wait(o_full[1], uses[1] & 1)
+                uses = [u + 1 for u in uses]
+                join.arrive()
+                yield from wait(join, joins & 1)
+                for i in range(2):
+                    assert result[i] == (k, (n_blk + 1 - i) // 2 - 1)
+                    read[i][k] = read[i].get(k, 0) + 1
+                joined.arrive()
+                yield from wait(joined, joins & 1)
+                joins += 1
+                o_empty[s].arrive()
+            yield
+
+    threads = [producer(), issuer()] + [softmax(w % 2) for w in range(2 * WARPS)]
+    speed = [rnd.choice([1, 1, 5, 25]) for _ in threads]              # (some are late)
+    alive, idle = list(range(len(threads))), 0
+    while alive:
+        if mma and rnd.random() < 0.4:
+            mma.pop(0)()
+            idle = 0
+        elif copies and rnd.random() < 0.4:
+            copies.pop(rnd.randrange(len(copies)))()
+            idle = 0
+        else:
+            t = rnd.choices(alive, [1 / speed[i] for i in alive])[0]
+            try:
+                next(threads[t])
+            except StopIteration:
+                alive.remove(t)
+                idle = 0
+            idle += 1
+            assert idle < 40000 or mma or copies, "nothing moves"
+
+
+@pytest.mark.parametrize("n_blk", [1, 2, 3, 4, 5, 6, 7, 16, 33])
+@pytest.mark.parametrize("split", [False, True])
+def test_prompt_attention_of_two_streams_always_finishes(n_blk, split):
+    for seed in range(10):
+        simulate_two_streams([(n_blk, split)], seed)
+        simulate_two_streams([(n_blk, split), (1, not split), (n_blk, not split)], seed)
+
+
+def test_prompt_attention_of_two_streams_item_behind_item():
+    for seed in range(60):
+        rnd = random.Random(seed)
+        simulate_two_streams([(rnd.choice([1, 1, 2, 3, 5, 8]), rnd.random() < 0.5) for _ in range(rnd.randint(2, 9))], seed)

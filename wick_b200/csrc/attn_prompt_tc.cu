@@ -1,22 +1,31 @@
 // Causal attention of a step's new tokens over the paged cache on the 5th-
 // generation tensor cores (tcgen05), bfloat16, head sizes 64 and 128.
 //
-// A block takes one query head and 128 consecutive new tokens of one sequence
-// (two of the step's 64-row work items) and walks over the keys in blocks of 128
-// (two cache pages):
+// The 128 rows of a tile are the query heads of one key head times as many consecutive tokens as
+// fit: 4 heads to a key head make 32 tokens, 5 make 25 (125 rows), 1 makes 128 (one TMA box of
+// heads x tokens either way).  A block runs two streams over blocks of 128 keys (two cache pages),
+// each with its own scores and its own result in tensor memory and four softmax warps:
+//   * two tiles of neighbouring tokens over all key blocks (a key or value tile is read twice), or
+//   * where the step is too small for that to fill the device, or the second tile has no tokens,
+//     ONE tile, even key blocks in one stream and odd ones in the other, joined at the end.
 //   * a producer thread fetches the query rows once and the key and value pages
-//     through a ring of six tiles (TMA, 64 x 64 boxes, 128-byte swizzle); a key
-//     tile is free again as soon as its scores are computed;
-//   * an issuing thread computes S = Q K^T into one of three 128-column buffers
-//     of tensor memory, up to three blocks ahead of the softmax, and accumulates
-//     O += P V (the values are the MN-major operand: their rows are keys);
-//   * eight warps own one query row per pair of threads (64 keys of a block each;
-//     the row's maximum crosses through shared memory): they read S from tensor
-//     memory, scale, mask (a key is visible up to the token's own position), and
-//     write P as pairs of bfloat16 back into tensor memory over the scores it
-//     came from, where the second product takes it from.  With three buffers the
-//     softmax of the next block never waits for a product: what bounds a block
-//     is the 16 instructions the tensor core takes for it (one every ~93 clocks).
+//     through a ring of five tiles (TMA, 64 x 64 boxes, 128-byte swizzle);
+//   * an issuing thread alternates between the streams: O += P V of one (the values are the
+//     MN-major operand: their rows are keys), the scores S = Q K^T of its next key block, then
+//     the other stream's, so that one stream's softmax runs beside the other's products;
+//   * a softmax thread owns a row of its stream: it reads 128 scores from tensor memory, scales,
+//     masks (a key is visible up to the token's own position), and writes P as pairs of bfloat16
+//     over the scores, where the second product takes it from.  The next scores overwrite P:
+//     tensor-core instructions of one thread execute in order.  That a stream's scores of step t + 1
+//     are complete therefore also says that its product of step t is.
+// A block an SM works through its items one behind the other: the next item's tiles and scores are under way during the
+// last one's epilogue.
+// What bounds it: a tile and key block take the tensor core 1,024 clocks (16 instructions of 64) and the
+// exponentials as many; a stream's chain of softmax (1,830 clocks), product, scores and the waits between them takes ~3,400 clocks for
+// both streams' blocks.  Before (a tile of one head's rows a block, two threads a row, one lane issuing) / now, us:
+// 2,048 tokens, 32 heads over 8 69 -> 43, 8,192 tokens 625 -> 453 (1.2 PFLOP/s); 16 prompts of 64 to 2,048 tokens, 40 over 8
+// 717 -> 529; 1,419 tokens behind 3,100 124 -> 105; 8 x 1,024, 64 over 8 336 -> 189; 64 tokens 7.2 -> 8.7 behind itself, but in a step,
+// where its start overlaps the kernel before, no longer than before.
 // O and the sum are scaled by a maximum that follows the true running maximum
 // lazily: only when a block's maximum exceeds it by more than 8 (in units of
 // log2 e) is O rescaled in tensor memory, so that after the first blocks of a row
@@ -28,6 +37,8 @@
 // window, each as one key and value (tiles of 64 blocks a sequence, laid out like cache
 // pages; their key blocks come before the window's), soft-caps the scores and multiplies
 // the result by a number per token and head.
+// Work items are dealt longest first (see find_longest_item): neighbouring block indexes are the key heads
+// of one item.
 // Every wait is bounded and reports through the status word.
 // Formulas: wick src/model.rs:520-553.  The plain forms of this computation are
 // attn_prompt_mma_kernel (attn_prompt_mma.cu) and attn_prompt_kernel (attn.cu).
@@ -48,30 +59,42 @@ namespace prompttc {
 
 constexpr bool SUPPORTED = WICK_HD == 64 || WICK_HD == 128;
 constexpr int HD = SUPPORTED ? WICK_HD : 64;           // other head sizes: the entry point refuses, the kernel is never launched
-constexpr int BQ = 128;                                // query rows of a block
+constexpr int BQ = 128;                                // rows of a tile
 constexpr int BK = 128;                                // keys of an inner step (two pages)
 constexpr int PANELS = HD / 64;                        // 64-column panels of a head row
 constexpr int PANEL_BYTES = 128 * 128;                 // 128 rows of 128 bytes
-constexpr int TILE_BYTES = PANELS * PANEL_BYTES;       // Q, or one block of keys or of values
-constexpr int NSLOT = 6;                               // key / value tiles in flight: 2 per score buffer (the ring of
-                                                       // tiles and the ring of score buffers turn together)
-constexpr int SMEM_BYTES = TILE_BYTES + NSLOT * TILE_BYTES + 1024;
-constexpr int THREADS = 320;                           // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-9: softmax
-constexpr int NBUF = 3;                                // score buffers
-static_assert(NSLOT == 2 * NBUF, "a tile slot is free when the scores (the product) of three blocks before are done");
-constexpr int HALF_K = BK / 2;                         // keys of a block that one softmax thread handles
-constexpr uint32_t TMEM_COLS = 512;                    // S0 | S1 | S2 | O; P (bfloat16 pairs) takes the place of the
-constexpr uint32_t COL_S = 0, COL_O = NBUF * BK;       // first 64 columns of the S buffer it was computed from
+constexpr int TILE_BYTES = PANELS * PANEL_BYTES;       // a tile of Q, or one block of keys or of values
+constexpr int LONG = 4;                                // key blocks of an item from which on its softmax is written out (8,192 tokens: 537 us looped, 453)
+constexpr int P_FIRST = 64;                            // keys of a block whose probabilities the product begins with
+constexpr int NSLOT = 5;                               // key / value tiles in flight
+constexpr int MAX_ITEMS = 16;                          // work items of a block
+// A work item: the sequence (-1: none), its place, new and cached tokens; the item's first token; the heads; key blocks.
+struct Item {
+    int b, tok0, q_len, start, q0, kvh, head0;
+    int jb0, n_pool, n_blk;                            // first block of keys; of the item's n_blk, those of blocks of positions
+    int split;                                         // one tile, its key blocks dealt to both streams
+    // Tiles come through the ring in the order in which the issuing thread uses them: K0 V0 K1 V1 ..., or, split,
+    // K0 K1 V0 K2 V1 K3 ... V(n-2) V(n-1): an item's 2 n_blk tiles, and the place of block j's values among them.
+    __device__ __forceinline__ int place_v(int j) const { return split ? min(2 * j + 2, 2 * n_blk - 1) : 2 * j + 1; }
+    __device__ __forceinline__ int block_of(int s, int t) const { return split ? 2 * t + s : t; }    // step t of stream s
+};
+// Behind the tiles in shared memory (which begins on a multiple of 1,024 bytes, and has no room for a shift):
+struct Shared {
+    float ml[2][2][BQ];                                // the streams' maxima and sums, where they share rows
+    uint64_t q_full, q_empty, full[NSLOT], empty[NSLOT], s_full[2], p_full[2][2], o_full[2], o_empty[2], join, joined;
+    Item items[MAX_ITEMS];
+    uint32_t tmem_slot;
+    int abort_flag;
+};
+constexpr int SMEM_BYTES = (2 + NSLOT) * TILE_BYTES + (int)sizeof(Shared);
+static_assert(SMEM_BYTES <= 227 * 1024, "a block's shared memory");
+constexpr int THREADS = 320;                           // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5 and 6-9: softmax
+constexpr uint32_t TMEM_COLS = 512;                    // S of both streams | O of both; P (bfloat16 pairs) takes the place of
+constexpr uint32_t COL_S = 0, COL_O = 2 * BK;          // the first 64 columns of the S it was computed from
 typedef __nv_bfloat16 bf16;
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// Two barriers at once (their polls overlap).
-__device__ __forceinline__ bool mbar_wait2(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, volatile int* abort_flag, int* status, int code) {
-    const bool ra = mbar_try_wait(a, pa), rb = mbar_try_wait(b, pb);
-    if (ra && rb) return true;
-    return (ra || mbar_wait(a, pa, abort_flag, status, code)) && (rb || mbar_wait(b, pb, abort_flag, status, code));
 }
 __device__ __forceinline__ void tc_ld32_nowait(uint32_t taddr, uint32_t* r) {
     asm volatile(
@@ -94,6 +117,13 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t* r) {
           "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // The issuing thread is one thread: what it computes per instruction is what limits
 // the rate of small products.  A shared-memory descriptor is therefore kept as two
@@ -105,6 +135,11 @@ __device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo_bytes) {
 // stride offset 1024 bytes (8 rows of 128 bytes), descriptor version 1 (bit 46), 128-byte swizzle (bits 61-63)
 constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 
+__device__ __forceinline__ bool elect_one() {                   // true in one lane of a whole warp
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // D (tensor memory) (+)= A (shared memory) * B (shared memory)
 template <int ACC>
 __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
@@ -118,14 +153,13 @@ __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t 
         : "memory");
 }
 // D (tensor memory) (+)= A (tensor memory: 128 lanes x 8 columns of bfloat16 pairs) * B (shared memory)
-template <int ACC>
-__device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc) {
+__device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, int acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
         "mov.b64 db, {%2, %3};\n\t"
         "setp.ne.b32 p, %5, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(DESC_HI), "r"(idesc), "n"(ACC)
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(DESC_HI), "r"(idesc), "r"(acc)
         : "memory");
 }
 template <int I, int N, typename F>
@@ -139,6 +173,12 @@ __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+__device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, uint64_t* bar, void* dst, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
 }
 // The softmax warps are bound by the number of instructions they issue: two products-and-sums,
 // two sums, or a maximum of three per instruction where sm_100 has one.
@@ -205,339 +245,599 @@ __device__ __forceinline__ float rcp(float x) {
     return y;
 }
 
+// Work items of R tokens, longest first: all items of the step in falling order of the key block that their first
+// token lies in (items of one sequence that share it, and sequences, in index order); this finds the item at place `rank`.
+// A warp takes the sequences 32 at a time (the first 32 are kept in registers); the key block is found by bisection over counts
+// (9 steps for 40,960 positions; one sequence needs none).
+struct Finder {
+    const int *cu_seqlens, *start_arr;
+    int n_seqs, R, tok0, q_len, start, top;                        // (lane l: sequence l; top: no item lies in this key block or beyond)
+    __device__ __forceinline__ Finder(const int* cu, const int* st, int n, int r) : cu_seqlens(cu), start_arr(st), n_seqs(n), R(r) {
+        const int s = threadIdx.x & 31;
+        tok0 = s < n ? cu[s] : 0;
+        q_len = s < n ? cu[s + 1] - tok0 : 0;
+        start = s < n ? st[s] : 0;
+        int t = (start + q_len) / BK + 1;
+#pragma unroll 1
+        for (int i = s + 32; i < n; i += 32) t = max(t, (st[i] + cu[i + 1] - cu[i]) / BK + 1);
+        top = (int)__reduce_max_sync(0xffffffffu, t);
+    }
+    // items of this lane's sequence of the chunk at s0, and those of them whose first token lies in key block k or a later one
+    __device__ __forceinline__ int items(int s0) const {
+        const int s = s0 + (int)(threadIdx.x & 31), n = s0 == 0 ? q_len : (s < n_seqs ? cu_seqlens[s + 1] - cu_seqlens[s] : 0);
+        return (n + R - 1) / R;
+    }
+    __device__ __forceinline__ int from(int s0, int n, int k) const {
+        const int s = s0 + (int)(threadIdx.x & 31), before = k * BK - (s0 == 0 ? start : (s < n_seqs ? start_arr[s] : 0));
+        return before > 0 ? max(0, n - (before + R - 1) / R) : n;
+    }
+    __device__ __forceinline__ int count(int k) const {
+        int c = 0;
+#pragma unroll 1
+        for (int s0 = 0; s0 < n_seqs; s0 += 32) c += from(s0, items(s0), k);
+        return (int)__reduce_add_sync(0xffffffffu, c);
+    }
+    // (every lane gets the item)
+    __device__ __forceinline__ Item find(int rank) const {
+        Item it;
+        it.b = -1;
+        int lo = 0, hi = top, above = 0;
+        if (n_seqs == 1) {
+            const int n = (__shfl_sync(0xffffffffu, q_len, 0) + R - 1) / R;
+            if (rank < n) it.b = 0, it.q0 = (n - 1 - rank) * R;
+        } else if (count(0) > rank) {
+#pragma unroll 1
+            while (hi - lo > 1) {                                  // count(lo) > rank >= count(hi) = above
+                const int mid = (lo + hi) >> 1, c = count(mid);
+                if (c > rank) lo = mid;
+                else hi = mid, above = c;
+            }
+            int left = rank - above;                               // place among the items of key block lo
+#pragma unroll 1
+            for (int s0 = 0; s0 < n_seqs; s0 += 32) {
+                const int all = items(s0), later = from(s0, all, lo + 1), n = from(s0, all, lo) - later;
+                int upto = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, upto, o);
+                    if ((int)(threadIdx.x & 31) >= o) upto += t;
+                }
+                const int total = __shfl_sync(0xffffffffu, upto, 31);
+                if (left < total) {
+                    const int l = __ffs(__ballot_sync(0xffffffffu, left < upto)) - 1;
+                    it.b = s0 + l;                                 // (all - later - n: the sequence's first item in lo)
+                    it.q0 = (__shfl_sync(0xffffffffu, all - later - upto, l) + left) * R;
+                    break;
+                }
+                left -= total;
+            }
+        }
+        if (it.b >= 0) {
+            if (it.b < 32) {
+                it.tok0 = __shfl_sync(0xffffffffu, tok0, it.b);
+                it.q_len = __shfl_sync(0xffffffffu, q_len, it.b);
+                it.start = __shfl_sync(0xffffffffu, start, it.b);
+            } else {
+                it.tok0 = cu_seqlens[it.b], it.q_len = cu_seqlens[it.b + 1] - it.tok0, it.start = start_arr[it.b];
+            }
+        }
+        return it;
+    }
+};
+
+// What follows from an item's place: `column` counts the step's tiles of heads.
+__device__ __forceinline__ void complete(Item& it, int column, int per_kv, int gs, int T, int tiles, int mask, int mask_size, int block) {
+    const int kv_len = it.start + it.q_len;
+    it.kvh = per_kv == 1 ? column : column / per_kv;                // (a group of more than 128 heads: several tiles of heads)
+    it.head0 = column * gs;
+    it.split = tiles == 1 || it.q0 + T >= it.q_len;
+    const int last_key = min(it.start + it.q0 + (it.split ? T : 2 * T) - 1, kv_len - 1);   // the last position any row of the item may see
+    // With a mask the first block of keys is the one that holds the first row's first visible key (the first
+    // visible key grows with the position); blocks are counted from there, j = 0 .. n_blk - 1, everywhere below.
+    it.jb0 = first_visible_key(it.start + it.q0, mask, mask_size) / BK;
+    // (EXTRA: the first n_pool key blocks hold blocks of positions; block j >= n_pool holds the keys from (j - n_pool + jb0) BK on)
+    it.n_pool = block > 0 ? (blocks_seen(last_key, mask_size, block) + BK - 1) / BK : 0;
+    it.n_blk = last_key / BK + 1 - it.jb0 + it.n_pool;
+}
+
 template <bool EXTRA>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                       bf16* __restrict__ out, const int* __restrict__ cu_seqlens, int n_seqs,
                       const int* __restrict__ start_arr,
-                      const int* __restrict__ page_table, int table_width, int n_tiles, int n_heads, int n_kv,
+                      const int* __restrict__ page_table, int table_width, int n_heads, int n_kv, int gs, int T, int columns, int per_kv, int tiles, int n_items,
                       float scale, int* status, int mask, int mask_size, const float* __restrict__ sink,
                       const __grid_constant__ CUtensorMap pool_map, const TcExtra X) {
-    extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t q_full, full[NSLOT];
-    __shared__ uint64_t s_full[NBUF], p_full[NBUF], pv_done[2], v_free[NBUF], x_bar[4];   // pv_done: even blocks, odd blocks
-    __shared__ bf16 mx_x[2][2][BQ];                            // the maxima the two halves of a row tell each other
-    __shared__ uint32_t tmem_slot;
-    __shared__ int abort_flag;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* q_s = smem_raw;                                       // two tiles of queries
+    uint8_t* kv_s = q_s + 2 * TILE_BYTES;                          // NSLOT tiles: keys and values of the blocks in flight
+    Shared& sh = *reinterpret_cast<Shared*>(kv_s + NSLOT * TILE_BYTES);
+    volatile int* abort_flag = &sh.abort_flag;
 
     pdl_trigger();
-    // longest first: the last work items of a sequence see the most keys
+    if (smem_u32(smem_raw) & 1023) {                               // (cannot be, see Shared)
+        if (threadIdx.x == 0) atomicCAS(status, 0, 7);
+        return;
+    }
     // (the step's description is written by the host before the step: no kernel produces it)
-    int b, q0;
-    find_work_item(cu_seqlens, n_seqs, 64, n_tiles - 1 - (int)blockIdx.x, b, q0);
-    if (b < 0 || q0 % BQ != 0) return;                             // the odd 64-row item belongs to its even neighbour's block
-    const int head = blockIdx.y, kvh = head / (n_heads / n_kv);
-    const int tok0 = cu_seqlens[b], q_len = cu_seqlens[b + 1] - tok0, start = start_arr[b];
-    const int kv_len = start + q_len;
-    const int rows = min(BQ, q_len - q0);
-    const int last_key = min(start + q0 + BQ - 1, kv_len - 1);     // the last position any row of the block may see
-    // With a mask the first block of keys is the one that holds the first row's first visible key (the first
-    // visible key grows with the position); blocks are counted from there, j = 0 .. n_blk - 1, everywhere below.
-    const int jb0 = first_visible_key(start + q0, mask, mask_size) / BK;
-    // (EXTRA: the first n_pool key blocks hold blocks of positions; block j >= n_pool holds the keys from (j + jw) BK on)
-    const int n_pool = EXTRA ? (blocks_seen(last_key, mask_size, X.block) + BK - 1) / BK : 0;
-    const int jw = jb0 - n_pool;
-    const int n_blk = last_key / BK + 1 - jw;
-
+    const int rows = T * gs;                                       // of a tile: T tokens times gs heads
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* q_s = base;
-    uint8_t* kv_s = q_s + TILE_BYTES;                              // NSLOT tiles: keys and values of the blocks in flight
+    // Item k of the block is the one at place(k) of all, the key heads of one item side by side, in falling order of length, dealt
+    // to and fro over the blocks.
+    auto place = [&](int k) { return k * (int)gridDim.x + (k & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x); };
 
     if (threadIdx.x == 0) {
-        abort_flag = 0;
-        mbar_init(&q_full, 1);
-        for (int s = 0; s < NSLOT; ++s) mbar_init(&full[s], 1);
-        for (int i = 0; i < NBUF; ++i) {
-            mbar_init(&s_full[i], 1);
-            // One arrival per softmax warp; a barrier per score buffer, since a warp may be up to
-            // two blocks ahead of another (never three: the scores of block j + 3 wait for P V of block j).
-            mbar_init(&p_full[i], 8);
+        sh.abort_flag = 0;
+        mbar_init(&sh.q_full, 1), mbar_init(&sh.q_empty, 1);
+        for (int i = 0; i < NSLOT; ++i) mbar_init(&sh.full[i], 1), mbar_init(&sh.empty[i], 1);
+        // Every waiter below sees every phase of the barrier it waits on, so that a parity is never ambiguous
+        // (full as seen by the softmax warps: see there).
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sh.s_full[i], 1), mbar_init(&sh.o_full[i], 1), mbar_init(&sh.o_empty[i], 4);
+            mbar_init(&sh.p_full[i][0], 4), mbar_init(&sh.p_full[i][1], 4);
         }
-        mbar_init(&pv_done[0], 1);
-        mbar_init(&pv_done[1], 1);
-        for (int i = 0; i < NBUF; ++i) mbar_init(&v_free[i], 1);
-        for (int i = 0; i < 4; ++i) mbar_init(&x_bar[i], 2);       // the two warps that share 32 rows
+        mbar_init(&sh.join, 8), mbar_init(&sh.joined, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == 0 && lane < 2 + (int)EXTRA) {
+        const CUtensorMap* map = lane == 0 ? &q_map : (lane == 1 ? &kv_map : &pool_map);
+        asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+    }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_slot)), "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (rows < BQ) {                                               // rows of the tiles that no query fills
+#pragma unroll 1
+        for (int i = threadIdx.x; i < 2 * PANELS * (BQ - rows) * 8; i += THREADS) {
+            const int panel = i / ((BQ - rows) * 8), at = i % ((BQ - rows) * 8);
+            *reinterpret_cast<uint4*>(q_s + panel * PANEL_BYTES + rows * 128 + at * 16) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    {
+        const Finder finder(cu_seqlens, start_arr, n_seqs, T * tiles);
+#pragma unroll 1
+        for (int k = warp; k < MAX_ITEMS; k += THREADS / 32) {      // (a warp each, up to the first that is none)
+            const int at = place(k);
+            Item it;
+            it.b = -1;
+            const int rank = at / columns;
+            if (rank < n_items) it = finder.find(rank);
+            if (it.b >= 0) complete(it, at - rank * columns, per_kv, gs, T, tiles, mask, mask_size, EXTRA ? X.block : 0);
+            if (lane == 0) sh.items[k] = it;
+            if (it.b < 0) break;
+        }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
-    pdl_wait();                                                    // q and the cache come from the kernel before this one
+    const uint32_t tmem = sh.tmem_slot;
+    // (item k, if there is one; the items of a block come in order, and none follows the first that is none)
+    auto any = [&](int k) { return k < MAX_ITEMS && sh.items[k].b >= 0; };
 
-    if (warp == 0) {
-        // ---------------- producer ----------------
-        // Items in order K_0, V_0, K_1, V_1, ...; item i lives in slot i % NSLOT.
-        if (lane == 0) {
-            mbar_expect_tx(&q_full, TILE_BYTES);
-            for (int pn = 0; pn < PANELS; ++pn) tma_load_2d(&q_map, &q_full, q_s + pn * PANEL_BYTES, head * HD + pn * 64, tok0 + q0);
-            for (int i = 0; i < 2 * n_blk; ++i) {
-                const int slot = i % NSLOT, j = i >> 1, is_v = i & 1;
-                // The slot held the keys (values) of block j - 3: free when that block's scores are
-                // computed (its P V product is complete), which is what s_full (v_free) says.  Each
-                // of these barriers completes one phase per visit of this thread, and its next phase
-                // needs the tile that is fetched after the wait: it can never be two phases on, which
-                // a parity could not tell from none.  (pv_done, which alternate blocks share, could:
-                // nothing holds the last two products back while this thread is late.)
-                if (j >= NBUF) {
-                    const int jp = j - NBUF;
-                    if (!mbar_wait(is_v ? &v_free[jp % NBUF] : &s_full[jp % NBUF], (jp / NBUF) & 1, &abort_flag, status, 7)) break;
-                }
-                mbar_expect_tx(&full[slot], TILE_BYTES);
-                if (EXTRA && j < n_pool) {
-                    for (int w = 0; w < 2; ++w) {
-                        const int page = b * X.pool_tiles + min(2 * j + w, X.pool_tiles - 1);
+    if (warp < 2) {
+        if (warp == 0) {
+            // ---------------- producer ----------------
+            // A lane holds a page number of each of two runs of 32 (read ahead, so that a copy never waits for one).
+            const bool one = elect_one();
+            bool ok = true;
+            int slot = 0, turn = 0;                                // of the ring
+#pragma unroll 1
+            for (int k = 0; ok && any(k); ++k) {
+                const Item& w = sh.items[k];
+                const int n_blk = w.n_blk, n_pool = w.n_pool, kvh = w.kvh;
+                const bool split = w.split;
+                auto pages = [&](int run) {
+                    const int at = 2 * w.jb0 + run * 32 + lane;
+                    return at < table_width ? page_table[(int64_t)w.b * table_width + at] : 0;
+                };
+                int even = pages(0), odd = pages(1);
+                if (k == 0) pdl_wait();                            // q and the cache come from the kernel before this one
+                else ok = __all_sync(0xffffffffu, mbar_wait(&sh.q_empty, (k - 1) & 1, abort_flag, status, 7));
+                if (!ok) break;
+                if (one) {
+                    const int n_q = w.split ? 1 : 2;
+                    mbar_expect_tx(&sh.q_full, n_q * PANELS * rows * 128);
+#pragma unroll 1
+                    for (int i = 0; i < n_q; ++i)
                         for (int pn = 0; pn < PANELS; ++pn)
-                            tma_load_2d(&pool_map, &full[slot], kv_s + slot * TILE_BYTES + pn * PANEL_BYTES + w * (kPage * 128), pn * 64,
-                                        ((page * 2 + is_v) * n_kv + kvh) * kPage);
-                    }
-                    continue;
+                            tma_load_3d(&q_map, &sh.q_full, q_s + i * TILE_BYTES + pn * PANEL_BYTES, pn * 64, w.head0, w.tok0 + w.q0 + i * T);
                 }
-                for (int w = 0; w < 2; ++w) {
-                    const int idx = 2 * (j + jw) + w;
-                    const int page = idx < table_width ? page_table[(int64_t)b * table_width + idx] : 0;
-                    for (int pn = 0; pn < PANELS; ++pn)
-                        tma_load_2d(&kv_map, &full[slot], kv_s + slot * TILE_BYTES + pn * PANEL_BYTES + w * (kPage * 128), pn * 64,
-                                    ((page * 2 + is_v) * n_kv + kvh) * kPage);
+#pragma unroll 1
+                for (int i = 0; i < 2 * n_blk; ++i) {
+                    const bool last = split && i == 2 * n_blk - 1;    // (split: the last two tiles are values, or the first keys and values)
+                    const int is_v = split ? (last || (i > 0 && !(i & 1))) : (i & 1);
+                    const int j = last ? n_blk - 1 : (split ? (is_v ? (i - 2) >> 1 : (i + 1) >> 1) : i >> 1);
+                    if (turn > 0 && !__all_sync(0xffffffffu, mbar_wait(&sh.empty[slot], (turn - 1) & 1, abort_flag, status, 7))) {
+                        ok = false;
+                        break;
+                    }
+                    const bool pooled = EXTRA && j < n_pool;
+                    const int at = 2 * (j - n_pool);             // the key block's first page of those from 2 jb0 on
+                    int page0, page1;
+                    if (pooled) {
+                        page0 = w.b * X.pool_tiles + min(2 * j, X.pool_tiles - 1);
+                        page1 = w.b * X.pool_tiles + min(2 * j + 1, X.pool_tiles - 1);
+                    } else {
+                        const int held = (at >> 5) & 1 ? odd : even;
+                        page0 = __shfl_sync(0xffffffffu, held, at & 31);
+                        page1 = __shfl_sync(0xffffffffu, held, (at + 1) & 31);
+                        if (is_v && at >= 32 && (at & 31) == 0) {  // (keys and values have left the run before)
+                            if ((at >> 5) & 1) even = pages((at >> 5) + 1);
+                            else odd = pages((at >> 5) + 1);
+                        }
+                    }
+                    if (one) {
+                        mbar_expect_tx(&sh.full[slot], TILE_BYTES);
+                        uint8_t* dst = kv_s + slot * TILE_BYTES;
+#pragma unroll 1
+                        for (int h = 0; h < 2; ++h)
+                            for (int pn = 0; pn < PANELS; ++pn)
+                                tma_load_2d(pooled ? &pool_map : &kv_map, &sh.full[slot], dst + pn * PANEL_BYTES + h * (kPage * 128), pn * 64,
+                                            (((h ? page1 : page0) * 2 + is_v) * n_kv + kvh) * kPage);
+                    }
+                    if (++slot == NSLOT) slot = 0, ++turn;
+                    __syncwarp();
                 }
             }
-        }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        // Block j: scores in S[j % 3], all blocks accumulate into the one O.
-        // (Measured on this part: the tensor core takes an instruction of this kind every
-        // ~93 clocks at best, whatever its width up to N = 128; 16 of them make a block.)
-        if (lane == 0) {
+        } else {
+            // ---------------- MMA issuer ----------------
+            // The whole warp walks through the steps and one elected lane issues: what an instruction needs stays in uniform
+            // registers.  (A branch of one lane needs tens of instructions for each, beside softmax warps that compete for
+            // the same scheduler: 86 to 146 clocks per instruction instead of the tensor core's 64.)
             // kind::f16, bfloat16 operands, float32 accumulator, M = 128
             const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BK >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
             const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
-            const uint32_t q_lo = desc_lo(smem_u32(q_s), 16);
+            const uint32_t q_lo0 = desc_lo(smem_u32(q_s), 16);
             const uint32_t k_lo0 = desc_lo(smem_u32(kv_s), 16), v_lo0 = desc_lo(smem_u32(kv_s), PANEL_BYTES);
-            auto issue_s = [&](int j) -> bool {
-                const int i = 2 * j, slot = i % NSLOT, buf = j % NBUF;
-                if (!mbar_wait(&full[slot], (i / NSLOT) & 1, &abort_flag, status, 7)) return false;
-                tc_fence_after();
-                const uint32_t k_lo = k_lo0 + slot * (TILE_BYTES >> 4), d = tmem + COL_S + buf * BK;
-                static_for<0, HD / 16>([&](auto ks) {
-                    constexpr uint32_t off = (((int)ks >> 2) * PANEL_BYTES + ((int)ks & 3) * 32) >> 4;
-                    mma_ss<((int)ks > 0)>(d, q_lo + off, k_lo + off, idesc_s);
-                });
-                tc_commit(&s_full[buf]);                                     // (also: the keys are read)
-                return true;
+            const bool one = elect_one();
+            bool ok = true;
+            int slot = 0, turn = 0;                                // of the ring
+            int steps0 = 0, steps1 = 0, uses0 = 0, uses1 = 0;      // steps and items of each stream so far
+            // the next tile of the ring, when it has come
+            auto take = [&](int& at) {
+                at = slot;
+                const bool here = __all_sync(0xffffffffu, mbar_wait(&sh.full[slot], turn & 1, abort_flag, status, 7));
+                if (++slot == NSLOT) slot = 0, ++turn;
+                return here;
             };
-            bool ok = mbar_wait(&q_full, 0, &abort_flag, status, 7);
-            for (int j = 0; j < NBUF && j < n_blk && ok; ++j) ok = issue_s(j);
-            for (int j = 0; j < n_blk && ok; ++j) {
-                const int i = 2 * j + 1, slot = i % NSLOT;
-                ok = ok && mbar_wait2(&p_full[j % NBUF], (j / NBUF) & 1, &full[slot], (i / NSLOT) & 1, &abort_flag, status, 7);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t v_lo = v_lo0 + slot * (TILE_BYTES >> 4), d = tmem + COL_O, pa = tmem + COL_S + (j % NBUF) * BK;
-                if (j > 0) mma_ts<1>(d, pa, v_lo, idesc_o);
-                else mma_ts<0>(d, pa, v_lo, idesc_o);
-                static_for<1, BK / 16>([&](auto ks) { mma_ts<1>(d, pa + (int)ks * 8, v_lo + (int)ks * (2048 >> 4), idesc_o); });
-                tc_commit(&pv_done[j & 1]);
-                tc_commit(&v_free[j % NBUF]);                                // the values are read: their tile is free
-                if (j + NBUF < n_blk) {
-                    // the scores of block j + 3 go where this block's P lies: only when it has been read
-                    ok = mbar_wait(&pv_done[j & 1], (j >> 1) & 1, &abort_flag, status, 7) && issue_s(j + NBUF);
+#pragma unroll 1
+            for (int k = 0; ok && any(k); ++k) {
+                const int n_blk = sh.items[k].n_blk;
+                const bool split = sh.items[k].split;
+                auto block_of = [&](int s, int t) { return split ? 2 * t + s : t; };
+                int k_at = 0, v_at = 0;                            // where the keys and values at hand lie (both streams read a tile, or one)
+                ok = __all_sync(0xffffffffu, mbar_wait(&sh.q_full, k & 1, abort_flag, status, 7));
+                // Turn t of stream s: the product of its step t, the scores of step t + 1.  Long items take the form in which the streams
+                // are told apart when the kernel is built (8,192 tokens: 537 us in the other, 453), short ones the shorter code.
+                auto turn = [&](auto form, int s, int t) {
+                    constexpr int UNROLL = decltype(form)::value;
+                    const int steps = s == 0 ? steps0 : steps1, uses = s == 0 ? uses0 : uses1;
+                    const bool more = block_of(s, t + 1) < n_blk;
+                    if (block_of(s, t) >= n_blk) return;
+                    if (t >= 0) {
+                        if (split || s == 0) ok = take(v_at);
+                        // (the result of the stream's item before has been read)
+                        if (ok && t == 0 && uses > 0) ok = __all_sync(0xffffffffu, mbar_wait(&sh.o_empty[s], (uses - 1) & 1, abort_flag, status, 7));
+                        const uint32_t v_lo = v_lo0 + v_at * (TILE_BYTES >> 4), d = tmem + COL_O + s * HD, pa = tmem + COL_S + s * BK;
+#pragma unroll UNROLL
+                        for (int part = 0; part < 2; ++part) {
+                            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&sh.p_full[s][part], steps & 1, abort_flag, status, 7));
+                            if (!ok) break;
+                            tc_fence_after();
+                            const uint32_t pp = pa + part * (P_FIRST / 2), vp = v_lo + part * (P_FIRST / 16) * (2048 >> 4);
+                            if (one) {
+                                mma_ts(d, pp, vp, idesc_o, t > 0 || part > 0);
+                                static_for<1, P_FIRST / 16>([&](auto ks) { mma_ts(d, pp + (int)ks * 8, vp + (int)ks * (2048 >> 4), idesc_o, 1); });
+                            }
+                        }
+                        if (!ok) return;
+                        if (one) {
+                            if (split || s == 1) tc_commit(&sh.empty[v_at]);   // a tile is free behind its last reader
+                            if (!more) tc_commit(&sh.o_full[s]);
+                        }
+                        if (s == 0) ++steps0, uses0 += more ? 0 : 1;
+                        else ++steps1, uses1 += more ? 0 : 1;
+                    }
+                    if (more) {
+                        if (split || s == 0) ok = take(k_at);
+                        if (!ok) return;
+                        tc_fence_after();
+                        const uint32_t k_lo = k_lo0 + k_at * (TILE_BYTES >> 4), q_lo = q_lo0 + (split ? 0 : s * (TILE_BYTES >> 4));
+                        const uint32_t d = tmem + COL_S + s * BK;
+                        if (one) {
+                            static_for<0, HD / 16>([&](auto ks) {
+                                constexpr uint32_t off = (((int)ks >> 2) * PANEL_BYTES + ((int)ks & 3) * 32) >> 4;
+                                mma_ss<((int)ks > 0)>(d, q_lo + off, k_lo + off, idesc_s);
+                            });
+                            tc_commit(&sh.s_full[s]);
+                            if (split || s == 1) {
+                                tc_commit(&sh.empty[k_at]);
+                                if (block_of(s, t + 1) == n_blk - 1) tc_commit(&sh.q_empty);   // (the item's last scores)
+                            }
+                        }
+                    }
+                    __syncwarp();
+                };
+                if (n_blk >= LONG) {
+#pragma unroll 1
+                    for (int t = -1; ok && block_of(0, t) < n_blk; ++t) {
+                        turn(std::integral_constant<int, 2>{}, 0, t);
+                        if (ok) turn(std::integral_constant<int, 2>{}, 1, t);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int i = -2; ok && block_of(0, i >> 1) < n_blk; ++i) turn(std::integral_constant<int, 1>{}, i & 1, i >> 1);
                 }
             }
         }
     } else {
-        // ---------------- softmax: a query row per pair of threads ----------------
-        // Warps 2-5 take keys 0-63 of a block, warps 6-9 keys 64-127 of the same rows
-        // (a warp reads the 32 lanes of tensor memory given by its index modulo 4).
-        const int quad = warp & 3, half = (warp - 2) >> 2;
-        const int r = quad * 32 + lane;
-        const int c_lo = half * HALF_K;
-        const int q_pos = start + q0 + r;
-        const int limit = min(q_pos, kv_len - 1);                   // last visible key position
-        const int vis = first_visible_key(limit, mask, mask_size);  // first visible key position
+        // ---------------- softmax: a row per thread ----------------
+        // (a warp reads the 32 lanes of tensor memory given by its index modulo 4)
+        pdl_wait();                                                 // (the result's and the gate's memory may be in use until then)
+        const int quad = warp & 3, s = (warp - 2) >> 2;             // s: the stream
+        const int r = quad * 32 + lane, row_tok = min(r, rows - 1) / gs, row_head = min(r, rows - 1) % gs;
         const bool capped = EXTRA && X.cap > 0.f;
         const float sl2 = capped ? 1.0f : scale * 1.4426950408889634f;   // (a capped score comes in units of log2 e)
         const float cap2 = EXTRA ? X.cap * 1.4426950408889634f : 0.f, z_of_s = capped ? scale / X.cap : 0.f,
                     two_s = 2.0f * 1.4426950408889634f * z_of_s;
-        const int n_seen = EXTRA ? blocks_seen(limit, mask_size, X.block) : 0;
-        const float sink2 = sink ? sink[head] * 1.4426950408889634f : -INFINITY;   // a score without a value
         const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
-        constexpr int OW = HD / 2;                                  // columns of O this thread rescales and stores
-        const uint32_t o_addr = lane_base + COL_O + half * OW;
-        // m: the maximum (in units of log2 e) that O and l are scaled by.  It follows
-        // the true running maximum lazily; l: this thread's part of the row's sum.
-        // (a sink: the scaling maximum starts there, and its share joins the row's sum at the end)
-        float m = sink2, l = 0.f;
+        const uint32_t s_addr = lane_base + COL_S + s * BK, o_addr = lane_base + COL_O + s * HD;
         bool ok = true;
-        for (int j = 0; j < n_blk; ++j) {
-            const int buf = j % NBUF, xb = j & 1, v_item = 2 * j + 1, v_slot = v_item % NSLOT;
-            const uint32_t s_addr = lane_base + COL_S + buf * BK;
-            ok = __all_sync(0xffffffffu, mbar_wait(&s_full[buf], (j / NBUF) & 1, &abort_flag, status, 7));
-            if (!ok) break;
-            tc_fence_after();
-            const bool pooled = EXTRA && j < n_pool;
-            const int key0 = (pooled ? j : j + jw) * BK + c_lo;
-            const int last = pooled ? n_seen - 1 : limit, first_key = pooled ? 0 : vis;
-            float s[HALF_K];
-            tc_ld32_nowait(s_addr + c_lo, reinterpret_cast<uint32_t*>(s));
-            tc_ld32_nowait(s_addr + c_lo + 32, reinterpret_cast<uint32_t*>(s + 32));
-            tc_ld_wait();
-            if (capped) {
-                // cap tanh(z), z = s / cap: by a polynomial where all of the warp's |z| are small (two products and sums an
-                // instruction), else as cap (1 - 2 / (1 + exp(2 z))), whose two special functions a score would bound the block.
-                float big = 0.f;
-#pragma unroll
-                for (int i = 0; i < HALF_K; i += 2) big = max3(big, fabsf(s[i]), fabsf(s[i + 1]));
-                if (__all_sync(0xffffffffu, big * z_of_s <= TANH_SMALL)) {
-                    const float2 zs = make_float2(z_of_s, z_of_s), c2 = make_float2(cap2, cap2);
-#pragma unroll
-                    for (int i = 0; i < HALF_K; i += 2) {
-                        const float2 z = mul2(make_float2(s[i], s[i + 1]), zs), q = mul2(z, z);
-                        float2 p = make_float2(TANH_C4, TANH_C4);
-                        p = fma2(p, q, make_float2(TANH_C3, TANH_C3));
-                        p = fma2(p, q, make_float2(TANH_C2, TANH_C2));
-                        p = fma2(p, q, make_float2(TANH_C1, TANH_C1));
-                        p = fma2(p, q, make_float2(TANH_C0, TANH_C0));
-                        const float2 r2 = mul2(mul2(p, z), c2);
-                        s[i] = r2.x;
-                        s[i + 1] = r2.y;
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < HALF_K; ++i) s[i] = fmaf(-2.0f * cap2, rcp(1.0f + ex2(s[i] * two_s)), cap2);
-                }
-            }
-            if (key0 + HALF_K - 1 > last || key0 < first_key) {
-#pragma unroll
-                for (int i = 0; i < HALF_K; ++i)
-                    if (key0 + i > last || key0 + i < first_key) s[i] = -INFINITY;
-            }
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-            for (int i = 0; i < HALF_K; i += 8) {
-                mx4[0] = max3(mx4[0], s[i], s[i + 1]);
-                mx4[1] = max3(mx4[1], s[i + 2], s[i + 3]);
-                mx4[2] = max3(mx4[2], s[i + 4], s[i + 5]);
-                mx4[3] = max3(mx4[3], s[i + 6], s[i + 7]);
-            }
-            // The row's other half: through shared memory and the pair's barrier.  Both sides
-            // round to bfloat16, so that both scale by the same number (the scaling maximum
-            // need not be the exact one).
-            const bf16 mx_mine = __float2bfloat16_rn(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])));
-            mx_x[xb][half][r] = mx_mine;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&x_bar[quad]);
-            ok = __all_sync(0xffffffffu, mbar_wait(&x_bar[quad], j & 1, &abort_flag, status, 7));
-            if (!ok) break;
-            const float mx = fmaxf(__bfloat162float(mx_mine), __bfloat162float(mx_x[xb][half ^ 1][r])) * sl2;
-            const bool grow = mx > m + 8.0f;
-            float alpha = 1.0f;
-            if (grow) {
-                alpha = ex2(m - mx);                                // 0 for the first keys a row sees
-                m = mx;
-            }
-            const float neg_m = m == -INFINITY ? 0.f : -m;          // a row that sees no key yet
-            if (j > 0 && __any_sync(0xffffffffu, grow)) {
-                // Rare.  O must hold the product of the block before.  (Its barrier serves every other
-                // block; that the scores of this block exist says that the product of block j - 3, the
-                // barrier's phase before, is complete: the parity is unambiguous although most blocks
-                // never wait here.)
-                ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, &abort_flag, status, 7));
+        int base = 0, step = 0, uses[2] = {0, 0}, joins = 0;        // tiles of earlier items; this stream's steps, both streams' items, joins so far
+#pragma unroll 1
+        for (int k = 0; ok && any(k); ++k) {
+            const Item& w = sh.items[k];
+            const int n_blk = w.n_blk, kv_len = w.start + w.q_len, n_pool = w.n_pool, jw = w.jb0 - n_pool;
+            const bool split = w.split;
+            const int tok = w.q0 + (split ? 0 : s * T) + row_tok, head = w.head0 + row_head;   // token (of the sequence) and head of the row
+            const int limit = min(w.start + tok, kv_len - 1);       // last visible key position
+            const int vis = first_visible_key(limit, mask, mask_size);  // first visible key position
+            const int n_seen = EXTRA ? blocks_seen(limit, mask_size, X.block) : 0;
+            const float sink2 = sink ? sink[head] * 1.4426950408889634f : -INFINITY;   // a score without a value
+            // m: the maximum (in units of log2 e) that O and l are scaled by.  It follows
+            // the true running maximum lazily; l: the row's sum.
+            // (a sink: the scaling maximum starts there, and its share joins the row's sum at the end)
+            float m = sink2, l = 0.f;
+            int t = 0;
+#pragma unroll 1
+            for (int j = split ? s : 0; j < n_blk; j += split ? 2 : 1, ++t) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&sh.s_full[s], step & 1, abort_flag, status, 7));
                 if (!ok) break;
+                ++step;
                 tc_fence_after();
-                {
-#pragma unroll
-                    for (int c = 0; c < OW; c += 32) {
-                        uint32_t raw[32];
-                        tc_ld32_nowait(o_addr + c, raw);
+                const bool pooled = EXTRA && j < n_pool;
+                const int key0 = (pooled ? j : j + jw) * BK;
+                const int last = pooled ? n_seen - 1 : limit, first_key = pooled ? 0 : vis;
+                // Three times over the scores: masks where there are any, the row's maximum, the probabilities, which take the place of scores
+                // already read.  In loops, except in long items: an item of a short prompt meets this code once, and each 128 bytes of it come
+                // from memory where weights have passed through the L2 cache since the layer before (the whole written out, 110 KB of code
+                // instead of 72: a prompt of 100 tokens took 7 us longer a layer).
+                if (capped || __any_sync(0xffffffffu, key0 + BK - 1 > last || key0 < first_key)) {
+#pragma unroll 1
+                    for (int c = 0; c < BK; c += 32) {
+                        float v[32];
+                        tc_ld32_nowait(s_addr + c, reinterpret_cast<uint32_t*>(v));
                         tc_ld_wait();
+                        if (capped) {
+                            // cap tanh(z), z = s / cap: by a polynomial where all of the warp's |z| are small (two products and sums an
+                            // instruction), else as cap (1 - 2 / (1 + exp(2 z))), whose two special functions a score would bound the block.
+                            float big = 0.f;
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) raw[i] = __float_as_uint(__uint_as_float(raw[i]) * alpha);
-                        tc_st32(o_addr + c, raw);
+                            for (int i = 0; i < 32; i += 2) big = max3(big, fabsf(v[i]), fabsf(v[i + 1]));
+                            if (__all_sync(0xffffffffu, big * z_of_s <= TANH_SMALL)) {
+                                const float2 zs = make_float2(z_of_s, z_of_s), c2 = make_float2(cap2, cap2);
+#pragma unroll
+                                for (int i = 0; i < 32; i += 2) {
+                                    const float2 z = mul2(make_float2(v[i], v[i + 1]), zs), q = mul2(z, z);
+                                    float2 p = make_float2(TANH_C4, TANH_C4);
+                                    p = fma2(p, q, make_float2(TANH_C3, TANH_C3));
+                                    p = fma2(p, q, make_float2(TANH_C2, TANH_C2));
+                                    p = fma2(p, q, make_float2(TANH_C1, TANH_C1));
+                                    p = fma2(p, q, make_float2(TANH_C0, TANH_C0));
+                                    const float2 r2 = mul2(mul2(p, z), c2);
+                                    v[i] = r2.x;
+                                    v[i + 1] = r2.y;
+                                }
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) v[i] = fmaf(-2.0f * cap2, rcp(1.0f + ex2(v[i] * two_s)), cap2);
+                            }
+                        }
+                        const int lo = first_key - key0 - c, hi = last - key0 - c;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (i > hi || i < lo) v[i] = -INFINITY;
+                        tc_st32(s_addr + c, reinterpret_cast<uint32_t*>(v));
                     }
                     tc_st_wait();
                 }
-            }
-            float2 sum2[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-            uint32_t packed[HALF_K / 2];
-            const float2 sl2_2 = make_float2(sl2, sl2), neg_m2 = make_float2(neg_m, neg_m);
+                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                float y[64];                                             // the scores read last
+#pragma unroll 1
+                for (int c = 0; c < BK; c += 64) {
+                    tc_ld32_nowait(s_addr + c, reinterpret_cast<uint32_t*>(y));
+                    tc_ld32_nowait(s_addr + c + 32, reinterpret_cast<uint32_t*>(y + 32));
+                    tc_ld_wait();
 #pragma unroll
-            for (int i = 0; i < HALF_K; i += 2) {
-                const float2 x = fma2(make_float2(s[i], s[i + 1]), sl2_2, neg_m2);
-                const float2 pp = make_float2(ex2(x.x), ex2(x.y));
-                sum2[(i >> 1) & 3] = add2(sum2[(i >> 1) & 3], pp);
-                __nv_bfloat162 hh = __floats2bfloat162_rn(pp.x, pp.y);      // key 2k in the low half, key 2k + 1 in the high half
-                packed[i >> 1] = *reinterpret_cast<uint32_t*>(&hh);
-            }
-            const float sum4[4] = {sum2[0].x + sum2[0].y, sum2[1].x + sum2[1].y, sum2[2].x + sum2[2].y, sum2[3].x + sum2[3].y};
-            // P over the scores it came from (the other half has its scores in registers: it passed the pair's barrier)
-            tc_st32(s_addr + half * (HALF_K / 2), packed);
-            tc_st_wait();
-            l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-            // value rows that hold no token yet are made zero before they are multiplied
-            const int valid = pooled ? BK : kv_len - (j + jw) * BK;  // (places without a block hold zeros)
-            if (valid < BK) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&full[v_slot], (v_item / NSLOT) & 1, &abort_flag, status, 7));
-                if (!ok) break;
-                const int first = max(valid, 0);
-                for (int i = threadIdx.x - 64; i < (BK - first) * (HD / 8); i += THREADS - 64) {
-                    const int row = first + i / (HD / 8), chunk = i % (HD / 8);
-                    *reinterpret_cast<uint4*>(kv_s + v_slot * TILE_BYTES + (chunk >> 3) * PANEL_BYTES + row * 128 +
-                                              (((chunk & 7) ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeros before the tensor core reads them
-            }
-            tc_fence_before();                                               // P and the rescaled O before it multiplies and accumulates
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[buf]);
-        }
-        // the last products, in their order (each wait with an unambiguous parity: see above)
-        if (ok && n_blk > 1) ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[(n_blk - 2) & 1], ((n_blk - 2) >> 1) & 1, &abort_flag, status, 7));
-        ok = ok && __all_sync(0xffffffffu, mbar_wait(&pv_done[(n_blk - 1) & 1], ((n_blk - 1) >> 1) & 1, &abort_flag, status, 7));
-        tc_fence_after();
-        float* l_x = reinterpret_cast<float*>(&mx_x[0][0][0]);       // free once every block's maxima have been read
-        if (ok) {
-            // the row's sum: this half's plus the other's, in a fixed order
-            l_x[half * BQ + r] = l;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&x_bar[quad]);
-            ok = __all_sync(0xffffffffu, mbar_wait(&x_bar[quad], n_blk & 1, &abort_flag, status, 7));
-        }
-        if (ok) {
-            // every lane takes part in the loads from tensor memory; only rows that exist are stored
-            const float l_row = l_x[r] + l_x[BQ + r] + (sink ? ex2(sink2 - m) : 0.f);   // (both halves scale by the same m)
-            const bool store = r < rows && l_row > 0.f;
-            float inv = store ? 1.0f / l_row : 0.f;
-            if (EXTRA && X.gate && store) inv *= X.gate[(int64_t)(tok0 + q0 + r) * n_heads + head];
-            bf16* dst = out + ((int64_t)(tok0 + q0 + r) * n_heads + head) * HD + half * OW;
-#pragma unroll
-            for (int c = 0; c < OW; c += 32) {
-                uint32_t raw[32];
-                tc_ld32_nowait(o_addr + c, raw);
-                tc_ld_wait();
-                if (store) {
-#pragma unroll
-                    for (int g4 = 0; g4 < 4; ++g4) {
-                        uint4 w;
-                        __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&w);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            hh[i] = __floats2bfloat162_rn(__uint_as_float(raw[8 * g4 + 2 * i]) * inv, __uint_as_float(raw[8 * g4 + 2 * i + 1]) * inv);
-                        *reinterpret_cast<uint4*>(dst + c + 8 * g4) = w;
+                    for (int i = 0; i < 64; i += 8) {
+                        mx4[0] = max3(mx4[0], y[i], y[i + 1]);
+                        mx4[1] = max3(mx4[1], y[i + 2], y[i + 3]);
+                        mx4[2] = max3(mx4[2], y[i + 4], y[i + 5]);
+                        mx4[3] = max3(mx4[3], y[i + 6], y[i + 7]);
                     }
                 }
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl2;
+                const bool grow = mx > m + 8.0f;
+                float alpha = 1.0f;
+                if (grow) {
+                    alpha = ex2(m - mx);                                // 0 for the first keys a row sees
+                    m = mx;
+                }
+                const float neg_m = m == -INFINITY ? 0.f : -m;          // a row that sees no key yet
+                if (t > 0 && __any_sync(0xffffffffu, grow)) {
+                    // Rare.  (O holds the product of the step before: the scores of this one say so.)
+#pragma unroll 1
+                    for (int c = 0; c < HD; c += 16) {
+                        float o[16];
+                        tc_ld16(o_addr + c, o);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] *= alpha;
+                        tc_st16(o_addr + c, reinterpret_cast<uint32_t*>(o));
+                    }
+                }
+                // value rows that hold no token yet are made zero before they are multiplied
+                const int valid = pooled ? BK : kv_len - (j + jw) * BK;  // (places without a block hold zeros)
+                if (valid < BK && (split || s == 0)) {
+                    // (The slot's phase before this one is complete: its tile was an earlier key block's keys, whose scores came
+                    // before these.  The one after needs the product that waits for this warp.)
+                    const int v_n = base + w.place_v(j), v_slot = v_n % NSLOT;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&sh.full[v_slot], (v_n / NSLOT) & 1, abort_flag, status, 7));
+                    if (!ok) break;
+                    const int first = max(valid, 0);
+#pragma unroll 1
+                    for (int i = r; i < (BK - first) * (HD / 8); i += BQ) {
+                        const int row = first + i / (HD / 8), chunk = i % (HD / 8);
+                        *reinterpret_cast<uint4*>(kv_s + v_slot * TILE_BYTES + (chunk >> 3) * PANEL_BYTES + row * 128 +
+                                                  (((chunk & 7) ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeros before the tensor core reads them
+                }
+                // P over the scores; the product begins with the first half
+                float2 sum2[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+                const float2 sl2_2 = make_float2(sl2, sl2), neg_m2 = make_float2(neg_m, neg_m);
+                auto probs = [&](int c, const float* v) {                // of the 32 scores from column c on
+                    uint32_t packed[16];
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        const float2 e = fma2(make_float2(v[i], v[i + 1]), sl2_2, neg_m2);
+                        const float2 pp = make_float2(ex2(e.x), ex2(e.y));
+                        sum2[(i >> 1) & 3] = add2(sum2[(i >> 1) & 3], pp);
+                        __nv_bfloat162 hh = __floats2bfloat162_rn(pp.x, pp.y);      // key 2k in the low half, key 2k + 1 in the high half
+                        packed[i >> 1] = *reinterpret_cast<uint32_t*>(&hh);
+                    }
+                    tc_st16(s_addr + c / 2, packed);
+                };
+                auto hand_over = [&](int part) {
+                    tc_st_wait();
+                    tc_fence_before();                                   // P and the rescaled O before it multiplies and accumulates
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh.p_full[s][part]);
+                };
+                if (n_blk >= LONG) {
+                    float z[32];
+                    tc_ld32_nowait(s_addr, reinterpret_cast<uint32_t*>(z));
+                    tc_ld_wait();
+                    probs(0, z);
+                    tc_ld32_nowait(s_addr + 32, reinterpret_cast<uint32_t*>(z));
+                    tc_ld_wait();
+                    probs(32, z);
+                    hand_over(0);
+                    probs(64, y);
+                    probs(96, y + 32);
+                    hand_over(1);
+                } else {
+#pragma unroll 1
+                    for (int part = 0; part < 2; ++part) {
+                        tc_ld32_nowait(s_addr + part * P_FIRST, reinterpret_cast<uint32_t*>(y));
+                        tc_ld32_nowait(s_addr + part * P_FIRST + 32, reinterpret_cast<uint32_t*>(y + 32));
+                        tc_ld_wait();
+                        probs(part * P_FIRST, y);
+                        probs(part * P_FIRST + 32, y + 32);
+                        hand_over(part);
+                    }
+                }
+                l = l * alpha + (((sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y)) + ((sum2[2].x + sum2[2].y) + (sum2[3].x + sum2[3].y)));
+            }
+            if (!ok) break;
+            base += 2 * n_blk;
+            // (rows of tokens beyond the sequence's end were computed from other tokens' queries and are left out here)
+            const bool store = r < rows && tok < w.q_len;
+            bf16* dst = out + ((int64_t)(w.tok0 + min(tok, w.q_len - 1)) * n_heads + head) * HD;
+            const float gate = EXTRA && X.gate && store ? X.gate[(int64_t)(w.tok0 + tok) * n_heads + head] : 1.0f;
+            auto put = [&](int c, const float* v) {                  // 32 numbers of the row from column c on
+#pragma unroll
+                for (int g4 = 0; g4 < 4; ++g4) {
+                    uint4 o;
+                    __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) hh[i] = __floats2bfloat162_rn(v[8 * g4 + 2 * i], v[8 * g4 + 2 * i + 1]);
+                    *reinterpret_cast<uint4*>(dst + c + 8 * g4) = o;
+                }
+            };
+            if (!split || n_blk == 1) {
+                // the row is the stream's own (of one key block: the even stream's)
+                if (!split || s == 0) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(&sh.o_full[s], uses[s] & 1, abort_flag, status, 7));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const float l_row = l + (sink ? ex2(sink2 - m) : 0.f);
+                    const float inv = l_row == 0.f ? 0.f : gate / l_row;
+#pragma unroll 1
+                    for (int c = 0; c < HD; c += 32) {               // (every lane takes part in the loads; only rows that exist are stored)
+                        float v[32];
+                        tc_ld32_nowait(o_addr + c, reinterpret_cast<uint32_t*>(v));
+                        tc_ld_wait();
+                        if (c + 32 == HD) {                          // read before the next item's product writes
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&sh.o_empty[s]);
+                        }
+                        if (store) {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) v[i] *= inv;
+                            put(c, v);
+                        }
+                        __syncwarp();
+                    }
+                }
+                ++uses[0];
+                uses[1] += split ? 0 : 1;
+            } else {
+                // both streams hold a part of every row: each stream's warps make half of the columns
+                ok = __all_sync(0xffffffffu, mbar_wait(&sh.o_full[0], uses[0] & 1, abort_flag, status, 7) &&
+                                                 mbar_wait(&sh.o_full[1], uses[1] & 1, abort_flag, status, 7));
+                if (!ok) break;
+                ++uses[0], ++uses[1];
+                sh.ml[s][0][r] = m;
+                sh.ml[s][1][r] = l;
                 __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.join);
+                ok = __all_sync(0xffffffffu, mbar_wait(&sh.join, joins & 1, abort_flag, status, 7));
+                if (!ok) break;
+                tc_fence_after();
+                const float m0 = sh.ml[0][0][r], m1 = sh.ml[1][0][r], mm = fmaxf(m0, m1);
+                const float f0 = m0 == -INFINITY ? 0.f : ex2(m0 - mm), f1 = m1 == -INFINITY ? 0.f : ex2(m1 - mm);
+                const float l_row = sh.ml[0][1][r] * f0 + sh.ml[1][1][r] * f1 + (sink ? ex2(sink2 - mm) : 0.f);
+                const float inv = l_row == 0.f ? 0.f : gate / l_row, i0 = f0 * inv, i1 = f1 * inv;
+                constexpr int HALF = HD / 2;
+#pragma unroll 1
+                for (int c = s * HALF; c < (s + 1) * HALF; c += 32) {
+                    float v[32], u[32];
+                    tc_ld32_nowait(lane_base + COL_O + c, reinterpret_cast<uint32_t*>(v));
+                    tc_ld32_nowait(lane_base + COL_O + HD + c, reinterpret_cast<uint32_t*>(u));
+                    tc_ld_wait();
+                    if (store) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = fmaf(u[i], i1, v[i] * i0);
+                        put(c, v);
+                    }
+                    __syncwarp();
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.joined);              // (both streams' warps have read both results)
+                ok = __all_sync(0xffffffffu, mbar_wait(&sh.joined, joins & 1, abort_flag, status, 7));
+                ++joins;
+                if (lane == 0) mbar_arrive(&sh.o_empty[s]);
             }
         }
     }
 
     tc_fence_before();
     __syncthreads();
-    if (abort_flag) {
+    if (sh.abort_flag) {
         const uint64_t t0 = global_ns();
         while (global_ns() - t0 < 2000000ull) __nanosleep(1000);   // copies in flight land before the block leaves
         __syncthreads();
@@ -555,6 +855,24 @@ using namespace wick;
 
 WICK_API int wick_attn_prompt_tc_supported() { return prompttc::SUPPORTED ? 1 : 0; }
 
+// Queries bfloat16 [tokens, heads, HD] as a TMA descriptor with boxes of 64 numbers x gs heads x T tokens: T gs rows of 128 bytes.
+static int make_heads_map(CUtensorMap* map, const void* ptr, long long tokens, int heads, int gs, int T) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    WICK_REQUIRE(fn != nullptr, "attention (tcgen05): the driver does not provide cuTensorMapEncodeTiled");
+    WICK_REQUIRE(((uintptr_t)ptr & 15) == 0, "attention (tcgen05): operand is not 16-byte aligned");
+    const int hd = prompttc::HD;
+    cuuint64_t dims[3] = {(cuuint64_t)hd, (cuuint64_t)heads, (cuuint64_t)tokens};
+    cuuint64_t strides[2] = {(cuuint64_t)hd * 2, (cuuint64_t)heads * hd * 2};
+    cuuint32_t box[3] = {64u, (cuuint32_t)gs, (cuuint32_t)T};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    WICK_REQUIRE(r == CUDA_SUCCESS, "attention (tcgen05): cuTensorMapEncodeTiled failed with code %d (tokens %lld, heads %d, box %d x %d)",
+                 (int)r, tokens, heads, gs, T);
+    return 0;
+}
+
 // q, out: bfloat16 [n_tokens, n_heads, HD]; kv: one schedule entry's cache, bfloat16
 // [kv_pages, 2, n_kv, 64, HD] (it already holds the new tokens' keys and values);
 // n_tiles: the step's 64-row work items (one per 64 new tokens of a sequence, numbered
@@ -568,8 +886,27 @@ static int attn_prompt_tc(const void* q, long long n_tokens, const void* kv, lon
     WICK_REQUIRE(n_heads > 0 && n_kv > 0 && n_heads % n_kv == 0, "attention: %d heads over %d kv heads", n_heads, n_kv);
     WICK_REQUIRE(n_heads <= 65535, "attention: %d heads is beyond the grid limit", n_heads);
     if (n_tiles == 0) return 0;
+    const int group = n_heads / n_kv;
+    int gs = 1;                                                    // heads of a tile: the divisor of the group that fills most rows
+    for (int g = 1; g <= min(group, BQ); ++g)
+        if (group % g == 0 && BQ / g * g >= BQ / gs * gs) gs = g;
+    const int T = BQ / gs, columns = n_heads / gs;
+    // the most work items of R tokens that sequences of n_tokens tokens (or of n_tiles 64-row items) can make
+    auto items = [&](long long R) { return (int)min((n_tokens + n_seqs * (R - 1)) / R, n_tiles * ((64 + R - 1) / R)); };
+    // Items of two tiles share every key and value tile; but as long as items of one tile find an SM each they take half as long
+    // (512 tokens, 32 heads over 8: 64 items of two 16.4 us, 128 of one 13.2), with up to two an SM they are no worse unless every
+    // sequence is one block of keys (2,048 tokens, 16 heads over 4: 39 and 31 us; 640 tokens, 32 over 8: 18.9 and 15.8; 16 x 64 tokens: 12.8
+    // and 16.8), and beyond, where the last round of two is the emptier one and the keys are many (1,419 tokens behind 3,100: 118 and 103;
+    // 4 x 700 alone, 16 over 4: 22.5 and 27.1).
+    const long long one = (long long)items(T) * columns, two = (long long)items(2 * T) * columns, sms = sm_count();
+    const long long keys = ((long long)table_width * kPage - n_tokens / max(n_seqs, 1) / 2) / BK;     // blocks of keys a tile sees, about
+    const int tiles = one <= sms || (one <= 2 * sms && keys >= 1) || (two <= 2 * sms && (one + sms - 1) / sms < 2 * ((two + sms - 1) / sms) && keys >= 16) ? 1 : 2;
+    const int n_items = items(T * tiles);
+    WICK_REQUIRE((long long)n_items * columns <= INT32_MAX / 2, "attention (tcgen05): %d work items of %d columns are too many", n_items, columns);
+    // a block an SM that works through its items one behind the other (more than MAX_ITEMS each: in several rounds)
+    const int rounds = ceil_div((long long)n_items * columns, (long long)MAX_ITEMS * sm_count()), blocks = min(n_items * columns, rounds * sm_count());
     CUtensorMap q_map, kv_map, pool_map;
-    if (int e = make_bf16_map(&q_map, q, n_tokens, (long long)n_heads * HD, BQ, "attention (tcgen05)")) return e;
+    if (int e = make_heads_map(&q_map, q, n_tokens, n_heads, gs, T)) return e;
     if (int e = make_bf16_map(&kv_map, kv, kv_pages * 2 * n_kv * kPage, HD, kPage, "attention (tcgen05)")) return e;
     pool_map = kv_map;
     TcExtra X = {0, 0, 0.f, nullptr};
@@ -586,9 +923,9 @@ static int attn_prompt_tc(const void* q, long long n_tokens, const void* kv, lon
         WICK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         raised[extra ? 1 : 0] = true;
     }
-    WICK_CUDA(launch(kernel, dim3(n_tiles, n_heads), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, q_map,
-                     kv_map, (bf16*)out, cu_seqlens, n_seqs, start, page_table, table_width, n_tiles, n_heads,
-                     n_kv, scale, status, mask, mask_size, sink, pool_map, X));
+    WICK_CUDA(launch(kernel, dim3(blocks), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, q_map,
+                     kv_map, (bf16*)out, cu_seqlens, n_seqs, start, page_table, table_width, n_heads,
+                     n_kv, gs, T, columns, group / gs, tiles, n_items, scale, status, mask, mask_size, sink, pool_map, X));
     return check_launch("attn_prompt_tc");
 }
 
