@@ -135,11 +135,6 @@ __device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo_bytes) {
 // stride offset 1024 bytes (8 rows of 128 bytes), descriptor version 1 (bit 46), 128-byte swizzle (bits 61-63)
 constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 
-__device__ __forceinline__ bool elect_one() {                   // true in one lane of a whole warp
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
 // D (tensor memory) (+)= A (shared memory) * B (shared memory)
 template <int ACC>
 __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {

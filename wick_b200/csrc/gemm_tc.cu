@@ -228,93 +228,99 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            uint32_t it = 0;                                 // 64-wide steps issued so far, over all tiles
-            bool ok = true;
-            for (int w = w_first; w < w_end && ok; w += w_step) {
-                int m0, n0, kb_begin, n_kb, z;
-                tile_coords(w, m0, n0, kb_begin, n_kb, z);
-                if constexpr (GROUPED) {                     // (from here on rows of the operands, not of the result)
-                    m0 += max(group, 0) * p.group_rows;
-                    n0 += max(group, 0) * p.group_b_rows;
-                }
-                // Coordinates of the box that holds rows row.. of k-block kb: in a row-major
-                // operand (kb * 64, row); in a packed one the tile (row / 128, kb) lies as
-                // 128 contiguous lines of 128 bytes.
-                auto load = [&](const CUtensorMap* map, int packed, int s, void* dst, int kb, int row) {
-                    if (packed) tma_load_2d(map, &full_bar[s], dst, 0, ((row >> 7) * k_blocks + kb) * 128 + (row & 127));
-                    else tma_load_2d(map, &full_bar[s], dst, kb * BK, row);
-                };
-                auto load_a = [&](int i, int s) {
-                    uint8_t* st = tiles + (size_t)s * stage_bytes;
-                    const int kb = kb_begin + i;
-                    load(ma, p.a_packed, s, st, kb, m0);
-                    if (a_tiles == 2) load(ma, p.a_packed, s, st + a_bytes, kb, m0 + pair_offset);
-                    if (GATED == 3) load(ma, p.a_packed, s, st + a_bytes / 2, kb, m0 + pair_offset);   // 64-row boxes
-                };
-                auto load_b = [&](int i, int s) {
-                    uint8_t* sb = tiles + (size_t)s * stage_bytes + a_tiles * a_bytes;
-                    const int kb = kb_begin + i;
-                    load(mb, p.b_packed, s, sb, kb, n0);
-                    if (p.b_packed && p.bn > 128) load(mb, p.b_packed, s, sb + 128 * BK * 2, kb, n0 + 128);   // 256 rows: two tiles
-                    if (b_tiles == 2) load(mb, p.b_packed, s, sb + b_bytes, kb, n0 + pair_offset);
-                };
-                int i = 0;
-                if (it == 0) {
-                    // The first ring of stages is free.  An operand that no kernel
-                    // writes (weights) is fetched before the preceding kernel has
-                    // finished; the other one only after pdl_wait.
-                    const int first = min(n_kb, p.stages);
-                    for (int j = 0; j < first; ++j) {
-                        mbar_expect_tx(&full_bar[j], stage_bytes);
-                        if (p.a_static) load_a(j, j);
-                        if (p.b_static) load_b(j, j);
+        // (Here and below the whole warp walks through the loop and one elected lane issues: what an instruction needs stays in uniform
+        // registers, where a branch of one lane moves it there for each.)
+        const bool one = elect_one();
+        int s = 0;                                           // the ring's next stage, how often the ring has been gone through
+        uint32_t round = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (int w = w_first; w < w_end && ok; w += w_step) {
+            int m0, n0, kb_begin, n_kb, z;
+            tile_coords(w, m0, n0, kb_begin, n_kb, z);
+            if constexpr (GROUPED) {                         // (from here on rows of the operands, not of the result)
+                m0 += max(group, 0) * p.group_rows;
+                n0 += max(group, 0) * p.group_b_rows;
+            }
+            // Coordinates of the box that holds rows row.. of k-block kb: in a row-major
+            // operand (kb * 64, row); in a packed one the tile (row / 128, kb) lies as
+            // 128 contiguous lines of 128 bytes.
+            auto load = [&](const CUtensorMap* map, int packed, int s, void* dst, int kb, int row) {
+                tma_load_2d(map, &full_bar[s], dst, packed ? 0 : kb * BK, packed ? ((row >> 7) * k_blocks + kb) * 128 + (row & 127) : row);
+            };
+            auto load_a = [&](int i, int s) {
+                uint8_t* st = tiles + (size_t)s * stage_bytes;
+                const int kb = kb_begin + i;
+                load(ma, p.a_packed, s, st, kb, m0);
+                if (a_tiles == 2) load(ma, p.a_packed, s, st + a_bytes, kb, m0 + pair_offset);
+                if (GATED == 3) load(ma, p.a_packed, s, st + a_bytes / 2, kb, m0 + pair_offset);   // 64-row boxes
+            };
+            auto load_b = [&](int i, int s) {
+                uint8_t* sb = tiles + (size_t)s * stage_bytes + a_tiles * a_bytes;
+                const int kb = kb_begin + i;
+                load(mb, p.b_packed, s, sb, kb, n0);
+                if (p.b_packed && p.bn > 128) load(mb, p.b_packed, s, sb + 128 * BK * 2, kb, n0 + 128);   // 256 rows: two tiles
+                if (b_tiles == 2) load(mb, p.b_packed, s, sb + b_bytes, kb, n0 + pair_offset);
+            };
+            // The first ring of stages is free.  An operand that no kernel
+            // writes (weights) is fetched before the preceding kernel has
+            // finished; the other one only after pdl_wait.
+            const int first = round == 0 && s == 0 ? min(n_kb, p.stages) : 0;
+#pragma unroll 1
+            for (int pass = first > 0 ? 0 : 2; pass < 3; ++pass) {
+                if (pass == 1) pdl_wait();
+                // pass 0: what is static of the first ring; 1: the rest of it; 2: everything behind it
+#pragma unroll 1
+                for (int i = pass == 2 ? first : 0; i < (pass == 2 ? n_kb : first); ++i) {
+                    int at = i;
+                    if (pass == 2) {
+                        at = s;
+                        if (round > 0) ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag, p.status, 1));
+                        if (!ok) break;
+                        if (++s == p.stages) s = 0, ++round;
                     }
-                    pdl_wait();
-                    for (int j = 0; j < first; ++j) {
-                        if (!p.a_static) load_a(j, j);
-                        if (!p.b_static) load_b(j, j);
+                    if (one) {
+                        if (pass != 1) mbar_expect_tx(&full_bar[at], stage_bytes);
+                        if (pass == 2 || (p.a_static != 0) == (pass == 0)) load_a(i, at);
+                        if (pass == 2 || (p.b_static != 0) == (pass == 0)) load_b(i, at);
                     }
-                    i = first;
-                    it = first;
+                    __syncwarp();
                 }
-                for (; i < n_kb; ++i, ++it) {
-                    const int s = it % p.stages;
-                    const uint32_t round = it / p.stages;
-                    if (!mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag, p.status, 1)) { ok = false; break; }
-                    mbar_expect_tx(&full_bar[s], stage_bytes);
-                    load_a(i, s);
-                    load_b(i, s);
+                if (pass == 1) {
+                    s = first;
+                    if (s == p.stages) s = 0, round = 1;
                 }
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            // kind::f16, A and B bfloat16 and k-major, float32 accumulator, M = 128, N = bn
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-            uint32_t it = 0;
-            bool ok = true;
-            int t = 0;
-            for (int w = w_first; w < w_end && ok; w += w_step, ++t) {
-                int m0, n0, kb_begin, n_kb, z;
-                tile_coords(w, m0, n0, kb_begin, n_kb, z);
-                const int buf = acc_bufs == 2 ? (t & 1) : 0;
-                const uint32_t use = acc_bufs == 2 ? (uint32_t)(t >> 1) : (uint32_t)t;   // how often this buffer was used before
-                if (t > 0) {
-                    ok = mbar_wait(&acc_empty[buf], (use & 1) ^ 1, &abort_flag, p.status, 5);  // the epilogue has drained it
-                    if (!ok) break;
-                    tc_fence_after();
-                }
-                const uint32_t d0 = tmem_base + buf * acc_cols;
-                for (int i = 0; i < n_kb; ++i, ++it) {
-                    const int s = it % p.stages;
-                    const uint32_t round = it / p.stages;
-                    ok = mbar_wait(&full_bar[s], round & 1, &abort_flag, p.status, 2);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t sa = smem_u32(tiles + (size_t)s * stage_bytes);
-                    const uint32_t sb = sa + a_tiles * a_bytes;
+        // kind::f16, A and B bfloat16 and k-major, float32 accumulator, M = 128, N = bn
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        const bool one = elect_one();
+        int s = 0;
+        uint32_t round = 0;
+        bool ok = true;
+        int t = 0;
+#pragma unroll 1
+        for (int w = w_first; w < w_end && ok; w += w_step, ++t) {
+            int m0, n0, kb_begin, n_kb, z;
+            tile_coords(w, m0, n0, kb_begin, n_kb, z);
+            const int buf = acc_bufs == 2 ? (t & 1) : 0;
+            const uint32_t use = acc_bufs == 2 ? (uint32_t)(t >> 1) : (uint32_t)t;   // how often this buffer was used before
+            if (t > 0) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (use & 1) ^ 1, &abort_flag, p.status, 5));  // the epilogue has drained it
+                if (!ok) break;
+                tc_fence_after();
+            }
+            const uint32_t d0 = tmem_base + buf * acc_cols;
+#pragma unroll 1
+            for (int i = 0; i < n_kb; ++i) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], round & 1, &abort_flag, p.status, 2));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t sa = smem_u32(tiles + (size_t)s * stage_bytes);
+                const uint32_t sb = sa + a_tiles * a_bytes;
+                if (one) {
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
                         const uint32_t acc = (i > 0 || k > 0) ? 1u : 0u;
@@ -323,16 +329,20 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
                         if (GATED == 1) tc_mma(d0 + p.bn, smem_desc(sa + a_bytes + k * UMMA_K * 2), db, idesc, acc);
                         if (GATED == 2) tc_mma(d0 + p.bn, da, smem_desc(sb + b_bytes + k * UMMA_K * 2), idesc, acc);
                     }
-                    tc_commit(&empty_bar[s]);      // the stage is free once these instructions have read it
+                    tc_commit(&empty_bar[s]);          // the stage is free once these instructions have read it
+                    if (i + 1 == n_kb) tc_commit(&acc_full[buf]);   // this tile's accumulator is complete
                 }
-                tc_commit(&acc_full[buf]);         // this tile's accumulator is complete
+                __syncwarp();
+                if (++s == p.stages) s = 0, ++round;
             }
+            if (n_kb <= 0 && one) tc_commit(&acc_full[buf]);
         }
     } else {
         // ---------------- epilogue: tensor memory -> global ----------------
         const int q = warp & 3;                    // this warp reads lanes 32q .. 32q+31
         pdl_wait();                                // the output may alias memory an earlier kernel still reads
         int t = 0;
+#pragma unroll 1
         for (int w = w_first; w < w_end; w += w_step, ++t) {
             int m0, n0, kb_begin, n_kb, z;
             tile_coords(w, m0, n0, kb_begin, n_kb, z);
@@ -358,6 +368,7 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
             if (JOINED) {
                 // column n of the accumulator at tiles[n][128 rows]
                 float* acc = reinterpret_cast<float*>(tiles);
+#pragma unroll 1
                 for (int c0 = 0; c0 < p.bn; c0 += 16) {
                     float v[16];
                     tc_ld16(lane_addr + c0, v);
@@ -373,6 +384,7 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
                 // memory.
                 const int mg = m0 + (q & 1) * 32 + lane, xrow = (q & 1) * 32 + lane;
                 const bool upper = q >= 2;
+#pragma unroll 1
                 for (int c0 = 0; c0 < p.bn; c0 += 16) {
                     float v[16];
                     if (ok && n_kb > 0) tc_ld16(lane_addr + c0, v);
@@ -400,6 +412,7 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");     // the exchange buffers are free for the next tile
             } else if (ok && n_kb > 0) {
+#pragma unroll 1
                 for (int c0 = 0; c0 < p.bn; c0 += 16) {
                     float v[16];
                     tc_ld16(lane_addr + c0, v);

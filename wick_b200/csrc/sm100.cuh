@@ -33,9 +33,9 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 // Bounded wait.  Returns false (and raises the block's abort flag) after limit_ns (~1 s).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
-                                          uint64_t limit_ns = 1000000000ull) {
-    if (mbar_try_wait(bar, parity)) return true;         // the common case costs one instruction
+// (The loop is a function of its own: a wait in place costs a few instructions.  The kernels of a layer then fit together into an SM's
+// instruction cache, which nothing else does for a step whose weights pass through the L2 cache between two uses of a kernel.)
+static __device__ __noinline__ bool mbar_wait_loop(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code, uint64_t limit_ns) {
     if (*abort_flag) return false;
     const uint64_t t0 = global_ns();
     for (uint32_t spin = 0;; ++spin) {
@@ -49,6 +49,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
             }
         }
     }
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
+                                          uint64_t limit_ns = 1000000000ull) {
+    if (mbar_try_wait(bar, parity)) return true;         // the common case costs one instruction
+    return mbar_wait_loop(bar, parity, abort_flag, status, code, limit_ns);
 }
 
 // global -> shared copy of `bytes` contiguous bytes (both addresses 16-byte
