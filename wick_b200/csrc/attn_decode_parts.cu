@@ -163,16 +163,24 @@ struct Walk {
     int is_v;                  // the tile of that page: keys (0) or values (1)
 };
 
-// cum, lens: the block's copies (shared memory) of the parts before each sequence and of the lengths.
+// cum, lens: the block's copies (shared memory) of the parts before each sequence and of the lengths.  PAIR: the walk holds
+// the one pair's sequence and head already, and its parts are counted from 0.
+template <bool PAIR>
 __device__ __forceinline__ void open_part(Walk& w, const int* cum, const int* lens, int n_kv) {
-    while (w.u >= cum[w.b + 1]) ++w.b;                 // (parts are visited in order: b only moves forward)
-    w.len = lens[w.b];
-    w.n_pages = (w.len + kPage - 1) / kPage;
+    if (!PAIR) {
+        while (w.u >= cum[w.b + 1]) ++w.b;             // (parts are visited in order: b only moves forward)
+        w.len = lens[w.b];
+        w.n_pages = (w.len + kPage - 1) / kPage;
+    }
     const int pp = pages_per_part(w.n_pages);
-    w.parts = (w.n_pages + pp - 1) / pp;
-    const int local = w.u - cum[w.b];
-    w.kvh = local / w.parts;
-    w.part = local % w.parts;
+    if (PAIR) {
+        w.part = w.u;
+    } else {
+        w.parts = (w.n_pages + pp - 1) / pp;
+        const int local = w.u - cum[w.b];
+        w.kvh = local / w.parts;
+        w.part = local % w.parts;
+    }
     w.page = w.part * pp;
     w.page_end = min(w.n_pages, w.page + pp);
     w.is_v = 0;
@@ -214,7 +222,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
     constexpr int TT = T;                              // tiles of a warp's ring
     constexpr int u_step = PAIR ? W : 1;               // from a warp's part to its next one
     extern __shared__ uint8_t smem_raw[];
-    __shared__ int cum[(PAIR ? 1 : MAX_SEQS) + 1];     // parts of the sequences before each sequence (times kv heads)
+    __shared__ int cum[PAIR ? 1 : MAX_SEQS + 1];       // parts of the sequences before each sequence (times kv heads)
     __shared__ int lens[PAIR ? 1 : MAX_SEQS];          // the sequences' lengths (0: left out)
     __shared__ uint64_t full[NW][TT];
     __shared__ int abort_flag;
@@ -226,12 +234,14 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
 
     if (tid == 0) {
         abort_flag = 0;
+#pragma unroll 1
         for (int w = 0; w < NW; ++w)
             for (int t = 0; t < TT; ++t) mbar_init(&full[w][t], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // b_base: the sequence that index 0 of cum / lens stands for (PAIR: the pair's own, the only one the block knows)
     int b_base = 0, u0 = 0, u1 = 0, my_parts = 0;
+    Walk pw, cw;                                       // where the copies are, where the computation is
     if (PAIR) {
         const int pair = (int)blockIdx.x;
         b_base = pair / n_kv;
@@ -240,17 +250,17 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         const bool fits = len > 0 && n_pages <= table_width && parts_of(n_pages) <= part_stride;
         if (len > 0 && !fits && tid == 0) atomicCAS(status, 0, 10);
         my_parts = fits ? parts_of(n_pages) : 0;
-        if (tid == 0) {
-            lens[0] = fits ? len : 0;
-            cum[0] = 0;
-            cum[1] = my_parts * n_kv;
-        }
-        u0 = (pair % n_kv) * my_parts + warp;          // this warp's parts: warp, warp + W, ...
-        u1 = (pair % n_kv) * my_parts + my_parts;
+        pw.len = len;
+        pw.n_pages = n_pages;
+        pw.parts = my_parts;
+        pw.kvh = pair % n_kv;
+        u0 = warp;                                     // this warp's parts: warp, warp + W, ...
+        u1 = my_parts;
     } else if (warp == 0) {
         // The step's lengths are in place before the step's first kernel starts (the host or
         // the kernel that prepares a step writes them; neither is the kernel before this one).
         int before = 0;
+#pragma unroll 1
         for (int s0 = 0; s0 < n_seqs; s0 += 32) {
             const int s = s0 + lane;
             int mine = 0;
@@ -285,17 +295,17 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
     const bool work = u0 < u1;                         // (PAIR: a warp without a part still helps with the rows and the merge)
 
     uint8_t* ring = tiles + (size_t)warp * TT * TILE_BYTES;
-    Walk pw, cw;                                       // where the copies are, where the computation is
     {
         int lo = 0, hi = (PAIR ? 1 : n_seqs) - 1;      // the sequence of part u0: the last b with cum[b] <= u0
-        while (lo < hi) {
+#pragma unroll 1
+        while (!PAIR && lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
             if (cum[mid] <= u0) lo = mid;
             else hi = mid - 1;
         }
         pw.u = u0;
         pw.b = lo;
-        if (work) open_part(pw, cum, lens, n_kv);
+        if (work) open_part<PAIR>(pw, cum, lens, n_kv);
         cw = pw;
     }
     // The page ids of a part: lane j holds the part's j-th page (a part of more than 32 pages
@@ -310,10 +320,10 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
     Walk nw = pw;                                      // the part after pw's
     int ids = work ? page_ids(pw) : 0, ids_next = 0, ids_first = pw.page;
     auto peek_next = [&]() {
+        nw = pw;
         nw.u = pw.u + u_step;
-        nw.b = pw.b;
         if (nw.u < u1) {
-            open_part(nw, cum, lens, n_kv);
+            open_part<PAIR>(nw, cum, lens, n_kv);
             ids_next = page_ids(nw);
         }
     };
@@ -358,6 +368,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         }
         return true;
     };
+#pragma unroll 1
     while (issue(false)) {}
     pdl_wait();                                        // the query rows (or the projection's sums they are made from)
     q = fresh(q);
@@ -435,32 +446,33 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         }
     };
 
+    // Rows ra and (if below end) rb of a pair's: the query heads' (0 .. group - 1), then the new key and value.
+    auto make = [&](int b, int kvh, int ra, int rb, int end) {
+        auto offset = [&](int ri) { return ri < group ? (int64_t)(kvh * group + ri) * HD : (int64_t)(n_heads + (ri - group) * n_kv + kvh) * HD; };
+        auto norm_w = [&](int ri) { return ri < group ? proj.q_w : (ri == group ? proj.k_w : (const float*)nullptr); };
+        auto dest = [&](int ri) { return rows_s[ri < group ? ri : NH + ri - group]; };
+        const int rc = min(rb, end - 1);
+        make_rows(b, offset(ra), offset(rc), rb < end, norm_w(ra), norm_w(rc), ra <= group, rb <= group, dest(ra), dest(rc));
+    };
     if (PAIR) {
-        if (PREP && my_parts > 0) {
-            // the pair's rows, a warp at one or two of them: query heads 0 .. group - 1, then the new key and value
-            const int kvh = (int)blockIdx.x % n_kv, n_rows = group + (proj.write_kv ? 2 : 0);
-            auto offset = [&](int ri) { return ri < group ? (int64_t)(kvh * group + ri) * HD : (int64_t)(n_heads + (ri - group) * n_kv + kvh) * HD; };
-            auto norm_w = [&](int ri) { return ri < group ? proj.q_w : (ri == group ? proj.k_w : (const float*)nullptr); };
-            auto dest = [&](int ri) { return ri < group ? rows_s[ri] : rows_s[NH + ri - group]; };
-            const int ra = warp, rb = warp + W;
-            if (ra < n_rows)
-                make_rows(b_base, offset(ra), offset(min(rb, n_rows - 1)), rb < n_rows, norm_w(ra), norm_w(min(rb, n_rows - 1)),
-                          ra <= group, rb <= group, dest(ra), dest(min(rb, n_rows - 1)));
-        }
+        // the pair's rows, a warp at one or two of them
+        const int n_rows = group + (proj.write_kv ? 2 : 0);
+        if (PREP && my_parts > 0 && warp < n_rows) make(b_base, (int)blockIdx.x % n_kv, warp, warp + W, n_rows);
         __syncthreads();
     }
 
+#pragma unroll 1
     while (cw.u < u1 && !dead) {
         const int b = b_base + cw.b, kvh = cw.kvh, pair = b * n_kv + kvh;
         const bool owner = PREP && proj.write_kv && cw.part == cw.parts - 1;   // this part ends with the new token
+        if (PREP && !PAIR) {
+            const int end = owner ? group + 2 : group;
+#pragma unroll 1
+            for (int ri = pair != q_of ? 0 : group; ri < end; ri += 2) make(b, kvh, ri, ri + 1, end);
+            __syncwarp();
+        }
         if (pair != q_of) {
             if (PREP) {
-                if (!PAIR) {
-                    for (int h = 0; h < group; h += 2)
-                        make_rows(b, (int64_t)(kvh * group + h) * HD, (int64_t)(kvh * group + h + 1) * HD, h + 1 < group, proj.q_w,
-                                  proj.q_w, true, true, rows_s[h], rows_s[h + 1]);
-                    __syncwarp();
-                }
 #pragma unroll
                 for (int ks = 0; ks < KS; ++ks) {
                     qb[ks][0] = r0 < group ? *reinterpret_cast<const uint32_t*>(&rows_s[r0][16 * ks + c0]) : 0u;
@@ -479,11 +491,6 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         }
         if (owner) {
             // the new token's key (normed, rotated) and value: into the cache, for the steps to come
-            if (!PAIR) {
-                make_rows(b, (int64_t)(n_heads + kvh) * HD, (int64_t)(n_heads + n_kv + kvh) * HD, true, proj.k_w, nullptr, true, false,
-                          rows_s[NH], rows_s[NH + 1]);
-                __syncwarp();
-            }
             const int pos = cw.len - 1;
             const int page = page_table[(int64_t)b * table_width + pos / kPage];
             if (page >= 0 && page < kv_pages && lane < 2 * (HD / 8)) {
@@ -498,21 +505,27 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
 #pragma unroll
         for (int mb = 0; mb < KS; ++mb) acc[mb][0] = acc[mb][1] = acc[mb][2] = acc[mb][3] = 0.f;
 
-        for (int page = cw.page; page < cw.page_end; ++page) {
+        float sc[4][4], mx0 = -INFINITY, mx1 = -INFINITY;      // a page's scores and their largest
+        bool ok = true;
+        // Two turns a page: its keys' scores; the probabilities and its values' product.  (Loops stay loops, one place starts copies: see mbar_wait_loop.)
+#pragma unroll 1
+        for (int turn = 2 * cw.page; turn < 2 * cw.page_end; ++turn) {
+            const int page = turn >> 1;
             const int keys_here = min(kPage, cw.len - page * kPage);
+#pragma unroll 1
             while (issue(true)) {}
-            // ---- scores S^T[key, head] of the page ----
-            uint32_t s = consumed % TT;
-            bool ok = mbar_wait(&full[warp][s], (consumed / TT) & 1, &abort_flag, status, 8);
-            const uint32_t k_base = smem_u32(ring + s * TILE_BYTES);
+            const uint32_t s = consumed % TT;
             const int new_row = (owner && page == cw.n_pages - 1) ? (cw.len - 1) % kPage : -1;
+            if (!(turn & 1)) {
+            // ---- scores S^T[key, head] of the page ----
+            ok = mbar_wait(&full[warp][s], (consumed / TT) & 1, &abort_flag, status, 8);
+            const uint32_t k_base = smem_u32(ring + s * TILE_BYTES);
             if (new_row >= 0 && ok) {
                 if (lane < HD / 8)
                     *reinterpret_cast<uint4*>(ring + s * TILE_BYTES + tile_off(new_row, lane)) = reinterpret_cast<const uint4*>(rows_s[NH])[lane];
                 __syncwarp();
             }
-            float sc[4][4];
-            float mx0 = -INFINITY, mx1 = -INFINITY;
+            mx0 = mx1 = -INFINITY;
             if (ok) {
 #pragma unroll
                 for (int mb = 0; mb < 4; ++mb) {
@@ -533,9 +546,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
                     mx1 = fmaxf(mx1, fmaxf(sc[mb][1], sc[mb][3]));
                 }
             }
-            __syncwarp();
-            ++consumed;                                // the keys are read: their tile may be filled again
-            while (issue(true)) {}
+            } else {
 #pragma unroll
             for (int o = 4; o < 32; o <<= 1) {
                 mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
@@ -575,7 +586,6 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
                 acc[mb][3] *= a1;
             }
             // ---- O^T[dim, head] += V^T[dim, key] P[key, head] ----
-            s = consumed % TT;
             ok = mbar_wait(&full[warp][s], (consumed / TT) & 1, &abort_flag, status, 8) && ok;
             uint8_t* v_tile = ring + s * TILE_BYTES;
             if (ok && new_row >= 0 && lane < HD / 8)
@@ -584,6 +594,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             if (ok && keys_here < kPage) {
                 // Rows of the last page that hold no token yet may be anything: make them zero,
                 // so that a zero weight times such a row stays zero.
+#pragma unroll 1
                 for (int i = lane; i < (kPage - keys_here) * (HD / 8); i += 32) {
                     const int row = keys_here + i / (HD / 8), chunk = i % (HD / 8);
                     *reinterpret_cast<uint4*>(v_tile + tile_off(row, chunk)) = make_uint4(0, 0, 0, 0);
@@ -603,9 +614,10 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
                     }
                 }
             }
-            __syncwarp();
-            ++consumed;                                // the values are read
             if (!ok) dead = true;
+            }
+            __syncwarp();
+            ++consumed;                                // the keys (values) are read: their tile may be filled again
         }
         if (dead) break;
 
@@ -646,12 +658,13 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             }
         }
         cw.u += u_step;
-        if (cw.u < u1) open_part(cw, cum, lens, n_kv);
+        if (cw.u < u1) open_part<PAIR>(cw, cum, lens, n_kv);
     }
     if (PAIR) {
         __syncthreads();                               // every part's record is written (and visible to this block)
         if (my_parts > 1 && !abort_flag) {
             const int pair = (int)blockIdx.x;
+#pragma unroll 1
             for (int h = warp; h < group; h += W) {
                 const float* first = partials + ((int64_t)pair * part_stride * group + h) * REC;
                 merge_head([&](int p, int i) { return ld_cg(first + (int64_t)p * group * REC + i); }, my_parts, lane,
