@@ -95,7 +95,6 @@ attn_latent_kernel(const Params P) {
     typedef Sizes<MT> Z;
     constexpr int HG = Z::HG, KSPLIT = Z::KSPLIT, KPW = Z::KPW, HPW = HG / WARPS;
     extern __shared__ __align__(128) uint8_t latent_smem[];
-    pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int R = P.R, r = P.r, pieces = (R / 8) | 1;
     bf16* tiles = reinterpret_cast<bf16*>(latent_smem);                                   // [STAGES][TK][pieces * 8]
@@ -118,6 +117,7 @@ attn_latent_kernel(const Params P) {
         const int kk = tid / TPK, c0 = tid % TPK, key = key_of(min(v_begin + i * TK + kk, v_end - 1));
         const bf16* src = P.store + ((int64_t)table[key / kPage] * kPage + key % kPage) * R;
         bf16* dst = tiles + ((int64_t)(i % STAGES) * TK + kk) * pieces * 8;
+#pragma unroll 1
         for (int c = c0; c < R / 8; c += TPK) cp16(dst + c * 8, src + c * 8);
     };
     auto settled = [&](int i) { return key_of(min(v_begin + (i + 1) * TK, v_end) - 1) < first_new; };    // rows of earlier steps only
@@ -270,6 +270,9 @@ attn_latent_kernel(const Params P) {
             }
         }
     }
+    // (Not earlier: a block fills its multiprocessor, so that all blocks of the merge that follows would be placed on the few that have none,
+    // and read their records through those: 4 tokens of 700 to 1,500 positions, the merge 10.3 us in a step.)
+    pdl_trigger();
     // maxima and sums to everyone, then the results: records, or finished here
     float *ms = corrs + HG, *ls = corrs + 2 * HG;
     if (lane == 0) {

@@ -635,10 +635,12 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
         else if (j < qr + r) ss[1] += sq;
     };
     if (TOGETHER) {
+#pragma unroll 1
         for (int j = tid * 4; j < W; j += blockDim.x * 4)                  // (the last group may reach behind W: the row has cols numbers)
             *reinterpret_cast<float4*>(row + j) = sum_parts4(mine + j, splits, split_stride);
         __syncthreads();
         if (tid < 256)
+#pragma unroll 1
             for (int j = tid * 4; j < qr + r; j += 1024) squares(j, *reinterpret_cast<const float4*>(row + j));
     } else if (((qr | r | cols) & 3) == 0 && (reinterpret_cast<size_t>(parts) & 15) == 0) {
 #pragma unroll 2
@@ -652,6 +654,7 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
             squares(j, v);
         }
     } else {
+#pragma unroll 1
         for (int j = tid; j < W; j += blockDim.x) {
             float v = mine[j];
             for (int s = 1; s < splits; ++s) v += mine[s * split_stride + j];
@@ -663,10 +666,12 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
     block_sums(ss, red);                            // (its barrier also makes the row whole; TOGETHER's further warps add zeros)
     const float fq = 1.0f / sqrtf(ss[0] / (float)qr + eps);
     if ((qr & 3) == 0) {
+#pragma unroll 1
         for (int j = tid * 4; j < qr; j += blockDim.x * 4)
             st4(cq_out + (int64_t)t * qr + j, (row[j] * fq) * q_w[j], (row[j + 1] * fq) * q_w[j + 1], (row[j + 2] * fq) * q_w[j + 2],
                 (row[j + 3] * fq) * q_w[j + 3]);
     } else {
+#pragma unroll 1
         for (int j = tid; j < qr; j += blockDim.x) st(cq_out + (int64_t)t * qr + j, (row[j] * fq) * q_w[j]);
     }
     if (r > 0) {
@@ -676,6 +681,7 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
             const int pg = page_table[(int64_t)seq_of_token[t] * table_width + pos / kPage];
             T* dst = rows + ((int64_t)pg * kPage + pos % kPage) * (r + dr);
             if (((r | dr | qr) & 3) == 0) {
+#pragma unroll 1
                 for (int j = tid * 4; j < r; j += blockDim.x * 4) {
                     const float4 v = *reinterpret_cast<const float4*>(row + qr + j);
                     const float a = (v.x * fc) * kv_w[j], b = (v.y * fc) * kv_w[j + 1], c = (v.z * fc) * kv_w[j + 2], d = (v.w * fc) * kv_w[j + 3];
@@ -683,6 +689,7 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
                     if (flat_c) st4(flat_c + (int64_t)t * r + j, a, b, c, d);
                 }
             } else {
+#pragma unroll 1
                 for (int j = tid; j < r; j += blockDim.x) {
                     const float c = (row[qr + j] * fc) * kv_w[j];
                     st(dst + j, c);
@@ -691,6 +698,7 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
             }
             const int half = dr >> 1;
             const float* kr = row + qr + r;
+#pragma unroll 1
             for (int i = tid; i < half; i += blockDim.x) {
                 const int j0 = pairing == 0 ? 2 * i : i, j1 = pairing == 0 ? 2 * i + 1 : i + half;
                 float u = kr[j0], v = kr[j1];
@@ -713,6 +721,7 @@ latent_finish_kernel(const float* __restrict__ parts, int splits, int64_t split_
             }
         }
     }
+#pragma unroll 1
     for (int j = tid; j < Hg; j += blockDim.x) gate_out[(int64_t)t * Hg + j] = 1.0f / (1.0f + expf(-row[qr + r + dr + j]));
 }
 
@@ -938,12 +947,14 @@ latent_absorb_few_kernel(const float* __restrict__ parts, int splits, int64_t sp
     cos_t = fresh(cos_t);
     sin_t = fresh(sin_t);
     if (vec) {
+#pragma unroll 1
         for (int idx = tid; idx < LAT_TT * (dq >> 2); idx += blockDim.x) {
             const int tt = idx / (dq >> 2), x = (idx - tt * (dq >> 2)) * 4;
             const float4 v = tt < n_t ? sum_parts4(parts + (int64_t)(t0 + tt) * W + h * dq + x, splits, split_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
             qh[x * LAT_TT + tt] = v.x; qh[(x + 1) * LAT_TT + tt] = v.y; qh[(x + 2) * LAT_TT + tt] = v.z; qh[(x + 3) * LAT_TT + tt] = v.w;
         }
     } else {
+#pragma unroll 1
         for (int idx = tid; idx < LAT_TT * dq; idx += blockDim.x) {
             const int tt = idx / dq, x = idx - tt * dq;
             float v = 0.f;
@@ -957,6 +968,7 @@ latent_absorb_few_kernel(const float* __restrict__ parts, int splits, int64_t sp
     __syncthreads();
     if (blockIdx.z == 0) {
         const int half = dr >> 1;
+#pragma unroll 1
         for (int idx = tid; idx < n_t * half; idx += blockDim.x) {
             const int tt = idx / half, i = idx - tt * half;
             const int p0 = pairing == 0 ? 2 * i : i, p1 = pairing == 0 ? 2 * i + 1 : i + half;
@@ -999,6 +1011,7 @@ latent_absorb_few_kernel(const float* __restrict__ parts, int splits, int64_t sp
 #pragma unroll
     for (int tt = 0; tt < LAT_TT; ++tt) *reinterpret_cast<float2*>(&sums[warp][tt][2 * lane]) = make_float2(acc[tt][0], acc[tt][1]);
     __syncthreads();
+#pragma unroll 1
     for (int idx = tid; idx < n_t * 64; idx += blockDim.x) {
         const int tt = idx >> 6, c = idx & 63, j = blockIdx.z * 64 + c;
         if (j >= r) continue;
@@ -1047,6 +1060,7 @@ latent_expand_few_kernel(const float* __restrict__ y, const T* __restrict__ uv, 
             gt = 1.0f / (1.0f + expf(-z));
         }
     }
+#pragma unroll 1
     for (int j = 2 * tid; j < r; j += 2 * blockDim.x) {
         float2 v[LAT_TT];                         // (all tokens' loads together)
 #pragma unroll

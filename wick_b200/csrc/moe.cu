@@ -348,6 +348,7 @@ moe_combine_table_kernel(const float* __restrict__ y, int y_splits, const int* _
             v[0] += *p;
         }
     };
+#pragma unroll 1
     for (int j = (blockIdx.y * blockDim.x + threadIdx.x) * V; j < width; j += gridDim.y * blockDim.x * V) {
         float sum[V], v[V];
 #pragma unroll
