@@ -205,7 +205,7 @@ struct Projection {
     int write_kv;
 };
 
-// PAIR: the form for few pairs (up to some 400; fewer for long sequences: the host decides by
+// PAIR: the form for few pairs, and for many long ones (the host decides by
 // measured rules).  A block takes one pair and its warps the pair's parts; the block makes the new
 // token's rows once, all warps at it (a row or two each, one trip to the L2 cache), and when
 // all parts are done its warps merge the pair's records, a head each: one launch.  Otherwise
@@ -762,10 +762,13 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
     // number of pairs, until the SMs that have a pair cannot keep the memory busy between them; the persistent
     // form costs about 9 us + the step's bytes at 5 TB/s.
     const bool pays = pages <= 16 || pairs >= 96 || (pairs >= 24 && pages <= 24) || (pairs >= 48 && pages <= 32);
-    // More pairs than SMs, up to some 400: the blocks run in waves; that still beats the persistent form, whose
-    // warps then have one or two parts each, unless the last wave is mostly empty.
+    // More pairs than SMs: the blocks run in waves, in which a long pair's block is followed by whatever is left; the persistent
+    // form deals parts in equal numbers, whatever their length, and its warps have one or two each up to some 400 pairs.  Beyond, where no
+    // sequence has more than 16 pages, the blocks' starts and ends cost more than that (64 x 64 to 400 positions: 26.5 us persistent, 29.1
+    // in waves; 56 x 1,000: 56 and 60); with longer ones 64 x 64 to 1,536 take 54 persistent and 50 in waves, 128 of them 105 and 86, 64 x
+    // 1,500 to 3,900 146 and 134, 64 x 1,500 81 and 74, 64 x 2,000 100 and 103, 256 x 100 to 1,500 179 and 162.
     const long long waves = (pairs + sms - 1) / sms;
-    const bool waves_pay = pairs <= 400 && pairs * 10 >= waves * sms * 6;
+    const bool waves_pay = (pairs <= 400 || pages > 16) && pairs * 10 >= waves * sms * 6;
     const bool pair_form = force >= 0 ? force == 1 : (pairs <= sms ? pays : waves_pay);
     if (pair_form) {
         // Few pairs of short parts: a block per pair, its warps at the pair's parts, merged by the block itself.
