@@ -64,7 +64,7 @@ constexpr int BK = 128;                                // keys of an inner step 
 constexpr int PANELS = HD / 64;                        // 64-column panels of a head row
 constexpr int PANEL_BYTES = 128 * 128;                 // 128 rows of 128 bytes
 constexpr int TILE_BYTES = PANELS * PANEL_BYTES;       // a tile of Q, or one block of keys or of values
-constexpr int LONG = 4;                                // key blocks of an item from which on its softmax is written out (8,192 tokens: 537 us looped, 453)
+constexpr int LONG = 9;                                // key blocks of an item from which on its softmax is written out (8,192 tokens: 537 us looped, 453)
 constexpr int P_FIRST = 64;                            // keys of a block whose probabilities the product begins with
 constexpr int NSLOT = 5;                               // key / value tiles in flight
 constexpr int MAX_ITEMS = 16;                          // work items of a block
@@ -243,15 +243,17 @@ __device__ __forceinline__ float rcp(float x) {
 // Work items of R tokens, longest first: all items of the step in falling order of the key block that their first
 // token lies in (items of one sequence that share it, and sequences, in index order); this finds the item at place `rank`.
 // A warp takes the sequences 32 at a time (the first 32 are kept in registers); the key block is found by bisection over counts
-// (9 steps for 40,960 positions; one sequence needs none).
+// (9 steps for 40,960 positions; one sequence needs none).  Not ordered: all items in index order.
 struct Finder {
     const int *cu_seqlens, *start_arr;
     int n_seqs, R, tok0, q_len, start, top;                        // (lane l: sequence l; top: no item lies in this key block or beyond)
-    __device__ __forceinline__ Finder(const int* cu, const int* st, int n, int r) : cu_seqlens(cu), start_arr(st), n_seqs(n), R(r) {
+    bool ordered;
+    __device__ __forceinline__ Finder(const int* cu, const int* st, int n, int r, bool o) : cu_seqlens(cu), start_arr(st), n_seqs(n), R(r), ordered(o) {
         const int s = threadIdx.x & 31;
         tok0 = s < n ? cu[s] : 0;
         q_len = s < n ? cu[s + 1] - tok0 : 0;
         start = s < n ? st[s] : 0;
+        if (!ordered) return;
         int t = (start + q_len) / BK + 1;
 #pragma unroll 1
         for (int i = s + 32; i < n; i += 32) t = max(t, (st[i] + cu[i + 1] - cu[i]) / BK + 1);
@@ -280,9 +282,9 @@ struct Finder {
         if (n_seqs == 1) {
             const int n = (__shfl_sync(0xffffffffu, q_len, 0) + R - 1) / R;
             if (rank < n) it.b = 0, it.q0 = (n - 1 - rank) * R;
-        } else if (count(0) > rank) {
+        } else if (!ordered || count(0) > rank) {
 #pragma unroll 1
-            while (hi - lo > 1) {                                  // count(lo) > rank >= count(hi) = above
+            while (ordered && hi - lo > 1) {                       // count(lo) > rank >= count(hi) = above
                 const int mid = (lo + hi) >> 1, c = count(mid);
                 if (c > rank) lo = mid;
                 else hi = mid, above = c;
@@ -290,7 +292,7 @@ struct Finder {
             int left = rank - above;                               // place among the items of key block lo
 #pragma unroll 1
             for (int s0 = 0; s0 < n_seqs; s0 += 32) {
-                const int all = items(s0), later = from(s0, all, lo + 1), n = from(s0, all, lo) - later;
+                const int all = items(s0), later = ordered ? from(s0, all, lo + 1) : 0, n = ordered ? from(s0, all, lo) - later : all;
                 int upto = n;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
@@ -340,7 +342,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                       bf16* __restrict__ out, const int* __restrict__ cu_seqlens, int n_seqs,
                       const int* __restrict__ start_arr,
-                      const int* __restrict__ page_table, int table_width, int n_heads, int n_kv, int gs, int T, int columns, int per_kv, int tiles, int n_items,
+                      const int* __restrict__ page_table, int table_width, int n_heads, int n_kv, int gs, int T, int columns, int per_kv, int tiles, int n_items, int ordered,
                       float scale, int* status, int mask, int mask_size, const float* __restrict__ sink,
                       const __grid_constant__ CUtensorMap pool_map, const TcExtra X) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -391,7 +393,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     {
-        const Finder finder(cu_seqlens, start_arr, n_seqs, T * tiles);
+        const Finder finder(cu_seqlens, start_arr, n_seqs, T * tiles, ordered != 0);
 #pragma unroll 1
         for (int k = warp; k < MAX_ITEMS; k += THREADS / 32) {      // (a warp each, up to the first that is none)
             const int at = place(k);
@@ -912,6 +914,8 @@ static int attn_prompt_tc(const void* q, long long n_tokens, const void* kv, lon
     } else {
         X.block = 0;
     }
+    // (up to four key blocks - every captured prompt step - the order is worth less than the ~2 us that finding it takes)
+    const int ordered = table_width > 4 * BK / kPage ? 1 : 0;
     auto kernel = extra ? attn_prompt_tc_kernel<true> : attn_prompt_tc_kernel<false>;
     static bool raised[2] = {false, false};
     if (!raised[extra ? 1 : 0]) {
@@ -920,7 +924,7 @@ static int attn_prompt_tc(const void* q, long long n_tokens, const void* kv, lon
     }
     WICK_CUDA(launch(kernel, dim3(blocks), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, q_map,
                      kv_map, (bf16*)out, cu_seqlens, n_seqs, start, page_table, table_width, n_heads,
-                     n_kv, gs, T, columns, group / gs, tiles, n_items, scale, status, mask, mask_size, sink, pool_map, X));
+                     n_kv, gs, T, columns, group / gs, tiles, n_items, ordered, scale, status, mask, mask_size, sink, pool_map, X));
     return check_launch("attn_prompt_tc");
 }
 
