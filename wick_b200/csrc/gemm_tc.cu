@@ -106,6 +106,11 @@ template <bool PERSIST, int GATED, bool TRANSPOSED, bool OUT_F32, bool GROUPED, 
 __device__ __forceinline__ void
 gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap* shared_a, const CUtensorMap* shared_b,
               const std::conditional_t<GROUPED, GroupedParams, GemmParams>& p) {
+    // A gated pair that shares a tile leaves its accumulator in the ring, which is idle by then, and all six warps finish the results from
+    // there, four neighbours a thread.  (Gate and up values lie in different warps' parts of tensor memory.  Crossing 16 columns at a time,
+    // with two barriers each and the four epilogue warps at work, 64 / 100 tokens x 2 x 12,288 outputs of 4,096 took 39.5 / 46.0 us; now 37.4 / 42.9.)
+    constexpr bool STAGED = GATED == 3 && !GROUPED && !OUT_F32 && !PERSIST;
+    static_assert(!JOINED || STAGED, "runs are joined where the accumulator is staged");
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full_bar[MAX_STAGES];
     __shared__ uint64_t empty_bar[MAX_STAGES];
@@ -114,7 +119,7 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
     __shared__ int ok_w[4];
-    __shared__ float xch[2][64][17];           // gated == 3: up values on their way to the warps that hold the gate values
+    __shared__ float xch[GATED == 3 && !STAGED ? 2 : 1][64][17];   // gated == 3: up values on their way to the warps that hold the gate values
 
     __shared__ unsigned uses[GROUPED ? 8 : 1];   // grouped: a bit per token that uses this block's matrix
     __shared__ unsigned named[RANKED ? NAMED_WORDS : 1];               // ranked: a bit per matrix that the step names
@@ -358,22 +363,27 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
             // One answer for the four epilogue warps, so that they leave the loop together.
             const bool ok_warp = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1, &abort_flag, p.status, 3));
             bool ok = ok_warp;
-            if (my_tiles > 1 || (GATED == 3 && !JOINED)) {            // (a block with one plain tile has nothing left to agree on)
+            if (my_tiles > 1 || (GATED == 3 && !STAGED)) {            // (a block with one plain tile has nothing left to agree on)
                 if (lane == 0) ok_w[q] = ok_warp ? 1 : 0;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 ok = ok_w[0] && ok_w[1] && ok_w[2] && ok_w[3];
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
             tc_fence_after();
-            if (JOINED) {
+            if constexpr (STAGED) {
                 // column n of the accumulator at tiles[n][128 rows]
-                float* acc = reinterpret_cast<float*>(tiles);
+                float* acc = reinterpret_cast<float*>(tiles) + q * 32 + lane;
 #pragma unroll 1
-                for (int c0 = 0; c0 < p.bn; c0 += 16) {
-                    float v[16];
-                    tc_ld16(lane_addr + c0, v);
+                for (int c0 = 0; c0 < p.bn; c0 += 32, acc += 32 * BM) {
+                    float v[32];
+                    tc_ld16_nowait(lane_addr + c0, v);
+                    tc_ld16_nowait(lane_addr + c0 + 16, v + 16);
+                    tc_wait_ld();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) acc[(c0 + j) * BM + q * 32 + lane] = v[j];
+                    for (int j = 0; j < 16; ++j) acc[j * BM] = v[j];
+                    if (c0 + 16 < p.bn)
+#pragma unroll
+                        for (int j = 16; j < 32; ++j) acc[j * BM] = v[j];
                 }
             } else if (GATED == 3) {
                 // Lanes 0-63 of the accumulator hold gate rows, lanes 64-127 the up rows of the
@@ -411,6 +421,32 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
                     }
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");     // the exchange buffers are free for the next tile
+            } else if (TRANSPOSED && GATED == 0 && !GROUPED) {
+                // 32 columns' loads at a time, then a store a column whose address moves by one addition (64 tokens x 6,144 and 4,096 outputs of
+                // 4,096, us: 16 at a time, an address and a test each 12.2 and 9.2, now 11.7 and 8.8)
+                if (ok && n_kb > 0) {
+                    typedef std::conditional_t<OUT_F32, float, __nv_bfloat16> Out;
+                    Out* o = (Out*)out_base + (long long)n0 * ldo + m;
+                    const int n_end = m < a_rows ? p.b_rows - n0 : 0;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < p.bn; c0 += 32) {
+                        float v[32];
+                        tc_ld16_nowait(lane_addr + c0, v);              // (tensor memory is allocated in multiples of 32 columns)
+                        tc_ld16_nowait(lane_addr + c0 + 16, v + 16);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int half = 0; half < 32; half += 16) {
+                            if (c0 + half + 16 <= n_end) {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j, o += ldo) st(o, v[half + j]);
+                            } else if (c0 + half < n_end) {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j, o += ldo)
+                                    if (c0 + half + j < n_end) st(o, v[half + j]);
+                            }
+                        }
+                    }
+                }
             } else if (ok && n_kb > 0) {
 #pragma unroll 1
                 for (int c0 = 0; c0 < p.bn; c0 += 16) {
@@ -471,11 +507,14 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
         }
     }
 
-    if constexpr (JOINED) {
-        static_assert(!GROUPED, "built for one matrix");
-        __syncwarp();
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        const int runs = (int)gridDim.z, rank = (int)blockIdx.z, m0 = (int)blockIdx.x * (BM / 2);
+    if constexpr (STAGED) {
+        if constexpr (JOINED) {
+            __syncwarp();
+            asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+        const int runs = JOINED ? (int)gridDim.z : 1, rank = JOINED ? (int)blockIdx.z : 0, m0 = (int)blockIdx.x * (BM / 2);
         const int n0 = blockIdx.y * p.bn;
         const uint32_t here = smem_u32(tiles);
         __nv_bfloat16* o = (__nv_bfloat16*)p.out;
@@ -495,9 +534,9 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
                 float g[V], u[V];
 #pragma unroll 8
                 for (int z = 0; z < runs; ++z) {
-                    uint32_t there;
+                    uint32_t there = here + 4u * (uint32_t)(n * BM + m);
                     float a[V], b[V];
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here + 4u * (uint32_t)(n * BM + m)), "r"(z));
+                    if (JOINED) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here + 4u * (uint32_t)(n * BM + m)), "r"(z));
                     load(there, a);
                     load(there + 2u * BM, b);
 #pragma unroll
@@ -516,9 +555,10 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
                         if (m0 + m + i < p.a_rows) at[i] = __float2bfloat16_rn(g[i]);
             }
         };
-        if (runs <= 4) finish(std::integral_constant<int, 4>());
+        if (!JOINED || runs <= 4) finish(std::integral_constant<int, 4>());
         else finish(std::integral_constant<int, 1>());
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // (nobody leaves while it is read)
+        if constexpr (JOINED)
+            asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // (nobody leaves while it is read)
     }
 
     tc_fence_before();
@@ -639,9 +679,9 @@ static int gemm_tc_host(const void* a, long long a_total_rows, int a_rows, const
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     if (stages > per_split) stages = per_split < 2 ? 2 : per_split;
     WICK_REQUIRE(stages >= 2, "gemm_tc: %d bytes of shared memory hold fewer than two stages of %d bytes", budget, stage_bytes);
-    const bool joined = gated == 3 && splits > 1;
-    if (joined && stages * stage_bytes < bn * BM * 4) stages = ceil_div(bn * BM * 4, stage_bytes);      // (the ring holds the accumulator at the end)
-    WICK_REQUIRE(!joined || stages <= MAX_STAGES, "gemm_tc: the joined tile does not fit the ring");
+    const bool joined = gated == 3 && splits > 1, staged = gated == 3 && !out_f32 && !G.n;
+    if (staged && stages * stage_bytes < bn * BM * 4) stages = ceil_div(bn * BM * 4, stage_bytes);      // (the ring holds the accumulator at the end)
+    WICK_REQUIRE(!staged || stages <= MAX_STAGES, "gemm_tc: the tile does not fit the ring");
     const int smem = stages * stage_bytes + 1024;
     GemmParams p;
     p.a_rows = a_rows; p.b_rows = b_rows; p.bn = bn; p.k_blocks = k_blocks; p.k_blocks_per_split = per_split;
