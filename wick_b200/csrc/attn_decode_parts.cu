@@ -454,6 +454,13 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         const int rc = min(rb, end - 1);
         make_rows(b, offset(ra), offset(rc), rb < end, norm_w(ra), norm_w(rc), ra <= group, rb <= group, dest(ra), dest(rc));
     };
+    // PAIR: the records stay in shared memory (through global scratch the merge waited for a trip to the L2 cache): a warp's last part in
+    // its ring, which is idle then, an earlier one behind the pair's rows.
+    static_assert(MAX_PARTS <= 2 * W && (MAX_PARTS - W) * NH * REC * 4 <= (W - 1) * ROWS_BYTES, "room for the records of parts that are not a warp's last");
+    auto record = [&](int part) {
+        return reinterpret_cast<float*>(part + W < my_parts ? tiles + (size_t)NW * TT * TILE_BYTES + ROWS_BYTES + (size_t)part * group * REC * 4
+                                                            : tiles + (size_t)(part % W) * TT * TILE_BYTES);
+    };
     if (PAIR) {
         // the pair's rows, a warp at one or two of them
         const int n_rows = group + (proj.write_kv ? 2 : 0);
@@ -639,7 +646,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             }
         } else {
             // the part's record, for the merge
-            float* rec = partials + ((int64_t)pair * part_stride + cw.part) * group * REC;
+            float* rec = PAIR ? record(cw.part) : partials + ((int64_t)pair * part_stride + cw.part) * group * REC;
 #pragma unroll
             for (int mb = 0; mb < KS; ++mb) {
                 const int d = 16 * mb + r0;
@@ -666,8 +673,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             const int pair = (int)blockIdx.x;
 #pragma unroll 1
             for (int h = warp; h < group; h += W) {
-                const float* first = partials + ((int64_t)pair * part_stride * group + h) * REC;
-                merge_head([&](int p, int i) { return ld_cg(first + (int64_t)p * group * REC + i); }, my_parts, lane,
+                merge_head([&](int p, int i) { return record(p)[h * REC + i]; }, my_parts, lane,
                            out + ((int64_t)(pair / n_kv) * n_heads + (pair % n_kv) * group + h) * HD);
             }
         }
