@@ -764,17 +764,18 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
     const int pages = ceil_div(max_kv_len > 0 ? max_kv_len : 1, kPage);
     static int force = -2;                             // WICK_B200_PAIR_DECODE=0/1: never / whenever possible (for measurements)
     if (force == -2) force = getenv("WICK_B200_PAIR_DECODE") ? atoi(getenv("WICK_B200_PAIR_DECODE")) : -1;
-    // Measured (8 kv heads of 128, one B200): a block per pair costs about 5 us + 0.4 us a page whatever the
-    // number of pairs, until the SMs that have a pair cannot keep the memory busy between them; the persistent
-    // form costs about 9 us + the step's bytes at 5 TB/s.
-    const bool pays = pages <= 16 || pairs >= 96 || (pairs >= 24 && pages <= 24) || (pairs >= 48 && pages <= 32);
-    // More pairs than SMs: the blocks run in waves, in which a long pair's block is followed by whatever is left; the persistent
-    // form deals parts in equal numbers, whatever their length, and its warps have one or two each up to some 400 pairs.  Beyond, where no
-    // sequence has more than 16 pages, the blocks' starts and ends cost more than that (64 x 64 to 400 positions: 26.5 us persistent, 29.1
-    // in waves; 56 x 1,000: 56 and 60); with longer ones 64 x 64 to 1,536 take 54 persistent and 50 in waves, 128 of them 105 and 86, 64 x
-    // 1,500 to 3,900 146 and 134, 64 x 1,500 81 and 74, 64 x 2,000 100 and 103, 256 x 100 to 1,500 179 and 162.
+    // Measured (8 kv heads of 128, one B200), us persistent / a block per pair.  Up to one pair an SM: a block's warps take a part each up to 24
+    // pages (8 pairs of 1,500 positions 15.0 / 11.0), beyond some take two, one after the other (1,800: 12.3 / 17.3; 64 pairs 18.4 / 19.5), which
+    // pays where there are pairs enough to keep the memory busy (96 pairs of 1,800, 3,900: 26.2 / 23.4, 42.7 / 41.5).
+    const bool pays = pages <= 24 || pairs >= 96;
+    // More pairs than SMs: the blocks run in waves, in which a long pair's block is followed by whatever is left, unless the last
+    // wave is mostly empty (160 pairs of 2,000: 43.8 / 48.6); the persistent form deals parts in equal numbers, whatever their length.  It
+    // is the better one where parts are so short that the blocks' starts and ends count (256 pairs of 100 positions 9.9 / 12.5, of 300 16.0 /
+    // 14.5; beyond some 400 pairs 64 to 400 positions 46.2 / 53.6, 64 to 600 89 / 87, 64 to 1,000 85.7 / 67.6, 640 73.7 / 68.1, 64 to
+    // 1,536 105 / 86).  Heads of 64 have twice the warps a block: 512 pairs of 640 26.2 / 30.2, of 64 to 1,500 36.5 / 36.8.
     const long long waves = (pairs + sms - 1) / sms;
-    const bool waves_pay = (pairs <= 400 || pages > 16) && pairs * 10 >= waves * sms * 6;
+    const int least = pairs <= 400 ? 4 : HD == 64 ? 17 : 9;
+    const bool waves_pay = pages >= least && pairs * 10 >= waves * sms * 6;
     const bool pair_form = force >= 0 ? force == 1 : (pairs <= sms ? pays : waves_pay);
     if (pair_form) {
         // Few pairs of short parts: a block per pair, its warps at the pair's parts, merged by the block itself.
