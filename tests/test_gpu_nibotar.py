@@ -302,6 +302,54 @@ def test_bulk_copy_decode_attention_equals_the_warp_kernel(mask, size, d, H, G, 
         assert (out.float() - ref.float()).abs().max().item() < (2e-5 if dtype == torch.float32 else 0.02), (mask, size, d)
 
 
+@pytest.mark.parametrize("d,H,G", [(128, 8, 2), (64, 6, 1), (128, 5, 5), (128, 16, 2)])
+@pytest.mark.parametrize("mask,size", [("block", 100), ("window", 64), ("window", 129), ("block", 1024), ("causal", 0)])
+def test_decode_attention_with_a_mask_on_tensor_cores(mask, size, d, H, G):
+    """Lengths at the edges of pages, of a mask's blocks and windows and of parts, few sequences (a block per pair of sequence and key
+    head) and many (persistent blocks and a merge): against 64 bits no further off than one rounding of the result to bfloat16 (2^-8 of
+    the largest), what hidden and unwritten rows hold (NaN) not seen.  A sequence's bits do not depend on the batch."""
+    g = torch.Generator().manual_seed(91)
+    lens = [1, 63, 64, 65, 100, 101, 128, 129, 200, 201, 640, 1023, 1024, 1025, 1100, 1700, 2111]
+    if G == 5:
+        lens = [70, 1, 700] * 22                       # 330 pairs, the most with 11 pages
+    n_pages = [(n + PAGE - 1) // PAGE for n in lens]
+    total = 1 + sum(n_pages)
+    kv = torch.full((total, 2, G, PAGE, d), float("nan"))
+    pages, nxt = [], 1
+    ks, vs = [], []
+    for n, c in zip(lens, n_pages):
+        pages.append(list(range(nxt, nxt + c)))
+        nxt += c
+        k, v = (torch.randn(n, G, d, generator=g).bfloat16().float() for _ in range(2))
+        p = torch.arange(n)
+        lo = (n - 1) // size * size if mask == "block" else (max(0, n - size) if mask == "window" else 0)
+        kv[torch.tensor(pages[-1])[p // PAGE], 0, :, p % PAGE] = torch.where((p >= lo)[:, None, None], k, torch.tensor(float("nan")))
+        kv[torch.tensor(pages[-1])[p // PAGE], 1, :, p % PAGE] = torch.where((p >= lo)[:, None, None], v, torch.tensor(float("nan")))
+        ks.append(k[lo:])
+        vs.append(v[lo:])
+    q = torch.randn(len(lens), H, d, generator=g).bfloat16()
+    sink = torch.randn(H, generator=g)
+    kvd = kv.bfloat16().to(DEV)
+
+    def step(which):
+        lay = BatchLayout(len(which), len(which), max(n_pages), 0)
+        host = np.zeros(lay.size, dtype=np.int32)
+        fill_host(lay, host, tokens=[[0]] * len(which), starts=[lens[i] - 1 for i in which], slots=list(range(len(which))),
+                  pages=[pages[i] for i in which], want=[[]] * len(which))
+        batch = StepBatch(lay, torch.from_numpy(host).to(DEV), q_lens=[1] * len(which), starts=[lens[i] - 1 for i in which])
+        return ops.attention_masked(q[which].to(DEV), kvd, batch, 0.2, n_kv=G, v_dim=d, mask=mask, mask_size=size,
+                                    sink=sink.to(DEV), kind="bulk").cpu()
+    out = step(list(range(len(lens))))
+    for i in range(len(lens)):
+        k, v = (x.double().repeat_interleave(H // G, 1) for x in (ks[i], vs[i]))
+        s = torch.einsum("hd,nhd->hn", q[i].double(), k) * 0.2
+        w = torch.softmax(torch.cat([s, sink.double()[:, None]], 1), 1)[:, :-1]
+        want = torch.einsum("hn,nhd->hd", w, v)
+        assert (out[i].double() - want).abs().max() <= 2 ** -8 * want.abs().max(), (lens[i], mask, size)
+    for i in (0, len(lens) // 2, len(lens) - 1):
+        assert torch.equal(step([i])[0], out[i]), lens[i]
+
+
 @pytest.mark.parametrize("size", [50, 64])
 def test_one_key_that_stands_out_shows_on_which_side_of_an_edge_it_lies(size):
     """Key j is made to dominate every query that sees it (its score is far above all others) and its value is

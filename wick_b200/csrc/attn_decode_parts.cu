@@ -118,14 +118,35 @@ __device__ __forceinline__ uint32_t ld_cg_u32(const void* p) {
 // 2^(a - b) for maxima that may be -inf (nothing seen yet): then the weight is 0.
 __device__ __forceinline__ float weight(float a, float b) { return a == -INFINITY ? 0.f : exp2f(a - b); }
 
+// What a token sees, and a score per head that joins the softmax's denominator without a value.
+struct Mask {
+    int kind, size;            // -1 nothing of this (and the form that holds it off), 0 every earlier key, 1 those of the token's own block of `size` positions, 2 the last `size` positions
+    const float* sink;         // float32 [n_heads], or null
+};
+__device__ __forceinline__ int first_visible_key(int p, const Mask& mk) {
+    return mk.kind == 1 ? p / mk.size * mk.size : (mk.kind == 2 ? max(0, p - mk.size + 1) : 0);
+}
+// Pages before the one that holds the first key that the token at the end of `len` positions sees.
+template <bool MASKED> __device__ __forceinline__ int skipped_pages(int len, const Mask& mk) {
+    return MASKED && len > 0 ? first_visible_key(len - 1, mk) / kPage : 0;
+}
+// p = t[0] + t[1] + t[2], each a bfloat16 number (the differences are exact).  For p in [0, 1].
+__device__ __forceinline__ void split3(float p, float (&t)[3]) {
+    t[0] = __bfloat162float(__float2bfloat16_rn(p));
+    p -= t[0];
+    t[1] = __bfloat162float(__float2bfloat16_rn(p));
+    t[2] = p - t[1];
+}
+
 // One head of a pair: its P parts' records folded in part order into a running maximum M, sum
 // l and accumulator o (a lane holds HD / 32 dims):
 //   M' = max(M, m_p);  l = l 2^(M - M') + l_p 2^(m_p - M');  o likewise;  out = o / l.
 // word(p, i) gives word i of part p's record (i < HD: the accumulator, HD: the maximum, HD + 1:
 // the sum).  Every product and sum is rounded on its own, so that the result does not depend on
 // which kernel this is compiled into.
+// sink2: a score in units of log2 e that joins the sum (-inf: none).
 template <typename Word>
-__device__ __forceinline__ void merge_head(Word word, int P, int lane, bf16* dst) {
+__device__ __forceinline__ void merge_head(Word word, int P, int lane, bf16* dst, float sink2) {
     float bo[MAX_PARTS][EPL], bm[MAX_PARTS], bl[MAX_PARTS];
 #pragma unroll
     for (int p = 0; p < MAX_PARTS; ++p) {
@@ -135,7 +156,7 @@ __device__ __forceinline__ void merge_head(Word word, int P, int lane, bf16* dst
 #pragma unroll
         for (int e = 0; e < EPL; ++e) bo[p][e] = word(pp, lane + 32 * e);
     }
-    float M = -INFINITY, l = 0.f, o[EPL];
+    float M = sink2, l = sink2 == -INFINITY ? 0.f : 1.f, o[EPL];
 #pragma unroll
     for (int e = 0; e < EPL; ++e) o[e] = 0.f;
 #pragma unroll
@@ -158,19 +179,21 @@ __device__ __forceinline__ void merge_head(Word word, int P, int lane, bf16* dst
 struct Walk {
     int u;                     // the part's number among all parts of the step
     int b, kvh, part;          // its sequence, kv head and number within the pair
-    int len, n_pages, parts;   // of sequence b
+    int len, n_pages, parts;   // of sequence b (pages: those with visible keys)
+    int skipped;               // pages before them
     int page, page_end;        // the page (of the sequence) it is at, and the part's end
     int is_v;                  // the tile of that page: keys (0) or values (1)
 };
 
 // cum, lens: the block's copies (shared memory) of the parts before each sequence and of the lengths.  PAIR: the walk holds
 // the one pair's sequence and head already, and its parts are counted from 0.
-template <bool PAIR>
-__device__ __forceinline__ void open_part(Walk& w, const int* cum, const int* lens, int n_kv) {
+template <bool PAIR, bool MASKED>
+__device__ __forceinline__ void open_part(Walk& w, const int* cum, const int* lens, int n_kv, const Mask& mk) {
     if (!PAIR) {
         while (w.u >= cum[w.b + 1]) ++w.b;             // (parts are visited in order: b only moves forward)
         w.len = lens[w.b];
-        w.n_pages = (w.len + kPage - 1) / kPage;
+        w.skipped = skipped_pages<MASKED>(w.len, mk);
+        w.n_pages = (w.len + kPage - 1) / kPage - w.skipped;
     }
     const int pp = pages_per_part(w.n_pages);
     if (PAIR) {
@@ -212,12 +235,14 @@ struct Projection {
 // (persistent form) all parts of the step are dealt to the warps of one block per SM, and the
 // merge kernel follows.  Which form runs changes no bit: a part is computed by one warp in the
 // same way, and the parts are folded in the same order with the same operations.
-template <bool PREP, bool PAIR>
+// MASKED: the token sees the keys from first_visible_key on, and a sink joins; probabilities enter the second product as the exact sum of
+// three bfloat16 numbers (the CUDA-core kernel that this form stands in for holds them in 32 bits).
+template <bool PREP, bool PAIR, bool MASKED = false>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16* q, Projection proj, bf16* __restrict__ out,
                          const int* __restrict__ kv_len_arr, const int* __restrict__ page_table, int table_width,
                          int n_seqs, int n_heads, int n_kv, float scale, float* partials, int part_stride, int kv_pages,
-                         int* status) {
+                         int* status, const Mask mk) {
     constexpr int NW = W;                              // warps of a block
     constexpr int TT = T;                              // tiles of a warp's ring
     constexpr int u_step = PAIR ? W : 1;               // from a warp's part to its next one
@@ -246,12 +271,13 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         const int pair = (int)blockIdx.x;
         b_base = pair / n_kv;
         const int len = kv_len_arr[b_base];            // (in place before the step's first kernel starts, see below)
-        const int n_pages = (len + kPage - 1) / kPage;
-        const bool fits = len > 0 && n_pages <= table_width && parts_of(n_pages) <= part_stride;
+        const int skipped = skipped_pages<MASKED>(len, mk), n_pages = (len + kPage - 1) / kPage - skipped;
+        const bool fits = len > 0 && n_pages + skipped <= table_width && parts_of(n_pages) <= part_stride;
         if (len > 0 && !fits && tid == 0) atomicCAS(status, 0, 10);
         my_parts = fits ? parts_of(n_pages) : 0;
         pw.len = len;
         pw.n_pages = n_pages;
+        pw.skipped = skipped;
         pw.parts = my_parts;
         pw.kvh = pair % n_kv;
         u0 = warp;                                     // this warp's parts: warp, warp + W, ...
@@ -266,8 +292,8 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             int mine = 0;
             if (s < n_seqs) {
                 const int len = kv_len_arr[s];
-                const int n_pages = (len + kPage - 1) / kPage;
-                if (len > 0 && n_pages <= table_width && parts_of(n_pages) <= part_stride) mine = parts_of(n_pages) * n_kv;
+                const int skipped = skipped_pages<MASKED>(len, mk), n_pages = (len + kPage - 1) / kPage - skipped;
+                if (len > 0 && n_pages + skipped <= table_width && parts_of(n_pages) <= part_stride) mine = parts_of(n_pages) * n_kv;
                 else if (len > 0) atomicCAS(status, 0, 10);      // longer than its page table or than the scratch allows: left out, and said so
                 lens[s] = mine ? len : 0;
             }
@@ -305,7 +331,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         }
         pw.u = u0;
         pw.b = lo;
-        if (work) open_part<PAIR>(pw, cum, lens, n_kv);
+        if (work) open_part<PAIR, MASKED>(pw, cum, lens, n_kv, mk);
         cw = pw;
     }
     // The page ids of a part: lane j holds the part's j-th page (a part of more than 32 pages
@@ -315,7 +341,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
     // warp meanwhile.
     auto page_ids = [&](const Walk& w) -> int {
         const int j = w.page + lane;
-        return j < w.page_end ? page_table[(int64_t)(b_base + w.b) * table_width + j] : 0;
+        return j < w.page_end ? page_table[(int64_t)(b_base + w.b) * table_width + (MASKED ? w.skipped : 0) + j] : 0;
     };
     Walk nw = pw;                                      // the part after pw's
     int ids = work ? page_ids(pw) : 0, ids_next = 0, ids_first = pw.page;
@@ -323,7 +349,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         nw = pw;
         nw.u = pw.u + u_step;
         if (nw.u < u1) {
-            open_part<PAIR>(nw, cum, lens, n_kv);
+            open_part<PAIR, MASKED>(nw, cum, lens, n_kv, mk);
             ids_next = page_ids(nw);
         }
     };
@@ -338,7 +364,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         if (dead || pw.u >= u1 || issued - consumed >= (uint32_t)TT) return false;
         if (!PREP && !after_wait && pw.page == pw.n_pages - 1) return false;   // (that kernel writes this page)
         const int j = pw.page - ids_first;
-        const int page = j < 32 ? __shfl_sync(0xffffffffu, ids, j) : page_table[(int64_t)(b_base + pw.b) * table_width + pw.page];
+        const int page = j < 32 ? __shfl_sync(0xffffffffu, ids, j) : page_table[(int64_t)(b_base + pw.b) * table_width + (MASKED ? pw.skipped : 0) + pw.page];
         if (page < 0 || page >= kv_pages) {            // a page outside the cache: give up, say so
             if (lane == 0) {
                 *(volatile int*)&abort_flag = 1;
@@ -518,7 +544,9 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
 #pragma unroll 1
         for (int turn = 2 * cw.page; turn < 2 * cw.page_end; ++turn) {
             const int page = turn >> 1;
-            const int keys_here = min(kPage, cw.len - page * kPage);
+            const int at = (MASKED ? cw.skipped + page : page) * kPage;     // the page's first position
+            const int keys_here = min(kPage, cw.len - at);
+            const int hidden = MASKED ? max(0, first_visible_key(cw.len - 1, mk) - at) : 0;   // keys before the first visible one
 #pragma unroll 1
             while (issue(true)) {}
             const uint32_t s = consumed % TT;
@@ -545,10 +573,10 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
                         mma16816(sc[mb], a, qb[ks][0], qb[ks][1]);
                     }
                     const int ka = 16 * mb + r0, kb = ka + 8;
-                    sc[mb][0] = ka < keys_here ? __fmul_rn(sc[mb][0], sl2) : -INFINITY;
-                    sc[mb][1] = ka < keys_here ? __fmul_rn(sc[mb][1], sl2) : -INFINITY;
-                    sc[mb][2] = kb < keys_here ? __fmul_rn(sc[mb][2], sl2) : -INFINITY;
-                    sc[mb][3] = kb < keys_here ? __fmul_rn(sc[mb][3], sl2) : -INFINITY;
+                    sc[mb][0] = ka < keys_here && (!MASKED || ka >= hidden) ? __fmul_rn(sc[mb][0], sl2) : -INFINITY;
+                    sc[mb][1] = ka < keys_here && (!MASKED || ka >= hidden) ? __fmul_rn(sc[mb][1], sl2) : -INFINITY;
+                    sc[mb][2] = kb < keys_here && (!MASKED || kb >= hidden) ? __fmul_rn(sc[mb][2], sl2) : -INFINITY;
+                    sc[mb][3] = kb < keys_here && (!MASKED || kb >= hidden) ? __fmul_rn(sc[mb][3], sl2) : -INFINITY;
                     mx0 = fmaxf(mx0, fmaxf(sc[mb][0], sc[mb][2]));
                     mx1 = fmaxf(mx1, fmaxf(sc[mb][1], sc[mb][3]));
                 }
@@ -563,7 +591,8 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             const float n0 = fmaxf(mr0, mx0), n1 = fmaxf(mr1, mx1);
             const float a0 = weight(mr0, n0), a1 = weight(mr1, n1);
             float l0 = 0.f, l1 = 0.f;
-            uint32_t pb[4][2];                         // P[key, head] as the 8-wide operand of the second product
+            constexpr int TERMS = MASKED ? 3 : 1;
+            uint32_t pb[TERMS][4][2];                  // P[key, head] as the 8-wide operand of the second product
             if (ok) {
 #pragma unroll
                 for (int mb = 0; mb < 4; ++mb) {
@@ -572,8 +601,18 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
                     l0 = __fadd_rn(l0, __fadd_rn(p0, p2));
                     l1 = __fadd_rn(l1, __fadd_rn(p1, p3));
                     // rows = keys (r0, r0 + 8), columns = heads (c0, c0 + 1) -> rows = heads, columns = keys
-                    pb[mb][0] = transpose8x8(pack_bf16(p0, p1));
-                    pb[mb][1] = transpose8x8(pack_bf16(p2, p3));
+                    if constexpr (MASKED) {
+                        float t0[3], t1[3], t2[3], t3[3];
+                        split3(p0, t0), split3(p1, t1), split3(p2, t2), split3(p3, t3);
+#pragma unroll
+                        for (int z = 0; z < TERMS; ++z) {
+                            pb[z][mb][0] = transpose8x8(pack_bf16(t0[z], t1[z]));
+                            pb[z][mb][1] = transpose8x8(pack_bf16(t2[z], t3[z]));
+                        }
+                    } else {
+                        pb[0][mb][0] = transpose8x8(pack_bf16(p0, p1));
+                        pb[0][mb][1] = transpose8x8(pack_bf16(p2, p3));
+                    }
                 }
             }
 #pragma unroll
@@ -598,6 +637,12 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             if (ok && new_row >= 0 && lane < HD / 8)
                 *reinterpret_cast<uint4*>(v_tile + tile_off(new_row, lane)) = reinterpret_cast<const uint4*>(rows_s[NH + 1])[lane];
             if (ok && new_row >= 0) __syncwarp();
+            if (MASKED && ok && hidden > 0) {            // (nothing that a hidden value holds reaches the sum)
+#pragma unroll 1
+                for (int i = lane; i < hidden * (HD / 8); i += 32)
+                    *reinterpret_cast<uint4*>(v_tile + tile_off(i / (HD / 8), i % (HD / 8))) = make_uint4(0, 0, 0, 0);
+                __syncwarp();
+            }
             if (ok && keys_here < kPage) {
                 // Rows of the last page that hold no token yet may be anything: make them zero,
                 // so that a zero weight times such a row stays zero.
@@ -617,7 +662,8 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
                     for (int mb = 0; mb < KS; ++mb) {
                         uint32_t a[4];
                         ldsm_x4_trans(a, v_base + tile_off(key, 2 * mb + ((lane >> 3) & 1)));
-                        mma16816(acc[mb], a, pb[j][0], pb[j][1]);
+#pragma unroll
+                        for (int z = TERMS - 1; z >= 0; --z) mma16816(acc[mb], a, pb[z][j][0], pb[z][j][1]);
                     }
                 }
             }
@@ -630,6 +676,21 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
 
         if (cw.parts == 1) {
             // the pair's only part: straight to the output rows
+            if (MASKED && mk.sink) {                     // the sink's share of each head's sum, all scaled by the larger of the two
+                auto join = [&](int c, float m, float& l, float& f) {
+                    const float s2 = mk.sink[kvh * group + min(c, group - 1)] * 1.4426950408889634f, n = fmaxf(m, s2);
+                    f = weight(m, n);
+                    l = __fadd_rn(__fmul_rn(l, f), weight(s2, n));
+                };
+                float f0, f1;
+                join(c0, mr0, lr0, f0);
+                join(c0 + 1, mr1, lr1, f1);
+#pragma unroll
+                for (int mb = 0; mb < KS; ++mb) {
+                    acc[mb][0] *= f0, acc[mb][2] *= f0;
+                    acc[mb][1] *= f1, acc[mb][3] *= f1;
+                }
+            }
             const float i0 = lr0 > 0.f ? __fdiv_rn(1.0f, lr0) : 0.f, i1 = lr1 > 0.f ? __fdiv_rn(1.0f, lr1) : 0.f;
             bf16* o0 = out + ((int64_t)b * n_heads + kvh * group + c0) * HD;
 #pragma unroll
@@ -665,7 +726,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             }
         }
         cw.u += u_step;
-        if (cw.u < u1) open_part<PAIR>(cw, cum, lens, n_kv);
+        if (cw.u < u1) open_part<PAIR, MASKED>(cw, cum, lens, n_kv, mk);
     }
     if (PAIR) {
         __syncthreads();                               // every part's record is written (and visible to this block)
@@ -674,7 +735,8 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
 #pragma unroll 1
             for (int h = warp; h < group; h += W) {
                 merge_head([&](int p, int i) { return record(p)[h * REC + i]; }, my_parts, lane,
-                           out + ((int64_t)(pair / n_kv) * n_heads + (pair % n_kv) * group + h) * HD);
+                           out + ((int64_t)(pair / n_kv) * n_heads + (pair % n_kv) * group + h) * HD,
+                           MASKED && mk.sink ? mk.sink[(pair % n_kv) * group + h] * 1.4426950408889634f : -INFINITY);
             }
         }
     }
@@ -691,7 +753,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
 // Pairs with one part were written by the first kernel and are skipped.
 __global__ void __launch_bounds__(128)
 attn_decode_merge_kernel(const float* partials, bf16* __restrict__ out, const int* __restrict__ kv_len_arr, int table_width,
-                         int n_seqs, int n_heads, int n_kv, int part_stride) {
+                         int n_seqs, int n_heads, int n_kv, int part_stride, const Mask mk) {
     pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int group = n_heads / n_kv;
@@ -699,15 +761,16 @@ attn_decode_merge_kernel(const float* partials, bf16* __restrict__ out, const in
     if (item >= n_seqs * n_heads) return;
     const int pair = item / group, h = item % group;
     const int len = kv_len_arr[pair / n_kv];           // (the step's lengths are in place before the step starts)
-    const int n_pages = (len + kPage - 1) / kPage;
-    if (len <= 0 || n_pages > table_width) return;
+    const int skipped = skipped_pages<true>(len, mk), n_pages = (len + kPage - 1) / kPage - skipped;
+    if (len <= 0 || n_pages + skipped > table_width) return;
     const int P = parts_of(n_pages);
     if (P < 2 || P > part_stride) return;
     pdl_wait();                                        // the records
     partials = fresh(partials);
     const float* first = partials + ((int64_t)pair * part_stride * group + h) * REC;
     merge_head([&](int p, int i) { return ld_cg(first + (int64_t)p * group * REC + i); }, P, lane,
-               out + ((int64_t)(pair / n_kv) * n_heads + (pair % n_kv) * group + h) * HD);
+               out + ((int64_t)(pair / n_kv) * n_heads + (pair % n_kv) * group + h) * HD,
+               mk.sink ? mk.sink[(pair % n_kv) * group + h] * 1.4426950408889634f : -INFINITY);
 }
 
 }  // namespace decodeparts
@@ -739,7 +802,7 @@ WICK_API long long wick_attn_decode_parts_scratch(int n_seqs, int n_heads, int n
 
 static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, const void* kv, long long kv_pages, void* out,
                         float* scratch, long long scratch_words, const int* kv_len, int n_seqs, int max_kv_len,
-                        const int* page_table, int table_width, int n_heads, int n_kv, float scale, int* status, void* s) {
+                        const int* page_table, int table_width, int n_heads, int n_kv, float scale, int* status, decodeparts::Mask mk, void* s) {
     using namespace decodeparts;
     WICK_REQUIRE(SUPPORTED, "attention decode: head_dim %d is not 64 or 128", (int)WICK_HD);
     WICK_REQUIRE(wick_attn_decode_parts_supported(n_seqs, n_heads, n_kv), "attention decode: %d sequences, %d heads over %d kv heads is beyond this kernel", n_seqs, n_heads, n_kv);
@@ -758,10 +821,14 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
         WICK_CUDA(cudaFuncSetAttribute(attn_decode_parts_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         WICK_CUDA(cudaFuncSetAttribute(attn_decode_parts_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         WICK_CUDA(cudaFuncSetAttribute(attn_decode_parts_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        WICK_CUDA(cudaFuncSetAttribute(attn_decode_parts_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        WICK_CUDA(cudaFuncSetAttribute(attn_decode_parts_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         raised = true;
     }
     const long long pairs = (long long)n_seqs * n_kv;
-    const int pages = ceil_div(max_kv_len > 0 ? max_kv_len : 1, kPage);
+    const bool masked = mk.kind >= 0;
+    int pages = ceil_div(max_kv_len > 0 ? max_kv_len : 1, kPage);            // (the most with visible keys)
+    if (mk.kind > 0) pages = min(pages, ceil_div(mk.size, kPage) + 1);
     static int force = -2;                             // WICK_B200_PAIR_DECODE=0/1: never / whenever possible (for measurements)
     if (force == -2) force = getenv("WICK_B200_PAIR_DECODE") ? atoi(getenv("WICK_B200_PAIR_DECODE")) : -1;
     // Measured (8 kv heads of 128, one B200), us persistent / a block per pair.  Up to one pair an SM: a block's warps take a part each up to 24
@@ -780,30 +847,38 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
     if (pair_form) {
         // Few pairs of short parts: a block per pair, its warps at the pair's parts, merged by the block itself.
         // (Longer parts, or more pairs than SMs, want the self-fed warps of the persistent form.)
-        if (prep)
+        if (masked)
+            WICK_CUDA(launch(attn_decode_parts_kernel<false, true, true>, dim3((unsigned)pairs), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, map,
+                             (const bf16*)q, proj, (bf16*)out, kv_len, page_table, table_width, n_seqs, n_heads, n_kv, scale, scratch,
+                             stride, (int)kv_pages, status, mk));
+        else if (prep)
             WICK_CUDA(launch(attn_decode_parts_kernel<true, true>, dim3((unsigned)pairs), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, map,
                              (const bf16*)q, proj, (bf16*)out, kv_len, page_table, table_width, n_seqs, n_heads, n_kv, scale, scratch,
-                             stride, (int)kv_pages, status));
+                             stride, (int)kv_pages, status, mk));
         else
             WICK_CUDA(launch(attn_decode_parts_kernel<false, true>, dim3((unsigned)pairs), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, map,
                              (const bf16*)q, proj, (bf16*)out, kv_len, page_table, table_width, n_seqs, n_heads, n_kv, scale, scratch,
-                             stride, (int)kv_pages, status));
+                             stride, (int)kv_pages, status, mk));
         return check_launch("attn_decode_parts (a block per pair)");
     }
     // As many blocks as there can be parts, up to one per SM (who computes a part changes no bit).
     const int grid = (int)(most < sms ? most : sms);
-    if (prep)
+    if (masked)
+        WICK_CUDA(launch(attn_decode_parts_kernel<false, false, true>, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, map,
+                         (const bf16*)q, proj, (bf16*)out, kv_len, page_table, table_width, n_seqs, n_heads, n_kv, scale, scratch,
+                         stride, (int)kv_pages, status, mk));
+    else if (prep)
         WICK_CUDA(launch(attn_decode_parts_kernel<true, false>, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, map,
                          (const bf16*)q, proj, (bf16*)out, kv_len, page_table, table_width, n_seqs, n_heads, n_kv, scale, scratch,
-                         stride, (int)kv_pages, status));
+                         stride, (int)kv_pages, status, mk));
     else
         WICK_CUDA(launch(attn_decode_parts_kernel<false, false>, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, map,
                          (const bf16*)q, proj, (bf16*)out, kv_len, page_table, table_width, n_seqs, n_heads, n_kv, scale, scratch,
-                         stride, (int)kv_pages, status));
+                         stride, (int)kv_pages, status, mk));
     if (int e = check_launch("attn_decode_parts")) return e;
     if (stride > 1) {
         WICK_CUDA(launch(attn_decode_merge_kernel, dim3(ceil_div((long long)n_seqs * n_heads, 4)), dim3(128), 0, (cudaStream_t)s,
-                         (const float*)scratch, (bf16*)out, kv_len, table_width, n_seqs, n_heads, n_kv, stride));
+                         (const float*)scratch, (bf16*)out, kv_len, table_width, n_seqs, n_heads, n_kv, stride, mk));
         return check_launch("attn_decode_merge");
     }
     return 0;
@@ -820,7 +895,18 @@ WICK_API int wick_attn_decode_parts_bf16(const void* q, const void* kv, long lon
                                          int* status, void* s) {
     decodeparts::Projection none = {};
     return launch_parts(false, q, none, kv, kv_pages, out, scratch, scratch_words, kv_len, n_seqs, max_kv_len, page_table,
-                        table_width, n_heads, n_kv, scale, status, s);
+                        table_width, n_heads, n_kv, scale, status, decodeparts::Mask{-1, 0, nullptr}, s);
+}
+
+// ... then the mask (0, or 1 / 2 with its size) and the sinks (float32 [n_heads] or null).
+WICK_API int wick_attn_decode_parts_masked_bf16(const void* q, const void* kv, long long kv_pages, void* out, float* scratch,
+                                                long long scratch_words, const int* kv_len, int n_seqs, int max_kv_len,
+                                                const int* page_table, int table_width, int n_heads, int n_kv, float scale,
+                                                int* status, int mask, int mask_size, const float* sink, void* s) {
+    WICK_REQUIRE(mask == 0 || ((mask == 1 || mask == 2) && mask_size > 0), "attention: mask %d of size %d", mask, mask_size);
+    decodeparts::Projection none = {};
+    return launch_parts(false, q, none, kv, kv_pages, out, scratch, scratch_words, kv_len, n_seqs, max_kv_len, page_table,
+                        table_width, n_heads, n_kv, scale, status, decodeparts::Mask{mask, mask_size, sink}, s);
 }
 
 // The same from the q/k/v projection's float32 partial sums [splits, n_seqs, (n_heads + 2 n_kv) HD]:
@@ -837,5 +923,5 @@ WICK_API int wick_attn_decode_parts_fused_bf16(const float* sums, int splits, co
     WICK_REQUIRE((q_w == nullptr) == (k_w == nullptr) && (cos_t == nullptr) == (sin_t == nullptr), "attention decode: q and k norm weights come together, and so do the rotation tables");
     Projection proj = {sums, splits, (int64_t)n_seqs * (n_heads + 2 * n_kv) * HD, q_w, k_w, eps, cos_t, sin_t, (bf16*)kv, write_kv};
     return launch_parts(true, nullptr, proj, kv, kv_pages, out, scratch, scratch_words, kv_len, n_seqs, max_kv_len, page_table,
-                        table_width, n_heads, n_kv, scale, status, s);
+                        table_width, n_heads, n_kv, scale, status, decodeparts::Mask{-1, 0, nullptr}, s);
 }

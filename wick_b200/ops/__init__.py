@@ -1162,6 +1162,15 @@ def attention_masked(q: torch.Tensor, kv: torch.Tensor, batch, scale: float, *, 
     if kind == "bulk":
         _need(d == v_dim and batch.is_decode, "the bulk-copy kernel takes one token per sequence and one head size")
         mk = batch.kv_bound
+        if q.dtype == torch.bfloat16 and attention_decode_parts_supported(batch.n_seqs, n_heads, n_kv, d, q.dtype):
+            need = attention_decode_parts_scratch(batch.n_seqs, n_heads, n_kv, d, mk)
+            ws = getattr(batch, "workspace", None)
+            scratch = ws.get("attention_decode", need, torch.float32) if ws is not None else \
+                torch.empty(need, dtype=torch.float32, device=q.device)
+            _attn(d).call("wick_attn_decode_parts_masked_bf16", "pplpplpiipiiifpiipp", _p(q), _p(kv), kv.shape[0], _p(out), _p(scratch),
+                          scratch.numel(), _p(batch.kv_len), n, mk, _p(batch.page_table), batch.table_width, n_heads, n_kv,
+                          float(scale), _p(status_tensor(q.device)), MASKS[mask], int(mask_size), _p(sink), _stream(), kernels=2 if mk > 128 else 1)
+            return out
         need = attention_decode_scratch_floats(batch.n_seqs, n_heads, d, mk, q.dtype)
         ws = getattr(batch, "workspace", None)
         scratch = ws.get("attention_decode", need, torch.float32) if ws is not None else \
