@@ -303,7 +303,7 @@ def test_bulk_copy_decode_attention_equals_the_warp_kernel(mask, size, d, H, G, 
 
 
 @pytest.mark.parametrize("d,H,G", [(128, 8, 2), (64, 6, 1), (128, 5, 5), (128, 16, 2)])
-@pytest.mark.parametrize("mask,size", [("block", 100), ("window", 64), ("window", 129), ("block", 1024), ("causal", 0)])
+@pytest.mark.parametrize("mask,size", [("block", 100), ("window", 64), ("window", 129), ("block", 1024)])
 def test_decode_attention_with_a_mask_on_tensor_cores(mask, size, d, H, G):
     """Lengths at the edges of pages, of a mask's blocks and windows and of parts, few sequences (a block per pair of sequence and key
     head) and many (persistent blocks and a merge): against 64 bits no further off than one rounding of the result to bfloat16 (2^-8 of
@@ -322,7 +322,7 @@ def test_decode_attention_with_a_mask_on_tensor_cores(mask, size, d, H, G):
         nxt += c
         k, v = (torch.randn(n, G, d, generator=g).bfloat16().float() for _ in range(2))
         p = torch.arange(n)
-        lo = (n - 1) // size * size if mask == "block" else (max(0, n - size) if mask == "window" else 0)
+        lo = (n - 1) // size * size if mask == "block" else max(0, n - size)
         kv[torch.tensor(pages[-1])[p // PAGE], 0, :, p % PAGE] = torch.where((p >= lo)[:, None, None], k, torch.tensor(float("nan")))
         kv[torch.tensor(pages[-1])[p // PAGE], 1, :, p % PAGE] = torch.where((p >= lo)[:, None, None], v, torch.tensor(float("nan")))
         ks.append(k[lo:])
