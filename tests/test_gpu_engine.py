@@ -353,6 +353,20 @@ def test_decode_batch_of_80_sequences(dtype, graphs):
 
 
 @pytest.mark.parametrize("graphs", [False, True])
+def test_decode_batch_beyond_what_the_decode_attention_by_parts_holds(graphs):
+    """1,025 sequences (the kernel by parts takes 1,024): prompts of one to three tokens, then two decode steps."""
+    name, n = "D", 1025
+    eng = make_engine(name, "bfloat16", max_tokens=n * 64, max_seqs=n, use_graphs=graphs)
+    poison_all(eng)
+    seqs = [random_tokens(vocab_of(name), 3 + i % 3, 6000 + i) for i in range(n)]
+    slots = [eng.open_seq() for _ in range(n)]
+    eng.step(slots, [s[:-2] for s in seqs], [[] for _ in seqs])
+    rows = [eng.step(slots, [[s[-k]] for s in seqs]).clone() for k in (2, 1)]
+    for i in (0, 1, 2, 511, 1023, 1024):
+        assert_logits_close(torch.stack([r[i] for r in rows]), plain_logits(name, seqs[i])[-2:], "bfloat16", f"sequence {i}")
+
+
+@pytest.mark.parametrize("graphs", [False, True])
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", ["D", "E"])
 def test_decoding_across_512_and_1024_cached_tokens(name, dtype, graphs):

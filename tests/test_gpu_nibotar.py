@@ -350,6 +350,26 @@ def test_decode_attention_with_a_mask_on_tensor_cores(mask, size, d, H, G):
         assert torch.equal(step([i])[0], out[i]), lens[i]
 
 
+@pytest.mark.parametrize("n", [1024, 1025, 1500])
+def test_a_masked_decode_step_of_more_sequences_than_the_kernel_by_parts_holds(n):
+    """1,024 sequences is the most that the kernel by parts takes; a step of more goes to the bulk-copy kernel."""
+    g = torch.Generator().manual_seed(92)
+    lens = [1 + i % 5 for i in range(n)]
+    kv = torch.randn(n + 1, 2, 2, PAGE, 64, generator=g).bfloat16().to(DEV)
+    q = torch.randn(n, 4, 64, generator=g).bfloat16().to(DEV)
+    sink = torch.randn(4, generator=g).to(DEV)
+    lay = BatchLayout(n, n, 1, 0)
+    host = np.zeros(lay.size, dtype=np.int32)
+    fill_host(lay, host, tokens=[[0]] * n, starts=[m - 1 for m in lens], slots=list(range(n)), pages=[[i + 1] for i in range(n)], want=[[]] * n)
+    batch = StepBatch(lay, torch.from_numpy(host).to(DEV), q_lens=[1] * n, starts=[m - 1 for m in lens])
+    for mask, size in (("block", 3), ("window", 2)):
+        kw = dict(n_kv=2, v_dim=64, mask=mask, mask_size=size, sink=sink)
+        out = ops.attention_masked(q, kv, batch, 0.2, **kw)
+        ref = ops.attention_masked(q, kv, batch, 0.2, kind="warp", **kw)
+        assert (out.float() - ref.float()).abs().max().item() < 0.02
+    ops.check_status()
+
+
 @pytest.mark.parametrize("size", [50, 64])
 def test_one_key_that_stands_out_shows_on_which_side_of_an_edge_it_lies(size):
     """Key j is made to dominate every query that sees it (its score is far above all others) and its value is

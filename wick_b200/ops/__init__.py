@@ -447,10 +447,11 @@ def attention_decode(q: torch.Tensor, kv: torch.Tensor, batch, scale: float, scr
 
 def attention_decode_parts_supported(n_seqs: int, n_heads: int, n_kv: int, head_dim: int, dtype: torch.dtype) -> bool:
     """Whether the tensor-core decode attention whose work is cut by each sequence's own
-    length takes this problem: bfloat16, head size 64 or 128, at most 8 query heads per kv head."""
-    if dtype != torch.bfloat16 or head_dim not in (64, 128) or n_kv <= 0 or n_heads % n_kv != 0 or n_heads // n_kv > 8:
+    length takes this problem: bfloat16, head size 64 or 128, at most 8 query heads per kv head, and
+    as many sequences as the library says (what is beyond it takes the other decode kernels)."""
+    if dtype != torch.bfloat16 or head_dim not in (64, 128):
         return False
-    return n_seqs <= 2048
+    return bool(_attn(head_dim)._lib.wick_attn_decode_parts_supported(n_seqs, n_heads, n_kv))
 
 
 def attention_decode_parts_scratch(n_seqs: int, n_heads: int, n_kv: int, head_dim: int, max_kv_len: int) -> int:
