@@ -1,8 +1,12 @@
 """The rules that send a call to one kernel or another, as far as they can be looked at without a GPU."""
+import os
+import re
+
 import pytest
 import torch
 
 from wick_b200 import ops
+from wick_b200.ops.build import CSRC
 
 
 @pytest.mark.parametrize("hd", [64, 128])
@@ -18,3 +22,44 @@ def test_decode_attention_by_parts_is_offered_only_what_its_library_takes(hd):
     assert not ops.attention_decode_parts_supported(1025, 8, 2, hd, torch.bfloat16)
     assert not ops.attention_decode_parts_supported(1, 8, 2, hd, torch.float32)
     assert not ops.attention_decode_parts_supported(1, 8, 2, 32, torch.bfloat16)
+
+
+def _enclosed(text, at, pair="{}"):
+    """The text from the bracket that opens at or behind ``at`` to the one that closes it."""
+    begin = at = text.index(pair[0], at)
+    depth = 0
+    while True:
+        depth += {pair[0]: 1, pair[1]: -1}.get(text[at], 0)
+        if depth == 0:
+            return text[begin:at + 1]
+        at += 1
+
+
+def _kernels():
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, f)) as fh:
+                text = re.sub(r"//[^\n]*", "", fh.read())
+            for m in re.finditer(r"__global__", text):
+                name = re.compile(r"\w+_kernel(?=\()").search(text, m.end())
+                args = _enclosed(text, name.end(), "()")
+                yield f, name.group(), _enclosed(text, name.end() + len(args))
+
+
+def test_no_kernel_that_lets_its_successor_start_ends_before_it_has_waited():
+    """A kernel waits for the one before it only (griddepcontrol.wait), so that one must not have ended before ITS predecessor has: no
+    thread may leave ahead of the wait.  (Were every thread to leave there, nothing would order the kernel behind it and the kernel
+    ahead of it.)"""
+    found = 0
+    for f, name, body in _kernels():
+        if "pdl_trigger" not in body:
+            continue
+        found += 1
+        while True:                                    # a lambda's own returns leave the lambda only
+            m = re.search(r"\[[&=]?\]\s*\([^()]*\)\s*(?:->\s*\w+\s*)?(?=\{)", body)
+            if not m:
+                break
+            body = body[:m.start()] + body[m.end() + len(_enclosed(body, m.end())):]
+        before = body[:body.index("return")] if "return" in body else body
+        assert "pdl_wait()" in before, f"{name} ({f}) may end before its wait"
+    assert found > 40, "the kernels' sources are not where they were"

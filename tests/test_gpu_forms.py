@@ -3,6 +3,9 @@
 Tolerances: a float32 sum of k products of numbers of order one and 1 / sqrt(k) differs from the exact one by a few 2^-24 times
 sqrt(k) of its own size at most, i.e. below 1e-5 for the sizes here; a result rounded to bfloat16 by 2^-9 of itself."""
 import math
+import os
+import subprocess
+import sys
 import types
 
 import numpy as np
@@ -16,6 +19,7 @@ from wick_b200.engine.batch import BatchLayout, StepBatch, fill_host  # noqa: E4
 
 DEV = "cuda"
 PAGE = 64
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def batch_of(q_lens, starts):
@@ -551,3 +555,49 @@ def test_poly_norm_forms(ff, n, splits):
     got = ops.poly_norm(parts, co, 1e-5, torch.float32)
     assert (got.double() - ref).abs().max() < 5e-6 * float(ref.abs().max())
     assert torch.equal(ops.poly_norm(parts, co, 1e-5, torch.bfloat16), got.bfloat16())
+
+
+# Decode attention and the product that reads it, one behind the other without a look in between, over several caches in turn.
+_ATTENTION_THEN_PRODUCT = """
+import sys
+sys.path[:0] = [{root!r}, {tests!r}]
+import torch
+from wick_b200 import ops
+from wick_b200.ops import gemm_tc as G
+from test_gpu_forms import DEV, batch_of
+lens, mask, size, heads, kv = {case!r}
+batch, pages, n_pages = batch_of([1] * len(lens), [n - 1 for n in lens])
+g = torch.Generator().manual_seed(5)
+store = [torch.randn(n_pages, 2, kv, 64, 64, generator=g).bfloat16().to(DEV) for _ in range(4)]
+q = [torch.randn(len(lens), heads, 64, generator=g).bfloat16().to(DEV) for _ in range(4)]
+plan = G.plan_for(torch.randn(256, heads * 64, generator=g).bfloat16().to(DEV))
+scratch = torch.empty(max(1, ops.attention_decode_parts_scratch(len(lens), heads, kv, 64, 4096)), device=DEV)
+att = torch.zeros(len(lens), heads, 64, dtype=torch.bfloat16, device=DEV)
+got = []
+torch.cuda.synchronize()
+for i in range(16):
+    if mask:
+        a = ops.attention_masked(q[i % 4], store[i % 4], batch, 0.2, n_kv=kv, v_dim=64, mask=mask, mask_size=size, kind="bulk")
+    else:
+        a = ops.attention_decode_parts(q[i % 4], store[i % 4], batch, 0.2, scratch, out=att, max_kv_len=4096)    # (sized as in a captured step)
+    got.append(plan.forward_delta(a.view(len(lens), -1)))
+ops.check_status()
+torch.save([x.cpu() for x in got], sys.argv[1])
+"""
+
+
+@pytest.mark.parametrize("case", [
+    ([700 + i for i in range(40)], "window", 64, 8, 4), ([64 + 65 * (i % 20) for i in range(40)], "window", 65, 8, 4),
+    ([1025 + i for i in range(40)], "block", 1024, 8, 4), ([100] * 64, None, 0, 16, 8)])
+def test_what_follows_a_decode_attention_with_nothing_to_merge_waits_for_it(case, tmp_path):
+    """More pairs of sequence and key head than multiprocessors, every pair in one part (its rows are written by the parts' kernel, the
+    merge behind it has nothing to do): the product that reads the rows gives the same bits with dependent launch and without."""
+    got = []
+    for off in ("0", "1"):
+        out = str(tmp_path / off)
+        run = subprocess.run([sys.executable, "-c", _ATTENTION_THEN_PRODUCT.format(root=ROOT, tests=os.path.join(ROOT, "tests"), case=case), out],
+                             env=dict(os.environ, WICK_B200_NO_PDL=off, WICK_B200_PAIR_DECODE="0"), capture_output=True, text=True, timeout=300)
+        assert run.returncode == 0, run.stderr[-2000:]
+        got.append(torch.load(out))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    assert all(torch.isfinite(a).all() for a in got[0])

@@ -316,7 +316,10 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         const int64_t S = (int64_t)gridDim.x * W, slot = (int64_t)warp * gridDim.x + blockIdx.x;
         u0 = (int)(slot * U / S);
         u1 = (int)((slot + 1) * U / S);
-        if (u0 >= u1) return;
+        if (u0 >= u1) {
+            pdl_wait();                                // (should no warp have a part: see the merge)
+            return;
+        }
     }
     const bool work = u0 < u1;                         // (PAIR: a warp without a part still helps with the rows and the merge)
 
@@ -758,14 +761,15 @@ attn_decode_merge_kernel(const float* partials, bf16* __restrict__ out, const in
     const int lane = threadIdx.x & 31;
     const int group = n_heads / n_kv;
     const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);       // (pair, head)
-    if (item >= n_seqs * n_heads) return;
-    const int pair = item / group, h = item % group;
-    const int len = kv_len_arr[pair / n_kv];           // (the step's lengths are in place before the step starts)
+    const int pair = item / group, h = item % group, b = min(pair / n_kv, n_seqs - 1);
+    const int len = kv_len_arr[b];                     // (the step's lengths are in place before the step starts)
     const int skipped = skipped_pages<true>(len, mk), n_pages = (len + kPage - 1) / kPage - skipped;
-    if (len <= 0 || n_pages + skipped > table_width) return;
+    // Before any warp leaves: the kernel after this one waits for this one only, and the rows of pairs with one part are written by the
+    // kernel before.  Where no warp had anything to merge, nothing would hold that one back until they are.
+    pdl_wait();
+    if (item >= n_seqs * n_heads || len <= 0 || n_pages + skipped > table_width) return;
     const int P = parts_of(n_pages);
     if (P < 2 || P > part_stride) return;
-    pdl_wait();                                        // the records
     partials = fresh(partials);
     const float* first = partials + ((int64_t)pair * part_stride * group + h) * REC;
     merge_head([&](int p, int i) { return ld_cg(first + (int64_t)p * group * REC + i); }, P, lane,
@@ -785,19 +789,29 @@ WICK_API int wick_attn_decode_parts_supported(int n_seqs, int n_heads, int n_kv)
     return n_seqs <= MAX_SEQS ? 1 : 0;
 }
 
-// Scratch for a step of n_seqs sequences of at most max_kv_len positions: float32 words for
-// every part's record.
-static int part_stride_for(int max_kv_len) {
-    using namespace decodeparts;
+// The most pages with visible keys that a sequence of at most max_kv_len positions has, and the most parts.
+static int pages_for(int max_kv_len, const decodeparts::Mask& mk) {
     const int pages = ceil_div(max_kv_len > 0 ? max_kv_len : 1, kPage);
+    return mk.kind > 0 ? min(pages, ceil_div(mk.size, kPage) + 1) : pages;
+}
+static int part_stride_for(int pages) {
+    using namespace decodeparts;
     if (pages <= PART_PAGES) return 1;
     const int halves = ceil_div(pages, PART_PAGES);
     return halves < MAX_PARTS ? halves : MAX_PARTS;
 }
 
+static long long scratch_for(int n_seqs, int n_heads, int n_kv, int stride) {
+    return (long long)n_seqs * n_kv * stride * (n_heads / n_kv) * decodeparts::REC;
+}
+
+// Scratch for a step of n_seqs sequences of at most max_kv_len positions: float32 words for every part's record.
 WICK_API long long wick_attn_decode_parts_scratch(int n_seqs, int n_heads, int n_kv, int max_kv_len) {
-    using namespace decodeparts;
-    return (long long)n_seqs * n_kv * part_stride_for(max_kv_len) * (n_heads / n_kv) * REC;
+    return scratch_for(n_seqs, n_heads, n_kv, part_stride_for(pages_for(max_kv_len, decodeparts::Mask{-1, 0, nullptr})));
+}
+// ... with a mask (1 / 2 with its size).
+WICK_API long long wick_attn_decode_parts_masked_scratch(int n_seqs, int n_heads, int n_kv, int max_kv_len, int mask, int mask_size) {
+    return scratch_for(n_seqs, n_heads, n_kv, part_stride_for(pages_for(max_kv_len, decodeparts::Mask{mask, mask_size, nullptr})));
 }
 
 static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, const void* kv, long long kv_pages, void* out,
@@ -808,11 +822,11 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
     WICK_REQUIRE(wick_attn_decode_parts_supported(n_seqs, n_heads, n_kv), "attention decode: %d sequences, %d heads over %d kv heads is beyond this kernel", n_seqs, n_heads, n_kv);
     WICK_REQUIRE(kv_pages > 0 && kv_pages * 2 * n_kv * kPage < (1ll << 31), "attention decode: a cache of %lld pages is beyond the kernel's 31-bit row index", kv_pages);
     if (n_seqs == 0) return 0;
-    const long long need = wick_attn_decode_parts_scratch(n_seqs, n_heads, n_kv, max_kv_len);
+    const int pages = pages_for(max_kv_len, mk), stride = part_stride_for(pages);
+    const long long need = scratch_for(n_seqs, n_heads, n_kv, stride);
     WICK_REQUIRE(scratch_words >= need, "attention decode: scratch of %lld words given, %lld needed", scratch_words, need);
     CUtensorMap map;
     if (int e = make_bf16_map(&map, kv, kv_pages * 2 * n_kv * kPage, HD, kPage, "attention decode")) return e;
-    const int stride = part_stride_for(max_kv_len);
     const long long most = (long long)n_seqs * n_kv * stride;
     const int sms = sm_count();
     static bool raised = false;
@@ -827,8 +841,6 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
     }
     const long long pairs = (long long)n_seqs * n_kv;
     const bool masked = mk.kind >= 0;
-    int pages = ceil_div(max_kv_len > 0 ? max_kv_len : 1, kPage);            // (the most with visible keys)
-    if (mk.kind > 0) pages = min(pages, ceil_div(mk.size, kPage) + 1);
     static int force = -2;                             // WICK_B200_PAIR_DECODE=0/1: never / whenever possible (for measurements)
     if (force == -2) force = getenv("WICK_B200_PAIR_DECODE") ? atoi(getenv("WICK_B200_PAIR_DECODE")) : -1;
     // Measured (8 kv heads of 128, one B200), us persistent / a block per pair.  Up to one pair an SM: a block's warps take a part each up to 24

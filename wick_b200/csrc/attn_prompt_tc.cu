@@ -354,6 +354,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     pdl_trigger();
     if (smem_u32(smem_raw) & 1023) {                               // (cannot be, see Shared)
         if (threadIdx.x == 0) atomicCAS(status, 0, 7);
+        pdl_wait();
         return;
     }
     // (the step's description is written by the host before the step: no kernel produces it)

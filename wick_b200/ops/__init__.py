@@ -462,6 +462,15 @@ def attention_decode_parts_scratch(n_seqs: int, n_heads: int, n_kv: int, head_di
     return int(f(n_seqs, n_heads, n_kv, max_kv_len))
 
 
+def attention_decode_parts_masked_scratch(n_seqs: int, n_heads: int, n_kv: int, head_dim: int, max_kv_len: int, mask: str,
+                                          mask_size: int) -> int:
+    """float32 words of scratch that the form with a mask needs: only pages with visible keys have parts."""
+    f = _attn(head_dim)._lib.wick_attn_decode_parts_masked_scratch
+    f.restype = ctypes.c_longlong
+    f.argtypes = [ctypes.c_int] * 6
+    return int(f(n_seqs, n_heads, n_kv, max_kv_len, MASKS[mask], mask_size))
+
+
 def attention_decode_parts(q: torch.Tensor, kv: torch.Tensor, batch, scale: float, scratch: torch.Tensor,
                            out: Optional[torch.Tensor] = None, max_kv_len: Optional[int] = None) -> torch.Tensor:
     """One new token per sequence over the cache (which already holds its key and value).
@@ -1169,13 +1178,14 @@ def attention_masked(q: torch.Tensor, kv: torch.Tensor, batch, scale: float, *, 
         # more, one sequence's chains of pages take longer than that: window of 2,048 13.3 / 19.9.)
         if q.dtype == torch.bfloat16 and mask != "causal" and mask_size <= 1024 and \
                 attention_decode_parts_supported(batch.n_seqs, n_heads, n_kv, d, q.dtype):
-            need = attention_decode_parts_scratch(batch.n_seqs, n_heads, n_kv, d, mk)
+            need = attention_decode_parts_masked_scratch(batch.n_seqs, n_heads, n_kv, d, mk, mask, int(mask_size))
             ws = getattr(batch, "workspace", None)
             scratch = ws.get("attention_decode", need, torch.float32) if ws is not None else \
                 torch.empty(need, dtype=torch.float32, device=q.device)
             _attn(d).call("wick_attn_decode_parts_masked_bf16", "pplpplpiipiiifpiipp", _p(q), _p(kv), kv.shape[0], _p(out), _p(scratch),
                           scratch.numel(), _p(batch.kv_len), n, mk, _p(batch.page_table), batch.table_width, n_heads, n_kv,
-                          float(scale), _p(status_tensor(q.device)), MASKS[mask], int(mask_size), _p(sink), _stream(), kernels=2 if mk > 128 else 1)
+                          float(scale), _p(status_tensor(q.device)), MASKS[mask], int(mask_size), _p(sink), _stream(),
+                          kernels=2 if need > n * n_heads * (d + 2) else 1)
             return out
         need = attention_decode_scratch_floats(batch.n_seqs, n_heads, d, mk, q.dtype)
         ws = getattr(batch, "workspace", None)
