@@ -229,6 +229,30 @@ def test_attention_over_rows_of_few_heads_stays_on_the_cuda_cores(H, R, tensor_c
         assert (out[t].double().cpu() - ref).abs().max() < 1e-5 * float(ref.abs().max())
 
 
+@pytest.mark.parametrize("bn", [16, 48, 80, 112])
+@pytest.mark.parametrize("rows, runs, dtype", [(100, 1, torch.float32), (131, 2, torch.float32), (100, 1, torch.bfloat16)])
+def test_products_whose_tokens_take_several_tiles_of_an_odd_width(bn, rows, runs, dtype):
+    """Weights on the 128-row side, the tokens in more than one tile of a width that is no multiple of 32: a tile writes its own
+    columns only."""
+    from wick_b200.ops import gemm_tc as G
+    n, k = 200, 320
+    g = torch.Generator().manual_seed(bn + rows)
+    w = (torch.randn(n, k, generator=g) / math.sqrt(k)).bfloat16().to(DEV)
+    x = torch.randn(rows, k, generator=g).bfloat16().to(DEV)
+    ref = x.double() @ w.double().T
+    for _ in range(20):
+        out = torch.full((runs, rows, n), float("nan"), dtype=dtype, device=DEV)
+        G.gemm_tc(w, n, x, rows, bn=bn, out=out, ldo=n, transposed=True, splits=runs, split_stride=rows * n, a_static=True)
+        assert (out.double().sum(0) - ref).abs().max() < (1e-5 if dtype == torch.float32 else 2 ** -8) * float(ref.abs().max())
+    if runs == 1 and dtype == torch.bfloat16:
+        w2 = (torch.randn(2 * 128, k, generator=g) / math.sqrt(k)).bfloat16().to(DEV)
+        out = torch.full((rows, 128), float("nan"), dtype=dtype, device=DEV)
+        G.gemm_tc(w2, 128, x, rows, bn=bn, out=out, ldo=128, gated=3, pair_offset=128, transposed=True, a_static=True)
+        ref = gated(x.double() @ w2.double().T)
+        assert (out.double() - ref).abs().max() < 2 ** -8 * max(1.0, float(ref.abs().max()))
+    G.check_status()
+
+
 @pytest.mark.parametrize("ff, width, t", [(64, 512, 1), (200, 1024, 16), (320, 2048, 17), (65, 576, 128), (1000, 264, 5)])
 def test_gated_products_of_few_tokens_joined_over_a_cluster(ff, width, t):
     """Few tiles of a gated pair: runs of the inner dimension meet inside the kernel; a token's bits do not depend on the others."""

@@ -427,7 +427,7 @@ gemm_tc_block(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensor
                 if (ok && n_kb > 0) {
                     typedef std::conditional_t<OUT_F32, float, __nv_bfloat16> Out;
                     Out* o = (Out*)out_base + (long long)n0 * ldo + m;
-                    const int n_end = m < a_rows ? p.b_rows - n0 : 0;
+                    const int n_end = m < a_rows ? min(p.bn, p.b_rows - n0) : 0;   // (bn may be an odd multiple of 16: what lies behind is not this tile's)
 #pragma unroll 1
                     for (int c0 = 0; c0 < p.bn; c0 += 32) {
                         float v[32];
