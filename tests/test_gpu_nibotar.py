@@ -350,6 +350,51 @@ def test_decode_attention_with_a_mask_on_tensor_cores(mask, size, d, H, G):
         assert torch.equal(step([i])[0], out[i]), lens[i]
 
 
+def decode_case(lens, d, H, G, seed, nan=True):
+    """Caches of these lengths (on pages in order; NaN where no token is), one token each: q, kv, a step of some of them."""
+    g = torch.Generator().manual_seed(seed)
+    counts = [(n + PAGE - 1) // PAGE for n in lens]
+    pages, nxt = [], 1
+    for c in counts:
+        pages.append(list(range(nxt, nxt + c)))
+        nxt += c
+    kv = torch.randn(nxt, 2, G, PAGE, d, generator=g)
+    for n, p in zip(lens, pages):
+        if n % PAGE:
+            kv[p[-1], :, :, n % PAGE:] = float("nan")
+    q = torch.randn(len(lens), H, d, generator=g).bfloat16()
+
+    def step(which):
+        lay = BatchLayout(len(which), len(which), max(counts), 0)
+        host = np.zeros(lay.size, dtype=np.int32)
+        fill_host(lay, host, tokens=[[0]] * len(which), starts=[lens[i] - 1 for i in which], slots=list(range(len(which))),
+                  pages=[pages[i] for i in which], want=[[]] * len(which))
+        return StepBatch(lay, torch.from_numpy(host).to(DEV), q_lens=[1] * len(which), starts=[lens[i] - 1 for i in which])
+    return q, kv.bfloat16(), pages, step
+
+
+@pytest.mark.parametrize("sinks", [False, True])
+@pytest.mark.parametrize("mask,size", [("block", 200), ("window", 150)])
+def test_infinite_values_and_numbers_that_are_none_in_masked_decode_attention(mask, size, sinks):
+    """An infinite value that a token sees makes its result infinite (of both signs: NaN), a NaN makes it NaN, as in the kernel
+    without tensor cores; those a token does not see show nowhere."""
+    lens, d, H, G = [130, 400, 401, 700, 64], 64, 4, 2
+    q, kv, pages, step = decode_case(lens, d, H, G, 31)
+    for seq, pos, value in ((0, 129, float("inf")), (1, 399, -float("inf")), (2, 400, float("inf")), (2, 399, -float("inf")), (3, 690, float("nan")),
+                            (3, 640, float("inf")), (4, 3, float("inf")), (1, 100, float("inf")), (3, 1, float("nan"))):
+        kv[pages[seq][pos // PAGE], 1, :, pos % PAGE, 7 + seq] = value
+    sink = torch.randn(H, generator=torch.Generator().manual_seed(3)).to(DEV) if sinks else None
+    kw = dict(n_kv=G, v_dim=d, mask=mask, mask_size=size, sink=sink)
+    batch = step(range(len(lens)))
+    out = ops.attention_masked(q.to(DEV), kv.to(DEV), batch, 0.2, kind="bulk", **kw).float().cpu()
+    ref = ops.attention_masked(q.to(DEV), kv.to(DEV), batch, 0.2, kind="warp", **kw).float().cpu()
+    odd = ~torch.isfinite(ref)
+    assert all(odd[i, :, 7 + i].all() and odd[i].sum() == H for i in range(len(lens)))
+    assert torch.equal(torch.isnan(out), torch.isnan(ref)) and torch.equal(out[odd & ~torch.isnan(ref)], ref[odd & ~torch.isnan(ref)])
+    assert (out - ref)[~odd].abs().max() < 0.02
+    ops.check_status()
+
+
 @pytest.mark.parametrize("n", [1024, 1025, 1500])
 def test_a_masked_decode_step_of_more_sequences_than_the_kernel_by_parts_holds(n):
     """1,024 sequences is the most that the kernel by parts takes; a step of more goes to the bulk-copy kernel."""

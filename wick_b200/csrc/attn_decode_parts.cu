@@ -31,6 +31,8 @@
 // Formulas: wick src/model.rs:520-553.
 #include <cuda.h>
 
+#include <cfloat>
+
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -658,16 +660,35 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             }
             if (ok) {
                 const uint32_t v_base = smem_u32(v_tile);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int key = 16 * j + (lane & 7) + (lane >> 4) * 8;
+                auto values = [&](int j, int mb, uint32_t (&a)[4]) {
+                    ldsm_x4_trans(a, v_base + tile_off(16 * j + (lane & 7) + (lane >> 4) * 8, 2 * mb + ((lane >> 3) & 1)));
+                };
+                if constexpr (MASKED) {
+                    // The first terms into the accumulator, the others' sums added to it where they are finite: an infinite value times its
+                    // weight is infinite, but times a term that is zero or negative it is not a number.
 #pragma unroll
                     for (int mb = 0; mb < KS; ++mb) {
-                        uint32_t a[4];
-                        ldsm_x4_trans(a, v_base + tile_off(key, 2 * mb + ((lane >> 3) & 1)));
+                        float rest[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                        for (int z = TERMS - 1; z >= 0; --z) mma16816(acc[mb], a, pb[z][j][0], pb[z][j][1]);
+                        for (int j = 0; j < 4; ++j) {
+                            uint32_t a[4];
+                            values(j, mb, a);
+                            mma16816(rest, a, pb[2][j][0], pb[2][j][1]);
+                            mma16816(rest, a, pb[1][j][0], pb[1][j][1]);
+                            mma16816(acc[mb], a, pb[0][j][0], pb[0][j][1]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[mb][i] += fabsf(rest[i]) <= FLT_MAX ? rest[i] : 0.f;
                     }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int mb = 0; mb < KS; ++mb) {
+                            uint32_t a[4];
+                            values(j, mb, a);
+                            mma16816(acc[mb], a, pb[0][j][0], pb[0][j][1]);
+                        }
                 }
             }
             if (!ok) dead = true;
