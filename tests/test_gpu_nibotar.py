@@ -395,6 +395,21 @@ def test_infinite_values_and_numbers_that_are_none_in_masked_decode_attention(ma
     ops.check_status()
 
 
+def test_a_sink_that_is_no_number_shows_in_masked_decode_attention():
+    """... and an infinite one: negative it takes no part, positive it leaves NaN, as in the kernel without tensor cores; the other
+    heads' rows are the same.  Sequences of one part and of several."""
+    lens, d, H, G = [70, 600], 64, 4, 2
+    q, kv, pages, step = decode_case(lens, d, H, G, 32)
+    batch = step(range(2))
+    sink = torch.tensor([0.5, float("nan"), float("inf"), -float("inf")])
+    kw = dict(n_kv=G, v_dim=d, mask="window", mask_size=500)
+    out = ops.attention_masked(q.to(DEV), kv.to(DEV), batch, 0.2, kind="bulk", sink=sink.to(DEV), **kw).float().cpu()
+    ref = ops.attention_masked(q.to(DEV), kv.to(DEV), batch, 0.2, kind="warp", sink=sink.to(DEV), **kw).float().cpu()
+    none = ops.attention_masked(q.to(DEV), kv.to(DEV), batch, 0.2, kind="bulk", **kw).float().cpu()
+    assert torch.isnan(ref[:, 1:3]).all() and torch.isnan(out[:, 1:3]).all()
+    assert (out - ref)[:, [0, 3]].abs().max() < 0.02 and (out[:, 3] - none[:, 3]).abs().max() < 0.01
+
+
 @pytest.mark.parametrize("n", [1024, 1025, 1500])
 def test_a_masked_decode_step_of_more_sequences_than_the_kernel_by_parts_holds(n):
     """1,024 sequences is the most that the kernel by parts takes; a step of more goes to the bulk-copy kernel."""

@@ -172,7 +172,7 @@ __device__ __forceinline__ void merge_head(Word word, int P, int lane, bf16* dst
             M = mn;
         }
     }
-    const float inv = l > 0.f ? __fdiv_rn(1.0f, l) : 0.f;
+    const float inv = l != 0.f ? __fdiv_rn(1.0f, l) : 0.f;     // (a sum that is no number shows)
 #pragma unroll
     for (int e = 0; e < EPL; ++e) dst[lane + 32 * e] = __float2bfloat16_rn(__fmul_rn(o[e], inv));
 }
@@ -715,7 +715,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
                     acc[mb][1] *= f1, acc[mb][3] *= f1;
                 }
             }
-            const float i0 = lr0 > 0.f ? __fdiv_rn(1.0f, lr0) : 0.f, i1 = lr1 > 0.f ? __fdiv_rn(1.0f, lr1) : 0.f;
+            const float i0 = lr0 != 0.f ? __fdiv_rn(1.0f, lr0) : 0.f, i1 = lr1 != 0.f ? __fdiv_rn(1.0f, lr1) : 0.f;   // (a sum that is no number shows)
             bf16* o0 = out + ((int64_t)b * n_heads + kvh * group + c0) * HD;
 #pragma unroll
             for (int mb = 0; mb < KS; ++mb) {
