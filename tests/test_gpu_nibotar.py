@@ -410,6 +410,35 @@ def test_a_sink_that_is_no_number_shows_in_masked_decode_attention():
     assert (out - ref)[:, [0, 3]].abs().max() < 0.02 and (out[:, 3] - none[:, 3]).abs().max() < 0.01
 
 
+@pytest.mark.parametrize("few", [True, False])
+def test_rows_of_sequences_without_a_position_are_zeros_in_masked_decode_attention(few, monkeypatch):
+    """A place of a captured step that no sequence holds (length 0), alone with others in a block per pair and among many in persistent
+    blocks; and one whose length lies beyond its page table, which is reported besides."""
+    real = torch.empty
+
+    def empty(*a, **k):
+        t = real(*a, **k)
+        return t.fill_(float("nan")) if t.is_cuda and t.is_floating_point() else t
+    lens, d, H, G = ([70, 600, 5] if few else [70, 30, 5] * 60), 64, 6, 3
+    q, kv, pages, step = decode_case(lens, d, H, G, 33)
+    batch = step(range(len(lens)))
+    gone = [1, len(lens) - 1]
+    kw = dict(n_kv=G, v_dim=d, mask="block", mask_size=512)
+    whole = ops.attention_masked(q.to(DEV), kv.to(DEV), batch, 0.2, kind="bulk", **kw)
+    batch.kv_len[gone[0]] = batch.kv_len[gone[1]] = 0
+    monkeypatch.setattr(torch, "empty", empty)
+    out = ops.attention_masked(q.to(DEV), kv.to(DEV), batch, 0.2, kind="bulk", **kw)
+    ops.check_status()
+    assert (out[gone] == 0).all()
+    rest = [i for i in range(len(lens)) if i not in gone]
+    assert torch.equal(out[rest], whole[rest])
+    batch.kv_len[gone[1]] = batch.table_width * PAGE + 1
+    out = ops.attention_masked(q.to(DEV), kv.to(DEV), batch, 0.2, kind="bulk", **kw)
+    with pytest.raises(ops.KernelError, match="a length or a page"):
+        ops.check_status()
+    assert (out[gone] == 0).all() and torch.equal(out[rest], whole[rest])
+
+
 @pytest.mark.parametrize("n", [1024, 1025, 1500])
 def test_a_masked_decode_step_of_more_sequences_than_the_kernel_by_parts_holds(n):
     """1,024 sequences is the most that the kernel by parts takes; a step of more goes to the bulk-copy kernel."""

@@ -312,6 +312,16 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
     }
     __syncthreads();
 
+    // MASKED, behind the wait: the rows of sequences that are left out are zeros.
+    auto clear_left_out = [&]() {
+        if (!MASKED) return;
+#pragma unroll 1
+        for (int s = PAIR ? 0 : warp * (int)gridDim.x + (int)blockIdx.x; s < (PAIR ? 1 : n_seqs); s += W * (int)gridDim.x)
+            if (PAIR ? my_parts == 0 && warp == 0 : lens[s] == 0) {
+                bf16* rows = out + (PAIR ? (int64_t)blockIdx.x * group : (int64_t)s * n_heads) * HD;   // (the pair's, or all of the sequence's)
+                for (int i = lane; i < (PAIR ? group : n_heads) * HD; i += 32) rows[i] = __float2bfloat16_rn(0.f);
+            }
+    };
     if (!PAIR) {
         // This warp's run of parts.
         const int U = cum[n_seqs];
@@ -320,6 +330,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         u1 = (int)((slot + 1) * U / S);
         if (u0 >= u1) {
             pdl_wait();                                // (should no warp have a part: see the merge)
+            clear_left_out();
             return;
         }
     }
@@ -403,6 +414,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
     while (issue(false)) {}
     pdl_wait();                                        // the query rows (or the projection's sums they are made from)
     q = fresh(q);
+    clear_left_out();
 
     const float sl2 = scale * 1.4426950408889634f;
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;     // accumulator rows r0, r0 + 8; columns c0, c0 + 1
