@@ -24,6 +24,19 @@ def test_decode_attention_by_parts_is_offered_only_what_its_library_takes(hd):
     assert not ops.attention_decode_parts_supported(1, 8, 2, 32, torch.bfloat16)
 
 
+def test_decode_attention_by_parts_refuses_query_rows_it_cannot_read():
+    """Rows are read two numbers at a time: an address that is no multiple of 4 is an error of the call, not of the device."""
+    lib = ops._attn(64)
+    for at, message in ((1 << 20, None), ((1 << 20) + 2, "multiple of 4 bytes")):
+        try:
+            lib.call("wick_attn_decode_parts_masked_bf16", "pplpplpiipiiifpiipp", at, 1 << 20, 4, 1 << 20, 1 << 20, 0 if message is None else 1 << 20,
+                     1 << 20, 1, 64, 1 << 20, 1, 4, 2, 0.1, 1 << 20, 2, 64, None, 0)
+            got = ""
+        except ops.KernelError as e:
+            got = str(e)
+        assert got and (message is None) == ("multiple of 4 bytes" not in got), got       # (the first call is refused for its scratch)
+
+
 def _enclosed(text, at, pair="{}"):
     """The text from the bracket that opens at or behind ``at`` to the one that closes it."""
     begin = at = text.index(pair[0], at)

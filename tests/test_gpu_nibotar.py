@@ -439,6 +439,19 @@ def test_rows_of_sequences_without_a_position_are_zeros_in_masked_decode_attenti
     assert (out[gone] == 0).all() and torch.equal(out[rest], whole[rest])
 
 
+def test_masked_decode_attention_takes_query_rows_that_begin_anywhere():
+    """Queries at an address that is no multiple of 4 bytes go to the kernel that reads them one number at a time."""
+    lens, d, H, G = [70, 600, 129], 64, 4, 2
+    q, kv, pages, step = decode_case(lens, d, H, G, 34)
+    flat = torch.zeros(q.numel() + 1, dtype=torch.bfloat16, device=DEV)
+    flat[1:] = q.flatten().to(DEV)
+    kw = dict(n_kv=G, v_dim=d, mask="window", mask_size=200)
+    odd = ops.attention_masked(flat[1:].view(q.shape), kv.to(DEV), step(range(3)), 0.2, **kw)
+    even = ops.attention_masked(q.to(DEV), kv.to(DEV), step(range(3)), 0.2, **kw)
+    ops.check_status()
+    assert (odd.float() - even.float()).abs().max() < 0.02
+
+
 @pytest.mark.parametrize("n", [1024, 1025, 1500])
 def test_a_masked_decode_step_of_more_sequences_than_the_kernel_by_parts_holds(n):
     """1,024 sequences is the most that the kernel by parts takes; a step of more goes to the bulk-copy kernel."""

@@ -855,6 +855,7 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
     WICK_REQUIRE(wick_attn_decode_parts_supported(n_seqs, n_heads, n_kv), "attention decode: %d sequences, %d heads over %d kv heads is beyond this kernel", n_seqs, n_heads, n_kv);
     WICK_REQUIRE(kv_pages > 0 && kv_pages * 2 * n_kv * kPage < (1ll << 31), "attention decode: a cache of %lld pages is beyond the kernel's 31-bit row index", kv_pages);
     if (n_seqs == 0) return 0;
+    WICK_REQUIRE(((uintptr_t)q & 3) == 0, "attention decode: query rows are read two numbers at a time and begin on no multiple of 4 bytes");
     const int pages = pages_for(max_kv_len, mk), stride = part_stride_for(pages);
     const long long need = scratch_for(n_seqs, n_heads, n_kv, stride);
     WICK_REQUIRE(scratch_words >= need, "attention decode: scratch of %lld words given, %lld needed", scratch_words, need);

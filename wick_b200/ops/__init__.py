@@ -1175,8 +1175,8 @@ def attention_masked(q: torch.Tensor, kv: torch.Tensor, batch, scale: float, *, 
         # Few visible keys: on the tensor cores, by parts.  (By the mask's size alone, so that a sequence's bits do not depend on the batch.
         # us, CUDA cores / by parts, 16 heads over 4 of 128, block of 1,024: 1 x 500 positions 8.6 / 6.7, 8 x 1,500 14.8 / 7.7, 64 x 300
         # 28.8 / 15.4, 160 x 1,000 139 / 80, but 1 x 4,000, whose block is nearly full, 10.8 / 12.5.  Where a token sees 2,048 positions and
-        # more, one sequence's chains of pages take longer than that: window of 2,048 13.3 / 19.9.)
-        if q.dtype == torch.bfloat16 and mask != "causal" and mask_size <= 1024 and \
+        # more, one sequence's chains of pages take longer than that: window of 2,048 13.3 / 19.9.  It reads the queries two numbers at a time.)
+        if q.dtype == torch.bfloat16 and mask != "causal" and mask_size <= 1024 and q.data_ptr() % 4 == 0 and \
                 attention_decode_parts_supported(batch.n_seqs, n_heads, n_kv, d, q.dtype):
             need = attention_decode_parts_masked_scratch(batch.n_seqs, n_heads, n_kv, d, mk, mask, int(mask_size))
             ws = getattr(batch, "workspace", None)
