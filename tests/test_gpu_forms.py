@@ -625,3 +625,24 @@ def test_what_follows_a_decode_attention_with_nothing_to_merge_waits_for_it(case
         got.append(torch.load(out))
     assert all(torch.equal(a, b) for a, b in zip(*got))
     assert all(torch.isfinite(a).all() for a in got[0])
+
+
+@pytest.mark.parametrize("d, heads, kv", [(64, 20, 4), (128, 16, 16)])
+@pytest.mark.parametrize("start, mask, size, pos, clean", [(0, "causal", 0, 200, (0, 128)), (64, "window", 16, 100, (128, 256)), (64, "block", 128, 300, (0, 128))])
+def test_prompt_rows_do_not_show_values_of_key_blocks_they_see_nothing_of(d, heads, kv, start, mask, size, pos, clean):
+    """Two tiles of 128 tokens a block: a value that is no number lies in a key block (128 positions) that only one of them sees."""
+    lens, starts = [256] * 16, [start] * 16
+    batch, pages, n_pages = batch_of(lens, starts)
+    g = torch.Generator().manual_seed(d + start)
+    store = torch.randn(n_pages, 2, kv, PAGE, d, generator=g).bfloat16()
+    for b, bad in ((0, float("nan")), (7, float("inf")), (15, -float("inf"))):
+        store[pages[b][pos // PAGE], 1, :, pos % PAGE] = bad
+    q = torch.randn(sum(lens), heads, d, generator=g).bfloat16()
+    out = ops.attention_masked(q.to(DEV), store.to(DEV), batch, 0.2, n_kv=kv, v_dim=d, mask=mask, mask_size=size, kind="tc").cpu()
+    ref = ops.attention_masked(q.to(DEV), store.to(DEV), batch, 0.2, n_kv=kv, v_dim=d, mask=mask, mask_size=size, kind="warp").cpu()
+    ops.check_status()
+    for b in range(16):
+        a, z = 256 * b + clean[0], 256 * b + clean[1]
+        assert torch.isfinite(ref[a:z].float()).all() and torch.isfinite(out[a:z].float()).all(), b
+        assert (out[a:z].float() - ref[a:z].float()).abs().max() < 0.02
+    assert not torch.isfinite(out[:256].float()).all(), "and those that see it show it"

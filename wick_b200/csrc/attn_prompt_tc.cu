@@ -78,6 +78,13 @@ struct Item {
     __device__ __forceinline__ int place_v(int j) const { return split ? min(2 * j + 2, 2 * n_blk - 1) : 2 * j + 1; }
     __device__ __forceinline__ int block_of(int s, int t) const { return split ? 2 * t + s : t; }    // step t of stream s
 };
+// The key blocks that a tile multiplies: those before `pool`, and those from `from` up to `to`.
+struct Seen {
+    int pool, from, to;
+    __device__ __forceinline__ bool has(int j) const { return j < pool || (j >= from && j < to); }
+    __device__ __forceinline__ int first() const { return pool > 0 ? 0 : from; }
+};
+constexpr int GUARDED = 4;                             // (of a form of the issuing loop, beside how far it is unrolled)
 // Behind the tiles in shared memory (which begins on a multiple of 1,024 bytes, and has no room for a shift):
 struct Shared {
     float ml[2][2][BQ];                                // the streams' maxima and sums, where they share rows
@@ -502,15 +509,27 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             };
 #pragma unroll 1
             for (int k = 0; ok && any(k); ++k) {
-                const int n_blk = sh.items[k].n_blk;
-                const bool split = sh.items[k].split;
+                const Item& w = sh.items[k];
+                const int n_blk = w.n_blk;
+                const bool split = w.split;
                 auto block_of = [&](int s, int t) { return split ? 2 * t + s : t; };
+                // Two tiles of more tokens together than a key block has keys: a tile multiplies no block that none of its rows sees a key of.
+                // (Such a block weighs nothing, but a value that is infinite or no number would show in rows that do not see it.)
+                const bool guard = !split && 2 * T > BK;
+                auto seen_by = [&](int s) {
+                    const int first = w.start + w.q0 + s * T, last = min(first + T, w.start + w.q_len) - 1, before = w.n_pool - w.jb0;
+                    return Seen{EXTRA ? (blocks_seen(last, mask_size, X.block) + BK - 1) / BK : 0,
+                                before + first_visible_key(first, mask, mask_size) / BK, before + last / BK + 1};
+                };
+                Seen seen0 = {}, seen1 = {};
+                if (guard) seen0 = seen_by(0), seen1 = seen_by(1);
                 int k_at = 0, v_at = 0;                            // where the keys and values at hand lie (both streams read a tile, or one)
                 ok = __all_sync(0xffffffffu, mbar_wait(&sh.q_full, k & 1, abort_flag, status, 7));
                 // Turn t of stream s: the product of its step t, the scores of step t + 1.  Long items take the form in which the streams
                 // are told apart when the kernel is built (8,192 tokens: 537 us in the other, 453), short ones the shorter code.
                 auto turn = [&](auto form, int s, int t) {
-                    constexpr int UNROLL = decltype(form)::value;
+                    constexpr int UNROLL = decltype(form)::value & 3;
+                    constexpr bool GUARD = decltype(form)::value >= GUARDED;
                     const int steps = s == 0 ? steps0 : steps1, uses = s == 0 ? uses0 : uses1;
                     const bool more = block_of(s, t + 1) < n_blk;
                     if (block_of(s, t) >= n_blk) return;
@@ -519,14 +538,21 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                         // (the result of the stream's item before has been read)
                         if (ok && t == 0 && uses > 0) ok = __all_sync(0xffffffffu, mbar_wait(&sh.o_empty[s], (uses - 1) & 1, abort_flag, status, 7));
                         const uint32_t v_lo = v_lo0 + v_at * (TILE_BYTES >> 4), d = tmem + COL_O + s * HD, pa = tmem + COL_S + s * BK;
+                        bool go = one;
+                        int begun = t;                             // (0: the stream's first product of the item)
+                        if constexpr (GUARD) {
+                            const Seen seen = s == 0 ? seen0 : seen1;
+                            go = one && seen.has(t);
+                            begun = t - seen.first();
+                        }
 #pragma unroll UNROLL
                         for (int part = 0; part < 2; ++part) {
                             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&sh.p_full[s][part], steps & 1, abort_flag, status, 7));
                             if (!ok) break;
                             tc_fence_after();
                             const uint32_t pp = pa + part * (P_FIRST / 2), vp = v_lo + part * (P_FIRST / 16) * (2048 >> 4);
-                            if (one) {
-                                mma_ts(d, pp, vp, idesc_o, t > 0 || part > 0);
+                            if (go) {
+                                mma_ts(d, pp, vp, idesc_o, begun > 0 || part > 0);
                                 static_for<1, P_FIRST / 16>([&](auto ks) { mma_ts(d, pp + (int)ks * 8, vp + (int)ks * (2048 >> 4), idesc_o, 1); });
                             }
                         }
@@ -558,15 +584,28 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                     }
                     __syncwarp();
                 };
-                if (n_blk >= LONG) {
+                auto looped = [&](auto form, int from, int to) {
 #pragma unroll 1
-                    for (int t = -1; ok && block_of(0, t) < n_blk; ++t) {
+                    for (int i = 2 * from; ok && i < 2 * to && block_of(0, i >> 1) < n_blk; ++i) turn(form, i & 1, i >> 1);
+                };
+                auto written_out = [&](int from, int to) {
+#pragma unroll 1
+                    for (int t = from; ok && t < to && block_of(0, t) < n_blk; ++t) {
                         turn(std::integral_constant<int, 2>{}, 0, t);
                         if (ok) turn(std::integral_constant<int, 2>{}, 1, t);
                     }
+                };
+                if (guard) {
+                    // (between the last block that either tile begins with and the first that either no longer sees: as without)
+                    const int lo = max(seen0.from, seen1.from) + 1, hi = max(lo, min(seen0.to, seen1.to));
+                    looped(std::integral_constant<int, GUARDED + 1>{}, -1, lo);
+                    if (n_blk >= LONG) written_out(lo, hi);
+                    else looped(std::integral_constant<int, 1>{}, lo, hi);
+                    looped(std::integral_constant<int, GUARDED + 1>{}, hi, n_blk);
+                } else if (n_blk >= LONG) {
+                    written_out(-1, n_blk);
                 } else {
-#pragma unroll 1
-                    for (int i = -2; ok && block_of(0, i >> 1) < n_blk; ++i) turn(std::integral_constant<int, 1>{}, i & 1, i >> 1);
+                    looped(std::integral_constant<int, 1>{}, -1, n_blk);
                 }
             }
         }
