@@ -646,3 +646,21 @@ def test_prompt_rows_do_not_show_values_of_key_blocks_they_see_nothing_of(d, hea
         assert torch.isfinite(ref[a:z].float()).all() and torch.isfinite(out[a:z].float()).all(), b
         assert (out[a:z].float() - ref[a:z].float()).abs().max() < 0.02
     assert not torch.isfinite(out[:256].float()).all(), "and those that see it show it"
+
+
+@pytest.mark.parametrize("heads, kv", [(64, 16), (64, 8), (40, 8)])
+def test_prompt_rows_of_a_step_of_few_tokens_do_not_depend_on_the_other_sequences(heads, kv):
+    """Up to 64 tokens in a step: a sequence's rows are the same bits alone and among others, however many items the step makes."""
+    d, lens, starts = 64, [33] + [1] * 31, [500] + [130 + 7 * i for i in range(31)]
+    batch, pages, n_pages = batch_of(lens, starts)
+    g = torch.Generator().manual_seed(heads)
+    store = torch.randn(n_pages, 2, kv, PAGE, d, generator=g).bfloat16().to(DEV)
+    q = torch.randn(sum(lens), heads, d, generator=g).bfloat16().to(DEV)
+    full = ops.attention_prompt(q, store, batch, 0.2)
+    at = 0
+    for b, n in enumerate(lens[:3]):
+        one, own, _ = batch_of([n], [starts[b]])
+        one.page_table.copy_(torch.tensor([pages[b]], dtype=torch.int32))
+        assert torch.equal(ops.attention_prompt(q[at:at + n].contiguous(), store, one, 0.2), full[at:at + n]), b
+        at += n
+    ops.check_status()

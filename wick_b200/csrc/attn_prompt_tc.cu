@@ -937,7 +937,8 @@ static int attn_prompt_tc(const void* q, long long n_tokens, const void* kv, lon
     // 4 x 700 alone, 16 over 4: 22.5 and 27.1).
     const long long one = (long long)items(T) * columns, two = (long long)items(2 * T) * columns, sms = sm_count();
     const long long keys = ((long long)table_width * kPage - n_tokens / max(n_seqs, 1) / 2) / BK;     // blocks of keys a tile sees, about
-    const int tiles = one <= sms || (one <= 2 * sms && keys >= 1) || (two <= 2 * sms && (one + sms - 1) / sms < 2 * ((two + sms - 1) / sms) && keys >= 16) ? 1 : 2;
+    // Steps of up to 64 tokens, in which no matrix product's sums depend on the other sequences, always take one tile: nor do these then.
+    const int tiles = n_tokens <= 64 || one <= sms || (one <= 2 * sms && keys >= 1) || (two <= 2 * sms && (one + sms - 1) / sms < 2 * ((two + sms - 1) / sms) && keys >= 16) ? 1 : 2;
     const int n_items = items(T * tiles);
     WICK_REQUIRE((long long)n_items * columns <= INT32_MAX / 2, "attention (tcgen05): %d work items of %d columns are too many", n_items, columns);
     // a block an SM that works through its items one behind the other (more than MAX_ITEMS each: in several rounds)
