@@ -73,6 +73,9 @@ def test_no_kernel_that_lets_its_successor_start_ends_before_it_has_waited():
             if not m:
                 break
             body = body[:m.start()] + body[m.end() + len(_enclosed(body, m.end())):]
-        before = body[:body.index("return")] if "return" in body else body
-        assert "pdl_wait()" in before, f"{name} ({f}) may end before its wait"
+        first = body.find("return")
+        if name == "attn_decode_parts_kernel":         # its warps without a part leave, where there are warps with one
+            assert "if (before == 0) pdl_wait();" in body[:first]
+            first = body.find("return", first + 1)
+        assert "pdl_wait()" in body[:first if first >= 0 else len(body)], f"{name} ({f}) may end before its wait"
     assert found > 40, "the kernels' sources are not where they were"

@@ -309,15 +309,17 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             before += __shfl_sync(0xffffffffu, upto, 31);
         }
         if (lane == 0) cum[0] = 0;
+        if (before == 0) pdl_wait();                   // (nobody has a part: see the merge)
     }
     __syncthreads();
 
-    // MASKED, behind the wait: the rows of sequences that are left out are zeros.
+    // MASKED: the rows of sequences that are left out are zeros.
     auto clear_left_out = [&]() {
         if (!MASKED) return;
 #pragma unroll 1
         for (int s = PAIR ? 0 : warp * (int)gridDim.x + (int)blockIdx.x; s < (PAIR ? 1 : n_seqs); s += W * (int)gridDim.x)
             if (PAIR ? my_parts == 0 && warp == 0 : lens[s] == 0) {
+                pdl_wait();
                 bf16* rows = out + (PAIR ? (int64_t)blockIdx.x * group : (int64_t)s * n_heads) * HD;   // (the pair's, or all of the sequence's)
                 for (int i = lane; i < (PAIR ? group : n_heads) * HD; i += 32) rows[i] = __float2bfloat16_rn(0.f);
             }
@@ -328,8 +330,9 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
         const int64_t S = (int64_t)gridDim.x * W, slot = (int64_t)warp * gridDim.x + blockIdx.x;
         u0 = (int)(slot * U / S);
         u1 = (int)((slot + 1) * U / S);
+        // A warp without a part leaves: a block that does makes room for the next kernel's (4 x 2,000 positions, 32 heads over 8: 15.4 us where
+        // all wait, 14.2).  Some warp has waited by then, or will.
         if (u0 >= u1) {
-            pdl_wait();                                // (should no warp have a part: see the merge)
             clear_left_out();
             return;
         }
@@ -672,9 +675,6 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
             }
             if (ok) {
                 const uint32_t v_base = smem_u32(v_tile);
-                auto values = [&](int j, int mb, uint32_t (&a)[4]) {
-                    ldsm_x4_trans(a, v_base + tile_off(16 * j + (lane & 7) + (lane >> 4) * 8, 2 * mb + ((lane >> 3) & 1)));
-                };
                 if constexpr (MASKED) {
                     // The first terms into the accumulator, the others' sums added to it where they are finite: an infinite value times its
                     // weight is infinite, but times a term that is zero or negative it is not a number.
@@ -684,7 +684,7 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             uint32_t a[4];
-                            values(j, mb, a);
+                            ldsm_x4_trans(a, v_base + tile_off(16 * j + (lane & 7) + (lane >> 4) * 8, 2 * mb + ((lane >> 3) & 1)));
                             mma16816(rest, a, pb[2][j][0], pb[2][j][1]);
                             mma16816(rest, a, pb[1][j][0], pb[1][j][1]);
                             mma16816(acc[mb], a, pb[0][j][0], pb[0][j][1]);
@@ -694,13 +694,15 @@ attn_decode_parts_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16*
                     }
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < 4; ++j) {
+                        const int key = 16 * j + (lane & 7) + (lane >> 4) * 8;
 #pragma unroll
                         for (int mb = 0; mb < KS; ++mb) {
                             uint32_t a[4];
-                            values(j, mb, a);
+                            ldsm_x4_trans(a, v_base + tile_off(key, 2 * mb + ((lane >> 3) & 1)));
                             mma16816(acc[mb], a, pb[0][j][0], pb[0][j][1]);
                         }
+                    }
                 }
             }
             if (!ok) dead = true;
@@ -797,11 +799,10 @@ attn_decode_merge_kernel(const float* partials, bf16* __restrict__ out, const in
     const int pair = item / group, h = item % group, b = min(pair / n_kv, n_seqs - 1);
     const int len = kv_len_arr[b];                     // (the step's lengths are in place before the step starts)
     const int skipped = skipped_pages<true>(len, mk), n_pages = (len + kPage - 1) / kPage - skipped;
+    const int P = item < n_seqs * n_heads && len > 0 && n_pages + skipped <= table_width ? parts_of(n_pages) : 0;
     // Before any warp leaves: the kernel after this one waits for this one only, and the rows of pairs with one part are written by the
     // kernel before.  Where no warp had anything to merge, nothing would hold that one back until they are.
     pdl_wait();
-    if (item >= n_seqs * n_heads || len <= 0 || n_pages + skipped > table_width) return;
-    const int P = parts_of(n_pages);
     if (P < 2 || P > part_stride) return;
     partials = fresh(partials);
     const float* first = partials + ((int64_t)pair * part_stride * group + h) * REC;
