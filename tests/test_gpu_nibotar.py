@@ -306,7 +306,7 @@ def test_bulk_copy_decode_attention_equals_the_warp_kernel(mask, size, d, H, G, 
 @pytest.mark.parametrize("mask,size", [("block", 100), ("window", 64), ("window", 129), ("block", 1024)])
 def test_decode_attention_with_a_mask_on_tensor_cores(mask, size, d, H, G):
     """Lengths at the edges of pages, of a mask's blocks and windows and of parts, few sequences (a block per pair of sequence and key
-    head) and many (persistent blocks and a merge): against 64 bits no further off than one rounding of the result to bfloat16 (2^-8 of
+    head) and many of one part each (persistent blocks without a merge; with one: the test below): against 64 bits no further off than one rounding of the result to bfloat16 (2^-8 of
     the largest), what hidden and unwritten rows hold (NaN) not seen.  A sequence's bits do not depend on the batch."""
     g = torch.Generator().manual_seed(91)
     lens = [1, 63, 64, 65, 100, 101, 128, 129, 200, 201, 640, 1023, 1024, 1025, 1100, 1700, 2111]
@@ -450,6 +450,61 @@ def test_masked_decode_attention_takes_query_rows_that_begin_anywhere():
     even = ops.attention_masked(q.to(DEV), kv.to(DEV), step(range(3)), 0.2, **kw)
     ops.check_status()
     assert (odd.float() - even.float()).abs().max() < 0.02
+
+
+@pytest.mark.parametrize("d,H,G,n,mask,size,most", [
+    (128, 16, 4, 40, "block", 1024, 1024), (64, 6, 3, 55, "block", 1024, 1024), (128, 5, 5, 33, "window", 1000, 2100), (64, 8, 1, 160, "window", 700, 1500),
+    (128, 8, 4, 130, "window", 129, 300), (64, 9, 3, 150, "window", 128, 300), (128, 4, 4, 104, "block", 448, 900)])
+def test_masked_decode_attention_of_persistent_blocks_with_a_merge(d, H, G, n, mask, size, most):
+    """More pairs of sequence and key head than multiprocessors, of 1 to 18 visible pages: the launcher takes persistent blocks, which
+    leave records for a merge.  Against 64 bits, and the same bits as the sequences alone (a block a pair, merged by itself), with a sink."""
+    g = torch.Generator().manual_seed(n)
+    lens = [1 + int(x) for x in torch.randint(0, most, (n,), generator=g)]
+    lens[:4] = [1, most, 64, min(most, 1030)]
+    sms, pairs = torch.cuda.get_device_properties(0).multi_processor_count, n * G
+    pages_seen = min((max(lens) + PAGE - 1) // PAGE, (size + PAGE - 1) // PAGE + 1)
+    waves = -(-pairs // sms)
+    least = 4 if pairs <= 400 else (17 if d == 64 else 9)
+    assert pairs > sms and (pages_seen < least or pairs * 10 < waves * sms * 6) and pages_seen > 2
+    q, kv, pages, step = decode_case(lens, d, H, G, 40 + n)
+    sink = torch.randn(H, generator=g)
+    kw = dict(n_kv=G, v_dim=d, mask=mask, mask_size=size, sink=sink.to(DEV), kind="bulk")
+    out = ops.attention_masked(q.to(DEV), kv.to(DEV), step(range(n)), 0.2, **kw).cpu()
+    ops.check_status()
+    for i, m in enumerate(lens):
+        if i < 12 or i % 7 == 0:
+            rows = kv[pages[i]].double().permute(1, 0, 3, 2, 4).reshape(2, -1, G, d)[:, :m]
+            lo = (m - 1) // size * size if mask == "block" else max(0, m - size)
+            k, v = (x[lo:].repeat_interleave(H // G, 1) for x in rows)
+            sc = torch.einsum("hd,nhd->hn", q[i].double(), k) * 0.2
+            w = torch.softmax(torch.cat([sc, sink.double()[:, None]], 1), 1)[:, :-1]
+            want = torch.einsum("hn,nhd->hd", w, v)
+            assert (out[i].double() - want).abs().max() <= 2 ** -8 * want.abs().max(), (m, mask, size)
+            assert torch.equal(ops.attention_masked(q[i:i + 1].to(DEV), kv.to(DEV), step([i]), 0.2, **kw).cpu()[0], out[i]), m
+
+
+@pytest.mark.parametrize("d,H,G", [(128, 8, 2), (64, 6, 3)])
+@pytest.mark.parametrize("mask,size", [("block", 1024), ("block", 1025), ("block", 2048), ("window", 1024), ("window", 1025), ("window", 2048)])
+def test_masked_decode_attention_on_both_sides_of_the_mask_size_that_decides(mask, size, d, H, G, monkeypatch):
+    """bfloat16 heads of 64 and 128: masks of up to 1,024 positions take the kernel by parts, larger ones the bulk-copy kernel, with
+    sinks, at lengths around the masks' edges."""
+    lens = [1, size - 1, size, size + 1, size + 64, 2 * size, 2 * size + 1, 2 * size - 63, 700]
+    q, kv, pages, step = decode_case(lens, d, H, G, size)
+    sink = torch.randn(H, generator=torch.Generator().manual_seed(6))
+    lib, called = ops._attn(d), []
+    call = lib.call
+    monkeypatch.setattr(lib, "call", lambda name, *a, **k: (called.append(name), call(name, *a, **k)))
+    out = ops.attention_masked(q.to(DEV), kv.to(DEV), step(range(len(lens))), 0.2, n_kv=G, v_dim=d, mask=mask, mask_size=size, sink=sink.to(DEV)).cpu()
+    ops.check_status()
+    assert called == ["wick_attn_decode_parts_masked_bf16" if size <= 1024 else "wick_attn_decode_masked_bf16"]
+    for i, m in enumerate(lens):
+        rows = kv[pages[i]].double().permute(1, 0, 3, 2, 4).reshape(2, -1, G, d)[:, :m]
+        lo = (m - 1) // size * size if mask == "block" else max(0, m - size)
+        k, v = (x[lo:].repeat_interleave(H // G, 1) for x in rows)
+        sc = torch.einsum("hd,nhd->hn", q[i].double(), k) * 0.2
+        w = torch.softmax(torch.cat([sc, sink.double()[:, None]], 1), 1)[:, :-1]
+        want = torch.einsum("hn,nhd->hd", w, v)
+        assert (out[i].double() - want).abs().max() <= 2 ** -8 * want.abs().max(), (m, mask, size)
 
 
 @pytest.mark.parametrize("n", [1024, 1025, 1500])

@@ -1173,9 +1173,12 @@ def attention_masked(q: torch.Tensor, kv: torch.Tensor, batch, scale: float, *, 
         _need(d == v_dim and batch.is_decode, "the bulk-copy kernel takes one token per sequence and one head size")
         mk = batch.kv_bound
         # Few visible keys: on the tensor cores, by parts.  (By the mask's size alone, so that a sequence's bits do not depend on the batch.
-        # us, CUDA cores / by parts, 16 heads over 4 of 128, block of 1,024: 1 x 500 positions 8.6 / 6.7, 8 x 1,500 14.8 / 7.7, 64 x 300
-        # 28.8 / 15.4, 160 x 1,000 139 / 80, but 1 x 4,000, whose block is nearly full, 10.8 / 12.5.  Where a token sees 2,048 positions and
-        # more, one sequence's chains of pages take longer than that: window of 2,048 13.3 / 19.9.  It reads the queries two numbers at a time.)
+        # A warp walks through its part's pages one by one, which one sequence that sees many positions has to wait for; many sequences gain
+        # at every size.  us, CUDA cores / by parts, heads of 128, one sequence whose block is full: 16 heads over 4, block of 1,024 10.3 / 10.8,
+        # 1,280 11.9 / 12.8, 1,536 13.8 / 15.3, 2,048 14.3 / 20.4; 32 over 8, 1,024 12.2 / 10.9, 1,536 14.3 / 15.5, 2,048 16.2 / 20.5; 8 over 8,
+        # 1,024 8.9 / 10.7; half full 16 over 4, 1,024 9.1 / 6.2, 2,048 10.9 / 12.4.  16 sequences of full blocks, 16 over 4: 1,024 22.8 / 11.2, 2,048
+        # 39.2 / 21.5; 64: 1,024 63.5 / 27.2, 2,048 115.9 / 45.5.  Heads of 64: 1,024 8.3 / 6.8, 2,048 11.1 / 10.9.)
+        # The queries are read two numbers at a time.
         if q.dtype == torch.bfloat16 and mask != "causal" and mask_size <= 1024 and q.data_ptr() % 4 == 0 and \
                 attention_decode_parts_supported(batch.n_seqs, n_heads, n_kv, d, q.dtype):
             need = attention_decode_parts_masked_scratch(batch.n_seqs, n_heads, n_kv, d, mk, mask, int(mask_size))
