@@ -664,3 +664,73 @@ def test_prompt_rows_of_a_step_of_few_tokens_do_not_depend_on_the_other_sequence
         assert torch.equal(ops.attention_prompt(q[at:at + n].contiguous(), store, one, 0.2), full[at:at + n]), b
         at += n
     ops.check_status()
+
+
+def prompt_case(lens, starts, d, heads, kv, seed):
+    """Sequences whose caches hold NaN behind their ends; queries; the step."""
+    batch, pages, n_pages = batch_of(lens, starts)
+    g = torch.Generator().manual_seed(seed)
+    store = torch.full((n_pages, 2, kv, PAGE, d), float("nan"))
+    for n, s, own in zip(lens, starts, pages):
+        for i, page in enumerate(own):
+            rows = min(PAGE, n + s - i * PAGE)
+            store[page, :, :, :rows] = torch.randn(2, kv, rows, d, generator=g)
+    q = torch.randn(sum(lens), heads, d, generator=g)
+    return q.bfloat16().to(DEV), store.bfloat16().to(DEV), batch
+
+
+def prompt_items(lens, heads, kv, tokens):
+    """Work items of a prompt step whose items are ``tokens`` tokens of 128 rows each: (items, those a multiprocessor gets)."""
+    group = heads // kv
+    gs = max(g for g in range(1, group + 1) if group % g == 0 and 128 % g == 0)
+    items = sum(-(-n // (tokens * (128 // gs))) for n in lens) * (heads // gs)
+    return items, items / torch.cuda.get_device_properties(0).multi_processor_count
+
+
+# 40 sequences (more than a warp's lanes), a few of more than eight blocks of 128 keys
+MANY = ([5 + 37 * (i % 23) for i in range(36)] + [700, 128, 129, 1], [(61 * i) % 300 for i in range(36)] + [1100, 1500, 0, 2000])
+
+
+@pytest.mark.parametrize("d, heads, kv, lens, starts, a_block", [
+    (128, 32, 8, *MANY, 4), (64, 16, 2, *MANY, 2), (128, 10, 2, *MANY, 1), (64, 6, 6, *MANY, 1),
+    (64, 64, 16, [400 + i for i in range(64)], [0] * 64, 16), (64, 6, 2, [300] * 100 + [1000], [0] * 100 + [300], 4)])
+@pytest.mark.parametrize("mask, size", [("causal", 0), ("block", 500), ("window", 300), ("window", 129)])
+def test_prompt_attention_of_two_tiles_a_block_item_behind_item(d, heads, kv, lens, starts, a_block, mask, size):
+    """Steps whose items are two tiles a block and several a block (more than 16: several rounds of blocks), one, two, four and eight
+    heads to a tile, of more than 32 sequences, of up to eight key blocks and of more, with masks and sinks; against the kernel that
+    takes row by row in float32.  A rounding to bfloat16 (8 bits) is off by at most 2^-8 of the number: the
+    probabilities' by 2^-8 of the largest value together, the two results' by 2^-8 of themselves each."""
+    one, each = prompt_items(lens, heads, kv, 1)
+    two, _ = prompt_items(lens, heads, kv, 2)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert one > 2 * sms and two > 2 * sms and two / sms > a_block, (one, two)
+    q, store, batch = prompt_case(lens, starts, d, heads, kv, heads + size)
+    sink = torch.randn(heads, generator=torch.Generator().manual_seed(1)).to(DEV)
+    for sk in (sink, None):
+        kw = dict(n_kv=kv, v_dim=d, mask=mask, mask_size=size, sink=sk)
+        out = ops.attention_masked(q, store, batch, d ** -0.5, kind="tc", **kw).float()
+        ref = ops.attention_masked(q, store, batch, d ** -0.5, kind="warp", **kw).float()
+        ops.check_status()
+        assert torch.isfinite(out).all()
+        assert ((out - ref).abs() <= 2 ** -8 * 6 + 2 ** -7 * ref.abs()).all()          # (values are normal: none is beyond 6)
+
+
+@pytest.mark.parametrize("d, heads, kv", [(64, 16, 4), (128, 6, 6), (64, 10, 2)])
+@pytest.mark.parametrize("window, block, cap", [(200, 16, 30.0), (130, 1, None), (0, 0, 5.0)])
+def test_prompt_attention_beside_blocks_of_two_tiles_a_block_item_behind_item(d, heads, kv, window, block, cap):
+    """The form with blocks of positions before the window, capped scores and a factor of the result, at the same kinds of steps."""
+    lens = [5 + 37 * (i % 23) for i in range(36)] + [1700, 128, 129, 1]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    lens = lens * (1 if prompt_items(lens, heads, kv, 2)[0] > 2 * sms else 4)
+    assert prompt_items(lens, heads, kv, 2)[0] > 2 * sms
+    q, store, batch = prompt_case(lens, [0] * len(lens), d, heads, kv, window + block)
+    flat = store.view(store.shape[0], -1)
+    gate = torch.rand(q.shape[0], heads, generator=torch.Generator().manual_seed(2)).to(DEV)
+    got = {}
+    for kind in ("tc", "rows"):
+        means = torch.full((store.shape[0], kv * ops.block_rows(block) * 2 * d), float("nan"), dtype=torch.bfloat16, device=DEV) if block else None
+        got[kind] = ops.attention_pooled(q, flat, batch, d ** -0.5, n_kv=kv, v_dim=d, window=window, store=means, block=block, soft_cap=cap,
+                                         gate=gate, kind=kind).float()
+    ops.check_status()
+    assert torch.isfinite(got["tc"]).all()
+    assert ((got["tc"] - got["rows"]).abs() <= 2 ** -8 * 6 + 2 ** -7 * got["rows"].abs()).all()
