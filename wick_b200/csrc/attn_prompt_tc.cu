@@ -344,7 +344,10 @@ __device__ __forceinline__ void complete(Item& it, int column, int per_kv, int g
     it.n_blk = last_key / BK + 1 - it.jb0 + it.n_pool;
 }
 
-template <bool EXTRA>
+// GUARD: two tiles an item, of more tokens together than a key block has keys.  A tile then multiplies no block that none of its rows sees
+// a key of: such a block weighs nothing, but a value that is infinite or no number would show in rows that do not see it.  (A kernel
+// of its own: with this in one kernel a step of a short prompt, which meets the code once a layer, took 2 us longer a layer.)
+template <bool EXTRA, bool GUARD>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                       bf16* __restrict__ out, const int* __restrict__ cu_seqlens, int n_seqs,
@@ -513,9 +516,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                 const int n_blk = w.n_blk;
                 const bool split = w.split;
                 auto block_of = [&](int s, int t) { return split ? 2 * t + s : t; };
-                // Two tiles of more tokens together than a key block has keys: a tile multiplies no block that none of its rows sees a key of.
-                // (Such a block weighs nothing, but a value that is infinite or no number would show in rows that do not see it.)
-                const bool guard = !split && 2 * T > BK;
+                const bool guard = GUARD && !split;
                 auto seen_by = [&](int s) {
                     const int first = w.start + w.q0 + s * T, last = min(first + T, w.start + w.q_len) - 1, before = w.n_pool - w.jb0;
                     return Seen{EXTRA ? (blocks_seen(last, mask_size, X.block) + BK - 1) / BK : 0,
@@ -529,7 +530,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                 // are told apart when the kernel is built (8,192 tokens: 537 us in the other, 453), short ones the shorter code.
                 auto turn = [&](auto form, int s, int t) {
                     constexpr int UNROLL = decltype(form)::value & 3;
-                    constexpr bool GUARD = decltype(form)::value >= GUARDED;
+                    constexpr bool SEEN_ONLY = decltype(form)::value >= GUARDED;
                     const int steps = s == 0 ? steps0 : steps1, uses = s == 0 ? uses0 : uses1;
                     const bool more = block_of(s, t + 1) < n_blk;
                     if (block_of(s, t) >= n_blk) return;
@@ -540,7 +541,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                         const uint32_t v_lo = v_lo0 + v_at * (TILE_BYTES >> 4), d = tmem + COL_O + s * HD, pa = tmem + COL_S + s * BK;
                         bool go = one;
                         int begun = t;                             // (0: the stream's first product of the item)
-                        if constexpr (GUARD) {
+                        if constexpr (SEEN_ONLY) {
                             const Seen seen = s == 0 ? seen0 : seen1;
                             go = one && seen.has(t);
                             begun = t - seen.first();
@@ -586,27 +587,25 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                 };
                 auto looped = [&](auto form, int from, int to) {
 #pragma unroll 1
-                    for (int i = 2 * from; ok && i < 2 * to && block_of(0, i >> 1) < n_blk; ++i) turn(form, i & 1, i >> 1);
+                    for (int i = 2 * from; ok && i < 2 * to; ++i) turn(form, i & 1, i >> 1);
                 };
                 auto written_out = [&](int from, int to) {
 #pragma unroll 1
-                    for (int t = from; ok && t < to && block_of(0, t) < n_blk; ++t) {
+                    for (int t = from; ok && t < to; ++t) {
                         turn(std::integral_constant<int, 2>{}, 0, t);
                         if (ok) turn(std::integral_constant<int, 2>{}, 1, t);
                     }
                 };
-                if (guard) {
+                const int turns = split ? (n_blk + 1) / 2 : n_blk;
+                int lo = -1, hi = turns;
+                if (GUARD && guard) {
                     // (between the last block that either tile begins with and the first that either no longer sees: as without)
-                    const int lo = max(seen0.from, seen1.from) + 1, hi = max(lo, min(seen0.to, seen1.to));
+                    lo = max(seen0.from, seen1.from) + 1, hi = max(lo, min(seen0.to, seen1.to));
                     looped(std::integral_constant<int, GUARDED + 1>{}, -1, lo);
-                    if (n_blk >= LONG) written_out(lo, hi);
-                    else looped(std::integral_constant<int, 1>{}, lo, hi);
-                    looped(std::integral_constant<int, GUARDED + 1>{}, hi, n_blk);
-                } else if (n_blk >= LONG) {
-                    written_out(-1, n_blk);
-                } else {
-                    looped(std::integral_constant<int, 1>{}, -1, n_blk);
                 }
+                if (n_blk >= LONG) written_out(lo, hi);
+                else looped(std::integral_constant<int, 1>{}, lo, hi);
+                if (GUARD && guard) looped(std::integral_constant<int, GUARDED + 1>{}, hi, turns);
             }
         }
     } else {
@@ -957,11 +956,14 @@ static int attn_prompt_tc(const void* q, long long n_tokens, const void* kv, lon
     }
     // (up to four key blocks - every captured prompt step - the order is worth less than the ~2 us that finding it takes)
     const int ordered = table_width > 4 * BK / kPage ? 1 : 0;
-    auto kernel = extra ? attn_prompt_tc_kernel<true> : attn_prompt_tc_kernel<false>;
-    static bool raised[2] = {false, false};
-    if (!raised[extra ? 1 : 0]) {
+    const bool guard = tiles == 2 && 2 * T > BK;
+    auto kernel = extra ? (guard ? attn_prompt_tc_kernel<true, true> : attn_prompt_tc_kernel<true, false>)
+                        : (guard ? attn_prompt_tc_kernel<false, true> : attn_prompt_tc_kernel<false, false>);
+    static bool raised[4] = {false, false, false, false};
+    bool& done = raised[(extra ? 2 : 0) + (guard ? 1 : 0)];
+    if (!done) {
         WICK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        raised[extra ? 1 : 0] = true;
+        done = true;
     }
     WICK_CUDA(launch(kernel, dim3(blocks), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, q_map,
                      kv_map, (bf16*)out, cu_seqlens, n_seqs, start, page_table, table_width, n_heads,
