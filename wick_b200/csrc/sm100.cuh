@@ -34,8 +34,14 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 // Bounded wait.  Returns false (and raises the block's abort flag) after limit_ns (~1 s).
 // (The loop is a function of its own: a wait in place costs a few instructions.  The kernels of a layer then fit together into an SM's
-// instruction cache, which nothing else does for a step whose weights pass through the L2 cache between two uses of a kernel.)
-static __device__ __noinline__ bool mbar_wait_loop(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code, uint64_t limit_ns) {
+// instruction cache, which nothing else does for a step whose weights pass through the L2 cache between two uses of a kernel.  A file whose
+// kernels run long can ask for waits in place: WICK_WAITS_IN_PLACE.)
+#ifdef WICK_WAITS_IN_PLACE
+#define WICK_WAIT_LOOP __forceinline__
+#else
+#define WICK_WAIT_LOOP __noinline__
+#endif
+static __device__ WICK_WAIT_LOOP bool mbar_wait_loop(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code, uint64_t limit_ns) {
     if (*abort_flag) return false;
     const uint64_t t0 = global_ns();
     for (uint32_t spin = 0;; ++spin) {
