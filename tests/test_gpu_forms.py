@@ -734,3 +734,18 @@ def test_prompt_attention_beside_blocks_of_two_tiles_a_block_item_behind_item(d,
     ops.check_status()
     assert torch.isfinite(got["tc"]).all()
     assert ((got["tc"] - got["rows"]).abs() <= 2 ** -8 * 6 + 2 ** -7 * got["rows"].abs()).all()
+
+
+@pytest.mark.parametrize("lens, starts", [([400], [0]), ([70, 1, 130], [900, 500, 800])])
+def test_prompt_rows_do_not_depend_on_the_width_of_the_page_table(lens, starts):
+    """A table of up to 16 pages (1,024 positions) takes the kernel without the code for long items, a wider one the kernel with it."""
+    d, heads, kv = 128, 8, 2
+    q, store, batch = prompt_case(lens, starts, d, heads, kv, 12)
+    assert batch.table_width <= 16
+    layout = BatchLayout(len(lens), sum(lens), 40, 0)
+    host = np.zeros(layout.size, dtype=np.int32)
+    fill_host(layout, host, tokens=[[0] * n for n in lens], starts=starts, slots=[1 + i for i in range(len(lens))],
+              pages=[[int(p) for p in row] for row in batch.page_table.cpu()], want=[[]] * len(lens))
+    wide = StepBatch(layout, torch.from_numpy(host).to(DEV), q_lens=lens, starts=starts)
+    assert torch.equal(ops.attention_prompt(q, store, batch, 0.1), ops.attention_prompt(q, store, wide, 0.1))
+    ops.check_status()

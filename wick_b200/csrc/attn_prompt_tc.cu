@@ -347,7 +347,9 @@ __device__ __forceinline__ void complete(Item& it, int column, int per_kv, int g
 // GUARD: two tiles an item, of more tokens together than a key block has keys.  A tile then multiplies no block that none of its rows sees
 // a key of: such a block weighs nothing, but a value that is infinite or no number would show in rows that do not see it.  (A kernel
 // of its own: with this in one kernel a step of a short prompt, which meets the code once a layer, took 2 us longer a layer.)
-template <bool EXTRA, bool GUARD>
+// LONGS: there can be items of LONG key blocks and more.  (Without them the code is 51 KB instead of 69: 400 tokens, 32 heads over 8
+// 9.9 us, now 9.5; 200 tokens 7.9 and 7.5; a step of 200 tokens on 6 8B layers 1,238 and 1,227, of 400 on 4 small ones 742 and 732.)
+template <bool EXTRA, bool GUARD, bool LONGS>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                       bf16* __restrict__ out, const int* __restrict__ cu_seqlens, int n_seqs,
@@ -603,7 +605,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                     lo = max(seen0.from, seen1.from) + 1, hi = max(lo, min(seen0.to, seen1.to));
                     looped(std::integral_constant<int, GUARDED + 1>{}, -1, lo);
                 }
-                if (n_blk >= LONG) written_out(lo, hi);
+                if (LONGS && n_blk >= LONG) written_out(lo, hi);
                 else looped(std::integral_constant<int, 1>{}, lo, hi);
                 if (GUARD && guard) looped(std::integral_constant<int, GUARDED + 1>{}, hi, turns);
             }
@@ -761,7 +763,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sh.p_full[s][part]);
                 };
-                if (n_blk >= LONG) {
+                if (LONGS && n_blk >= LONG) {
                     float z[32];
                     tc_ld32_nowait(s_addr, reinterpret_cast<uint32_t*>(z));
                     tc_ld_wait();
@@ -957,10 +959,12 @@ static int attn_prompt_tc(const void* q, long long n_tokens, const void* kv, lon
     // (up to four key blocks - every captured prompt step - the order is worth less than the ~2 us that finding it takes)
     const int ordered = table_width > 4 * BK / kPage ? 1 : 0;
     const bool guard = tiles == 2 && 2 * T > BK;
-    auto kernel = extra ? (guard ? attn_prompt_tc_kernel<true, true> : attn_prompt_tc_kernel<true, false>)
-                        : (guard ? attn_prompt_tc_kernel<false, true> : attn_prompt_tc_kernel<false, false>);
-    static bool raised[4] = {false, false, false, false};
-    bool& done = raised[(extra ? 2 : 0) + (guard ? 1 : 0)];
+    // (all items are short: of a table of so few pages, every captured step's among them)
+    const bool shorts = !extra && !guard && (long long)table_width * kPage <= (LONG - 1) * BK;
+    auto kernel = extra ? (guard ? attn_prompt_tc_kernel<true, true, true> : attn_prompt_tc_kernel<true, false, true>)
+                        : (guard ? attn_prompt_tc_kernel<false, true, true> : (shorts ? attn_prompt_tc_kernel<false, false, false> : attn_prompt_tc_kernel<false, false, true>));
+    static bool raised[5] = {false, false, false, false, false};
+    bool& done = raised[shorts ? 4 : (extra ? 2 : 0) + (guard ? 1 : 0)];
     if (!done) {
         WICK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         done = true;
