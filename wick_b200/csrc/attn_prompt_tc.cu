@@ -1,9 +1,9 @@
 // Causal attention of a step's new tokens over the paged cache on the 5th-
 // generation tensor cores (tcgen05), bfloat16, head sizes 64 and 128.
 //
-// The 128 rows of a tile are the query heads of one key head times as many consecutive tokens as
-// fit: 4 heads to a key head make 32 tokens, 5 make 25 (125 rows), 1 makes 128 (one TMA box of
-// heads x tokens either way).  A block runs two streams over blocks of 128 keys (two cache pages),
+// The 128 rows of a tile are query heads of one key head times consecutive tokens: as many heads as fill it with whole
+// tokens, i.e. the largest power of two that divides their number (4 heads to a key head: 4 x 32 tokens; 5 or 1: 1 x 128; one
+// TMA box of heads x tokens either way).  A block runs two streams over blocks of 128 keys (two cache pages),
 // each with its own scores and its own result in tensor memory and four softmax warps:
 //   * two tiles of neighbouring tokens over all key blocks (a key or value tile is read twice), or
 //   * where the step is too small for that to fill the device, or the second tile has no tokens,
@@ -22,10 +22,11 @@
 // last one's epilogue.
 // What bounds it: a tile and key block take the tensor core 1,024 clocks (16 instructions of 64) and the
 // exponentials as many; a stream's chain of softmax (1,830 clocks), product, scores and the waits between them takes ~3,400 clocks for
-// both streams' blocks.  Before (a tile of one head's rows a block, two threads a row, one lane issuing) / now, us:
-// 2,048 tokens, 32 heads over 8 69 -> 43, 8,192 tokens 625 -> 453 (1.2 PFLOP/s); 16 prompts of 64 to 2,048 tokens, 40 over 8
-// 717 -> 529; 1,419 tokens behind 3,100 124 -> 105; 8 x 1,024, 64 over 8 336 -> 189; 64 tokens 7.2 -> 8.7 behind itself, but in a step,
-// where its start overlaps the kernel before, no longer than before.
+// both streams' blocks.  Before (a tile of one head's rows a block, two threads a row, one lane issuing) / now, us alone, one behind the
+// other: 2,048 tokens, 32 heads over 8 67 / 42, 8,192 tokens 654 / 517 (at the power cap); 16 prompts of 64 to 2,048 tokens, 40 over 8
+// 472 / 355; 1,419 tokens behind 3,100 118 / 94; 8 x 1,024, 64 over 8 336 / 190.  Short prompts have a thread for 128 scores where they had
+// two: 64 tokens, 32 over 8 5.8 / 6.3, 200 7.2 / 7.5, 400 9.8 / 9.5, 16 over 4 400 9.0 / 9.3, 1,000 14.4 / 14.9; a whole step of 64 tokens is 2 to 5 %
+// shorter than before all the same, one of 200 or 400 0.3 to 0.7 % longer.
 // O and the sum are scaled by a maximum that follows the true running maximum
 // lazily: only when a block's maximum exceeds it by more than 8 (in units of
 // log2 e) is O rescaled in tensor memory, so that after the first blocks of a row
@@ -37,8 +38,8 @@
 // window, each as one key and value (tiles of 64 blocks a sequence, laid out like cache
 // pages; their key blocks come before the window's), soft-caps the scores and multiplies
 // the result by a number per token and head.
-// Work items are dealt longest first (see find_longest_item): neighbouring block indexes are the key heads
-// of one item.
+// Work items are dealt longest first (see Finder): neighbouring block indexes are the key heads of one item.  Steps of several
+// sequences whose page table has up to eight pages deal them in index order.
 // Every wait is bounded and reports through the status word.
 // Formulas: wick src/model.rs:520-553.  The plain forms of this computation are
 // attn_prompt_mma_kernel (attn_prompt_mma.cu) and attn_prompt_kernel (attn.cu).
@@ -76,7 +77,6 @@ struct Item {
     // Tiles come through the ring in the order in which the issuing thread uses them: K0 V0 K1 V1 ..., or, split,
     // K0 K1 V0 K2 V1 K3 ... V(n-2) V(n-1): an item's 2 n_blk tiles, and the place of block j's values among them.
     __device__ __forceinline__ int place_v(int j) const { return split ? min(2 * j + 2, 2 * n_blk - 1) : 2 * j + 1; }
-    __device__ __forceinline__ int block_of(int s, int t) const { return split ? 2 * t + s : t; }    // step t of stream s
 };
 // The key blocks that a tile multiplies: those before `pool`, and those from `from` up to `to`.
 struct Seen {
@@ -370,7 +370,6 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
         return;
     }
     // (the step's description is written by the host before the step: no kernel produces it)
-    const int rows = T * gs;                                       // of a tile: T tokens times gs heads
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Item k of the block is the one at place(k) of all, the key heads of one item side by side, in falling order of length, dealt
     // to and fro over the blocks.
@@ -396,14 +395,6 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_slot)), "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    if (rows < BQ) {                                               // rows of the tiles that no query fills
-#pragma unroll 1
-        for (int i = threadIdx.x; i < 2 * PANELS * (BQ - rows) * 8; i += THREADS) {
-            const int panel = i / ((BQ - rows) * 8), at = i % ((BQ - rows) * 8);
-            *reinterpret_cast<uint4*>(q_s + panel * PANEL_BYTES + rows * 128 + at * 16) = make_uint4(0, 0, 0, 0);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     {
         const Finder finder(cu_seqlens, start_arr, n_seqs, T * tiles, ordered != 0);
@@ -448,7 +439,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                 if (!ok) break;
                 if (one) {
                     const int n_q = w.split ? 1 : 2;
-                    mbar_expect_tx(&sh.q_full, n_q * PANELS * rows * 128);
+                    mbar_expect_tx(&sh.q_full, n_q * TILE_BYTES);
 #pragma unroll 1
                     for (int i = 0; i < n_q; ++i)
                         for (int pn = 0; pn < PANELS; ++pn)
@@ -493,9 +484,8 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             }
         } else {
             // ---------------- MMA issuer ----------------
-            // The whole warp walks through the steps and one elected lane issues: what an instruction needs stays in uniform
-            // registers.  (A branch of one lane needs tens of instructions for each, beside softmax warps that compete for
-            // the same scheduler: 86 to 146 clocks per instruction instead of the tensor core's 64.)
+            // The whole warp walks through the steps and one elected lane issues.  (Issued in a branch of one lane, beside busy softmax
+            // warps, an instruction took 86 to 146 clocks instead of the tensor core's 64.)
             // kind::f16, bfloat16 operands, float32 accumulator, M = 128
             const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BK >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
             const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
@@ -615,7 +605,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
         // (a warp reads the 32 lanes of tensor memory given by its index modulo 4)
         pdl_wait();                                                 // (the result's and the gate's memory may be in use until then)
         const int quad = warp & 3, s = (warp - 2) >> 2;             // s: the stream
-        const int r = quad * 32 + lane, row_tok = min(r, rows - 1) / gs, row_head = min(r, rows - 1) % gs;
+        const int r = quad * 32 + lane, row_tok = r / gs, row_head = r % gs;    // (a tile is T tokens of gs heads, T gs = 128)
         const bool capped = EXTRA && X.cap > 0.f;
         const float sl2 = capped ? 1.0f : scale * 1.4426950408889634f;   // (a capped score comes in units of log2 e)
         const float cap2 = EXTRA ? X.cap * 1.4426950408889634f : 0.f, z_of_s = capped ? scale / X.cap : 0.f,
@@ -630,6 +620,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             const int n_blk = w.n_blk, kv_len = w.start + w.q_len, n_pool = w.n_pool, jw = w.jb0 - n_pool;
             const bool split = w.split;
             const int tok = w.q0 + (split ? 0 : s * T) + row_tok, head = w.head0 + row_head;   // token (of the sequence) and head of the row
+            const bool store = tok < w.q_len;                       // (rows of tokens beyond the sequence's end are left out)
             const int limit = min(w.start + tok, kv_len - 1);       // last visible key position
             const int vis = first_visible_key(limit, mask, mask_size);  // first visible key position
             const int n_seen = EXTRA ? blocks_seen(limit, mask_size, X.block) : 0;
@@ -791,7 +782,6 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             if (!ok) break;
             base += 2 * n_blk;
             // (rows of tokens beyond the sequence's end were computed from other tokens' queries and are left out here)
-            const bool store = r < rows && tok < w.q_len;
             bf16* dst = out + ((int64_t)(w.tok0 + min(tok, w.q_len - 1)) * n_heads + head) * HD;
             const float gate = EXTRA && X.gate && store ? X.gate[(int64_t)(w.tok0 + tok) * n_heads + head] : 1.0f;
             auto put = [&](int c, const float* v) {                  // 32 numbers of the row from column c on
@@ -925,9 +915,8 @@ static int attn_prompt_tc(const void* q, long long n_tokens, const void* kv, lon
     WICK_REQUIRE(n_heads <= 65535, "attention: %d heads is beyond the grid limit", n_heads);
     if (n_tiles == 0) return 0;
     const int group = n_heads / n_kv;
-    int gs = 1;                                                    // heads of a tile: the divisor of the group that fills most rows
-    for (int g = 1; g <= min(group, BQ); ++g)
-        if (group % g == 0 && BQ / g * g >= BQ / gs * gs) gs = g;
+    int gs = 1;                                                    // heads of a tile: as many as fill its rows with whole tokens
+    while (group % (2 * gs) == 0 && 2 * gs <= BQ) gs *= 2;
     const int T = BQ / gs, columns = n_heads / gs;
     // the most work items of R tokens that sequences of n_tokens tokens (or of n_tiles 64-row items) can make
     auto items = [&](long long R) { return (int)min((n_tokens + n_seqs * (R - 1)) / R, n_tiles * ((64 + R - 1) / R)); };
