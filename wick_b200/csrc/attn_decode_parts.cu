@@ -4,24 +4,24 @@
 //
 // How the work is cut depends on each sequence's OWN length and on nothing else, so a
 // sequence's output bits do not depend on the batch it is in:
-//   * the pages of a (sequence, kv head) pair are cut into PARTS of pages_per_part(n)
-//     consecutive pages (two, i.e. 128 positions, up to 64 pages; more for longer
-//     sequences, so that a pair never has more than 32 parts);
+//   * the pages of a (sequence, kv head) pair are cut into PARTS of consecutive pages: two,
+//     i.e. 128 positions, up to 16 pages, more for longer sequences, so that a pair never has
+//     more than MAX_PARTS = 8 parts (with a mask: its visible pages, evenly, see parts_of);
 //   * a part is computed by ONE warp, page by page in order (scores with the keys on
 //     the 16-row side of mma.sync, the probabilities turned into the second product's
 //     operand inside the warp with movmatrix, running maximum, sum and accumulator in
-//     registers); it leaves its result (accumulator, maximum, sum per head) in global
-//     scratch;
-//   * a second, small kernel (attn_decode_merge_kernel, a warp per pair and head) merges
-//     a pair's parts in part order and writes the output rows.  A pair with one part is
-//     written directly by the first kernel.
-// Which warp computes which part is a matter of scheduling only: all parts of the step,
-// in the order (sequence, kv head, part), are dealt in equal contiguous runs to the
-// warps of the grid (three warps a block at head size 128, one block per SM, blocks
-// first so that few parts spread over many SMs).  Every warp feeds itself: a private
-// ring of four tiles (a tile is one page of keys or of values of one kv head, fetched
-// by TMA into 128-byte-swizzled shared memory), filled up to four tiles ahead across
-// the boundaries of its parts.  No warp waits for another one; the only waits are on
+//     registers); it leaves a record (accumulator, maximum, sum per head);
+//   * a pair's records are merged in part order, a warp per head.  A pair with one part is
+//     written directly.
+// Which warp computes which part is a matter of scheduling only, in one of two forms (see
+// launch_parts): a block per pair, whose warps (six at head size 128, twelve at 64) take the
+// pair's parts and merge its records in shared memory; or persistent blocks, one per SM, to whose
+// warps all parts of the step, in the order (sequence, kv head, part), are dealt in equal
+// contiguous runs, with the records in global scratch and a second, small kernel for the merge
+// (attn_decode_merge_kernel).  Every warp feeds itself: a private
+// ring of two tiles (a tile is one page of keys or of values of one kv head, fetched
+// by TMA into 128-byte-swizzled shared memory), filled ahead across
+// the boundaries of its parts.  While parts are computed no warp waits for another one; the only waits are on
 // a warp's own copies, and they are bounded.
 //
 // The kernel before this one (qk_norm_rope_append_kernel) has normed and rotated the
@@ -896,8 +896,6 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
     const bool waves_pay = pages >= least && pairs * 10 >= waves * sms * 6;
     const bool pair_form = force >= 0 ? force == 1 : (pairs <= sms ? pays : waves_pay);
     if (pair_form) {
-        // Few pairs of short parts: a block per pair, its warps at the pair's parts, merged by the block itself.
-        // (Longer parts, or more pairs than SMs, want the self-fed warps of the persistent form.)
         if (masked)
             WICK_CUDA(launch(attn_decode_parts_kernel<false, true, true>, dim3((unsigned)pairs), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)s, map,
                              (const bf16*)q, proj, (bf16*)out, kv_len, page_table, table_width, n_seqs, n_heads, n_kv, scale, scratch,
@@ -939,7 +937,7 @@ static int launch_parts(bool prep, const void* q, decodeparts::Projection proj, 
 // [kv_pages, 2, n_kv, 64, HD], the new token's key and value already in it; kv_len: positions
 // per sequence including the new token; scratch: float32 (see above); status: device int (code
 // 8 if a warp gave up waiting for its copies, 10 if a length or a page lies outside what it was
-// given).  Two launches: the parts, then (if any sequence can have more than one part) the merge.
+// given).  One launch (a block per pair), or the parts and, if any sequence can have more than one part, the merge.
 WICK_API int wick_attn_decode_parts_bf16(const void* q, const void* kv, long long kv_pages, void* out, float* scratch,
                                          long long scratch_words, const int* kv_len, int n_seqs, int max_kv_len,
                                          const int* page_table, int table_width, int n_heads, int n_kv, float scale,
