@@ -25,7 +25,7 @@
 // both streams' blocks.  Before (a tile of one head's rows a block, two threads a row, one lane issuing) / now, us alone, one behind the
 // other: 2,048 tokens, 32 heads over 8 67 / 42, 8,192 tokens 654 / 517 (at the power cap); 16 prompts of 64 to 2,048 tokens, 40 over 8
 // 472 / 355; 1,419 tokens behind 3,100 118 / 94; 8 x 1,024, 64 over 8 336 / 190.  Short prompts have a thread for 128 scores where they had
-// two: 64 tokens, 32 over 8 5.8 / 6.3, 200 7.2 / 7.5, 400 9.8 / 9.5, 16 over 4 400 9.0 / 9.3, 1,000 14.4 / 14.9; a whole step of 64 tokens is 2 to 5 %
+// two: 64 tokens, 32 over 8 5.8 / 6.2, 200 7.2 / 7.4, 400 9.8 / 9.4, 16 over 4 400 9.0 / 9.3, 1,000 14.4 / 14.9; a whole step of 64 tokens is 2 to 5 %
 // shorter than before all the same, one of 200 or 400 0.3 to 0.7 % longer.
 // O and the sum are scaled by a maximum that follows the true running maximum
 // lazily: only when a block's maximum exceeds it by more than 8 (in units of
@@ -639,49 +639,37 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                 const bool pooled = EXTRA && j < n_pool;
                 const int key0 = (pooled ? j : j + jw) * BK;
                 const int last = pooled ? n_seen - 1 : limit, first_key = pooled ? 0 : vis;
-                // Three times over the scores: masks where there are any, the row's maximum, the probabilities, which take the place of scores
+                // Twice over the scores: masks where there are any and the row's maximum (in two passes of their own 1 to 5 % of the kernel's time
+                // more: 400 tokens, 40 heads over 8 12.8 us, now 12.5; 300 with a cap and blocks 16.3 and 15.2), the probabilities, which take the place of scores
                 // already read.  In loops, except in long items: an item of a short prompt meets this code once, and each 128 bytes of it come
                 // from memory where weights have passed through the L2 cache since the layer before (the whole written out, 110 KB of code
                 // instead of 72: a prompt of 100 tokens took 7 us longer a layer).
-                if (capped || __any_sync(0xffffffffu, key0 + BK - 1 > last || key0 < first_key)) {
-#pragma unroll 1
-                    for (int c = 0; c < BK; c += 32) {
-                        float v[32];
-                        tc_ld32_nowait(s_addr + c, reinterpret_cast<uint32_t*>(v));
-                        tc_ld_wait();
-                        if (capped) {
-                            // cap tanh(z), z = s / cap: by a polynomial where all of the warp's |z| are small (two products and sums an
-                            // instruction), else as cap (1 - 2 / (1 + exp(2 z))), whose two special functions a score would bound the block.
-                            float big = 0.f;
+                const bool changed = capped || __any_sync(0xffffffffu, key0 + BK - 1 > last || key0 < first_key);
+                auto cap = [&](float* v) {                                // of 32 scores
+                    // cap tanh(z), z = s / cap: by a polynomial where all of the warp's |z| are small (two products and sums an
+                    // instruction), else as cap (1 - 2 / (1 + exp(2 z))), whose two special functions a score would bound the block.
+                    float big = 0.f;
 #pragma unroll
-                            for (int i = 0; i < 32; i += 2) big = max3(big, fabsf(v[i]), fabsf(v[i + 1]));
-                            if (__all_sync(0xffffffffu, big * z_of_s <= TANH_SMALL)) {
-                                const float2 zs = make_float2(z_of_s, z_of_s), c2 = make_float2(cap2, cap2);
+                    for (int i = 0; i < 32; i += 2) big = max3(big, fabsf(v[i]), fabsf(v[i + 1]));
+                    if (__all_sync(0xffffffffu, big * z_of_s <= TANH_SMALL)) {
+                        const float2 zs = make_float2(z_of_s, z_of_s), c2 = make_float2(cap2, cap2);
 #pragma unroll
-                                for (int i = 0; i < 32; i += 2) {
-                                    const float2 z = mul2(make_float2(v[i], v[i + 1]), zs), q = mul2(z, z);
-                                    float2 p = make_float2(TANH_C4, TANH_C4);
-                                    p = fma2(p, q, make_float2(TANH_C3, TANH_C3));
-                                    p = fma2(p, q, make_float2(TANH_C2, TANH_C2));
-                                    p = fma2(p, q, make_float2(TANH_C1, TANH_C1));
-                                    p = fma2(p, q, make_float2(TANH_C0, TANH_C0));
-                                    const float2 r2 = mul2(mul2(p, z), c2);
-                                    v[i] = r2.x;
-                                    v[i + 1] = r2.y;
-                                }
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) v[i] = fmaf(-2.0f * cap2, rcp(1.0f + ex2(v[i] * two_s)), cap2);
-                            }
+                        for (int i = 0; i < 32; i += 2) {
+                            const float2 z = mul2(make_float2(v[i], v[i + 1]), zs), q = mul2(z, z);
+                            float2 p = make_float2(TANH_C4, TANH_C4);
+                            p = fma2(p, q, make_float2(TANH_C3, TANH_C3));
+                            p = fma2(p, q, make_float2(TANH_C2, TANH_C2));
+                            p = fma2(p, q, make_float2(TANH_C1, TANH_C1));
+                            p = fma2(p, q, make_float2(TANH_C0, TANH_C0));
+                            const float2 r2 = mul2(mul2(p, z), c2);
+                            v[i] = r2.x;
+                            v[i + 1] = r2.y;
                         }
-                        const int lo = first_key - key0 - c, hi = last - key0 - c;
+                    } else {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (i > hi || i < lo) v[i] = -INFINITY;
-                        tc_st32(s_addr + c, reinterpret_cast<uint32_t*>(v));
+                        for (int i = 0; i < 32; ++i) v[i] = fmaf(-2.0f * cap2, rcp(1.0f + ex2(v[i] * two_s)), cap2);
                     }
-                    tc_st_wait();
-                }
+                };
                 float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                 float y[64];                                             // the scores read last
 #pragma unroll 1
@@ -689,6 +677,15 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                     tc_ld32_nowait(s_addr + c, reinterpret_cast<uint32_t*>(y));
                     tc_ld32_nowait(s_addr + c + 32, reinterpret_cast<uint32_t*>(y + 32));
                     tc_ld_wait();
+                    if (changed) {
+                        if (capped) cap(y), cap(y + 32);
+                        const int lo = first_key - key0 - c, hi = last - key0 - c;
+#pragma unroll
+                        for (int i = 0; i < 64; ++i)
+                            if (i > hi || i < lo) y[i] = -INFINITY;
+                        tc_st32(s_addr + c, reinterpret_cast<uint32_t*>(y));
+                        tc_st32(s_addr + c + 32, reinterpret_cast<uint32_t*>(y + 32));
+                    }
 #pragma unroll
                     for (int i = 0; i < 64; i += 8) {
                         mx4[0] = max3(mx4[0], y[i], y[i + 1]);
@@ -697,6 +694,7 @@ attn_prompt_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                         mx4[3] = max3(mx4[3], y[i + 6], y[i + 7]);
                     }
                 }
+                if (changed) tc_st_wait();
                 const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl2;
                 const bool grow = mx > m + 8.0f;
                 float alpha = 1.0f;
